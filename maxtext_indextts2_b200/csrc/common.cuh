@@ -71,6 +71,18 @@ __device__ __forceinline__ void timeline_end(int idx) {
   if (idx >= 0) d_timeline[4 + 3 * idx + 2] = globaltimer_ns();
 }
 
+// True in one lane of the (whole) warp.  Warps that issue TMA loads or tcgen05 instructions wait together and issue in this lane: a branch
+// on the lane number makes the compiler guard every issue against divergence.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t is;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(is));
+  return is != 0;
+}
+
 // ---------------------------------------------------------------------------------
 // programmatic dependent launch
 // ---------------------------------------------------------------------------------

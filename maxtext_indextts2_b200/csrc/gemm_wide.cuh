@@ -1,0 +1,304 @@
+// GEMM of steps with more than 256 rows (prompts and long portions of prompts): all rows of the step in one launch.
+//
+//   acc[r, n] = sum_k A[r, k] * W[n, k]        both operands K-major bf16, fp32 accumulation in TMEM
+//
+// gemm_rows.cuh takes at most 256 rows per launch, so a prompt of 4096 rows read every weight tile sixteen times and paid sixteen
+// launches, pipeline fills and drains per projection: 20 % of the bf16 rate.  Here two CTAs of a cluster (a TPC's two SMs) work on one
+// tile of 256 rows x BN columns with cta_group::2 MMAs (M = 256): CTA c of the pair holds rows 128 c .. of A and half of the
+// weight tile's rows, so that an SM takes in 16 KB + BN * 64 B per k block of 64 for BN * 2^15 multiply-adds.  One pair per TPC walks the
+// tiles (rows fastest, so that the pairs at work share weight tiles in L2), the accumulators are double-buffered (2 x 256 TMEM
+// columns): the eight epilogue warps of each CTA drain a tile under the next tile's MMAs.
+//
+// BN is chosen per shape (wide_tile_columns) so that the tiles fill whole waves of pairs.
+//
+// Bound: the tensor pipe at BN = 256 (0.28 us per k block of a tile; 4096 x 2048 x 4096 in 47 us, 1.45 PFLOP/s, 0.91 of the 1.59 that
+// cuBLAS reaches in a burst; gemm_rows.cuh in sixteen launches: 257 us), below that the round of barrier, four MMAs and commit
+// (0.16 us per k block).  That round took 0.29 us as long as the issuing threads were picked by `lane == 0`.
+//
+//   warp 0    TMA: its CTA's half of both operands into a ring of stages, both halves counted on the leader's barrier
+//   warp 1    the leader's issues tcgen05.mma and commits (multicast to both CTAs' barriers)
+//   warps 2-9 epilogue: a thread owns one row (TMEM lane) and half of the tile's columns
+//
+// The epilogue is a class with  prepare(tile)  (what a thread needs of its row, read while the tile's MMAs run) and
+// operator()(tile, n, prepared, load)  where load(c, v) reads the accumulator's 16 columns c .. c + 15.
+#pragma once
+
+#include "gemm_rows.cuh"
+
+namespace mtx {
+
+constexpr int kPairThreads = 320;
+constexpr int kPairRows = 256;    // rows of a pair's tile
+constexpr int kPairMaxCols = 256;
+constexpr int kPairMaxStages = 12;
+constexpr int kPairABytes = 128 * kBlockK * 2;  // a CTA's part of an A stage
+
+struct WideParams {
+  int rows, n, k;
+  int bn;      // columns of a tile: a multiple of 32, at most 256
+  int stages;  // depth of the ring
+  int first;   // columns of a tile's first half (the epilogue warps 2-5; the warps 6-9 take the rest)
+};
+
+struct WideSmemTail {
+  uint64_t full[kPairMaxStages];
+  uint64_t empty[kPairMaxStages];
+  uint64_t tmem_full[2];
+  uint64_t tmem_empty[2];
+  uint32_t tmem_base;
+  uint32_t pad;
+};
+
+__host__ __device__ inline size_t wide_stage_bytes(int bn) { return size_t(kPairABytes) + size_t(bn / 2) * kBlockK * 2; }
+__host__ __device__ inline size_t wide_smem_bytes(int bn, int stages) { return 1024 + stages * wide_stage_bytes(bn) + sizeof(WideSmemTail) + 16; }
+// as many stages as an SM's shared memory holds: a stage comes round in one to two microseconds (TMA, the leader's barrier, the MMAs, the
+// commit back to both CTAs) whatever its size, so narrow tiles want more of them
+inline int wide_stages(int bn) {
+  const int n = int((227 * 1024 - wide_smem_bytes(bn, 0)) / wide_stage_bytes(bn));
+  return n < kPairMaxStages ? n : kPairMaxStages;
+}
+
+// what an epilogue thread works on: its row, and the columns [c0, c1) of the tile that starts at column n0 of the output
+struct WideTile {
+  int row;
+  bool valid;
+  int n0, c0, c1;
+  int slice;  // index of this run of columns among all the runs of a row: 2 * tile + half
+};
+
+// ---- cta_group::2 forms ----------------------------------------------------------------------------------------------------
+
+constexpr uint32_t kPairLeaderMask = 0xFEFFFFFFu;  // a shared::cluster address with the pair's low rank bit cleared: the leader's copy
+
+// 2-D tiled load into this CTA's shared memory; the bytes count on the LEADER's barrier
+__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* tm, int c0, int c1, uint64_t* bar, uint64_t hint) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint"
+      " [%0], [%1, {%3, %4}], [%2], %5;"
+      :
+      : "r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(tm)), "r"(smem_u32(bar) & kPairLeaderMask), "r"(c0), "r"(c1), "l"(hint)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t* dst_smem, uint32_t ncols) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void tmem_relinquish_pair() { asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      :
+      : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// arrives on the barrier at this offset in both CTAs of the pair once the MMAs issued so far are done
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "h"(uint16_t(3))
+               : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_leader(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(smem_u32(bar) & kPairLeaderMask) : "memory");
+}
+
+// ---- the kernel ----------------------------------------------------------------------------------------------------------------
+
+template <class EPI>
+__global__ void __launch_bounds__(kPairThreads, 1)
+gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_a, const WideParams p, const EPI epi) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  const int stage_bytes = int(wide_stage_bytes(p.bn)), half_n = p.bn / 2;
+  WideSmemTail* tail = reinterpret_cast<WideSmemTail*>(smem + size_t(p.stages) * stage_bytes);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = int(blockIdx.x) & 1, pair = int(blockIdx.x) >> 1, pairs = int(gridDim.x) >> 1;  // (the cluster is two CTAs along x)
+  const int m_tiles = (p.rows + kPairRows - 1) / kPairRows, n_tiles = (p.n + p.bn - 1) / p.bn, tiles = m_tiles * n_tiles;
+  const int nkb = p.k / kBlockK;
+  const int my_tiles = pair < tiles ? (tiles - pair + pairs - 1) / pairs : 0;
+  const int F = my_tiles * nkb;
+
+  griddep_launch_dependents();
+  if (warp == 0 && lane == 0) {
+    tma_prefetch_desc(&tm_w);
+    tma_prefetch_desc(&tm_a);
+    for (int s = 0; s < p.stages; ++s) {
+      mbar_init(&tail->full[s], 1);
+      mbar_init(&tail->empty[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&tail->tmem_full[b], 1);
+      mbar_init(&tail->tmem_empty[b], 16);  // the eight epilogue warps of both CTAs
+    }
+    fence_barrier_init();
+  }
+  if (warp == 1) {
+    tmem_alloc_pair(&tail->tmem_base, 512);
+    tmem_relinquish_pair();
+  }
+  tcgen05_fence_before();
+  cluster_sync_all();
+  tcgen05_fence_after();
+  const uint32_t tmem_base = tail->tmem_base;
+
+  if (warp == 0) {
+    // (the whole warp counts and waits, one elected lane issues: a branch on the lane number makes the compiler guard every issue against
+    // divergence.  Stage, phase, k block and tile are counted, not divided out of a fill number.)
+    const bool issuer = elect_one();
+    int s = 0, kb = 0, m = pair % m_tiles, nt = pair / m_tiles;
+    uint32_t phase = 1;
+    const int m_step = pairs % m_tiles, n_step = pairs / m_tiles;
+    auto w_load = [&](int stage, int k, int n) {
+      if (rank == 0) mbar_expect_tx(&tail->full[stage], uint32_t(2 * stage_bytes));
+      tma_load_2d_pair(smem + stage * stage_bytes + kPairABytes, &tm_w, k * kBlockK, n * p.bn + rank * half_n, &tail->full[stage], kEvictLast);
+    };
+    auto a_load = [&](int stage, int k, int mt) {
+      tma_load_2d_pair(smem + stage * stage_bytes, &tm_a, k * kBlockK, mt * kPairRows + rank * 128, &tail->full[stage], kEvictLast);
+    };
+    // the first tile's weights do not depend on the previous kernel
+    const int pre = my_tiles == 0 ? 0 : (nkb < p.stages ? nkb : p.stages);
+    if (issuer)
+      for (int f = 0; f < pre; ++f) w_load(f, f, nt);
+    griddep_wait();
+    if (issuer)
+      for (int f = 0; f < pre; ++f) a_load(f, f, m);
+    for (int f = 0; f < F; ++f) {
+      if (f >= pre) {
+        mbar_wait(&tail->empty[s], phase);
+        if (issuer) {
+          w_load(s, kb, nt);
+          a_load(s, kb, m);
+        }
+      }
+      if (++s == p.stages) s = 0, phase ^= 1;
+      if (++kb == nkb) {
+        kb = 0;
+        nt += n_step;
+        m += m_step;
+        if (m >= m_tiles) m -= m_tiles, ++nt;
+      }
+    }
+    // the commits of the last stages arrive on this CTA's barriers too: they have to be there before it may leave
+    const int last = F < p.stages ? F : p.stages;
+    for (int f = 0; f < last; ++f) {
+      if (s == 0) s = p.stages, phase ^= 1;
+      --s;
+      mbar_wait(&tail->empty[s], phase ^ 1);
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (rank == 0) {
+      const bool issuer = elect_one();
+      const uint32_t idesc = umma_idesc_bf16(kPairRows, p.bn);
+      const uint64_t d0 = umma_desc_sw128(smem);
+      const uint32_t step = uint32_t(stage_bytes) >> 4;  // descriptors count in 16-byte units
+      int s = 0;
+      uint32_t phase = 0;
+      for (int j = 0; j < my_tiles; ++j) {
+        const int buf = j & 1;
+        if (j >= 2) mbar_wait(&tail->tmem_empty[buf], ((j >> 1) & 1) ^ 1);
+        tcgen05_fence_after();
+        const uint32_t acc = tmem_base + uint32_t(buf * kPairMaxCols);
+        for (int i = 0; i < nkb; ++i) {
+          mbar_wait(&tail->full[s], phase);
+          tcgen05_fence_after();
+          if (issuer) {
+            const uint64_t da = d0 + uint64_t(uint32_t(s) * step), dw = da + uint64_t(kPairABytes >> 4);
+#pragma unroll
+            for (int kk = 0; kk < kBlockK / kUmmaK; ++kk) umma_bf16_pair(acc, da + uint64_t(kk * 2), dw + uint64_t(kk * 2), idesc, uint32_t((i | kk) != 0));
+            umma_commit_pair(&tail->empty[s]);
+          }
+          if (++s == p.stages) s = 0, phase ^= 1;
+        }
+        if (issuer) umma_commit_pair(&tail->tmem_full[buf]);
+      }
+    }
+    __syncwarp();
+  } else {
+    const int half = (warp - 2) >> 2, quarter = warp & 3;
+    const int c0 = half == 0 ? 0 : p.first, c1 = half == 0 ? p.first : p.bn;
+    griddep_wait();  // side inputs (residual rows, row statistics) come from earlier kernels
+    for (int j = 0; j < my_tiles; ++j) {
+      const int t = pair + j * pairs, buf = j & 1;
+      WideTile w;
+      w.row = (t % m_tiles) * kPairRows + rank * 128 + quarter * 32 + lane;
+      w.valid = w.row < p.rows;
+      w.n0 = (t / m_tiles) * p.bn;
+      w.c0 = c0;
+      w.c1 = w.n0 + c1 < p.n ? c1 : (w.n0 + c0 < p.n ? p.n - w.n0 : c0);
+      w.slice = 2 * (t / m_tiles) + half;
+      const uint32_t taddr = tmem_base + (uint32_t(quarter * 32) << 16) + uint32_t(buf * kPairMaxCols);
+      const auto pre = epi.prepare(w);
+      mbar_wait(&tail->tmem_full[buf], (j >> 1) & 1);
+      tcgen05_fence_after();
+      epi(w, p.n, pre, [&](int c, float (&v)[16]) { tmem_ld_x16(taddr + uint32_t(c), v); });
+      tcgen05_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_leader(&tail->tmem_empty[buf]);
+    }
+  }
+  tcgen05_fence_before();
+  cluster_sync_all();  // the pair's shared memory and TMEM are in use until both CTAs are done
+  tcgen05_fence_after();
+  if (warp == 1) tmem_dealloc_pair(tmem_base, 512);
+}
+
+// ---- epilogues of the decoder engine (the row fragments of gemm_rows.cuh) -------------------------------------------------------
+
+template <int KIND>
+struct WideEpi {
+  EpiArgs e;
+
+  // the row's 1 / rms from the partial sums of squares that a residual epilogue left, eight loads at a time
+  __device__ __forceinline__ float prepare(const WideTile& w) const {
+    if (KIND == EPI_RESIDUAL || e.ss_in == nullptr || !w.valid) return 1.0f;
+    float tot = 0.0f;
+#pragma unroll 8
+    for (int t = 0; t < e.ss_tiles; ++t) tot += __ldcg(e.ss_in + (long long)t * e.ss_pitch + w.row);
+    return 1.0f / sqrtf(tot / float(e.ss_dim) + e.ss_eps);
+  }
+
+  template <class LD>
+  __device__ __forceinline__ void operator()(const WideTile& w, int n, float rs, LD&& ld16) const {
+    if (KIND == EPI_STORE_BF16) {
+      for (int c = w.c0; c < w.c1; c += 16) {
+        float v[16];
+        ld16(c, v);
+        rows_scale16(v, rs);
+        if (w.valid) rows_epi_store(e, n, w.row, w.n0 + c, v);
+      }
+    } else if (KIND == EPI_RESIDUAL) {
+      float sq = 0.0f;
+      for (int c = w.c0; c < w.c1; c += 16) {
+        float v[16];
+        ld16(c, v);
+        if (w.valid) sq += rows_epi_residual(e, n, w.row, w.n0 + c, v);
+      }
+      if (e.ss_out != nullptr && w.valid && w.n0 + w.c0 < n) e.ss_out[(long long)w.slice * e.ss_pitch + w.row] = sq;
+    } else if (KIND == EPI_SWIGLU) {
+      for (int c = w.c0; c < w.c1; c += 32) {
+        float g[16], u[16];
+        ld16(c, g);
+        ld16(c + 16, u);
+        rows_scale16(g, rs);
+        rows_scale16(u, rs);
+        if (w.valid) rows_epi_swiglu(e, n, w.row, w.n0 + c, g, u);
+      }
+    } else if (KIND == EPI_QKV_ROPE) {
+      const int half = e.d >> 1;
+      for (int h = w.c0; h < w.c1; h += e.d)
+        for (int d = 0; d < half; d += 16) {
+          float lo[16], hi[16];
+          ld16(h + d, lo);
+          ld16(h + d + half, hi);
+          rows_scale16(lo, rs);
+          rows_scale16(hi, rs);
+          if (w.valid) rows_epi_qkv(e, n, w.row, (w.n0 + h) / e.d, d, lo, hi);
+        }
+    }
+  }
+};
+
+}  // namespace mtx

@@ -13,6 +13,7 @@
 #include "../../include/mtx_b200.h"
 #include "gemm_rows.cuh"
 #include "gemm_umma.cuh"
+#include "gemm_wide.cuh"
 
 namespace mtx {
 // one instance per library, whichever translation unit touches it
@@ -120,6 +121,7 @@ bool use_pdl() {
 }
 
 thread_local int g_cluster_y = 1;  // cluster size along grid.y for the next launch (split-K GEMM)
+thread_local int g_cluster_x = 1;  // ... along grid.x (CTA pairs)
 thread_local bool g_cooperative = false;  // next launch is cooperative: all its CTAs are co-resident or the launch fails
 
 template <typename... KArgs, typename... Args>
@@ -141,9 +143,9 @@ int launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStr
     attr[na].val.programmaticStreamSerializationAllowed = 1;
     ++na;
   }
-  if (g_cluster_y > 1) {
+  if (g_cluster_y > 1 || g_cluster_x > 1) {
     attr[na].id = cudaLaunchAttributeClusterDimension;
-    attr[na].val.clusterDim.x = 1;
+    attr[na].val.clusterDim.x = unsigned(g_cluster_x);
     attr[na].val.clusterDim.y = unsigned(g_cluster_y);
     attr[na].val.clusterDim.z = 1;
     ++na;
@@ -308,6 +310,52 @@ int single_gemm(const void* x, const void* w, int rows, int n, int k, EpiArgs ea
   }
   MTX_TRY(make_map(&tx, x, k, r_tile, r_tile));
   return launch_gemm<EPI>(tw, tx, p, ea, plan_gemm(n, k, r_tile, 148, EPI), st);
+}
+
+// ---- steps of more than 256 rows: gemm_wide.cuh ------------------------------------------------
+// Columns of a pair's tile.  A k block costs a pair about 128 + bn parts of time (measured with the grid full: 0.17 / 0.19 / 0.22 / 0.32 us
+// at 64 / 128 / 160 / 256 columns), so the best bn is the one whose waves of tiles over the pairs cost least in all: 4000 x 1280 x 5120
+// takes 38.7 us on tiles of 160 columns (two waves of 74 pairs, 64 tiles each) and 55.8 us on 256 (80 tiles).  `unit`: columns that
+// one epilogue thread has to hold together (a head of a rotated projection, else 32).
+int wide_tile_columns(int rows, int n, int unit, int pairs) {
+  const int m_tiles = (rows + kPairRows - 1) / kPairRows;
+  int best = 0;
+  long long cost = 0;
+  for (int bn = kPairMaxCols; bn >= 64; bn -= 32) {
+    if (bn % unit != 0) continue;
+    const long long waves = ((long long)m_tiles * ((n + bn - 1) / bn) + pairs - 1) / pairs;
+    if (best == 0 || waves * (128 + bn) < cost) {
+      best = bn;
+      cost = waves * (128 + bn);
+    }
+  }
+  return best;
+}
+
+// epi(x[rows, k] . w[n, k]^T), n a multiple of 32 (and of unit), k of 64, 16-byte aligned operands
+template <class EPI>
+int launch_wide(const void* x, const void* w, int rows, int n, int k, int unit, const EPI& epi, int num_sms, cudaStream_t st) {
+  static bool attr_set = false;  // per template instance
+  if (!attr_set) {
+    MTX_CUDA(cudaFuncSetAttribute(gemm_wide_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    attr_set = true;
+  }
+  const int pairs = num_sms / 2;
+  WideParams p;
+  p.rows = rows;
+  p.n = n;
+  p.k = k;
+  p.bn = wide_tile_columns(rows, n, unit, pairs);
+  p.stages = wide_stages(p.bn);
+  p.first = (p.bn / unit + 1) / 2 * unit;
+  CUtensorMap tw, tx;
+  MTX_TRY(make_map(&tw, w, k, n, uint32_t(p.bn / 2)));
+  MTX_TRY(make_map(&tx, x, k, rows, 128));
+  const int tiles = ((rows + kPairRows - 1) / kPairRows) * ((n + p.bn - 1) / p.bn);
+  g_cluster_x = 2;
+  const int rc = launch(gemm_wide_kernel<EPI>, dim3(2 * (tiles < pairs ? tiles : pairs)), dim3(kPairThreads), wide_smem_bytes(p.bn, p.stages), st, tw, tx, p, epi);
+  g_cluster_x = 1;
+  return rc;
 }
 
 }  // namespace

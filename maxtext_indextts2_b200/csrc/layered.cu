@@ -13,6 +13,7 @@
 #include "../../include/mtx_b200.h"
 #include "layer_ops.cuh"
 #include "linear_any.cuh"
+#include "linear_wide.cuh"
 #include "grouped_gemm.cuh"
 #include "window_attention.cuh"
 #include "window_attention_mma.cuh"
@@ -233,27 +234,42 @@ __global__ void act_bf16_kernel(const bf16* src, bf16* act, int n, long long ldo
   }
 }
 
-// the same product on the tcgen05 GEMM: the bf16 result stays in e->obf (256-row blocks)
+// steps of more than 256 rows run the pair GEMM, all rows in one launch (gemm_rows.cuh needs a launch per 256 rows: 257 rows of a
+// 1792 x 1280 projection take 12 us against 21)
+bool takes_wide(int rows) { return rows > 256; }
+
+// the same product on a tcgen05 GEMM: the bf16 result stays in e->obf
 int run_umma_raw(mtx_layered* e, const void* a, const void* w, int rows, int n, int k, cudaStream_t st) {
-  bf16* tmp = static_cast<bf16*>(e->obf);
-  for (int r0 = 0; r0 < rows; r0 += 256) {
-    const int nr = rows - r0 < 256 ? rows - r0 : 256;
-    EpiArgs ea;
-    memset(&ea, 0, sizeof(ea));
-    ea.out = tmp + size_t(r0) * n;
-    ea.ld_out = n;
-    MTX_TRY(single_gemm<EPI_STORE_BF16>(static_cast<const bf16*>(a) + size_t(r0) * k, w, nr, n, k, ea, st));
-  }
-  return MTX_OK;
+  EpiArgs ea;
+  memset(&ea, 0, sizeof(ea));
+  ea.out = static_cast<bf16*>(e->obf);
+  ea.ld_out = n;
+  if (!takes_wide(rows)) return single_gemm<EPI_STORE_BF16>(a, w, rows, n, k, ea, st);
+  WideEpi<EPI_STORE_BF16> epi;
+  epi.e = ea;
+  return launch_wide(a, w, rows, n, k, 32, epi, e->num_sms, st);
 }
 
 // ... then the epilogue as a row kernel
 template <int EPI>
 int run_linear_umma(mtx_layered* e, const void* a, const void* w, const float* bias, float* out, void* act, int rows, int n, int k, cudaStream_t st,
                     float limit = 0.0f, long long ldo = 0, int silu0 = 0, int silu1 = 0) {
+  constexpr bool gated = EPI == LIN_GATED || EPI == LIN_GATED_CLAMP, narrow = gated || EPI == LIN_ACT || EPI == LIN_RELU2 || EPI == LIN_GELU;
+  if (takes_wide(rows)) {  // the epilogue works on the accumulator itself
+    WideLinEpi<EPI> epi;
+    epi.bias = bias;
+    epi.out = out;
+    epi.act = static_cast<bf16*>(act);
+    epi.ldo = ldo > 0 ? ldo : (gated ? n / 2 : n);
+    epi.limit = limit;
+    epi.silu0 = silu0;
+    epi.silu1 = silu1;
+    const void* dst = narrow ? act : static_cast<const void*>(out);
+    if (epi.ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0 && (reinterpret_cast<uintptr_t>(bias) & 15) == 0)
+      return launch_wide(a, w, rows, n, k, 32, epi, e->num_sms, st);
+  }
   MTX_TRY(run_umma_raw(e, a, w, rows, n, k, st));
   const bf16* tmp = static_cast<const bf16*>(e->obf);
-  constexpr bool gated = EPI == LIN_GATED || EPI == LIN_GATED_CLAMP;
   const long long total = (long long)rows * (gated ? n / 2 : n);
   const int blocks = int((total + 255) / 256 < 148 * 8 ? (total + 255) / 256 : 148 * 8);
   const long long groups = total / 8;  // (n is a multiple of 128)
