@@ -342,56 +342,71 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   const int F = my_tiles * nkb;  // ring fills of this CTA: fill f = (tile f / nkb, k-block kb0 + f % nkb)
 
   if (warp == 0) {
-    // ===== TMA producer =====
-    if (lane == 0) {
-      auto w_load = [&](int f) {
-        const int s = f % p.stages, n0 = (first_tile + (f / nkb) * tile_stride) * kTileN, kb = kb0 + f % nkb;
-        mbar_expect_tx(&tail->full[s], uint32_t(stage_bytes));
-        tma_load_2d(smem + size_t(s) * stage_bytes, &tm_w, kb * kBlockK, n0, &tail->full[s], kEvictFirst);
-      };
-      auto x_load = [&](int f) {
-        const int s = f % p.stages, kb = kb0 + f % nkb;
-        tma_load_2d(smem + size_t(s) * stage_bytes + kWTileBytes, &tm_x, kb * kBlockK, row_base, &tail->full[s], kEvictLast);
-      };
-      const int pre = F < p.stages ? F : p.stages;
-      for (int f = 0; f < pre; ++f) w_load(f);  // weights do not depend on the previous kernel
-      griddep_wait();
-      if (trace) trace[1] = clock64() - t_start;
-      for (int f = 0; f < pre; ++f) x_load(f);
-      for (int f = pre; f < F; ++f) {
-        mbar_wait(&tail->empty[f % p.stages], ((f / p.stages) & 1) ^ 1);
-        w_load(f);
-        x_load(f);
+    // ===== TMA producer: the whole warp counts and waits, one elected lane issues (see elect_one) =====
+    const bool issuer = elect_one();
+    int s = 0, kb = 0, tile = first_tile;  // the next fill: stage, k-block of the unit, tile
+    uint32_t phase = 1;
+    auto w_load = [&]() {
+      mbar_expect_tx(&tail->full[s], uint32_t(stage_bytes));
+      tma_load_2d(smem + s * stage_bytes, &tm_w, (kb0 + kb) * kBlockK, tile * kTileN, &tail->full[s], kEvictFirst);
+    };
+    auto x_load = [&]() { tma_load_2d(smem + s * stage_bytes + kWTileBytes, &tm_x, (kb0 + kb) * kBlockK, row_base, &tail->full[s], kEvictLast); };
+    auto next = [&]() {
+      if (++s == p.stages) s = 0, phase ^= 1;
+      if (++kb == nkb) kb = 0, tile += tile_stride;
+    };
+    const int pre = F < p.stages ? F : p.stages;
+    for (int f = 0; f < pre; ++f) {  // weights do not depend on the previous kernel
+      if (issuer) w_load();
+      next();
+    }
+    griddep_wait();
+    if (trace && issuer) trace[1] = clock64() - t_start;
+    s = kb = 0, tile = first_tile, phase = 1;
+    for (int f = 0; f < pre; ++f) {
+      if (issuer) x_load();
+      next();
+    }
+    for (int f = pre; f < F; ++f) {
+      mbar_wait(&tail->empty[s], phase);
+      if (issuer) {
+        w_load();
+        x_load();
       }
+      next();
     }
     __syncwarp();
   } else if (warp == 1) {
-    // ===== MMA issuer =====
-    if (lane == 0) {
-      const uint32_t idesc = umma_idesc_bf16(128, kTileN);
-      int f = 0;
-      for (int j = 0; j < my_tiles; ++j) {
-        const uint32_t buf = split ? 0u : uint32_t(j & 1);
-        if (j >= 2) mbar_wait(&tail->tmem_empty[buf], ((j >> 1) & 1) ^ 1);
+    // ===== MMA issuer (the same division of the warp) =====
+    const bool issuer = elect_one();
+    const uint32_t idesc = umma_idesc_bf16(128, kTileN);
+    const uint64_t d0 = umma_desc_sw128(smem);
+    const uint32_t step = uint32_t(stage_bytes) >> 4;  // descriptors count in 16-byte units
+    int s = 0;
+    uint32_t phase = 0;
+    for (int j = 0; j < my_tiles; ++j) {
+      const uint32_t buf = split ? 0u : uint32_t(j & 1);
+      if (j >= 2) mbar_wait(&tail->tmem_empty[buf], ((j >> 1) & 1) ^ 1);
+      tcgen05_fence_after();
+      for (int i = 0; i < nkb; ++i) {
+        mbar_wait(&tail->full[s], phase);
         tcgen05_fence_after();
-        for (int i = 0; i < nkb; ++i, ++f) {
-          const int s = f % p.stages;
-          mbar_wait(&tail->full[s], (f / p.stages) & 1);
-          tcgen05_fence_after();
-          if (trace && f == 0) trace[2] = clock64() - t_start;
-          const uint64_t dw = umma_desc_sw128(smem + size_t(s) * stage_bytes);
+        if (issuer) {
+          if (trace && i == 0 && j == 0) trace[2] = clock64() - t_start;
+          const uint64_t dw = d0 + uint64_t(uint32_t(s) * step);
           for (int mb = 0; mb < mblocks; ++mb) {
-            const uint64_t dx = umma_desc_sw128(smem + size_t(s) * stage_bytes + kWTileBytes + size_t(mb) * 128 * kBlockK * 2);
+            const uint64_t dx = dw + uint64_t((kWTileBytes + mb * 128 * kBlockK * 2) >> 4);
             const uint32_t acc = tmem_base + buf * uint32_t(acc_cols) + uint32_t(mb) * 128u;
 #pragma unroll
             for (int kk = 0; kk < kBlockK / kUmmaK; ++kk) umma_bf16(acc, dx + uint64_t(kk * 2), dw + uint64_t(kk * 2), idesc, uint32_t((i | kk) != 0));
           }
           umma_commit(&tail->empty[s]);
         }
-        umma_commit(&tail->tmem_full[buf]);
+        if (++s == p.stages) s = 0, phase ^= 1;
       }
-      if (trace) trace[3] = clock64() - t_start;
+      if (issuer) umma_commit(&tail->tmem_full[buf]);
     }
+    if (trace && issuer) trace[3] = clock64() - t_start;
     __syncwarp();
   } else {
     // ===== epilogue: eight warps; warp w reads TMEM lanes 32 (w % 4) .., warps of quarter pairs split the row blocks =====

@@ -365,47 +365,55 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   const uint32_t tmem_base = tail->tmem_base;
 
   if (warp == 0) {
-    // ===== TMA producer =====
-    if (lane == 0) {
-      const int pre = nkb < p.stages ? nkb : p.stages;
-      if (trace) trace[0] = clock64() - t_start;
+    // ===== TMA producer: the whole warp counts and waits, one elected lane issues (see elect_one) =====
+    const bool issuer = elect_one();
+    const int pre = nkb < p.stages ? nkb : p.stages;
+    if (trace && issuer) trace[0] = clock64() - t_start;
+    if (issuer)
       for (int i = 0; i < pre; ++i) {  // weights do not depend on the previous kernel
         mbar_expect_tx(&tail->full[i], uint32_t(stage_bytes));
-        tma_load_2d(smem + size_t(i) * stage_bytes, &tm_w, (kb0 + i) * kBlockK, n0, &tail->full[i], kEvictFirst);
+        tma_load_2d(smem + i * stage_bytes, &tm_w, (kb0 + i) * kBlockK, n0, &tail->full[i], kEvictFirst);
       }
-      griddep_wait();
-      if (trace) trace[1] = clock64() - t_start;
-      for (int i = 0; i < pre; ++i)
-        tma_load_2d(smem + size_t(i) * stage_bytes + kWTileBytes, &tm_x, (kb0 + i) * kBlockK, 0, &tail->full[i], kEvictLast);
-      for (int i = pre; i < nkb; ++i) {
-        const int s = i % p.stages;
-        mbar_wait(&tail->empty[s], ((i / p.stages) & 1) ^ 1);
+    griddep_wait();
+    if (trace && issuer) trace[1] = clock64() - t_start;
+    if (issuer)
+      for (int i = 0; i < pre; ++i) tma_load_2d(smem + i * stage_bytes + kWTileBytes, &tm_x, (kb0 + i) * kBlockK, 0, &tail->full[i], kEvictLast);
+    int s = 0;
+    uint32_t phase = 0;  // (the first refill waits for the first fill's MMAs)
+    for (int i = pre; i < nkb; ++i) {
+      mbar_wait(&tail->empty[s], phase);
+      if (issuer) {
         if (trace && i < 30) trace[2 + i] = clock64() - t_start;
         mbar_expect_tx(&tail->full[s], uint32_t(stage_bytes));
-        tma_load_2d(smem + size_t(s) * stage_bytes, &tm_w, (kb0 + i) * kBlockK, n0, &tail->full[s], kEvictFirst);
-        tma_load_2d(smem + size_t(s) * stage_bytes + kWTileBytes, &tm_x, (kb0 + i) * kBlockK, 0, &tail->full[s], kEvictLast);
+        tma_load_2d(smem + s * stage_bytes, &tm_w, (kb0 + i) * kBlockK, n0, &tail->full[s], kEvictFirst);
+        tma_load_2d(smem + s * stage_bytes + kWTileBytes, &tm_x, (kb0 + i) * kBlockK, 0, &tail->full[s], kEvictLast);
       }
+      if (++s == p.stages) s = 0, phase ^= 1;
     }
     __syncwarp();
   } else if (warp == 1) {
-    // ===== MMA issuer =====
-    if (lane == 0) {
-      const uint32_t idesc = umma_idesc_bf16(kTileN, p.r_tile);
-      for (int i = 0; i < nkb; ++i) {
-        const int s = i % p.stages;
-        mbar_wait(&tail->full[s], (i / p.stages) & 1);
-        tcgen05_fence_after();
+    // ===== MMA issuer (the same division of the warp) =====
+    const bool issuer = elect_one();
+    const uint32_t idesc = umma_idesc_bf16(kTileN, p.r_tile);
+    const uint64_t d0 = umma_desc_sw128(smem);
+    const uint32_t step = uint32_t(stage_bytes) >> 4;  // descriptors count in 16-byte units
+    int s = 0;
+    uint32_t phase = 0;
+    for (int i = 0; i < nkb; ++i) {
+      mbar_wait(&tail->full[s], phase);
+      tcgen05_fence_after();
+      if (issuer) {
         if (trace && i < 30) trace[40 + i] = clock64() - t_start;
-        const uint64_t da = umma_desc_sw128(smem + size_t(s) * stage_bytes);
-        const uint64_t db = umma_desc_sw128(smem + size_t(s) * stage_bytes + kWTileBytes);
+        const uint64_t da = d0 + uint64_t(uint32_t(s) * step), db = da + uint64_t(kWTileBytes >> 4);
 #pragma unroll
         for (int kk = 0; kk < kBlockK / kUmmaK; ++kk)
           umma_bf16(tmem_base, da + uint64_t(kk * 2), db + uint64_t(kk * 2), idesc, uint32_t((i | kk) != 0));
         umma_commit(&tail->empty[s]);
       }
-      umma_commit(&tail->tmem_full);
-      if (trace) trace[39] = clock64() - t_start;
+      if (++s == p.stages) s = 0, phase ^= 1;
     }
+    if (issuer) umma_commit(&tail->tmem_full);
+    if (trace && issuer) trace[39] = clock64() - t_start;
     __syncwarp();
   }
 

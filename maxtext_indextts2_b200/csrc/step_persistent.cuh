@@ -1410,51 +1410,53 @@ step_persistent_kernel(const __grid_constant__ CUtensorMap tm_wqkv, const __grid
   if (warp == 0) {
     // =================================== weight producer =================================
     // Runs ahead of the grid barriers, bounded only by the ring: a stage is refilled as soon as the MMAs that
-    // read it have completed.
-    if (lane == 0) {
-      PkCursor c;
-      pk_cursor_init(c);
-      for_each_unit([&](int l, int ph, int tile, int kb0, int kb1) {
-        const CUtensorMap* tmw = ph == PK_QKV ? &tm_wqkv : ph == PK_OPROJ ? &tm_wo : ph == PK_UP ? &tm_w01 : ph == PK_DOWN ? &tm_wout : &tm_wlogits;
-        const int n_ph = ph == PK_QKV ? p.qkv_n : ph == PK_UP ? 2 * p.M : ph == PK_LOGITS ? 0 : p.E;
-        const int row = l * n_ph + tile * kTileN;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (c.uses) mbar_wait(&tail->empty[c.s], c.par ^ 1);
+    // read it have completed.  (The whole warp counts and waits, one elected lane issues: see elect_one.)
+    const bool issuer = elect_one();
+    PkCursor c;
+    pk_cursor_init(c);
+    for_each_unit([&](int l, int ph, int tile, int kb0, int kb1) {
+      const CUtensorMap* tmw = ph == PK_QKV ? &tm_wqkv : ph == PK_OPROJ ? &tm_wo : ph == PK_UP ? &tm_w01 : ph == PK_DOWN ? &tm_wout : &tm_wlogits;
+      const int n_ph = ph == PK_QKV ? p.qkv_n : ph == PK_UP ? 2 * p.M : ph == PK_LOGITS ? 0 : p.E;
+      const int row = l * n_ph + tile * kTileN;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (c.uses) mbar_wait(&tail->empty[c.s], c.par ^ 1);
+        if (issuer) {
           mbar_expect_tx(&tail->full_w[c.s], uint32_t(kWTileBytes));
           tma_load_2d(ring + size_t(c.s) * kPkStageBytes, tmw, kb * kBlockK, row, &tail->full_w[c.s], kEvictFirst);
-          pk_cursor_next(c);
         }
-      });
-    }
+        pk_cursor_next(c);
+      }
+    });
     __syncwarp();
   } else if (warp == 1) {
     // =================================== MMA issuer =====================================
-    if (lane == 0) {
-      const uint32_t idesc = umma_idesc_bf16(kTileN, p.r_tile);
-      PkCursor c;
-      pk_cursor_init(c);
-      uint32_t uc = 0;
-      for_each_unit([&](int, int, int, int kb0, int kb1) {
-        const uint32_t buf = uc % kPkAccBufs;
-        const uint32_t acc = tmem_base + buf * uint32_t(p.r_tile);
-        if (uc >= uint32_t(kPkAccBufs)) mbar_wait(&tail->tmem_empty[buf], ((uc / kPkAccBufs) & 1) ^ 1);
+    const bool issuer = elect_one();
+    const uint32_t idesc = umma_idesc_bf16(kTileN, p.r_tile);
+    const uint64_t d0 = umma_desc_sw128(ring);
+    PkCursor c;
+    pk_cursor_init(c);
+    uint32_t uc = 0;
+    for_each_unit([&](int, int, int, int kb0, int kb1) {
+      const uint32_t buf = uc % kPkAccBufs;
+      const uint32_t acc = tmem_base + buf * uint32_t(p.r_tile);
+      if (uc >= uint32_t(kPkAccBufs)) mbar_wait(&tail->tmem_empty[buf], ((uc / kPkAccBufs) & 1) ^ 1);
+      tcgen05_fence_after();
+      for (int kb = kb0; kb < kb1; ++kb) {
+        mbar_wait(&tail->full_w[c.s], c.par);
+        mbar_wait(&tail->xready[c.s], c.par);
         tcgen05_fence_after();
-        for (int kb = kb0; kb < kb1; ++kb) {
-          mbar_wait(&tail->full_w[c.s], c.par);
-          mbar_wait(&tail->xready[c.s], c.par);
-          tcgen05_fence_after();
-          const uint64_t da = umma_desc_sw128(ring + size_t(c.s) * kPkStageBytes);
-          const uint64_t db = umma_desc_sw128(ring + size_t(c.s) * kPkStageBytes + kWTileBytes);
+        if (issuer) {
+          const uint64_t da = d0 + uint64_t(uint32_t(c.s) * uint32_t(kPkStageBytes >> 4)), db = da + uint64_t(kWTileBytes >> 4);
 #pragma unroll
           for (int kk = 0; kk < kBlockK / kUmmaK; ++kk)
             umma_bf16(acc, da + uint64_t(kk * 2), db + uint64_t(kk * 2), idesc, uint32_t((kb > kb0) || kk > 0));
           umma_commit(&tail->empty[c.s]);
-          pk_cursor_next(c);
         }
-        umma_commit(&tail->tmem_full[buf]);
-        ++uc;
-      });
-    }
+        pk_cursor_next(c);
+      }
+      if (issuer) umma_commit(&tail->tmem_full[buf]);
+      ++uc;
+    });
     __syncwarp();
   } else if (warp < 6) {
     // =================================== epilogue warps ==================================
@@ -1823,15 +1825,18 @@ step_persistent_kernel(const __grid_constant__ CUtensorMap tm_wqkv, const __grid
       pk_wait_flag(&tail->bar_done, pk_need(layer, ph, p.L));
       fence_proxy_async_all();  // activations written with generic stores by other CTAs, read through TMA
       evx.on = layer == 1;
+      const bool issuer = elect_one();
       for (int u = 0; u < nu; ++u) {
         const int kb0 = ph == PK_LOGITS ? 0 : tab.u[ph][u].kb0, kb1 = ph == PK_LOGITS ? kb_e : tab.u[ph][u].kb1;
         for (int kb = kb0; kb < kb1; ++kb) {
           if (cur.uses) mbar_wait(&tail->empty[cur.s], cur.par ^ 1);
-          pk_ev(evx, 100 * ph + 1);
-          uint64_t* bar = xform ? &tail->full_x[cur.s] : &tail->xready[cur.s];
-          if (!xform) mbar_arrive(&tail->full_x[cur.s]);  // keep every barrier of the stage in step
-          mbar_expect_tx(bar, uint32_t(x_bytes));
-          tma_load_2d(ring + size_t(cur.s) * kPkStageBytes + kWTileBytes, tmx, kb * kBlockK, 0, bar, kEvictLast);
+          if (issuer) {
+            pk_ev(evx, 100 * ph + 1);
+            uint64_t* bar = xform ? &tail->full_x[cur.s] : &tail->xready[cur.s];
+            if (!xform) mbar_arrive(&tail->full_x[cur.s]);  // keep every barrier of the stage in step
+            mbar_expect_tx(bar, uint32_t(x_bytes));
+            tma_load_2d(ring + size_t(cur.s) * kPkStageBytes + kWTileBytes, tmx, kb * kBlockK, 0, bar, kEvictLast);
+          }
           pk_cursor_next(cur);
         }
       }
@@ -1930,7 +1935,7 @@ step_persistent_kernel(const __grid_constant__ CUtensorMap tm_wqkv, const __grid
       const bool xform = (ph == PK_QKV || ph == PK_UP) && !p.fold;
       if (xformer && xform) {
         transform_phase(ph, layer);
-      } else if (xproducer && lane == 0) {
+      } else if (xproducer) {
         x_phase(ph, layer);
       } else {
         pk_cursor_skip(cur, tab.kbs[ph]);
@@ -1986,7 +1991,7 @@ step_persistent_kernel(const __grid_constant__ CUtensorMap tm_wqkv, const __grid
       }
       __syncwarp();
     }
-    if (xproducer && lane == 0) x_phase(PK_LOGITS, p.L);
+    if (xproducer) x_phase(PK_LOGITS, p.L);
     __syncwarp();
   }
 
