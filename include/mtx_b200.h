@@ -250,6 +250,11 @@ int mtx_profile_decode_step(mtx_engine* e, int rows, mtx_stream stream, float* c
 int mtx_prefill_chunk(mtx_engine* e, const int32_t* tokens, int count, int start_pos, int slot, int sample_last,
                       int32_t* first_token, float* logits_out, float* first_log_prob, mtx_stream stream);
 
+/* The same for any number of positions, up to max_prefill_len in all: long prompts run through the layers in passes of thousands of rows.
+ * `draw_row` (0..255): which of the prefill's noise rows the draw of the first token uses; mtx_prefill_chunk uses its last row's index. */
+int mtx_prefill_rows(mtx_engine* e, const int32_t* tokens, int count, int start_pos, int slot, int sample_last, int draw_row, int32_t* first_token,
+                     float* logits_out, float* first_log_prob, mtx_stream stream);
+
 /* MaxEngine.insert (maxengine.py:1166-1192, _insert_jit :1045-1164): the first n_rows cache rows of a prefix (k_src / v_src
  * [L, Hkv, n_src_rows, D] bf16, what prefill left) into the prefill segment of decode slot `slot`, every layer and head in one
  * launch, and the slot's bookkeeping: prefill_len = n_rows, ar_lengths = 0, next_pos / generated / tokens as given.  The AR ring

@@ -341,6 +341,8 @@ def _declare(lib) -> None:
   lib.mtx_profile_decode_step.argtypes = [vp, i32, vp, c.POINTER(c.c_float), c.POINTER(c.c_int32)]
   lib.mtx_prefill_chunk.restype = i32
   lib.mtx_prefill_chunk.argtypes = [vp, vp, i32, i32, i32, i32, vp, vp, vp, vp]
+  lib.mtx_prefill_rows.restype = i32
+  lib.mtx_prefill_rows.argtypes = [vp, vp, i32, i32, i32, i32, i32, vp, vp, vp, vp]
   lib.mtx_insert_prefix.restype = i32
   lib.mtx_insert_prefix.argtypes = [vp, vp, vp, i32, i32, i32, i32, i32, i32, vp]
   lib.mtx_rmsnorm.restype = i32

@@ -21,6 +21,7 @@
 #include "gemma3_kernels.cuh"
 #include "paged_kv.cuh"
 #include "prefill_attention.cuh"
+#include "prefill_flash.cuh"
 #include "sampling.cuh"
 #include "step_kernels.cuh"
 #include "step_persistent.cuh"
@@ -52,6 +53,7 @@ struct mtx_engine {
   mtx_model_config cfg;
   int num_sms = 148;
   int max_r_tile = 16;
+  int pf_rows = 0;  // rows that one pass over a long prompt takes (0: prompts fit the 256-row steps)
   int qkv_n = 0;
   int attn_max_chunks = 0;
   bool bound = false;
@@ -132,9 +134,15 @@ bool kvq_fp8(const mtx_model_config& c) { return c.kv_quant >= 3; }
 bool is_paged(const mtx_model_config& c) { return c.paged_num_pages > 0; }
 bool staged_prefill(const mtx_model_config& c) { return c.kv_quant != 0 || is_paged(c); }
 
+// A long prompt's rows go through the layers together, at most kPfMaxRows of them (a 4096-row pass of a 10240-wide feed-forward holds 84 MB of
+// activations and leaves no wave of the GEMMs short; longer prompts take several passes).
+constexpr int kPfMaxRows = 4096;
+// most slices of a row that the residual epilogues of such a pass leave sums of squares of: two per tile of at least 64 columns
+size_t pf_slices(int emb_dim) { return 2 * size_t((emb_dim + 63) / 64); }
+
 WsLayout layout_workspace(const mtx_engine* e) {
   const mtx_model_config& c = e->cfg;
-  const size_t rt = e->max_r_tile;
+  const size_t rt = e->max_r_tile > e->pf_rows ? e->max_r_tile : e->pf_rows;
   WsLayout L;
   size_t off = 0;
   auto take = [&](size_t bytes) {
@@ -199,8 +207,9 @@ WsLayout layout_workspace(const mtx_engine* e) {
     L.pk_attn_part_o = take(pairs * kPkMaxParts * ((G * c.head_dim + 2 * G + 3) / 4 * 4) * 4);
     L.pk_tile_prefix = take((pk_rows + 1) * 4);
     L.pk_attn_info = take(64);
-    L.rows_ss_x = take(rt * ss_tiles * 4);
-    L.rows_ss_h = take(rt * ss_tiles * 4);
+    const size_t slices = e->pf_rows > 0 ? pf_slices(c.emb_dim) : ss_tiles;  // partial sums of squares per row
+    L.rows_ss_x = take(rt * slices * 4);
+    L.rows_ss_h = take(rt * slices * 4);
     L.cand_counters = take(64);
     L.par_M = take(size_t(c.max_rows) * 4);
     L.par_cand_count = take(size_t(c.max_rows) * 4);
@@ -346,6 +355,40 @@ int launch_prefill_attention(mtx_engine* e, int layer, int rows, int start_pos, 
   }
   if (c.head_dim == 64) return launch(prefill_attn_kernel<64>, grid, block, smem, st, e->tm_k, e->tm_v, p);
   return launch(prefill_attn_kernel<128>, grid, block, smem, st, e->tm_k, e->tm_v, p);
+}
+
+// The same for a pass of more than 256 rows (prefill_flash.cuh).  The 16-position CTAs above keep more SMs busy when positions are few: 256 rows
+// of 20 heads take 22 us there.
+template <int D>
+int launch_prefill_flash(mtx_engine* e, const CUtensorMap& tm_q, const PrefillFlashParams& p, cudaStream_t st) {
+  static bool attr_set = false;  // per head size
+  if (!attr_set) {
+    MTX_CUDA(cudaFuncSetAttribute(prefill_flash_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(prefill_flash_smem_bytes<D>())));
+    attr_set = true;
+  }
+  constexpr int rows_cta = FlashShape<D>::NQ * 128;
+  return launch(prefill_flash_kernel<D>, dim3(p.hq, (p.rows + rows_cta - 1) / rows_cta), dim3(FlashShape<D>::kThreads), prefill_flash_smem_bytes<D>(), st, tm_q,
+                e->tm_k, e->tm_v, p);
+}
+int launch_prefill_flash(mtx_engine* e, int layer, int rows, int start_pos, int slot, cudaStream_t st) {
+  const mtx_model_config& c = e->cfg;
+  const int planes = staged_prefill(c) ? 1 : c.num_slots;
+  CUtensorMap tm_q;
+  MTX_TRY(make_map(&tm_q, e->q, uint64_t(c.num_q_heads) * c.head_dim, rows, 128));
+  PrefillFlashParams p;
+  memset(&p, 0, sizeof(p));
+  p.out = e->attn;
+  p.rows = rows;
+  p.start_pos = start_pos;
+  p.hq = c.num_q_heads;
+  p.hkv = c.num_kv_heads;
+  p.T = c.max_target_len;
+  p.plane_row0 = (layer * planes + slot) * c.num_kv_heads * c.max_target_len;
+  p.softcap = c.attn_softcap;
+  p.window = layer_is_local(e, layer) ? c.sliding_window : 0;
+  if (c.head_dim == 64) return launch_prefill_flash<64>(e, tm_q, p, st);
+  if (c.head_dim == 128) return launch_prefill_flash<128>(e, tm_q, p, st);
+  return launch_prefill_flash<256>(e, tm_q, p, st);
 }
 
 // ---- persistent step kernel: work tables and launch -------------------------------------------
@@ -588,6 +631,229 @@ int launch_persistent(mtx_engine* e, int rows, const XMaps& xm, const EpiArgs& l
 // Noise row of a prefill draw: outside the rows of any decode step (< 256), one block of 256 rows per prefill call.
 int prefill_noise_row(const mtx_engine* e) { return 0x40000000 + int(e->prefill_draws % 0x100000u) * 256; }
 
+const char* const kTwoPassNeedsLogits = "nucleus / topk sampling read the materialised logits: decode_state.logits (or logits_out) must be set";
+
+// The prompt's last row `x` -> final norm, logits, the first token.  Only this row goes through the logits projection (a step of 256 prompt
+// rows spent 277 us on the logits of all of them; one row streams the 676 MB of weights in 110).  `draw_row`: the draw's row in the
+// prefill's noise block.
+int enqueue_last_logits(mtx_engine* e, const bf16* x, int draw_row, int32_t* first_token, float* prefill_logits, float* first_log_prob, cudaStream_t st) {
+  const mtx_model_config& c = e->cfg;
+  const int E = c.emb_dim;
+  const bool two_pass = e->strategy == MTX_SAMPLE_NUCLEUS || e->strategy == MTX_SAMPLE_TOPK;
+  if (two_pass && prefill_logits == nullptr) return fail(MTX_ERR_ARG, "%s", kTwoPassNeedsLogits);
+  const int noise_row = prefill_noise_row(e) + draw_row;
+  g_class = KC_RMSNORM;
+  MTX_TRY(launch(rmsnorm_kernel<false>, dim3(1), dim3(128), 0, st, x, (const int*)nullptr, (const bf16*)nullptr, static_cast<const bf16*>(e->w.final_norm),
+                 (bf16*)nullptr, e->n, E, c.rms_eps));
+  GemmParams gp;
+  memset(&gp, 0, sizeof(gp));
+  gp.rows = 1;
+  gp.r_tile = 16;
+  gp.n = c.vocab_size;
+  gp.k = E;
+  const GemmPlan plan = plan_gemm(c.vocab_size, E, 16, e->num_sms, EPI_LOGITS, 1);
+  EpiArgs ea;
+  memset(&ea, 0, sizeof(ea));
+  ea.logits_out = prefill_logits;
+  ea.ld_logits = c.vocab_size;
+  ea.logits_only_row = 0;
+  ea.part_score = e->part_score;
+  ea.part_idx = e->part_idx;
+  ea.part_raw = e->part_raw;
+  ea.part_max = e->part_max;
+  ea.part_sum = e->part_sum;
+  ea.n_tiles = plan.n_tiles;
+  ea.vocab_offset = c.vocab_offset;
+  ea.scale = c.logits_scale;
+  ea.softcap = c.final_softcap;
+  ea.inv_temp = 1.0f / e->temperature;
+  ea.round_bf16 = c.logits_round_bf16;
+  ea.gumbel = e->strategy == MTX_SAMPLE_WEIGHTED ? 1 : 0;
+  ea.want_lse = first_log_prob != nullptr && !two_pass ? 1 : 0;
+  ea.rng_state = e->s.rng_state;
+  ea.row_offset = noise_row;
+  XMaps* xm;
+  MTX_TRY(get_xmaps(e, 16, &xm));
+  g_class = KC_LOGITS;
+  MTX_TRY(launch_gemm<EPI_LOGITS>(e->tm_logits, xm->n, gp, ea, plan, st));
+  g_class = KC_FINALIZE;
+  FinalizeArgs fa;
+  memset(&fa, 0, sizeof(fa));
+  fa.part_score = e->part_score;
+  fa.part_idx = e->part_idx;
+  fa.part_raw = e->part_raw;
+  fa.part_max = e->part_max;
+  fa.part_sum = e->part_sum;
+  fa.n_tiles = plan.n_tiles;
+  fa.rows = 1;
+  fa.stride_r = plan.n_tiles;
+  fa.stride_t = 1;
+  if (two_pass) {  // inference_utils.py:87-111 on the row the GEMM just wrote; one candidate
+    SampleArgs sa;
+    memset(&sa, 0, sizeof(sa));
+    sa.logits = prefill_logits;
+    sa.ld = c.vocab_size;
+    sa.vocab = c.vocab_size;
+    sa.vocab_offset = c.vocab_offset;
+    sa.mode = e->strategy;
+    sa.top_k = e->top_k;
+    sa.nucleus_p = e->nucleus_p;
+    sa.inv_temp = 1.0f / e->temperature;
+    sa.rng_state = e->s.rng_state;
+    sa.row_offset = noise_row;
+    sa.out_score = e->part_score;
+    sa.out_idx = e->part_idx;
+    sa.out_raw = e->part_raw;
+    sa.out_max = e->part_max;
+    sa.out_sum = e->part_sum;
+    MTX_TRY(launch(sample_rows_kernel, dim3(1), dim3(kSampleThreads), 0, st, sa));
+    fa.n_tiles = 1;
+    fa.stride_r = 1;
+  }
+  fa.mode = 1;
+  fa.have_lse = two_pass || first_log_prob != nullptr ? 1 : 0;
+  fa.log_prob = first_log_prob;
+  fa.rng_state = e->s.rng_state;
+  fa.first_token = first_token;
+  return launch(finalize_kernel, dim3(1), dim3(kFinalizeThreads), 0, st, fa);
+}
+
+// The layers over `rows` (more than 256, at most pf_rows) prompt positions from start_pos on, all rows in every launch: the projections
+// on the pair GEMM (gemm_wide.cuh), RMSNorm fused into them as in the 65..256-row steps when its scales are folded.  e->x holds the
+// result.
+int enqueue_prefill_pass(mtx_engine* e, int rows, const int32_t* tokens, int start_pos, int slot, cudaStream_t st) {
+  const mtx_model_config& c = e->cfg;
+  const bool gemma3 = c.decoder_block == 1, fused = c.norm_scales_folded != 0;
+  const int planes = staged_prefill(c) ? 1 : c.num_slots;
+  if (staged_prefill(c)) slot = 0;
+  const int E = c.emb_dim, HD = c.num_q_heads * c.head_dim, M = c.mlp_dim, L = c.num_layers, pitch = e->pf_rows;
+  const size_t kv_layer = size_t(planes) * c.num_kv_heads * c.max_target_len * c.head_dim;
+  const bf16 *wqkv = static_cast<const bf16*>(e->w.wqkv), *wo = static_cast<const bf16*>(e->w.wo), *w01 = static_cast<const bf16*>(e->w.w01),
+             *wout = static_cast<const bf16*>(e->w.wout);
+  PrepareArgs pa;
+  memset(&pa, 0, sizeof(pa));
+  pa.chunk_tokens = tokens;
+  pa.start_pos = start_pos;
+  pa.slot = slot;
+  pa.D = c.head_dim;
+  pa.emb_rows = c.embedding_rows;
+  pa.rope_timescale = e->rope_timescale;
+  pa.window = gemma3 ? c.sliding_window : 0;
+  pa.rope_timescale_w = e->rope_timescale_w;
+  g_class = KC_PREPARE;
+  MTX_TRY(launch(prefill_rows_kernel, dim3(rows), dim3(128), 0, st, pa, e->rd));
+  // sums of squares of a row: one from the embedding gather, one per 128 features from post_norm_residual_kernel, one per slice from the
+  // residual epilogues (whose tiles have the same columns for both of their projections: rows and E are)
+  const int tiles128 = (E + 127) / 128, slices = 2 * ((E + wide_tile_columns(rows, E, 32, e->num_sms / 2) - 1) / wide_tile_columns(rows, E, 32, e->num_sms / 2));
+  int ss_x = 1;
+  const int ss_post = gemma3 ? tiles128 : slices;
+  auto norm_in = [&](EpiArgs& ea, const float* ss, int n) {
+    ea.ss_in = fused ? ss : nullptr;
+    ea.ss_tiles = n;
+    ea.ss_pitch = pitch;
+    ea.ss_dim = E;
+    ea.ss_eps = c.rms_eps;
+  };
+  g_class = KC_RMSNORM;
+  const bf16 *attn_norm = static_cast<const bf16*>(e->w.attn_norm), *mlp_norm = static_cast<const bf16*>(e->w.mlp_norm);
+  if (fused)
+    MTX_TRY(launch(embed_gather_ss_kernel, dim3(rows), dim3(128), 0, st, (const int*)e->rd.token, static_cast<const bf16*>(e->w.embedding), e->x,
+                   e->rows_ss_x, 1, pitch, E));
+  else
+    MTX_TRY(launch(rmsnorm_kernel<true>, dim3(rows), dim3(128), 0, st, (const bf16*)nullptr, (const int*)e->rd.token, static_cast<const bf16*>(e->w.embedding),
+                   attn_norm, e->x, e->n, E, c.rms_eps));
+  for (int l = 0; l < L; ++l) {
+    g_class = KC_QKV;
+    const bool local = layer_is_local(e, l);
+    if (gemma3) {
+      WideEpi<EPI_STORE_BF16> qkv;
+      memset(&qkv, 0, sizeof(qkv));
+      qkv.e.out = e->qkv_tmp;
+      qkv.e.ld_out = e->qkv_n;
+      norm_in(qkv.e, e->rows_ss_x, ss_x);
+      MTX_TRY(launch_wide(e->x, wqkv + size_t(l) * e->qkv_n * E, rows, e->qkv_n, E, 32, qkv, e->num_sms, st));
+      QkNormArgs qa;
+      memset(&qa, 0, sizeof(qa));
+      qa.qkv = e->qkv_tmp;
+      qa.q_scale = static_cast<const bf16*>(e->w.q_norm) + size_t(l) * c.head_dim;
+      qa.k_scale = static_cast<const bf16*>(e->w.k_norm) + size_t(l) * c.head_dim;
+      qa.rope_cs = local ? e->rd.rope_cs_w : e->rd.rope_cs;
+      qa.plane = e->rd.plane;
+      qa.write_row = e->rd.write_row;
+      qa.q_out = e->q;
+      qa.k_cache = static_cast<bf16*>(e->s.k_cache) + kv_layer * l;
+      qa.v_cache = static_cast<bf16*>(e->s.v_cache) + kv_layer * l;
+      qa.hq = c.num_q_heads;
+      qa.hkv = c.num_kv_heads;
+      qa.d = c.head_dim;
+      qa.t_alloc = c.max_target_len;
+      qa.eps = c.rms_eps;
+      qa.q_scalar = c.query_scalar;
+      MTX_TRY(launch(qk_norm_rope_append_kernel, dim3(rows, c.num_q_heads + 2 * c.num_kv_heads), dim3(c.head_dim / 2), 0, st, qa));
+    } else {
+      WideEpi<EPI_QKV_ROPE> qkv;
+      memset(&qkv, 0, sizeof(qkv));
+      qkv.e.q_out = e->q;
+      qkv.e.k_cache = static_cast<bf16*>(e->s.k_cache) + kv_layer * l;
+      qkv.e.v_cache = static_cast<bf16*>(e->s.v_cache) + kv_layer * l;
+      qkv.e.plane = e->rd.plane;
+      qkv.e.write_row = e->rd.write_row;
+      qkv.e.rope_cs = e->rd.rope_cs;
+      qkv.e.hq = c.num_q_heads;
+      qkv.e.hkv = c.num_kv_heads;
+      qkv.e.d = c.head_dim;
+      qkv.e.t_alloc = c.max_target_len;
+      norm_in(qkv.e, e->rows_ss_x, ss_x);
+      MTX_TRY(launch_wide(fused ? e->x : e->n, wqkv + size_t(l) * e->qkv_n * E, rows, e->qkv_n, E, c.head_dim, qkv, e->num_sms, st));
+    }
+    g_class = KC_ATTENTION;
+    MTX_TRY(launch_prefill_flash(e, l, rows, start_pos, slot, st));
+    // h = x + [norm](attn . wo),  x = h + [norm](act . wout)
+    auto project = [&](const bf16* a, const bf16* w, int k, const bf16* resid, bf16* out, float* ss, const void* post_scale) -> int {
+      if (gemma3) {
+        WideEpi<EPI_STORE_BF16> st_epi;
+        memset(&st_epi, 0, sizeof(st_epi));
+        st_epi.e.out = e->n;
+        st_epi.e.ld_out = E;
+        MTX_TRY(launch_wide(a, w, rows, E, k, 32, st_epi, e->num_sms, st));
+        g_class = KC_RMSNORM;
+        return launch(post_norm_residual_kernel, dim3(rows), dim3(128), 0, st, (const bf16*)e->n, resid, static_cast<const bf16*>(post_scale) + size_t(l) * E, out, ss,
+                      pitch, E, c.rms_eps);
+      }
+      WideEpi<EPI_RESIDUAL> re;
+      memset(&re, 0, sizeof(re));
+      re.e.out = out;
+      re.e.resid = resid;
+      re.e.ld_out = E;
+      re.e.ss_out = fused ? ss : nullptr;
+      re.e.ss_pitch = pitch;
+      return launch_wide(a, w, rows, E, k, 32, re, e->num_sms, st);
+    };
+    g_class = KC_OUTPROJ;
+    MTX_TRY(project(e->attn, wo + size_t(l) * E * HD, HD, e->x, e->h, e->rows_ss_h, e->w.post_attn_norm));
+    g_class = KC_RMSNORM;
+    if (!fused)
+      MTX_TRY(launch(rmsnorm_kernel<false>, dim3(rows), dim3(128), 0, st, (const bf16*)e->h, (const int*)nullptr, (const bf16*)nullptr, mlp_norm + size_t(l) * E,
+                     (bf16*)nullptr, e->n, E, c.rms_eps));
+    WideEpi<EPI_SWIGLU> up;
+    memset(&up, 0, sizeof(up));
+    up.e.out = e->act;
+    up.e.ld_out = M;
+    up.e.act_gelu = gemma3 ? 1 : 0;
+    norm_in(up.e, e->rows_ss_h, ss_post);
+    g_class = KC_MLP_UP;
+    MTX_TRY(launch_wide(fused ? e->h : e->n, w01 + size_t(l) * 2 * M * E, rows, 2 * M, E, 32, up, e->num_sms, st));
+    g_class = KC_MLP_DOWN;
+    MTX_TRY(project(e->act, wout + size_t(l) * E * M, M, e->h, e->x, e->rows_ss_x, e->w.post_ffw_norm));
+    ss_x = ss_post;
+    g_class = KC_RMSNORM;
+    if (!fused && l + 1 < L)
+      MTX_TRY(launch(rmsnorm_kernel<false>, dim3(rows), dim3(128), 0, st, (const bf16*)e->x, (const int*)nullptr, (const bf16*)nullptr,
+                     attn_norm + size_t(l + 1) * E, (bf16*)nullptr, e->n, E, c.rms_eps));
+  }
+  return MTX_OK;
+}
+
 int enqueue_step(mtx_engine* e, int mode, int rows, const int32_t* chunk_tokens, int start_pos, int slot, int want_logits,
                  int32_t* first_token, float* prefill_logits, cudaStream_t st, float* cand_out = nullptr, float* first_log_prob = nullptr) {
   const mtx_model_config& c = e->cfg;
@@ -760,7 +1026,7 @@ int enqueue_step(mtx_engine* e, int mode, int rows, const int32_t* chunk_tokens,
       MTX_TRY(launch(post_norm_residual_kernel, dim3(rows), dim3(128), 0, st, (const bf16*)e->n, (const bf16*)e->h,
                      static_cast<const bf16*>(e->w.post_ffw_norm) + size_t(l) * E, e->x, e->rows_ss_x, e->max_r_tile, E, c.rms_eps));
     }
-    if (want_logits)
+    if (want_logits && mode == 0)
       MTX_TRY(launch(rmsnorm_kernel<false>, dim3(rows), dim3(128), 0, st, (const bf16*)e->x, (const int*)nullptr, (const bf16*)nullptr,
                      static_cast<const bf16*>(e->w.final_norm), (bf16*)nullptr, e->n, E, c.rms_eps));
   } else if (!mega) {
@@ -891,22 +1157,23 @@ int enqueue_step(mtx_engine* e, int mode, int rows, const int32_t* chunk_tokens,
 
     g_class = KC_RMSNORM;
     const bf16* next_scale = l + 1 < L ? attn_norm + size_t(l + 1) * E : static_cast<const bf16*>(e->w.final_norm);
-    if ((l + 1 < L && !fused_norm) || (l + 1 == L && want_logits))
+    if ((l + 1 < L && !fused_norm) || (l + 1 == L && want_logits && mode == 0))
       MTX_TRY(launch(rmsnorm_kernel<false>, dim3(rows), dim3(128), 0, st, (const bf16*)e->x, (const int*)nullptr,
                      (const bf16*)nullptr, next_scale, (bf16*)nullptr, e->n, E, c.rms_eps));
   }
 
   }
 
+  if (want_logits && mode == 1)
+    return enqueue_last_logits(e, e->x + size_t(rows - 1) * E, rows - 1, first_token, prefill_logits, first_log_prob, st);
   if (want_logits) {
     const bool two_pass = e->strategy == MTX_SAMPLE_NUCLEUS || e->strategy == MTX_SAMPLE_TOPK;
-    if (two_pass && (mode == 0 ? e->s.logits == nullptr : prefill_logits == nullptr))
-      return fail(MTX_ERR_ARG, "nucleus / topk sampling read the materialised logits: decode_state.logits (or logits_out) must be set");
+    if (two_pass && e->s.logits == nullptr) return fail(MTX_ERR_ARG, "%s", kTwoPassNeedsLogits);
     EpiArgs ea;
     memset(&ea, 0, sizeof(ea));
-    ea.logits_out = mode == 0 ? e->s.logits : prefill_logits;
+    ea.logits_out = e->s.logits;
     ea.ld_logits = c.vocab_size;
-    ea.logits_only_row = mode == 0 ? -1 : rows - 1;
+    ea.logits_only_row = -1;
     ea.part_score = e->part_score;
     ea.part_idx = e->part_idx;
     ea.part_raw = e->part_raw;
@@ -919,14 +1186,14 @@ int enqueue_step(mtx_engine* e, int mode, int rows, const int32_t* chunk_tokens,
     ea.inv_temp = 1.0f / e->temperature;
     ea.round_bf16 = c.logits_round_bf16;
     ea.gumbel = e->strategy == MTX_SAMPLE_WEIGHTED ? 1 : 0;
-    float* lp_out = mode == 0 ? e->s.log_prob : first_log_prob;
+    float* lp_out = e->s.log_prob;
     // decode steps with top-k / nucleus run the all-SM sampler, which starts from the per-tile (max, sum exp) partials
-    const bool par_sampler = two_pass && mode == 0 && cand_out == nullptr && env_int("MTX_PAR_SAMPLER", 1) != 0;
+    const bool par_sampler = two_pass && cand_out == nullptr && env_int("MTX_PAR_SAMPLER", 1) != 0;
     // vocab-parallel top-k / nucleus: the shard's 64 candidates come from the same all-SM radix descent (par_collect_kernel)
-    const bool par_collect = two_pass && mode == 0 && cand_out != nullptr && env_int("MTX_PAR_COLLECT", 1) != 0;
+    const bool par_collect = two_pass && cand_out != nullptr && env_int("MTX_PAR_COLLECT", 1) != 0;
     ea.want_lse = (((lp_out != nullptr || cand_out != nullptr) && !two_pass) || par_sampler || par_collect) ? 1 : 0;
     ea.rng_state = e->s.rng_state;
-    ea.row_offset = mode == 0 ? 0 : prefill_noise_row(e);
+    ea.row_offset = 0;
     gp.n = c.vocab_size;
     gp.k = E;
     g_class = KC_LOGITS;
@@ -952,7 +1219,6 @@ int enqueue_step(mtx_engine* e, int mode, int rows, const int32_t* chunk_tokens,
     fa.stride_r = plan_logits.n_tiles;
     fa.stride_t = 1;
     fa.cand_out = cand_out;
-    int finalize_rows = rows;
     auto par_args = [&](ParSampleArgs& ps) {
       memset(&ps, 0, sizeof(ps));
       ps.logits = e->s.logits;
@@ -1052,7 +1318,7 @@ int enqueue_step(mtx_engine* e, int mode, int rows, const int32_t* chunk_tokens,
       // inference_utils.py:87-111 on the logits the GEMM just wrote; one candidate per row
       SampleArgs sa;
       memset(&sa, 0, sizeof(sa));
-      sa.logits = mode == 0 ? e->s.logits : prefill_logits;
+      sa.logits = e->s.logits;
       sa.ld = c.vocab_size;
       sa.vocab = c.vocab_size;
       sa.vocab_offset = c.vocab_offset;
@@ -1061,19 +1327,17 @@ int enqueue_step(mtx_engine* e, int mode, int rows, const int32_t* chunk_tokens,
       sa.nucleus_p = e->nucleus_p;
       sa.inv_temp = 1.0f / e->temperature;
       sa.rng_state = e->s.rng_state;
-      sa.row_offset = mode == 0 ? 0 : prefill_noise_row(e) + rows - 1;
+      sa.row_offset = 0;
       sa.out_score = e->part_score;
       sa.out_idx = e->part_idx;
       sa.out_raw = e->part_raw;
       sa.out_max = e->part_max;
       sa.out_sum = e->part_sum;
-      finalize_rows = mode == 0 ? rows : 1;
-      MTX_TRY(launch(sample_rows_kernel, dim3(finalize_rows), dim3(kSampleThreads), 0, st, sa));
+      MTX_TRY(launch(sample_rows_kernel, dim3(rows), dim3(kSampleThreads), 0, st, sa));
       fa.n_tiles = 1;
       fa.stride_r = 1;
-      fa.rows = finalize_rows;
     }
-    fa.mode = cand_out != nullptr ? 2 : mode;
+    fa.mode = cand_out != nullptr ? 2 : 0;
     fa.have_lse = (two_pass || lp_out != nullptr || cand_out != nullptr) ? 1 : 0;
     fa.tokens = e->s.tokens;
     fa.next_pos = e->s.next_pos;
@@ -1085,8 +1349,7 @@ int enqueue_step(mtx_engine* e, int mode, int rows, const int32_t* chunk_tokens,
     fa.rng_state = e->s.rng_state;
     fa.num_slots = c.num_slots;
     fa.R = c.max_target_len - c.max_prefill_len;
-    fa.first_token = first_token;
-    MTX_TRY(launch(finalize_kernel, dim3(finalize_rows), dim3(kFinalizeThreads), 0, st, fa));
+    MTX_TRY(launch(finalize_kernel, dim3(rows), dim3(kFinalizeThreads), 0, st, fa));
   }
   return MTX_OK;
 }
@@ -1155,6 +1418,10 @@ int mtx_engine_create(const mtx_model_config* cfg, mtx_engine** out) {
   e->max_r_tile = round_rows(c.max_rows);
   if (c.kv_quant && e->max_r_tile < 128) e->max_r_tile = 128;  // every step of an int8 engine runs the 128-row-block GEMM
   if (c.decoder_block == 1 && e->max_r_tile < 128) e->max_r_tile = 128;  // and so does every step of the gemma3 block
+  if (c.max_prefill_len > 256) {
+    const int rows = (c.max_prefill_len + 255) / 256 * 256;
+    e->pf_rows = rows < kPfMaxRows ? rows : kPfMaxRows;
+  }
   e->qkv_n = (c.num_q_heads + 2 * c.num_kv_heads) * c.head_dim;
   e->attn_max_chunks = attn_max_chunks(c.max_prefill_len, c.max_target_len);
   e->rope_timescale_host.resize(c.head_dim / 2);
@@ -1680,6 +1947,35 @@ int mtx_prefill_chunk(mtx_engine* e, const int32_t* tokens, int count, int start
   }
   return enqueue_step(e, 1, count, tokens, start_pos, slot, sample_last, first_token, logits_out, static_cast<cudaStream_t>(stream), nullptr,
                       first_log_prob);
+}
+
+int mtx_prefill_rows(mtx_engine* e, const int32_t* tokens, int count, int start_pos, int slot, int sample_last, int draw_row, int32_t* first_token,
+                     float* logits_out, float* first_log_prob, mtx_stream stream) {
+  if (!e || !e->bound) return fail(MTX_ERR_ARG, "engine is not bound");
+  if (count < 1 || start_pos < 0 || count > e->cfg.max_prefill_len - start_pos) return fail(MTX_ERR_ARG, "prompt positions exceed max_prefill_len");
+  if (slot < 0 || slot >= e->cfg.num_slots) return fail(MTX_ERR_ARG, "slot out of range");
+  if (sample_last && first_token == nullptr) return fail(MTX_ERR_ARG, "first_token is null");
+  if (draw_row < 0 || draw_row >= 256) return fail(MTX_ERR_ARG, "draw_row %d outside [0, 256)", draw_row);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (sample_last) {
+    ++e->prefill_draws;
+    e->last_prefill_rows = draw_row + 1;
+  }
+  const bf16* last = nullptr;
+  for (int at = 0; at < count;) {
+    const int left = count - at, small = e->cfg.max_rows;
+    int n;
+    if (e->pf_rows > 0 && left > 256) {
+      n = left < e->pf_rows ? left : e->pf_rows;
+      MTX_TRY(enqueue_prefill_pass(e, n, tokens + at, start_pos + at, slot, st));
+    } else {
+      n = left < small ? left : small;
+      MTX_TRY(enqueue_step(e, 1, n, tokens + at, start_pos + at, slot, 0, nullptr, nullptr, st));
+    }
+    last = e->x + size_t(n - 1) * e->cfg.emb_dim;
+    at += n;
+  }
+  return sample_last ? enqueue_last_logits(e, last, draw_row, first_token, logits_out, first_log_prob, st) : MTX_OK;
 }
 
 int mtx_insert_prefix(mtx_engine* e, const void* k_src, const void* v_src, int n_rows, int n_src_rows, int slot, int next_pos, int generated,

@@ -245,20 +245,80 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   if (warp == 1) tmem_dealloc_pair(tmem_base, 512);
 }
 
-// ---- epilogues of the decoder engine (the row fragments of gemm_rows.cuh) -------------------------------------------------------
+// ---- epilogues of the decoder engine --------------------------------------------------------------------------------------------
+// What gemm_rows.cuh's fragments compute, with the arithmetic between the accumulator and the stored value in fp32 and one rounding
+// at the end (those round every intermediate array to bf16; against float64 this side is the closer one).
+
+// the row's 1 / rms from the partial sums of squares that a residual epilogue left
+__device__ __forceinline__ float wide_rstd(const EpiArgs& e, int row) {
+  float tot = 0.0f;
+#pragma unroll 8
+  for (int t = 0; t < e.ss_tiles; ++t) tot += __ldcg(e.ss_in + (long long)t * e.ss_pitch + row);
+  return 1.0f / sqrtf(tot / float(e.ss_dim) + e.ss_eps);
+}
+
+// out = bf16(resid + acc); returns the sum of squares of the stored values
+__device__ __forceinline__ float wide_residual(const EpiArgs& e, int r, int n0, const float (&v)[16]) {
+  const long long o = (long long)r * e.ld_out + n0;
+  const uint4 ra = *reinterpret_cast<const uint4*>(e.resid + o), rb = *reinterpret_cast<const uint4*>(e.resid + o + 8);
+  const uint32_t w[8] = {ra.x, ra.y, ra.z, ra.w, rb.x, rb.y, rb.z, rb.w};
+  uint32_t s[8];
+  float sq = 0.0f;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    s[j] = pack_bf16x2(bf16_lo(w[j]) + v[2 * j], bf16_hi(w[j]) + v[2 * j + 1]);
+    sq += bf16_lo(s[j]) * bf16_lo(s[j]) + bf16_hi(s[j]) * bf16_hi(s[j]);
+  }
+  *reinterpret_cast<uint4*>(e.out + o) = make_uint4(s[0], s[1], s[2], s[3]);
+  *reinterpret_cast<uint4*>(e.out + o + 8) = make_uint4(s[4], s[5], s[6], s[7]);
+  return sq;
+}
+
+// 16 gates and the 16 values that belong to them
+__device__ __forceinline__ void wide_gate(const EpiArgs& e, int r, int n0, const float (&g)[16], const float (&u)[16]) {
+  float o[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    const float a = g[j];
+    const float act = e.act_gelu ? a * 0.5f * (1.0f + tanhf(0.7978845608028654f * (a + 0.044715f * a * a * a))) : __fdividef(a, 1.0f + __expf(-a));
+    o[j] = act * u[j];
+  }
+  frag_store_bf16(e.out + (long long)r * e.ld_out + (n0 >> 1), o);
+}
+
+// dims d0 .. d0 + 15 of a head's first half and the same of its second half (d0 + D / 2): rotated queries, appended keys and values
+__device__ __forceinline__ void wide_qkv(const EpiArgs& e, int r, int head, int d0, float (&a)[16], float (&b)[16]) {
+  const int D = e.d, half = D >> 1;
+  if (head < e.hq + e.hkv) {
+    const float4* cs = reinterpret_cast<const float4*>(e.rope_cs + (long long)r * half + d0);
+#pragma unroll
+    for (int j = 0; j < 16; j += 2) {
+      const float4 c = cs[j >> 1];
+      const float a0 = a[j], b0 = b[j], a1 = a[j + 1], b1 = b[j + 1];
+      a[j] = a0 * c.x - b0 * c.y;
+      b[j] = b0 * c.x + a0 * c.y;
+      a[j + 1] = a1 * c.z - b1 * c.w;
+      b[j + 1] = b1 * c.z + a1 * c.w;
+    }
+  }
+  bf16* dst;
+  if (head < e.hq) {
+    dst = e.q_out + (long long)r * (e.hq * D) + head * D + d0;
+  } else {
+    const int wr = e.write_row[r];
+    if (wr < 0) return;
+    const int kvh = (head - e.hq) % e.hkv;
+    dst = (head < e.hq + e.hkv ? e.k_cache : e.v_cache) + (((long long)e.plane[r] * e.hkv + kvh) * e.t_alloc + wr) * D + d0;
+  }
+  frag_store_bf16(dst, a);
+  frag_store_bf16(dst + half, b);
+}
 
 template <int KIND>
 struct WideEpi {
   EpiArgs e;
 
-  // the row's 1 / rms from the partial sums of squares that a residual epilogue left, eight loads at a time
-  __device__ __forceinline__ float prepare(const WideTile& w) const {
-    if (KIND == EPI_RESIDUAL || e.ss_in == nullptr || !w.valid) return 1.0f;
-    float tot = 0.0f;
-#pragma unroll 8
-    for (int t = 0; t < e.ss_tiles; ++t) tot += __ldcg(e.ss_in + (long long)t * e.ss_pitch + w.row);
-    return 1.0f / sqrtf(tot / float(e.ss_dim) + e.ss_eps);
-  }
+  __device__ __forceinline__ float prepare(const WideTile& w) const { return KIND == EPI_RESIDUAL || e.ss_in == nullptr || !w.valid ? 1.0f : wide_rstd(e, w.row); }
 
   template <class LD>
   __device__ __forceinline__ void operator()(const WideTile& w, int n, float rs, LD&& ld16) const {
@@ -274,9 +334,9 @@ struct WideEpi {
       for (int c = w.c0; c < w.c1; c += 16) {
         float v[16];
         ld16(c, v);
-        if (w.valid) sq += rows_epi_residual(e, n, w.row, w.n0 + c, v);
+        if (w.valid) sq += wide_residual(e, w.row, w.n0 + c, v);
       }
-      if (e.ss_out != nullptr && w.valid && w.n0 + w.c0 < n) e.ss_out[(long long)w.slice * e.ss_pitch + w.row] = sq;
+      if (e.ss_out != nullptr && w.valid) e.ss_out[(long long)w.slice * e.ss_pitch + w.row] = sq;
     } else if (KIND == EPI_SWIGLU) {
       for (int c = w.c0; c < w.c1; c += 32) {
         float g[16], u[16];
@@ -284,7 +344,7 @@ struct WideEpi {
         ld16(c + 16, u);
         rows_scale16(g, rs);
         rows_scale16(u, rs);
-        if (w.valid) rows_epi_swiglu(e, n, w.row, w.n0 + c, g, u);
+        if (w.valid) wide_gate(e, w.row, w.n0 + c, g, u);
       }
     } else if (KIND == EPI_QKV_ROPE) {
       const int half = e.d >> 1;
@@ -295,7 +355,7 @@ struct WideEpi {
           ld16(h + d + half, hi);
           rows_scale16(lo, rs);
           rows_scale16(hi, rs);
-          if (w.valid) rows_epi_qkv(e, n, w.row, (w.n0 + h) / e.d, d, lo, hi);
+          if (w.valid) wide_qkv(e, w.row, (w.n0 + h) / e.d, d, lo, hi);
         }
     }
   }

@@ -229,6 +229,29 @@ __global__ void prepare_rows_kernel(const PrepareArgs a, const RowDesc rd) {
   timeline_end(tl);
 }
 
+// The same descriptors for the rows of a long prompt (positions start_pos + r of one sequence; no attention work list): one CTA per row.
+__global__ void __launch_bounds__(128) prefill_rows_kernel(const PrepareArgs a, const RowDesc rd) {
+  griddep_launch_dependents();
+  griddep_wait();
+  const int r = blockIdx.x, pos = a.start_pos + r, half = a.D / 2;
+  if (threadIdx.x == 0) {
+    int token = a.chunk_tokens[r];
+    if (a.emb_rows > 0) token = token < 0 ? 0 : (token >= a.emb_rows ? a.emb_rows - 1 : token);
+    rd.token[r] = token;
+    rd.pos[r] = pos;
+    rd.plane[r] = a.slot;
+    rd.write_row[r] = pos;
+  }
+  for (int i = threadIdx.x; i < half; i += blockDim.x) {
+    const float ang = float(pos) / a.rope_timescale[i];
+    rd.rope_cs[(long long)r * half + i] = make_float2(bf16r(cosf(ang)), bf16r(sinf(ang)));
+    if (a.window > 0) {
+      const float angw = float(pos) / a.rope_timescale_w[i];
+      rd.rope_cs_w[(long long)r * half + i] = make_float2(bf16r(cosf(angw)), bf16r(sinf(angw)));
+    }
+  }
+}
+
 // RMSNorm (normalizations.py:57-69), optionally fused with the embedding gather
 // (embeddings.py:154: embedding.astype(bf16)[tokens]).  One CTA per row.
 //   y   = bf16(x32 * rsqrt(mean(x32^2) + eps));  out = bf16(y * bf16(scale))

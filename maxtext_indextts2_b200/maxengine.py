@@ -7,7 +7,7 @@ method                 reference                                    here
 =====================  ==========================================  =====================
 ``load_params``        maxengine.py:218                             repack for K-major streaming, upload
 ``init_decode_state``  maxengine.py:1370-1453                       zero the device state
-``prefill``            maxengine.py:533-574 (``_prefill_jit`` :400)  ``mtx_prefill_chunk``
+``prefill``            maxengine.py:533-574 (``_prefill_jit`` :400)  ``mtx_prefill_rows``
 ``insert``             maxengine.py:1166-1192 (``_insert_jit`` :1045)  device copies
 ``bulk_insert``        maxengine.py:946                              loop over ``insert``
 ``generate``           maxengine.py:838-866 (``_generate_jit`` :868)  ``mtx_decode_step[_graph]``
@@ -661,23 +661,21 @@ class MaxEngine:
       self._k[:, self._staging, :, :start_position].copy_(pk[:, :, :start_position])
       self._v[:, self._staging, :, :start_position].copy_(pv[:, :, :start_position])
     want_logits = self._logits is not None or self._vp_world > 1
-    for start in range(0, true_length, self._chunk):
-      count = min(self._chunk, true_length - start)
-      last = start + count == true_length
-      _lib.check(
-          self.lib.mtx_prefill_chunk(
-              self._handle,
-              ctypes.c_void_p(self._prefill_tokens.data_ptr() + 4 * start),
-              count,
-              start_position + start,
-              self._staging,
-              1 if last else 0,
-              ctypes.c_void_p(self._first_token.data_ptr()),
-              ctypes.c_void_p(self._prefill_logits.data_ptr()) if (want_logits and last) else None,
-              ctypes.c_void_p(self._first_log_prob.data_ptr()) if (self._first_log_prob is not None and last) else None,
-              self._stream(),
-          )
-      )
+    _lib.check(
+        self.lib.mtx_prefill_rows(
+            self._handle,
+            ctypes.c_void_p(self._prefill_tokens.data_ptr()),
+            true_length,
+            start_position,
+            self._staging,
+            1,
+            (true_length - 1) % self._chunk,  # (the draw's noise row: the last position's place in its chunk)
+            ctypes.c_void_p(self._first_token.data_ptr()),
+            ctypes.c_void_p(self._prefill_logits.data_ptr()) if want_logits else None,
+            ctypes.c_void_p(self._first_log_prob.data_ptr()) if self._first_log_prob is not None else None,
+            self._stream(),
+        )
+    )
     if self._vp_world > 1:
       # first token (not on the decode hot path): the shards' logits of the last prompt position are gathered into the full
       # row and sampled with the configured strategy by the same kernel on every rank

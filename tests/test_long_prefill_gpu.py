@@ -1,0 +1,51 @@
+"""Prompts of more than 256 tokens: one pass over all rows (csrc/gemm_wide.cuh, csrc/prefill_flash.cuh) against the same prompt in portions of
+at most 200 tokens, which run the 256-row kernels.  Lengths at the edges of the 128- and 256-row tiles, every head size, sliding windows
+that start and end inside a tile, unfolded norm scales, a paged and an 8-bit engine (their prompts go through a staging plane)."""
+
+import pytest
+import torch
+
+from maxtext_indextts2_b200 import maxengine, pyconfig
+
+pytestmark = pytest.mark.gpu
+
+
+def _config(block, dim, **kw):
+  base = dict(base_num_decoder_layers=2, base_emb_dim=192, base_num_query_heads=6, base_num_kv_heads=2, head_dim=dim, base_mlp_dim=320, vocab_size=512,
+              per_device_batch_size=2, max_prefill_predict_length=832, max_target_length=900, weight_dtype="bfloat16", scan_layers=False,
+              attention="dot_product", materialize_logits=True, use_chunked_prefill=True)
+  if block == "gemma3":
+    base.update(model_name="gemma3-4b", sliding_window_size=150)
+  base.update(kw)
+  return pyconfig.initialize(None, **base)
+
+
+CASES = [("llama2", 64, {}), ("llama2", 128, {}), ("llama2", 64, dict(fold_norm_scales=False)), ("llama2", 64, dict(attn_logits_soft_cap=5.0)),
+         ("llama2", 64, dict(quantize_kvcache=True, kv_quant_axis="dkv")),
+         ("llama2", 64, dict(attention="paged", pagedattn_num_pages=120, pagedattn_tokens_per_page=16)),
+         ("gemma3", 64, {}), ("gemma3", 128, {}), ("gemma3", 256, {}), ("gemma3", 256, dict(sliding_window_size=64))]
+
+
+@pytest.mark.parametrize("block,dim,kw", CASES)
+def test_one_pass_against_portions(block, dim, kw):
+  cfg = _config(block, dim, **kw)
+  engine = maxengine.MaxEngine(cfg)
+  params = engine.load_params(on_device_init=True, norm_jitter=0.1)
+  engine.init_decode_state()
+  for n in (257, 384, 513, 831):
+    toks = torch.randint(0, cfg.vocab_size, (n,), generator=torch.Generator().manual_seed(n))
+    whole, _ = engine.prefill(params=params, padded_tokens=toks, true_length=n, slot=0)
+    prefix, done = None, 0
+    while done < n:
+      m = min(200, n - done)
+      before = maxengine.ExistingPrefix(cache=prefix["cache"], common_prefix_tokens=toks[:done]) if done else None
+      prefix, _ = engine.prefill(params=params, padded_tokens=toks[done : done + m], true_length=m, existing_prefix=before, slot=0)
+      done += m
+    for name in ("key", "value"):
+      got, want = whole["cache"][name].double(), prefix["cache"][name].double()  # [L, heads, n, D]
+      assert got.shape == want.shape
+      # bf16 activations through at most two layers: 2^-9 for each of about ten roundings
+      err = ((got - want).square().mean((0, 1, 3)) / want.square().mean()).sqrt()
+      assert float(err.max()) < 4e-2, (n, name, int(err.argmax()))
+    a, b = whole["logits"].double(), prefix["logits"].double()
+    assert float((a - b).norm() / b.norm()) < 4e-2, n
