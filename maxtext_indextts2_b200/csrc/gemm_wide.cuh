@@ -6,8 +6,8 @@
 // launches, pipeline fills and drains per projection: 20 % of the bf16 rate.  Here two CTAs of a cluster (a TPC's two SMs) work on one
 // tile of 256 rows x BN columns with cta_group::2 MMAs (M = 256): CTA c of the pair holds rows 128 c .. of A and half of the
 // weight tile's rows, so that an SM takes in 16 KB + BN * 64 B per k block of 64 for BN * 2^15 multiply-adds.  One pair per TPC walks the
-// tiles (rows fastest, so that the pairs at work share weight tiles in L2), the accumulators are double-buffered (2 x 256 TMEM
-// columns): the eight epilogue warps of each CTA drain a tile under the next tile's MMAs.
+// tiles (rows fastest, so that the pairs at work share weight tiles in L2), the 512 TMEM columns hold as many accumulators as fit (two of
+// 256 columns, four of 128): the eight epilogue warps of each CTA drain a tile under the next tiles' MMAs.
 //
 // BN is chosen per shape (wide_tile_columns) so that the tiles fill whole waves of pairs.
 //
@@ -21,6 +21,14 @@
 //
 // The epilogue is a class with  prepare(tile)  (what a thread needs of its row, read while the tile's MMAs run) and
 // operator()(tile, n, prepared, load)  where load(c, v) reads the accumulator's 16 columns c .. c + 15.
+//
+// Segments: gemm_rows.cuh cuts the k blocks of a narrow projection over a cluster and adds the parts in order.  With `segments` set to that
+// number a tile's k range is accumulated in the same parts, which the epilogue threads add in registers, so that a row's result is bit
+// for bit what the 256-row steps give it, however many rows its step has.  Such an epilogue works on one fragment of 16 columns at a
+// time (kFragments; fragment(tile, n, column, values)).
+// Grouped (GROUPED; the experts of a routed feed-forward): the rows are slots, group g's are [group_off[g], group_off[g + 1]) (known on the
+// device only) and its weight the rows g * n .. of W.  The pairs walk the groups' row tiles one group after the other; a group's last tile
+// reads the next group's rows and drops their results.
 #pragma once
 
 #include "gemm_rows.cuh"
@@ -31,20 +39,24 @@ constexpr int kPairThreads = 320;
 constexpr int kPairRows = 256;    // rows of a pair's tile
 constexpr int kPairMaxCols = 256;
 constexpr int kPairMaxStages = 12;
+constexpr int kPairMaxAcc = 8;    // accumulators in TMEM (tiles of 64 columns)
 constexpr int kPairABytes = 128 * kBlockK * 2;  // a CTA's part of an A stage
 
 struct WideParams {
   int rows, n, k;
   int bn;      // columns of a tile: a multiple of 32, at most 256
   int stages;  // depth of the ring
+  int segments;  // parts that a tile's k blocks are accumulated in (1, or an epilogue with kFragments)
+  const int* group_off;  // GROUPED: [groups + 1]
+  int groups;
   int first;   // columns of a tile's first half (the epilogue warps 2-5; the warps 6-9 take the rest)
 };
 
 struct WideSmemTail {
   uint64_t full[kPairMaxStages];
   uint64_t empty[kPairMaxStages];
-  uint64_t tmem_full[2];
-  uint64_t tmem_empty[2];
+  uint64_t tmem_full[kPairMaxAcc];
+  uint64_t tmem_empty[kPairMaxAcc];
   uint32_t tmem_base;
   uint32_t pad;
 };
@@ -106,7 +118,7 @@ __device__ __forceinline__ void mbar_arrive_leader(uint64_t* bar) {
 
 // ---- the kernel ----------------------------------------------------------------------------------------------------------------
 
-template <class EPI>
+template <class EPI, bool GROUPED>
 __global__ void __launch_bounds__(kPairThreads, 1)
 gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_a, const WideParams p, const EPI epi) {
   extern __shared__ uint8_t smem_raw[];
@@ -115,10 +127,8 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   WideSmemTail* tail = reinterpret_cast<WideSmemTail*>(smem + size_t(p.stages) * stage_bytes);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = int(blockIdx.x) & 1, pair = int(blockIdx.x) >> 1, pairs = int(gridDim.x) >> 1;  // (the cluster is two CTAs along x)
-  const int m_tiles = (p.rows + kPairRows - 1) / kPairRows, n_tiles = (p.n + p.bn - 1) / p.bn, tiles = m_tiles * n_tiles;
   const int nkb = p.k / kBlockK;
-  const int my_tiles = pair < tiles ? (tiles - pair + pairs - 1) / pairs : 0;
-  const int F = my_tiles * nkb;
+  const int n_acc = 512 / p.bn;
 
   griddep_launch_dependents();
   if (warp == 0 && lane == 0) {
@@ -128,7 +138,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       mbar_init(&tail->full[s], 1);
       mbar_init(&tail->empty[s], 1);
     }
-    for (int b = 0; b < 2; ++b) {
+    for (int b = 0; b < n_acc; ++b) {
       mbar_init(&tail->tmem_full[b], 1);
       mbar_init(&tail->tmem_empty[b], 16);  // the eight epilogue warps of both CTAs
     }
@@ -143,33 +153,67 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   tcgen05_fence_after();
   const uint32_t tmem_base = tail->tmem_base;
 
+  int m_tiles = (p.rows + kPairRows - 1) / kPairRows;
+  if (GROUPED) {
+    griddep_wait();  // the slot ranges come from the kernel before
+    m_tiles = 0;
+    for (int g = 0; g < p.groups; ++g) m_tiles += (p.group_off[g + 1] - p.group_off[g] + kPairRows - 1) / kPairRows;
+  }
+  const int n_tiles = (p.n + p.bn - 1) / p.bn, tiles = m_tiles * n_tiles;
+  const int my_tiles = pair < tiles ? (tiles - pair + pairs - 1) / pairs : 0;
+  const int F = my_tiles * nkb;
+  // row tile m: its first row, how many rows follow from there, the row of W where its weight begins
+  struct Rows {
+    int row0, left, w0;
+  };
+  auto rows_of = [&](int m) {
+    Rows r = {m * kPairRows, p.rows - m * kPairRows, 0};
+    if (GROUPED) {
+      int off = p.group_off[0];
+      for (int g = 0; g < p.groups; ++g) {
+        const int end = p.group_off[g + 1], nt = (end - off + kPairRows - 1) / kPairRows;
+        if (m < nt) {
+          r.row0 = off + m * kPairRows;
+          r.left = end - r.row0;
+          r.w0 = g * p.n;
+          break;
+        }
+        m -= nt;
+        off = end;
+      }
+    }
+    return r;
+  };
+
   if (warp == 0) {
     // (the whole warp counts and waits, one elected lane issues: a branch on the lane number makes the compiler guard every issue against
     // divergence.  Stage, phase, k block and tile are counted, not divided out of a fill number.)
     const bool issuer = elect_one();
-    int s = 0, kb = 0, m = pair % m_tiles, nt = pair / m_tiles;
+    const int m_div = m_tiles > 0 ? m_tiles : 1;  // (no slots at all: no tiles)
+    int s = 0, kb = 0, m = pair % m_div, nt = pair / m_div;
     uint32_t phase = 1;
-    const int m_step = pairs % m_tiles, n_step = pairs / m_tiles;
-    auto w_load = [&](int stage, int k, int n) {
+    const int m_step = pairs % m_div, n_step = pairs / m_div;
+    Rows at = rows_of(m_tiles > 0 ? m : 0);
+    auto w_load = [&](int stage, int k) {
       if (rank == 0) mbar_expect_tx(&tail->full[stage], uint32_t(2 * stage_bytes));
-      tma_load_2d_pair(smem + stage * stage_bytes + kPairABytes, &tm_w, k * kBlockK, n * p.bn + rank * half_n, &tail->full[stage], kEvictLast);
+      tma_load_2d_pair(smem + stage * stage_bytes + kPairABytes, &tm_w, k * kBlockK, at.w0 + nt * p.bn + rank * half_n, &tail->full[stage], kEvictLast);
     };
-    auto a_load = [&](int stage, int k, int mt) {
-      tma_load_2d_pair(smem + stage * stage_bytes, &tm_a, k * kBlockK, mt * kPairRows + rank * 128, &tail->full[stage], kEvictLast);
+    auto a_load = [&](int stage, int k) {
+      tma_load_2d_pair(smem + stage * stage_bytes, &tm_a, k * kBlockK, at.row0 + rank * 128, &tail->full[stage], kEvictLast);
     };
     // the first tile's weights do not depend on the previous kernel
     const int pre = my_tiles == 0 ? 0 : (nkb < p.stages ? nkb : p.stages);
     if (issuer)
-      for (int f = 0; f < pre; ++f) w_load(f, f, nt);
-    griddep_wait();
+      for (int f = 0; f < pre; ++f) w_load(f, f);
+    if (!GROUPED) griddep_wait();
     if (issuer)
-      for (int f = 0; f < pre; ++f) a_load(f, f, m);
+      for (int f = 0; f < pre; ++f) a_load(f, f);
     for (int f = 0; f < F; ++f) {
       if (f >= pre) {
         mbar_wait(&tail->empty[s], phase);
         if (issuer) {
-          w_load(s, kb, nt);
-          a_load(s, kb, m);
+          w_load(s, kb);
+          a_load(s, kb);
         }
       }
       if (++s == p.stages) s = 0, phase ^= 1;
@@ -178,6 +222,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         nt += n_step;
         m += m_step;
         if (m >= m_tiles) m -= m_tiles, ++nt;
+        if (f + 1 < F) at = rows_of(m);
       }
     }
     // the commits of the last stages arrive on this CTA's barriers too: they have to be there before it may leave
@@ -194,14 +239,15 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       const uint32_t idesc = umma_idesc_bf16(kPairRows, p.bn);
       const uint64_t d0 = umma_desc_sw128(smem);
       const uint32_t step = uint32_t(stage_bytes) >> 4;  // descriptors count in 16-byte units
-      int s = 0;
-      uint32_t phase = 0;
-      for (int j = 0; j < my_tiles; ++j) {
-        const int buf = j & 1;
-        if (j >= 2) mbar_wait(&tail->tmem_empty[buf], ((j >> 1) & 1) ^ 1);
+      int s = 0, buf = 0;
+      uint32_t phase = 0, acc_phase = 1;
+      for (int j = 0, seg = 0; j < my_tiles * p.segments; ++j) {  // (tile, segment)
+        mbar_wait(&tail->tmem_empty[buf], acc_phase);
         tcgen05_fence_after();
-        const uint32_t acc = tmem_base + uint32_t(buf * kPairMaxCols);
-        for (int i = 0; i < nkb; ++i) {
+        const uint32_t acc = tmem_base + uint32_t(buf * p.bn);
+        const int n_seg = (seg + 1) * nkb / p.segments - seg * nkb / p.segments;
+        if (++seg == p.segments) seg = 0;
+        for (int i = 0; i < n_seg; ++i) {
           mbar_wait(&tail->full[s], phase);
           tcgen05_fence_after();
           if (issuer) {
@@ -213,30 +259,68 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
           if (++s == p.stages) s = 0, phase ^= 1;
         }
         if (issuer) umma_commit_pair(&tail->tmem_full[buf]);
+        if (++buf == n_acc) buf = 0, acc_phase ^= 1;
       }
     }
     __syncwarp();
   } else {
     const int half = (warp - 2) >> 2, quarter = warp & 3;
     const int c0 = half == 0 ? 0 : p.first, c1 = half == 0 ? p.first : p.bn;
-    griddep_wait();  // side inputs (residual rows, row statistics) come from earlier kernels
+    if (!GROUPED) griddep_wait();  // side inputs (residual rows, row statistics) come from earlier kernels
+    int buf = 0;
+    uint32_t acc_phase = 0;
+    auto release = [&]() {  // this warp is done with the accumulator
+      tcgen05_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_leader(&tail->tmem_empty[buf]);
+      if (++buf == n_acc) buf = 0, acc_phase ^= 1;
+    };
     for (int j = 0; j < my_tiles; ++j) {
-      const int t = pair + j * pairs, buf = j & 1;
+      const int t = pair + j * pairs;
       WideTile w;
-      w.row = (t % m_tiles) * kPairRows + rank * 128 + quarter * 32 + lane;
-      w.valid = w.row < p.rows;
+      const Rows at = rows_of(t % m_tiles);
+      const int local = rank * 128 + quarter * 32 + lane;
+      w.row = at.row0 + local;
+      w.valid = local < at.left;
       w.n0 = (t / m_tiles) * p.bn;
       w.c0 = c0;
       w.c1 = w.n0 + c1 < p.n ? c1 : (w.n0 + c0 < p.n ? p.n - w.n0 : c0);
       w.slice = 2 * (t / m_tiles) + half;
-      const uint32_t taddr = tmem_base + (uint32_t(quarter * 32) << 16) + uint32_t(buf * kPairMaxCols);
+      const uint32_t lanes = tmem_base + (uint32_t(quarter * 32) << 16);
+      if constexpr (EPI::kFragments) {
+        if (p.segments > 1) {
+          float acc[kPairMaxCols / 32][16];
+          for (int seg = 0; seg < p.segments; ++seg) {
+            const uint32_t taddr = lanes + uint32_t(buf * p.bn + w.c0);
+            mbar_wait(&tail->tmem_full[buf], acc_phase);
+            tcgen05_fence_after();
+#pragma unroll
+            for (int i = 0; i < kPairMaxCols / 32; i += 2)  // (32 columns in flight: what the registers beside the sums hold)
+              if (w.c0 + 16 * i < w.c1) {
+                uint32_t v[2][16];
+                tmem_ld_x16_issue(taddr + uint32_t(16 * i), v[0]);
+                tmem_ld_x16_issue(taddr + uint32_t(16 * i + 16), v[1]);
+                tmem_ld_wait();
+#pragma unroll
+                for (int x = 0; x < 32; ++x) {
+                  const float y = __uint_as_float(v[x >> 4][x & 15]);
+                  acc[i + (x >> 4)][x & 15] = seg == 0 ? y : acc[i + (x >> 4)][x & 15] + y;
+                }
+              }
+            release();
+          }
+#pragma unroll
+          for (int i = 0; i < kPairMaxCols / 32; ++i)
+            if (w.c0 + 16 * i < w.c1 && w.valid) epi.fragment(w, p.n, w.c0 + 16 * i, acc[i]);
+          continue;
+        }
+      }
+      const uint32_t taddr = lanes + uint32_t(buf * p.bn);
       const auto pre = epi.prepare(w);
-      mbar_wait(&tail->tmem_full[buf], (j >> 1) & 1);
+      mbar_wait(&tail->tmem_full[buf], acc_phase);
       tcgen05_fence_after();
       epi(w, p.n, pre, [&](int c, float (&v)[16]) { tmem_ld_x16(taddr + uint32_t(c), v); });
-      tcgen05_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_leader(&tail->tmem_empty[buf]);
+      release();
     }
   }
   tcgen05_fence_before();
@@ -316,7 +400,10 @@ __device__ __forceinline__ void wide_qkv(const EpiArgs& e, int r, int head, int 
 
 template <int KIND>
 struct WideEpi {
+  static constexpr bool kFragments = KIND == EPI_STORE_BF16;
   EpiArgs e;
+
+  __device__ __forceinline__ void fragment(const WideTile& w, int n, int c, const float (&v)[16]) const { rows_epi_store(e, n, w.row, w.n0 + c, v); }
 
   __device__ __forceinline__ float prepare(const WideTile& w) const { return KIND == EPI_RESIDUAL || e.ss_in == nullptr || !w.valid ? 1.0f : wide_rstd(e, w.row); }
 

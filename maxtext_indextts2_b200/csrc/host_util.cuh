@@ -334,26 +334,57 @@ int wide_tile_columns(int rows, int n, int unit, int pairs) {
 
 // epi(x[rows, k] . w[n, k]^T), n a multiple of 32 (and of unit), k of 64, 16-byte aligned operands
 template <class EPI>
-int launch_wide(const void* x, const void* w, int rows, int n, int k, int unit, const EPI& epi, int num_sms, cudaStream_t st) {
+int launch_wide(const void* x, const void* w, int rows, int n, int k, int unit, const EPI& epi, int num_sms, cudaStream_t st, int segments = 1) {
   static bool attr_set = false;  // per template instance
   if (!attr_set) {
-    MTX_CUDA(cudaFuncSetAttribute(gemm_wide_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    MTX_CUDA(cudaFuncSetAttribute(gemm_wide_kernel<EPI, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     attr_set = true;
   }
   const int pairs = num_sms / 2;
   WideParams p;
+  memset(&p, 0, sizeof(p));
   p.rows = rows;
   p.n = n;
   p.k = k;
   p.bn = wide_tile_columns(rows, n, unit, pairs);
   p.stages = wide_stages(p.bn);
+  p.segments = segments;
   p.first = (p.bn / unit + 1) / 2 * unit;
   CUtensorMap tw, tx;
   MTX_TRY(make_map(&tw, w, k, n, uint32_t(p.bn / 2)));
   MTX_TRY(make_map(&tx, x, k, rows, 128));
   const int tiles = ((rows + kPairRows - 1) / kPairRows) * ((n + p.bn - 1) / p.bn);
   g_cluster_x = 2;
-  const int rc = launch(gemm_wide_kernel<EPI>, dim3(2 * (tiles < pairs ? tiles : pairs)), dim3(kPairThreads), wide_smem_bytes(p.bn, p.stages), st, tw, tx, p, epi);
+  const int rc = launch(gemm_wide_kernel<EPI, false>, dim3(2 * (tiles < pairs ? tiles : pairs)), dim3(kPairThreads), wide_smem_bytes(p.bn, p.stages), st, tw, tx, p, epi);
+  g_cluster_x = 1;
+  return rc;
+}
+
+// the grouped form: at most `slots` rows of x in all, w [groups, n, k]
+template <class EPI>
+int launch_wide_grouped(const void* x, const void* w, const int* group_off, int groups, int slots, int n, int k, const EPI& epi, int num_sms, cudaStream_t st) {
+  static bool attr_set = false;  // per template instance
+  if (!attr_set) {
+    MTX_CUDA(cudaFuncSetAttribute(gemm_wide_kernel<EPI, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    attr_set = true;
+  }
+  const int pairs = num_sms / 2;
+  WideParams p;
+  memset(&p, 0, sizeof(p));
+  p.rows = slots;
+  p.n = n;
+  p.k = k;
+  p.bn = wide_tile_columns(slots + groups * (kPairRows / 2), n, 32, pairs);  // (a group's last tile is half empty on average)
+  p.stages = wide_stages(p.bn);
+  p.segments = 1;
+  p.group_off = group_off;
+  p.groups = groups;
+  p.first = (p.bn / 32 + 1) / 2 * 32;
+  CUtensorMap tw, tx;
+  MTX_TRY(make_map(&tw, w, k, uint64_t(groups) * n, uint32_t(p.bn / 2)));
+  MTX_TRY(make_map(&tx, x, k, slots, 128));
+  g_cluster_x = 2;
+  const int rc = launch(gemm_wide_kernel<EPI, true>, dim3(2 * pairs), dim3(kPairThreads), wide_smem_bytes(p.bn, p.stages), st, tw, tx, p, epi);
   g_cluster_x = 1;
   return rc;
 }

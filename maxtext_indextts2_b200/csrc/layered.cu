@@ -237,6 +237,8 @@ __global__ void act_bf16_kernel(const bf16* src, bf16* act, int n, long long ldo
 // steps of more than 256 rows run the pair GEMM, all rows in one launch (gemm_rows.cuh needs a launch per 256 rows: 257 rows of a
 // 1792 x 1280 projection take 12 us against 21)
 bool takes_wide(int rows) { return rows > 256; }
+// ... and accumulate as a full 256-row step does, so that a prompt's results do not change with the step's length
+int wide_segments(int n, int k) { return plan_rows(n, k, 256, 148, EPI_STORE_BF16).splits; }
 
 // the same product on a tcgen05 GEMM: the bf16 result stays in e->obf
 int run_umma_raw(mtx_layered* e, const void* a, const void* w, int rows, int n, int k, cudaStream_t st) {
@@ -247,7 +249,7 @@ int run_umma_raw(mtx_layered* e, const void* a, const void* w, int rows, int n, 
   if (!takes_wide(rows)) return single_gemm<EPI_STORE_BF16>(a, w, rows, n, k, ea, st);
   WideEpi<EPI_STORE_BF16> epi;
   epi.e = ea;
-  return launch_wide(a, w, rows, n, k, 32, epi, e->num_sms, st);
+  return launch_wide(a, w, rows, n, k, 32, epi, e->num_sms, st, wide_segments(n, k));
 }
 
 // ... then the epilogue as a row kernel
@@ -266,7 +268,7 @@ int run_linear_umma(mtx_layered* e, const void* a, const void* w, const float* b
     epi.silu1 = silu1;
     const void* dst = narrow ? act : static_cast<const void*>(out);
     if (epi.ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0 && (reinterpret_cast<uintptr_t>(bias) & 15) == 0)
-      return launch_wide(a, w, rows, n, k, 32, epi, e->num_sms, st);
+      return launch_wide(a, w, rows, n, k, 32, epi, e->num_sms, st, wide_segments(n, k));
   }
   MTX_TRY(run_umma_raw(e, a, w, rows, n, k, st));
   const bf16* tmp = static_cast<const bf16*>(e->obf);
@@ -893,6 +895,27 @@ int run_softmax_attention(mtx_layered* e, SoftmaxAttnArgs<T>& sa, const mtx_ragg
   return MTX_OK;
 }
 
+// do a routed feed-forward's products over that many (row, choice) slots take the pair GEMM?  (its tiles have 256 rows: at least half a tile
+// per expert)
+bool takes_wide_grouped(int slots, int groups, int n, int k) { return slots >= 128 * groups && n % 32 == 0 && k % 64 == 0; }
+
+// the expert that every token uses: into e->y, or e->obf
+template <typename T>
+int shared_expert(mtx_layered* e, const mtx_moe_desc& m, const T* xa, int rows, float shared_limit, cudaStream_t st, const bf16** shared_bf16) {
+  const int E = e->cfg.width;
+  if (shared_bf16) *shared_bf16 = nullptr;
+  if (m.shared_ff > 0) {
+    MTX_TRY((linear<T, LIN_GATED_CLAMP>(e, xa, m.shared_gate_up, nullptr, nullptr, e->act, rows, 2 * m.shared_ff, E, st, shared_limit)));
+    if (sizeof(T) == 2 && shared_bf16 && takes_umma(e, rows, E, m.shared_ff)) {
+      MTX_TRY(run_umma_raw(e, e->act, m.shared_down, rows, E, m.shared_ff, st));
+      *shared_bf16 = static_cast<const bf16*>(e->obf);
+    } else {
+      MTX_TRY((linear<T, LIN_PLAIN>(e, e->act, m.shared_down, nullptr, e->y, nullptr, rows, E, m.shared_ff, st)));
+    }
+  }
+  return MTX_OK;
+}
+
 // A routed feed-forward of the rows `xa` up to its experts' outputs: router, choice, sort, the chosen experts' products into e->moe_y (slot
 // e->moe_slot of every (row, choice)), the shared expert's product into e->y, or -- shared_bf16 given and the tcgen05 projection
 // taken -- left as bf16 in e->obf (*shared_bf16 points there, else it is null).
@@ -924,20 +947,32 @@ int routed_experts(mtx_layered* e, const mtx_moe_desc& m, const T* xa, int rows,
   // (identity experts get slot ranges behind the others': no product reads them)
   MTX_TRY(launch(moe_sort_kernel, dim3(1), dim3(1024), sizeof(int) * (2 * n_all + 1), st, (const int*)e->moe_chosen, entries, m.top, n_all, e->moe_off, e->moe_slot,
                  e->moe_row));
+  // many rows per expert (a prompt portion): the pair GEMM over the slots' rows, gathered once into the plane that the down products fill
+  // later.  16384 slots of 16 experts, 2048 -> 2 x 1024 -> 2048: 631 + 351 us on the mma.sync kernel of grouped_gemm.cuh, whose sums it repeats
+  // bit for bit (both add 16 products at a time in order of k).
+  if constexpr (sizeof(T) == 2) {
+    if (takes_wide_grouped(entries, m.experts, 2 * m.ff, E) && takes_wide_grouped(entries, m.experts, E, m.ff)) {
+      const int grid = e->num_sms * 8;
+      MTX_TRY(launch(moe_gather_kernel, dim3(grid), dim3(256), 0, st, reinterpret_cast<const uint4*>(xa), (const int*)e->moe_row, (const int*)(e->moe_off + m.experts),
+                     E / 8, reinterpret_cast<uint4*>(e->moe_y)));
+      WideLinEpi<LIN_GATED_CLAMP, false> up;
+      memset(&up, 0, sizeof(up));
+      up.act = static_cast<bf16*>(e->moe_act);
+      up.ldo = m.ff;
+      up.limit = limit;
+      MTX_TRY(launch_wide_grouped(e->moe_y, m.w_gate_up, e->moe_off, m.experts, entries, 2 * m.ff, E, up, e->num_sms, st));
+      WideLinEpi<LIN_PLAIN, false> down;
+      memset(&down, 0, sizeof(down));
+      down.out = e->moe_y;
+      down.ldo = E;
+      MTX_TRY(launch_wide_grouped(e->moe_act, m.w_down, e->moe_off, m.experts, entries, E, m.ff, down, e->num_sms, st));
+      return shared_expert<T>(e, m, xa, rows, shared_limit, st, shared_bf16);
+    }
+  }
   MTX_TRY((linear_grouped<T, LIN_GATED_CLAMP>(xa, e->moe_row, m.w_gate_up, (long long)2 * m.ff * E, e->moe_off, m.experts, nullptr, e->moe_act, entries, 2 * m.ff,
                                               E, limit, st)));
   MTX_TRY((linear_grouped<T, LIN_PLAIN>(e->moe_act, nullptr, m.w_down, (long long)E * m.ff, e->moe_off, m.experts, e->moe_y, nullptr, entries, E, m.ff, 0.0f, st)));
-  if (shared_bf16) *shared_bf16 = nullptr;
-  if (m.shared_ff > 0) {
-    MTX_TRY((linear<T, LIN_GATED_CLAMP>(e, xa, m.shared_gate_up, nullptr, nullptr, e->act, rows, 2 * m.shared_ff, E, st, shared_limit)));
-    if (sizeof(T) == 2 && shared_bf16 && takes_umma(e, rows, E, m.shared_ff)) {
-      MTX_TRY(run_umma_raw(e, e->act, m.shared_down, rows, E, m.shared_ff, st));
-      *shared_bf16 = static_cast<const bf16*>(e->obf);
-    } else {
-      MTX_TRY((linear<T, LIN_PLAIN>(e, e->act, m.shared_down, nullptr, e->y, nullptr, rows, E, m.shared_ff, st)));
-    }
-  }
-  return MTX_OK;
+  return shared_expert<T>(e, m, xa, rows, shared_limit, st, shared_bf16);
 }
 
 // a MTX_MIXER_COMPOSITE layer with MTX_NORM_SANDWICH norms; xa holds wnorm(x, norm1) on entry

@@ -180,6 +180,17 @@ __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* chosen, int e
   }
 }
 
+// the rows that the slots read, side by side for the pair GEMM: dst[s] = src[a_row[s]], `pieces` 16-byte pieces per row, for the slots below *n
+__global__ void __launch_bounds__(256) moe_gather_kernel(const uint4* src, const int* a_row, const int* n, int pieces, uint4* dst) {
+  griddep_wait();
+  const int slots = *n;
+  for (int s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); s < slots; s += gridDim.x * (blockDim.x >> 5)) {
+    const uint4* from = src + size_t(a_row[s]) * pieces;
+    uint4* to = dst + size_t(s) * pieces;
+    for (int c = threadIdx.x & 31; c < pieces; c += 32) to[c] = from[c];
+  }
+}
+
 __global__ void __launch_bounds__(256) moe_combine_kernel(const float* ye, const int* slot_of, const float* weight, int top, int width, int add, float* y) {
   griddep_wait();
   const int r = blockIdx.x;

@@ -21,8 +21,26 @@ def _model(name, width):
     layers = [ligidra.attention_layer(4, 2, 64, window=64, pool=16, mlp=ligidra.moe_ff(4, 4, 128, shared_ff=ff)),
               ligidra.delta_layer(4, 2, 32, 64, mlp=ligidra.moe_ff(4, 4, 128, shared_ff=ff))]
     return ligidra, ligidra.model_dict(width, 384, layers, side_dim=64)
-  layers = [zakelorn.parallel_layer(zakelorn.attention_part(4, 2, 64, window=64, keep_first=4), zakelorn.lightning_part(4, 64), mlp=zakelorn.dense_ff(ff))] * 2
+  ffs = [zakelorn.dense_ff(ff), zakelorn.moe_ff(5, 4, 96, identity=1, groups=2, keep=2)]  # unequal experts, slots beyond their ranges
+  layers = [zakelorn.parallel_layer(zakelorn.attention_part(4, 2, 64, window=64, keep_first=4), zakelorn.lightning_part(4, 64), mlp=f) for f in ffs]
   return zakelorn, zakelorn.model_dict(width, 384, layers)
+
+
+@pytest.mark.parametrize("name", ["kifusun", "gugidra", "zakelorn"])
+def test_long_steps_repeat_short_ones(name):
+  """A row's bits do not depend on how many rows its step has: 768 rows at once against three steps of 256."""
+  design, model = _model(name, 256)
+  toks = np.random.Generator(np.random.PCG64(1)).integers(0, model["vocab"], size=768).tolist()
+  out = []
+  for rows in (768, 256):
+    cfg = pyconfig.from_model_dict(model, dtype="bfloat16", per_device_batch_size=2, max_target_length=800, pagedattn_tokens_per_page=16,
+                                   pagedattn_num_pages=60, max_step_rows=rows)
+    engine = maxengine.MaxEngine(cfg)
+    engine.load_params(design.random_tensors(cfg, seed=3))
+    state = engine.init_decode_state()
+    engine.step([(0, toks, [])])
+    out.append([t.clone() for t in state["cache"]["key_pages"][:1]])
+  assert all(torch.equal(a, b) for a, b in zip(*out))
 
 
 @pytest.mark.parametrize("name", ["kifusun", "gugidra", "ligidra", "zakelorn"])
