@@ -52,6 +52,7 @@ struct mtx_layered {
   int max_part_cols = 0;       // columns of the partial results of layers with two score maps (float32 engines keep one part of them)
   // composite mixers, sandwich norms, routed feed-forwards
   bool sandwich = false;
+  int max_rec_n = 0;           // mLSTM: heads x dim
   int max_rec_o = 0, max_rec_aux = 0, max_moe_top = 0, max_moe_experts = 0, max_moe_ff = 0;
   float *x0 = nullptr, *rec_o = nullptr, *rec_aux = nullptr, *moe_logits = nullptr, *moe_weight = nullptr, *moe_y = nullptr;
   int *moe_chosen = nullptr, *moe_slot = nullptr, *moe_row = nullptr, *moe_off = nullptr;
@@ -66,6 +67,7 @@ struct mtx_layered {
   int max_rec_gate = 0, max_rec_z = 0;
   bool outlayer = false;  // MTX_NORM_OUT_LAYER layers
   float *rec_gate = nullptr, *rec_z = nullptr;
+  float* rec_n = nullptr;  // mLSTM: new n [groups, heads, dim], then new m [groups, heads]
 };
 
 namespace {
@@ -75,7 +77,7 @@ size_t elem(const mtx_layered* e) { return e->cfg.float32 ? 4 : 2; }
 struct LWs {
   size_t x, y, qkv, v_shared, xa, q, attn, act, wanted, obf, attn_part, total;
   size_t smax_ml, x0, rec_o, rec_aux, moe_logits, moe_weight, moe_y, moe_chosen, moe_slot, moe_row, moe_off, moe_act;
-  size_t h, xb, lat_q, lat_o, rec_gate, rec_z;
+  size_t h, xb, lat_q, lat_o, rec_gate, rec_z, rec_n;
 };
 
 LWs layered_layout(const mtx_layered* e) {
@@ -118,6 +120,7 @@ LWs layered_layout(const mtx_layered* e) {
   L.xb = take(e->parallel || e->prenorm ? R * c.width * es : 4);
   L.rec_gate = take(R * size_t(e->max_rec_gate > 0 ? e->max_rec_gate : 1) * 4);
   L.rec_z = take(R * size_t(e->max_rec_z > 0 ? e->max_rec_z : 1) * 4);
+  L.rec_n = take(size_t(c.num_groups > 0 ? c.num_groups : 1) * size_t(e->max_rec_n) * 2 * 4 + 4);
   L.lat_q = take(R * size_t(e->max_lat_q > 0 ? e->max_lat_q : 1) * 4);
   L.lat_o = take(R * size_t(e->max_lat_o > 0 ? e->max_lat_o : 1) * es);
   L.total = off;
@@ -1066,6 +1069,10 @@ int composite_layer(mtx_layered* e, int li, const mtx_ragged_batch& b, cudaStrea
     ra.state_s = r.state_s;
     ra.state_n = r.state_n;
     ra.state_m = r.state_m;
+    if (r.kind == MTX_REC_MLSTM) {
+      ra.next_n = e->rec_n;
+      ra.next_m = e->rec_n + size_t(c.num_groups) * r.heads * r.dim;
+    }
     ra.run_row0 = b.run_row0;
     ra.group = b.group;
     ra.pos = b.pos;
@@ -1092,6 +1099,12 @@ int composite_layer(mtx_layered* e, int li, const mtx_ragged_batch& b, cudaStrea
     oa.gate_silu = r.gate_silu;
     oa.eps = c.eps;
     oa.out_scale = r.out_scale;
+    oa.group = b.group;
+    oa.next_n = ra.next_n;
+    oa.next_m = ra.next_m;
+    oa.state_n = r.state_n;
+    oa.state_m = r.state_m;
+    oa.dim = r.dim;
     MTX_TRY(launch(recurrent_out_kernel<T>, dim3(rows), dim3(256), 0, st, oa));
   }
   MTX_TRY((linear<T, LIN_PLAIN>(e, mix, l.wo, nullptr, e->y, nullptr, rows, E, cc.k_out, st)));
@@ -2002,6 +2015,7 @@ int check_composite(mtx_layered* e, int i) {
     if (r.kind == MTX_REC_MLSTM && (!r.state_n || !r.state_m || !r.gate_bias || !(r.gate_cap > 0.0f))) return fail(MTX_ERR_ARG, "layer %d: mLSTM state / gate bias / cap missing", i);
     if (r.heads * r.vdim > e->max_rec_o) e->max_rec_o = r.heads * r.vdim;
     const int aux = r.kind == MTX_REC_GLA ? r.heads * r.dim : 2 * r.heads;
+    if (r.kind == MTX_REC_MLSTM && r.heads * r.dim > e->max_rec_n) e->max_rec_n = r.heads * r.dim;
     if (aux > e->max_rec_aux) e->max_rec_aux = aux;
   }
   const CompositeCols cc = composite_cols(l);
@@ -2385,6 +2399,7 @@ int mtx_layered_bind(mtx_layered* e, void* workspace, size_t workspace_bytes) {
   e->lat_o = base + L.lat_o;
   e->rec_gate = reinterpret_cast<float*>(base + L.rec_gate);
   e->rec_z = reinterpret_cast<float*>(base + L.rec_z);
+  e->rec_n = reinterpret_cast<float*>(base + L.rec_n);
   e->bound = true;
   return MTX_OK;
 }

@@ -248,6 +248,10 @@ struct RecScanArgs {
   float* state_s;      // [slots, heads, vdim, dim]: a value column's dim entries are contiguous
   float* state_n;      // mLSTM [slots, heads, dim]
   float* state_m;      // mLSTM [slots, heads]
+  // mLSTM: where the new n and m go, same layout (the CTAs of one head share them: one of them may be done before another has read the state's).
+  // recurrent_out_kernel puts them into the state.
+  float* next_n;
+  float* next_m;
   const int* run_row0; // [n_runs + 1]
   const int* group;
   const int* pos;
@@ -614,21 +618,22 @@ __global__ void __launch_bounds__(CB * SL) recurrent_scan_kernel(const RecScanAr
     __syncthreads();  // the stage is free for the next iteration's load
   }
   const bool write_n = KIND == REC_MLSTM && blockIdx.z == 0 && jl == 0;
+  float* gn_next = KIND == REC_MLSTM ? a.next_n + (size_t(slot) * H + h) * d : nullptr;
 #pragma unroll
   for (int i4 = 0; i4 < RPT; i4 += 4) {
     const int r = channel(i4);
     if (vec) {
       if (r < d && col_ok) *reinterpret_cast<float4*>(gs + r) = make_float4(S[i4], S[i4 + 1], S[i4 + 2], S[i4 + 3]);
-      if (write_n && r < d) *reinterpret_cast<float4*>(gn + r) = make_float4(N[i4], N[i4 + 1], N[i4 + 2], N[i4 + 3]);
+      if (write_n && r < d) *reinterpret_cast<float4*>(gn_next + r) = make_float4(N[i4], N[i4 + 1], N[i4 + 2], N[i4 + 3]);
     } else {
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         if (r + e < d && col_ok) gs[r + e] = S[i4 + e];
-        if (write_n && r + e < d) gn[r + e] = N[i4 + e];
+        if (write_n && r + e < d) gn_next[r + e] = N[i4 + e];
       }
     }
   }
-  if (write_n && tid == 0) a.state_m[size_t(slot) * H + h] = m;
+  if (write_n && tid == 0) a.next_m[size_t(slot) * H + h] = m;
 }
 
 template <typename T>
@@ -643,12 +648,22 @@ struct RecOutArgs {
   int out_col;
   int heads, vdim, gate_silu;
   float eps, out_scale;
+  // mLSTM (else null): the CTA of a run's last row puts the run's new n [slots, heads, dim] and m [slots, heads] into the state
+  const int* group;
+  const float *next_n, *next_m;
+  float *state_n, *state_m;
+  int dim;
 };
 
 // one CTA per row, a warp per head
 template <typename T>
 __global__ void __launch_bounds__(256) recurrent_out_kernel(const RecOutArgs<T> a) {
   griddep_wait();
+  if (a.next_n && (blockIdx.x + 1 == gridDim.x || a.group[blockIdx.x + 1] != a.group[blockIdx.x])) {
+    const size_t at = size_t(a.group[blockIdx.x]) * a.heads;
+    for (int i = threadIdx.x; i < a.heads * a.dim; i += blockDim.x) a.state_n[at * a.dim + i] = a.next_n[at * a.dim + i];
+    for (int i = threadIdx.x; i < a.heads; i += blockDim.x) a.state_m[at + i] = a.next_m[at + i];
+  }
   const int r = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5, dv = a.vdim;
   for (int h = warp; h < a.heads; h += nw) {
     const float* o = a.o + size_t(r) * a.heads * dv + h * dv;

@@ -1,0 +1,35 @@
+"""The recurrences' walks (csrc/recurrent_mixers.cuh) where CTAs of one head share state."""
+
+import numpy as np
+import pytest
+import torch
+
+from maxtext_indextts2_b200 import gugidra as g
+from maxtext_indextts2_b200 import maxengine, pyconfig
+
+pytestmark = pytest.mark.gpu
+
+
+def tokens(n, seed):
+  return np.random.Generator(np.random.PCG64(seed)).integers(0, 320, size=n).tolist()
+
+
+def test_many_slots_decode_like_each_alone():
+  """A decode step of more (slot, head, column block) CTAs than run at once: every CTA of a head reads the mLSTM's normaliser and running
+  maximum of the state, whichever of them is done first."""
+  cfg = g.model_dict(256, 320, [g.parallel_layer(4, 2, 64, 8, 64, 128)])
+  config = lambda slots: pyconfig.from_model_dict(cfg, dtype="float32", per_device_batch_size=slots, max_target_length=64, pagedattn_tokens_per_page=16,
+                                                  pagedattn_num_pages=4 * slots + 2)
+  tensors = g.random_tensors(config(1), seed=2)
+  many, one = (maxengine.MaxEngine(config(n)) for n in (64, 1))
+  for e in (many, one):
+    e.load_params(tensors)
+    e.init_decode_state()
+  prompt, then = tokens(9, 5), tokens(64, 6)
+  many.step([(s, prompt, []) for s in range(64)])
+  got = many.step([(s, [then[s]], [0]) for s in range(64)])
+  for s in range(0, 64, 9):
+    one.release_pages(0)
+    one.step([(0, prompt, [])])
+    want = one.step([(0, [then[s]], [0])])
+    assert float((got[s] - want[0]).abs().max() / want[0].abs().max()) < 3e-5  # (fp32 sums in another order, as in the design's own tests)
