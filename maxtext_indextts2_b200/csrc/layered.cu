@@ -651,6 +651,17 @@ int launch_rec_scan_cb(const RecScanArgs& ra, int n_runs, cudaStream_t st) {
   return fail(MTX_ERR_UNSUPPORTED, "recurrence: dim %d", ra.dim);
 }
 
+template <int KIND, int RPT>
+int launch_rec_walk(const RecScanArgs& ra, int n_runs, cudaStream_t st) {
+  const size_t smem = rec_walk_smem_bytes(KIND, ra.dim);
+  static size_t have = 0;  // per instantiation
+  if (smem > 48 * 1024 && smem > have) {
+    MTX_CUDA(cudaFuncSetAttribute(recurrent_walk_kernel<KIND, RPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    have = smem;
+  }
+  return launch(recurrent_walk_kernel<KIND, RPT>, dim3(n_runs, ra.heads, (ra.vdim + kWalkCols - 1) / kWalkCols), dim3(kWalkCols * kWalkSlices), smem, st, ra);
+}
+
 // A walk is bound by latency, so what counts is how many warps share an SM.  16 value columns per CTA when that still gives every
 // SM two CTAs, else 8; and when even 8-column CTAs with 8 slices per column leave the thread slots of the GPU mostly empty (one
 // prompt: heads x vdim columns in all), a column is cut into 16 slices.
@@ -661,6 +672,16 @@ int launch_rec_scan(mtx_layered* e, RecScanArgs& ra, int n_runs, int rows, cudaS
   static const int force_sl = env_int("MTX_REC_SLICES", 0);
   const bool fine = force_sl ? force_sl == 16 : (!wide && ra.dim >= 64 && columns * 8 < 512LL * e->num_sms);
   ra.chunk = rec_chunk_tokens(ra.dim, wide ? 16 : 8, fine ? 16 : 8, rows == n_runs, rec_vectors(KIND));
+  // runs of a chunk of tokens and more: the walk that reduces once per chunk
+  if constexpr (KIND == REC_GLA || KIND == REC_MLSTM) {
+    static const int walk = env_int("MTX_REC_WALK", 1);
+    if (walk && fine && ra.vec4 && ra.dim <= 256 && rows >= kWalkTokens * n_runs) {
+      const int rpt = rec_rpt(ra.dim, kWalkSlices);
+      if (rpt == 4) return launch_rec_walk<KIND, 4>(ra, n_runs, st);
+      if (rpt == 8) return launch_rec_walk<KIND, 8>(ra, n_runs, st);
+      return launch_rec_walk<KIND, 16>(ra, n_runs, st);
+    }
+  }
   if (fine && ra.dim >= 16) return launch_rec_scan_cb<KIND, 8, 16>(ra, n_runs, st);
   return wide ? launch_rec_scan_cb<KIND, 16, 8>(ra, n_runs, st) : launch_rec_scan_cb<KIND, 8, 8>(ra, n_runs, st);
 }

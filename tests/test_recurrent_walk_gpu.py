@@ -1,4 +1,4 @@
-"""The recurrences' walks (csrc/recurrent_mixers.cuh) where CTAs of one head share state."""
+"""The recurrences' walks (csrc/recurrent_mixers.cuh) where CTAs of one head share state, and the walk of long runs against the one of short ones."""
 
 import numpy as np
 import pytest
@@ -33,3 +33,20 @@ def test_many_slots_decode_like_each_alone():
     one.step([(0, prompt, [])])
     want = one.step([(0, [then[s]], [0])])
     assert float((got[s] - want[0]).abs().max() / want[0].abs().max()) < 3e-5  # (fp32 sums in another order, as in the design's own tests)
+
+
+def test_long_walk_repeats_short_portions():
+  """Runs of 16 tokens and more (one reduction per chunk of tokens) leave the bits that the token-by-token walk of portions of 10 leaves."""
+  for kind in ("gla", "parallel"):
+    layer = g.gla_layer(4, 64, 64) if kind == "gla" else g.parallel_layer(4, 2, 32, 2, 128, 64)
+    cfg = g.model_dict(256, 320, [layer])
+    config = pyconfig.from_model_dict(cfg, dtype="float32", per_device_batch_size=1, max_target_length=128, pagedattn_tokens_per_page=16, pagedattn_num_pages=10)
+    tensors, toks, states = g.random_tensors(config, seed=4), tokens(90, 5), []
+    for portion in (90, 10):
+      engine = maxengine.MaxEngine(config)
+      engine.load_params(tensors)
+      state = engine.init_decode_state()
+      for at in range(0, 90, portion):
+        logits = engine.step([(0, toks[at : at + portion], [portion - 1])])
+      states.append([t.clone() for t in state["cache"]["recurrent_state"]] + [logits])
+    assert all(torch.equal(a, b) for a, b in zip(*states))
