@@ -19,6 +19,7 @@
 #include "window_attention_mma.cuh"
 #include "window_attention_decode.cuh"
 #include "softmax_attention.cuh"
+#include "softmax_flash.cuh"
 #include "multi_attention.cuh"
 #include "recurrent_mixers.cuh"
 #include "decayed_sums.cuh"
@@ -875,6 +876,50 @@ int launch_multi_decode(mtx_layered* e, SoftmaxAttnArgs<bf16>& sa, const MultiDe
   return MTX_OK;
 }
 
+// rows of a page that one copy of a key tile takes: a page or the largest part of it that cuts the tile evenly (8 rows: the swizzle's period)
+int paged_flash_box(int tokens_per_page, int key_tile) {
+  int box = key_tile;
+  while (box > 1 && tokens_per_page % box != 0) box /= 2;
+  return box;
+}
+
+// Long runs -- at least 128 rows (half a CTA's) per run on average; shorter runs leave the tcgen05 tiles' rows empty, and the 16-row tiles of
+// softmax_attention_mma_kernel fill the chip -- of layers whose windows are longer than any sequence, if they have one.
+bool takes_paged_flash(const SoftmaxAttnArgs<bf16>& sa, const mtx_ragged_batch& b) {
+  static const int on = env_int("MTX_SOFTMAX_FLASH", 1);
+  auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  const int key_tile = sa.dim == 256 ? 32 : 64;
+  return on && (sa.dim == 64 || sa.dim == 128 || sa.dim == 256) && sa.pool == 0 && sa.chunk == 0 &&
+         (sa.window == 0 || sa.window >= sa.max_pages * sa.tokens_per_page) && b.n_runs > 0 && sa.rows >= 128 * b.n_runs && paged_flash_box(sa.tokens_per_page, key_tile) >= 8 && aligned(sa.q) && aligned(sa.k_pages) && aligned(sa.v_pages);
+}
+
+template <int D>
+int launch_paged_flash_t(const SoftmaxAttnArgs<bf16>& sa, const mtx_ragged_batch& b, cudaStream_t st) {
+  typedef PagedFlashShape<D> F;
+  static bool attr_set = false;  // per head size
+  if (!attr_set) {
+    MTX_CUDA(cudaFuncSetAttribute(paged_flash_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(paged_flash_smem_bytes<D>())));
+    attr_set = true;
+  }
+  PagedFlashArgs p;
+  p.a = sa;
+  p.run_row0 = b.run_row0;
+  p.n_runs = b.n_runs;
+  p.box = paged_flash_box(sa.tokens_per_page, F::KT);
+  CUtensorMap tm_q, tm_k, tm_v;
+  const uint64_t pool_rows = uint64_t(sa.kv_heads) * sa.num_pages * sa.tokens_per_page;
+  MTX_TRY(make_map(&tm_q, sa.q, uint64_t(sa.heads) * D, sa.rows, 128));
+  MTX_TRY(make_map(&tm_k, sa.k_pages, D, pool_rows, p.box));
+  MTX_TRY(make_map(&tm_v, sa.v_pages, D, pool_rows, p.box));
+  return launch(paged_flash_kernel<D>, dim3(sa.heads, sa.rows / (F::NQ * 128) + b.n_runs), dim3(F::kThreads), paged_flash_smem_bytes<D>(), st, tm_q, tm_k, tm_v, p);
+}
+
+int launch_paged_flash(const SoftmaxAttnArgs<bf16>& sa, const mtx_ragged_batch& b, cudaStream_t st) {
+  if (sa.dim == 64) return launch_paged_flash_t<64>(sa, b, st);
+  if (sa.dim == 128) return launch_paged_flash_t<128>(sa, b, st);
+  return launch_paged_flash_t<256>(sa, b, st);
+}
+
 // causal softmax attention of the step's rows over the paged cache: the tensor-core kernels for bf16 engines whose head sizes they
 // are built for (single-token steps: the transposed kernels), else the fp32 row kernel
 template <typename T>
@@ -892,6 +937,7 @@ int run_softmax_attention(mtx_layered* e, SoftmaxAttnArgs<T>& sa, const mtx_ragg
     if (use_softmax_mma() && sa.ld_out % 2 == 0) {
       if (plan.ok && !multi_shape) {
         if (b.n_tiles == sa.rows && decode_arm) return launch_softmax_decode(e, sa, plan.d16, st);
+        if (takes_paged_flash(sa, b)) return launch_paged_flash(sa, b, st);
         return launch_softmax_mma(e, sa, plan, b.n_tiles, b.n_tiles == sa.rows, st);
       }
       if (sa.pool == 0 && !sa.slopes && sa.softcap == 0.0f && sa.scale > 0.0f) {
