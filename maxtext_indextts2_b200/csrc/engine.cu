@@ -357,7 +357,39 @@ int launch_prefill_attention(mtx_engine* e, int layer, int rows, int start_pos, 
   return launch(prefill_attn_kernel<128>, grid, block, smem, st, e->tm_k, e->tm_v, p);
 }
 
-// The same for a pass of more than 256 rows (prefill_flash.cuh).  The 16-position CTAs above keep more SMs busy when positions are few: 256 rows
+// Prompt positions with heads of 256 (attention_wide.cuh): groups of positions share the K / V tiles.  Where the 256-row steps cut a position's keys
+// over several work items (fewer (position, kv head) pairs than CTAs are worth filling), they stay with decode_attn_wide_kernel.
+bool takes_prompt_wide(const mtx_engine* e, int rows) {
+  const mtx_model_config& c = e->cfg;
+  return c.head_dim == 256 &&
+         attn_tiles_per_item(rows, c.num_kv_heads, c.max_prefill_len, c.max_target_len, attn_target_items(e->num_sms)) >= attn_max_tiles(c.max_prefill_len, c.max_target_len);
+}
+
+int launch_prompt_wide(mtx_engine* e, int layer, int rows, int start_pos, int slot, cudaStream_t st) {
+  const mtx_model_config& c = e->cfg;
+  const int planes = staged_prefill(c) ? 1 : c.num_slots;
+  static bool attr_set = false;
+  if (!attr_set) {
+    MTX_CUDA(cudaFuncSetAttribute(prompt_attn_wide_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(attn_wide_smem_bytes(256))));
+    attr_set = true;
+  }
+  PromptWideParams p;
+  memset(&p, 0, sizeof(p));
+  p.q = e->q;
+  p.out = e->attn;
+  p.rows = rows;
+  p.start_pos = start_pos;
+  p.hq = c.num_q_heads;
+  p.hkv = c.num_kv_heads;
+  p.T = c.max_target_len;
+  p.plane_row0 = (layer * planes + slot) * c.num_kv_heads * c.max_target_len;
+  p.softcap = c.attn_softcap;
+  p.window = layer_is_local(e, layer) ? c.sliding_window : 0;
+  const int np = 8 / (p.hq / p.hkv), items = (rows + 64 * np - 1) / (64 * np) * 64 * p.hkv;
+  return launch(prompt_attn_wide_kernel<256>, dim3(items < e->num_sms ? items : e->num_sms), dim3(kWideThreads), attn_wide_smem_bytes(256), st, e->tm_k, e->tm_v, p);
+}
+
+// The same for a pass of more than 256 rows of the llama block (prefill_flash.cuh).  The 16-position CTAs above keep more SMs busy when positions are few: 256 rows
 // of 20 heads take 22 us there.
 template <int D>
 int launch_prefill_flash(mtx_engine* e, const CUtensorMap& tm_q, const PrefillFlashParams& p, cudaStream_t st) {
@@ -385,10 +417,7 @@ int launch_prefill_flash(mtx_engine* e, int layer, int rows, int start_pos, int 
   p.T = c.max_target_len;
   p.plane_row0 = (layer * planes + slot) * c.num_kv_heads * c.max_target_len;
   p.softcap = c.attn_softcap;
-  p.window = layer_is_local(e, layer) ? c.sliding_window : 0;
-  if (c.head_dim == 64) return launch_prefill_flash<64>(e, tm_q, p, st);
-  if (c.head_dim == 128) return launch_prefill_flash<128>(e, tm_q, p, st);
-  return launch_prefill_flash<256>(e, tm_q, p, st);
+  return c.head_dim == 64 ? launch_prefill_flash<64>(e, tm_q, p, st) : launch_prefill_flash<128>(e, tm_q, p, st);
 }
 
 // ---- persistent step kernel: work tables and launch -------------------------------------------
@@ -721,12 +750,16 @@ int enqueue_last_logits(mtx_engine* e, const bf16* x, int draw_row, int32_t* fir
 // The layers over `rows` (more than 256, at most pf_rows) prompt positions from start_pos on, all rows in every launch: the projections
 // on the pair GEMM (gemm_wide.cuh), RMSNorm fused into them as in the 65..256-row steps when its scales are folded.  e->x holds the
 // result.
+// The gemma3 block's passes (a multiple of 256 rows) repeat the bits of its 256-row steps: the GEMMs add up K in the steps' segments, the attention
+// kernels keep the steps' key tiles.  Its logits are products with the embedding table, the largest of them around 10 and rounded to bf16
+// (steps of 1/16), so that a last bit elsewhere moves the first token's log-probability by 6 %.
 int enqueue_prefill_pass(mtx_engine* e, int rows, const int32_t* tokens, int start_pos, int slot, cudaStream_t st) {
   const mtx_model_config& c = e->cfg;
   const bool gemma3 = c.decoder_block == 1, fused = c.norm_scales_folded != 0;
   const int planes = staged_prefill(c) ? 1 : c.num_slots;
   if (staged_prefill(c)) slot = 0;
   const int E = c.emb_dim, HD = c.num_q_heads * c.head_dim, M = c.mlp_dim, L = c.num_layers, pitch = e->pf_rows;
+  auto segments = [&](int n, int k) { return gemma3 ? plan_rows(n, k, 256, e->num_sms, EPI_STORE_BF16).splits : 1; };
   const size_t kv_layer = size_t(planes) * c.num_kv_heads * c.max_target_len * c.head_dim;
   const bf16 *wqkv = static_cast<const bf16*>(e->w.wqkv), *wo = static_cast<const bf16*>(e->w.wo), *w01 = static_cast<const bf16*>(e->w.w01),
              *wout = static_cast<const bf16*>(e->w.wout);
@@ -766,12 +799,12 @@ int enqueue_prefill_pass(mtx_engine* e, int rows, const int32_t* tokens, int sta
     g_class = KC_QKV;
     const bool local = layer_is_local(e, l);
     if (gemma3) {
-      WideEpi<EPI_STORE_BF16> qkv;
+      WideEpi<EPI_STORE_BF16, true> qkv;
       memset(&qkv, 0, sizeof(qkv));
       qkv.e.out = e->qkv_tmp;
       qkv.e.ld_out = e->qkv_n;
       norm_in(qkv.e, e->rows_ss_x, ss_x);
-      MTX_TRY(launch_wide(e->x, wqkv + size_t(l) * e->qkv_n * E, rows, e->qkv_n, E, 32, qkv, e->num_sms, st));
+      MTX_TRY(launch_wide(e->x, wqkv + size_t(l) * e->qkv_n * E, rows, e->qkv_n, E, 32, qkv, e->num_sms, st, segments(e->qkv_n, E)));
       QkNormArgs qa;
       memset(&qa, 0, sizeof(qa));
       qa.qkv = e->qkv_tmp;
@@ -807,7 +840,9 @@ int enqueue_prefill_pass(mtx_engine* e, int rows, const int32_t* tokens, int sta
       MTX_TRY(launch_wide(fused ? e->x : e->n, wqkv + size_t(l) * e->qkv_n * E, rows, e->qkv_n, E, c.head_dim, qkv, e->num_sms, st));
     }
     g_class = KC_ATTENTION;
-    MTX_TRY(launch_prefill_flash(e, l, rows, start_pos, slot, st));
+    if (!gemma3) MTX_TRY(launch_prefill_flash(e, l, rows, start_pos, slot, st));
+    else if (c.head_dim == 256) MTX_TRY(launch_prompt_wide(e, l, rows, start_pos, slot, st));
+    else MTX_TRY(launch_prefill_attention(e, l, rows, start_pos, slot, st));
     // h = x + [norm](attn . wo),  x = h + [norm](act . wout)
     auto project = [&](const bf16* a, const bf16* w, int k, const bf16* resid, bf16* out, float* ss, const void* post_scale) -> int {
       if (gemma3) {
@@ -815,7 +850,7 @@ int enqueue_prefill_pass(mtx_engine* e, int rows, const int32_t* tokens, int sta
         memset(&st_epi, 0, sizeof(st_epi));
         st_epi.e.out = e->n;
         st_epi.e.ld_out = E;
-        MTX_TRY(launch_wide(a, w, rows, E, k, 32, st_epi, e->num_sms, st));
+        MTX_TRY(launch_wide(a, w, rows, E, k, 32, st_epi, e->num_sms, st, segments(E, k)));
         g_class = KC_RMSNORM;
         return launch(post_norm_residual_kernel, dim3(rows), dim3(128), 0, st, (const bf16*)e->n, resid, static_cast<const bf16*>(post_scale) + size_t(l) * E, out, ss,
                       pitch, E, c.rms_eps);
@@ -835,14 +870,16 @@ int enqueue_prefill_pass(mtx_engine* e, int rows, const int32_t* tokens, int sta
     if (!fused)
       MTX_TRY(launch(rmsnorm_kernel<false>, dim3(rows), dim3(128), 0, st, (const bf16*)e->h, (const int*)nullptr, (const bf16*)nullptr, mlp_norm + size_t(l) * E,
                      (bf16*)nullptr, e->n, E, c.rms_eps));
-    WideEpi<EPI_SWIGLU> up;
+    EpiArgs up;
     memset(&up, 0, sizeof(up));
-    up.e.out = e->act;
-    up.e.ld_out = M;
-    up.e.act_gelu = gemma3 ? 1 : 0;
-    norm_in(up.e, e->rows_ss_h, ss_post);
+    up.out = e->act;
+    up.ld_out = M;
+    up.act_gelu = gemma3 ? 1 : 0;
+    norm_in(up, e->rows_ss_h, ss_post);
     g_class = KC_MLP_UP;
-    MTX_TRY(launch_wide(fused ? e->h : e->n, w01 + size_t(l) * 2 * M * E, rows, 2 * M, E, 32, up, e->num_sms, st));
+    const bf16 *up_x = fused ? e->h : e->n, *up_w = w01 + size_t(l) * 2 * M * E;
+    if (gemma3) MTX_TRY(launch_wide(up_x, up_w, rows, 2 * M, E, 32, WideEpi<EPI_SWIGLU, true>{up}, e->num_sms, st, segments(2 * M, E)));
+    else MTX_TRY(launch_wide(up_x, up_w, rows, 2 * M, E, 32, WideEpi<EPI_SWIGLU>{up}, e->num_sms, st));
     g_class = KC_MLP_DOWN;
     MTX_TRY(project(e->act, wout + size_t(l) * E * M, M, e->h, e->x, e->rows_ss_x, e->w.post_ffw_norm));
     ss_x = ss_post;
@@ -989,6 +1026,7 @@ int enqueue_step(mtx_engine* e, int mode, int rows, const int32_t* chunk_tokens,
       // averages every allocated cache row, valid or not: nothing a caller can rely on.)
       if (mode == 0 && local) MTX_CUDA(cudaMemsetAsync(e->attn, 0, size_t(rows) * HD * 2, st));
       if (mode == 1 && c.head_dim != 256) MTX_TRY(launch_prefill_attention(e, l, rows, start_pos, slot, st));
+      else if (mode == 1 && takes_prompt_wide(e, rows)) MTX_TRY(launch_prompt_wide(e, l, rows, start_pos, slot, st));
       else MTX_TRY(launch_attention(e, l, rows, st, mode));  // (head_dim 256: prompt positions run as decode rows)
 
       // h = x + rms_norm(dense(attn))
@@ -1965,8 +2003,9 @@ int mtx_prefill_rows(mtx_engine* e, const int32_t* tokens, int count, int start_
   for (int at = 0; at < count;) {
     const int left = count - at, small = e->cfg.max_rows;
     int n;
-    if (e->pf_rows > 0 && left > 256) {
-      n = left < e->pf_rows ? left : e->pf_rows;
+    const int wide = left < e->pf_rows ? left : e->pf_rows, take = e->cfg.decoder_block == 1 ? wide / 256 * 256 : wide;
+    if (take > 256 && (e->cfg.head_dim != 256 || takes_prompt_wide(e, 256))) {
+      n = take;
       MTX_TRY(enqueue_prefill_pass(e, n, tokens + at, start_pos + at, slot, st));
     } else {
       n = left < small ? left : small;

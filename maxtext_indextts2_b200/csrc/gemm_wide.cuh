@@ -290,6 +290,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       if constexpr (EPI::kFragments) {
         if (p.segments > 1) {
           float acc[kPairMaxCols / 32][16];
+          const auto pre = epi.prepare(w);
           for (int seg = 0; seg < p.segments; ++seg) {
             const uint32_t taddr = lanes + uint32_t(buf * p.bn + w.c0);
             mbar_wait(&tail->tmem_full[buf], acc_phase);
@@ -310,8 +311,8 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
             release();
           }
 #pragma unroll
-          for (int i = 0; i < kPairMaxCols / 32; ++i)
-            if (w.c0 + 16 * i < w.c1 && w.valid) epi.fragment(w, p.n, w.c0 + 16 * i, acc[i]);
+          for (int i = 0; i < kPairMaxCols / 32; i += 2)
+            if (w.c0 + 16 * i < w.c1 && w.valid) epi.fragment(w, p.n, pre, w.c0 + 16 * i, acc[i], acc[i + 1]);
           continue;
         }
       }
@@ -331,7 +332,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
 
 // ---- epilogues of the decoder engine --------------------------------------------------------------------------------------------
 // What gemm_rows.cuh's fragments compute, with the arithmetic between the accumulator and the stored value in fp32 and one rounding
-// at the end (those round every intermediate array to bf16; against float64 this side is the closer one).
+// at the end (those round every intermediate array to bf16; against float64 this side is the closer one); STEP: with their roundings.
 
 // the row's 1 / rms from the partial sums of squares that a residual epilogue left
 __device__ __forceinline__ float wide_rstd(const EpiArgs& e, int row) {
@@ -363,9 +364,7 @@ __device__ __forceinline__ void wide_gate(const EpiArgs& e, int r, int n0, const
   float o[16];
 #pragma unroll
   for (int j = 0; j < 16; ++j) {
-    const float a = g[j];
-    const float act = e.act_gelu ? a * 0.5f * (1.0f + tanhf(0.7978845608028654f * (a + 0.044715f * a * a * a))) : __fdividef(a, 1.0f + __expf(-a));
-    o[j] = act * u[j];
+    o[j] = __fdividef(g[j], 1.0f + __expf(-g[j])) * u[j];
   }
   frag_store_bf16(e.out + (long long)r * e.ld_out + (n0 >> 1), o);
 }
@@ -398,14 +397,28 @@ __device__ __forceinline__ void wide_qkv(const EpiArgs& e, int r, int head, int 
   frag_store_bf16(dst + half, b);
 }
 
-template <int KIND>
+template <int KIND, bool STEP = false>
 struct WideEpi {
-  static constexpr bool kFragments = KIND == EPI_STORE_BF16;
+  static constexpr bool kFragments = KIND == EPI_STORE_BF16 || (KIND == EPI_SWIGLU && STEP);
   EpiArgs e;
 
-  __device__ __forceinline__ void fragment(const WideTile& w, int n, int c, const float (&v)[16]) const { rows_epi_store(e, n, w.row, w.n0 + c, v); }
+  __device__ __forceinline__ float prepare(const WideTile& w) const {
+    if (KIND == EPI_RESIDUAL || e.ss_in == nullptr || !w.valid) return 1.0f;
+    return STEP ? rows_rstd(e, w.row) : wide_rstd(e, w.row);
+  }
 
-  __device__ __forceinline__ float prepare(const WideTile& w) const { return KIND == EPI_RESIDUAL || e.ss_in == nullptr || !w.valid ? 1.0f : wide_rstd(e, w.row); }
+  // 32 columns of a row
+  __device__ __forceinline__ void fragment(const WideTile& w, int n, float rs, int c, float (&a)[16], float (&b)[16]) const {
+    rows_scale16(a, rs);
+    rows_scale16(b, rs);
+    if (KIND == EPI_SWIGLU) {
+      if (STEP) rows_epi_swiglu(e, n, w.row, w.n0 + c, a, b);
+      else wide_gate(e, w.row, w.n0 + c, a, b);
+    } else {
+      rows_epi_store(e, n, w.row, w.n0 + c, a);
+      rows_epi_store(e, n, w.row, w.n0 + c + 16, b);
+    }
+  }
 
   template <class LD>
   __device__ __forceinline__ void operator()(const WideTile& w, int n, float rs, LD&& ld16) const {
@@ -429,9 +442,7 @@ struct WideEpi {
         float g[16], u[16];
         ld16(c, g);
         ld16(c + 16, u);
-        rows_scale16(g, rs);
-        rows_scale16(u, rs);
-        if (w.valid) wide_gate(e, w.row, w.n0 + c, g, u);
+        if (w.valid) fragment(w, n, rs, c, g, u);
       }
     } else if (KIND == EPI_QKV_ROPE) {
       const int half = e.d >> 1;

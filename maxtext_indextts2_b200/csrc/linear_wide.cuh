@@ -21,8 +21,13 @@ struct WideLinEpi {
 
   __device__ __forceinline__ int prepare(const WideTile&) const { return 0; }
 
-  // 16 columns of a row
-  __device__ __forceinline__ void fragment(const WideTile& w, int n, int c, float (&v)[16]) const {
+  // 32 columns of a row
+  __device__ __forceinline__ void fragment(const WideTile& w, int n, int, int c, float (&a)[16], float (&b)[16]) const {
+    columns(w, n, c, a);
+    columns(w, n, c + 16, b);
+  }
+  // 16 of them
+  __device__ __forceinline__ void columns(const WideTile& w, int n, int c, float (&v)[16]) const {
     constexpr bool gated = EPI == LIN_GATED || EPI == LIN_GATED_CLAMP, narrow = gated || EPI == LIN_ACT || EPI == LIN_RELU2 || EPI == LIN_GELU;
 #pragma unroll
     for (int j = 0; ROUND && j < 16; j += 2) {
@@ -77,7 +82,7 @@ struct WideLinEpi {
     for (int c = w.c0; c < w.c1; c += 16) {
       float v[16];
       ld16(c, v);
-      if (w.valid) fragment(w, n, c, v);
+      if (w.valid) columns(w, n, c, v);
     }
   }
 };

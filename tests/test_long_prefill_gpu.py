@@ -49,3 +49,22 @@ def test_one_pass_against_portions(block, dim, kw):
       assert float(err.max()) < 4e-2, (n, name, int(err.argmax()))
     a, b = whole["logits"].double(), prefix["logits"].double()
     assert float((a - b).norm() / b.norm()) < 4e-2, n
+
+
+@pytest.mark.parametrize("dim,kw", [(64, {}), (128, {"sliding_window_size": 256}), (256, {}), (256, {"sliding_window_size": 256}), (256, {"sliding_window_size": 300})])
+def test_gemma3_pass_repeats_steps(dim, kw):
+  """The gemma3 block in one pass leaves the bits of its 256-token steps: windows that no, some and all positions fill, a length at which a group of
+  positions holds some of either kind, and a remainder behind the pass."""
+  cfg = _config("gemma3", dim, **kw)
+  engine = maxengine.MaxEngine(cfg)
+  params = engine.load_params(on_device_init=True, norm_jitter=0.1)
+  engine.init_decode_state()
+  toks = torch.randint(0, cfg.vocab_size, (831,), generator=torch.Generator().manual_seed(2))
+  whole, _ = engine.prefill(params=params, padded_tokens=toks, true_length=831, slot=0)
+  prefix = None
+  for at in range(0, 831, 256):
+    m = min(256, 831 - at)
+    before = maxengine.ExistingPrefix(cache=prefix["cache"], common_prefix_tokens=toks[:at]) if at else None
+    prefix, _ = engine.prefill(params=params, padded_tokens=toks[at : at + m], true_length=m, existing_prefix=before, slot=0)
+  for name in ("key", "value"):
+    assert torch.equal(whole["cache"][name], prefix["cache"][name])
