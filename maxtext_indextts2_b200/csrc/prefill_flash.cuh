@@ -10,14 +10,13 @@
 // The accumulator is brought to a new maximum only when a position's maximum grew by more than 2^8 (its probabilities then reach 2^8 instead of 1;
 // their relative rounding is the same), which after the first tiles is hardly ever: a rescale reads and writes D columns of TMEM.
 //
-//   D = 64, 128:  NQ = 2, KT = 128: the MMAs of one half of the positions run under the softmax of the other
-//   D = 256:      NQ = 1, KT = 64 (the accumulator takes 256 of the 512 TMEM columns, Q, K and V 192 KB): two S buffers, the next tile's S
-//                 is issued before this tile's P V
+//   D = 64:   NQ = 1, KT = 128, half of the TMEM: two CTAs per SM, each under the other's MMAs.  20 heads x 16 CTAs of 256 positions (NQ = 2, one CTA
+//             per SM) left SMs idle behind the longest ones: 87 us for 4000 positions, 72 so
+//   D = 128:  NQ = 2, KT = 128: the MMAs of one half of the positions run under the softmax of the other
 //
 // Bound: the special-function units at D = 64 (one exp2 per score: 16 per SM and clock), 4000 positions x 20 heads: 36 us at least.
 // The mma.sync kernel (prefill_attention.cuh), 256 rows per launch, reads every tile for 16 positions at a time: 787 us for the same.  With the
-// projections on the pair GEMM a prompt of 4000 tokens (24 layers) went from 37.1 to 6.8 ms, 3001 tokens through six gemma3 layers with heads of
-// 256 from 17.5 to 3.7 ms.
+// projections on the pair GEMM a prompt of 4000 tokens (24 layers) went from 37.1 to 6.4 ms.
 #pragma once
 
 #include "attention.cuh"
@@ -34,17 +33,15 @@ struct PrefillFlashParams {
   int hq, hkv, T;
   int plane_row0;  // cache row of (layer, plane, kv head 0, position 0) in the K / V tensor maps; kv head h adds h * T
   float softcap;
-  int window;      // > 0: a query sees the keys (position - window, position]
 };
 
 template <int D>
 struct FlashShape {
-  static constexpr int NQ = D == 256 ? 1 : 2, KT = D == 256 ? 64 : 128;
-  static constexpr int kStages = D == 64 ? 4 : 2;
-  static constexpr int kThreads = 64 + NQ * 128;
-  static constexpr int kQBytes = 128 * D * 2, kTileBytes = KT * D * 2;  // a Q tile; a K or a V tile
-  static constexpr int kSBufs = 2;                                       // S of each Q tile (NQ = 2), or of alternate key tiles (NQ = 1)
-  static constexpr int kOCol = kSBufs * KT;                              // first TMEM column of the accumulators
+  static constexpr int NQ = D == 64 ? 1 : 2, KT = 128;
+  static constexpr int kStages = 2;
+  static constexpr int kThreads = 64 + NQ * 128, kCtas = D == 64 ? 2 : 1;  // CTAs per SM
+  static constexpr int kQBytes = 128 * D * 2, kTileBytes = KT * D * 2;    // a Q tile; a K or a V tile
+  static constexpr int kOCol = NQ * KT, kTmemCols = 512 / kCtas;           // first TMEM column of the accumulators; columns in all
 };
 
 struct FlashTail {
@@ -69,7 +66,7 @@ __device__ __forceinline__ float flash_ex2(float x) {
 
 // grid (query heads, ceil(rows / (NQ * 128))); blockIdx.y counts from the last positions, whose CTAs have the most keys
 template <int D>
-__global__ void __launch_bounds__(FlashShape<D>::kThreads, 1)
+__global__ void __launch_bounds__(FlashShape<D>::kThreads, FlashShape<D>::kCtas)
 prefill_flash_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                      const PrefillFlashParams p) {
   typedef FlashShape<D> F;
@@ -83,15 +80,12 @@ prefill_flash_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   const int head = blockIdx.x, h = head / (p.hq / p.hkv);
   const int q0 = (int(gridDim.y) - 1 - int(blockIdx.y)) * NQ * 128;
   const int plane_row = p.plane_row0 + h * p.T;
-  // key tiles of the 128 positions from q0 + 128 t on: [first[t], last[t]]; none when the pass has no such rows
-  int first[NQ], last[NQ], lo = 1 << 30, hi = -1;
+  // key tiles of the 128 positions from q0 + 128 t on: 0 .. last[t]; none when the pass has no such rows
+  int last[NQ], hi = -1;
 #pragma unroll
   for (int t = 0; t < NQ; ++t) {
     const int r0 = q0 + 128 * t, r1 = (r0 + 128 < p.rows ? r0 + 128 : p.rows) - 1;
-    const int k0 = p.window > 0 && p.start_pos + r0 - p.window + 1 > 0 ? p.start_pos + r0 - p.window + 1 : 0;
-    first[t] = r1 >= r0 ? k0 / KT : 1 << 30;
     last[t] = r1 >= r0 ? (p.start_pos + r1) / KT : -1;
-    lo = first[t] < lo ? first[t] : lo;
     hi = last[t] > hi ? last[t] : hi;
   }
 
@@ -114,7 +108,7 @@ prefill_flash_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     fence_barrier_init();
   }
   if (warp == 1) {
-    tmem_alloc(&tail->tmem_base, 512);
+    tmem_alloc(&tail->tmem_base, F::kTmemCols);
     tmem_relinquish();
   }
   tcgen05_fence_before();
@@ -132,7 +126,7 @@ prefill_flash_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     }
     int s = 0;
     uint32_t phase = 1;
-    for (int j = lo; j <= hi; ++j) {
+    for (int j = 0; j <= hi; ++j) {
       mbar_wait(&tail->empty[s], phase);
       if (issuer) {
         uint8_t* st = ring + s * 2 * F::kTileBytes;
@@ -151,86 +145,90 @@ prefill_flash_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     const uint32_t idesc_s = umma_idesc_bf16(128, KT), idesc_o = umma_idesc_bf16(128, D) | kIdescBMajorMN;
     const uint64_t dq = umma_desc_sw128(sq), dk = umma_desc_sw128(ring);
     const uint32_t ring_addr = smem_u32(ring);
-    // S of Q tile t from the K tile of `stage`, into the TMEM buffer `buf`
-    auto issue_s = [&](int t, int stage, int buf) {
+    // S of Q tile t from the K tile of `stage`
+    auto issue_s = [&](int t, int stage) {
       if (!issuer) return;
 #pragma unroll
       for (int c = 0; c < CH; ++c)
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
-          umma_bf16(tmem + buf * KT, dq + uint64_t((t * F::kQBytes + c * 16384 + kk * 32) >> 4), dk + uint64_t((stage * 2 * F::kTileBytes + c * KT * 128 + kk * 32) >> 4),
+          umma_bf16(tmem + t * KT, dq + uint64_t((t * F::kQBytes + c * 16384 + kk * 32) >> 4), dk + uint64_t((stage * 2 * F::kTileBytes + c * KT * 128 + kk * 32) >> 4),
                     idesc_s, uint32_t((c | kk) != 0));
-      umma_commit(&tail->s_full[buf]);
+      umma_commit(&tail->s_full[t]);
     };
-    // O of Q tile t += P (over S in buffer `buf`) times the V tile of `stage`
-    auto issue_o = [&](int t, int stage, int buf, bool start) {
+    // O of Q tile t += P (over its S) times the V tile of `stage`
+    auto issue_o = [&](int t, int stage, bool start) {
       if (!issuer) return;
 #pragma unroll
       for (int kk = 0; kk < KT / 16; ++kk)
-        umma_bf16_ts(tmem + F::kOCol + t * D, tmem + buf * KT + kk * 8, umma_desc_sw128_mn(ring_addr + stage * 2 * F::kTileBytes + F::kTileBytes + kk * 2048, KT * 128), idesc_o,
+        umma_bf16_ts(tmem + F::kOCol + t * D, tmem + t * KT + kk * 8, umma_desc_sw128_mn(ring_addr + stage * 2 * F::kTileBytes + F::kTileBytes + kk * 2048, KT * 128), idesc_o,
                      uint32_t(!start || kk != 0));
     };
     mbar_wait(&tail->q_full, 0);
     int s = 0;
-    uint32_t par = 0, seen[2] = {0, 0};  // seen[b]: parity of the next P in buffer b
-    if (lo <= hi) {
+    uint32_t par = 0;
+    if (hi >= 0) {
       mbar_wait(&tail->k_full[0], 0);
       tcgen05_fence_after();
 #pragma unroll
       for (int t = 0; t < NQ; ++t)
-        if (first[t] == lo) issue_s(t, 0, NQ == 2 ? t : 0);
+        if (last[t] >= 0) issue_s(t, 0);
     }
-    for (int j = lo; j <= hi; ++j) {
+    for (int j = 0; j <= hi; ++j) {
       const int s1 = s + 1 == F::kStages ? 0 : s + 1;
       const uint32_t par1 = s1 == 0 ? par ^ 1 : par;
       if (j < hi) {
         mbar_wait(&tail->k_full[s1], par1);
         tcgen05_fence_after();
-        if (NQ == 1) issue_s(0, s1, (j + 1 - lo) & 1);  // under this tile's softmax
+      }
+      mbar_wait(&tail->v_full[s], par);
+      const int beyond = p.start_pos + p.rows - j * KT;  // the tile's first key that the prompt does not have
+      if (beyond < KT) {                                 // rows of no key may hold anything, and 0 * NaN is not 0
+        uint8_t* v = ring + s * 2 * F::kTileBytes + F::kTileBytes;
+        for (int c = 0; c < CH; ++c)
+          for (int b = beyond * 128 + lane * 16; b < KT * 128; b += 512) *reinterpret_cast<uint4*>(v + c * KT * 128 + b) = make_uint4(0, 0, 0, 0);
+        fence_proxy_async();
+        __syncwarp();
       }
 #pragma unroll
       for (int t = 0; t < NQ; ++t) {
-        const int buf = NQ == 2 ? t : (j - lo) & 1;
-        if (j >= first[t] && j <= last[t]) {
-          mbar_wait(&tail->p_ready[buf], seen[buf]);
-          seen[buf] ^= 1;
-          mbar_wait(&tail->v_full[s], par);
+        if (j <= last[t]) {
+          mbar_wait(&tail->p_ready[t], j & 1);
           tcgen05_fence_after();
-          issue_o(t, s, buf, j == first[t]);
-          if (issuer && (NQ == 1 || j == last[t])) umma_commit(&tail->o_done[t]);
+          issue_o(t, s, j == 0);
+          if (issuer && j == last[t]) umma_commit(&tail->o_done[t]);
         }
-        if (NQ == 2 && j < hi && j + 1 >= first[t] && j + 1 <= last[t]) issue_s(t, s1, t);
+        if (j < last[t]) issue_s(t, s1);
       }
       if (issuer) umma_commit(&tail->empty[s]);
       s = s1;
       par = par1;
     }
     // the commits to the ring's barriers have to be in before the CTA may leave
-    const int n = hi - lo + 1, tail_n = n < F::kStages ? (n > 0 ? n : 0) : F::kStages;
+    const int tail_n = hi + 1 < F::kStages ? hi + 1 : F::kStages;
     for (int i = 0; i < tail_n; ++i) {
       if (s == 0) s = F::kStages, par ^= 1;
       --s;
       mbar_wait(&tail->empty[s], par);
     }
   } else {
-    const int t = NQ == 2 ? (warp - 2) >> 2 : 0, quarter = warp & 3;
+    const int t = (warp - 2) >> 2, quarter = warp & 3;
     const int row = q0 + 128 * t + quarter * 32 + lane, pos = p.start_pos + row;
-    const int pos_lo = p.start_pos + q0 + 128 * t + quarter * 32, pos_hi = pos_lo + 31;  // of the warp
+    const int pos_lo = p.start_pos + q0 + 128 * t + quarter * 32;  // the warp's first position
     const uint32_t lanes = tmem + (uint32_t(quarter * 32) << 16), acc = lanes + F::kOCol + t * D;
     float m = -INFINITY, l = 0.0f;  // the maximum that the accumulator stands at (times log2 e), the sum
-    int f = 0, la = -1;
+    int la = -1;
 #pragma unroll
     for (int i = 0; i < NQ; ++i)
-      if (i == t) f = first[i], la = last[i];
-    for (int j = f; j <= la; ++j) {
-      const int i = j - f, buf = NQ == 2 ? t : i & 1;
-      mbar_wait(&tail->s_full[buf], NQ == 2 ? (i & 1) : ((i >> 1) & 1));
+      if (i == t) la = last[i];
+    for (int j = 0; j <= la; ++j) {
+      mbar_wait(&tail->s_full[t], j & 1);
       tcgen05_fence_after();
       float x[KT];
       {
         uint32_t raw[KT / 32][32];
 #pragma unroll
-        for (int c = 0; c < KT / 32; ++c) tmem_ld_x32(lanes + buf * KT + c * 32, raw[c]);
+        for (int c = 0; c < KT / 32; ++c) tmem_ld_x32(lanes + t * KT + c * 32, raw[c]);
         tmem_wait_ld();
 #pragma unroll
         for (int c = 0; c < KT; ++c) x[c] = __uint_as_float(raw[c / 32][c % 32]);
@@ -240,11 +238,11 @@ prefill_flash_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         for (int c = 0; c < KT; ++c) x[c] = tanhf(x[c] / p.softcap) * p.softcap;
       }
       const int key0 = j * KT;
-      if (key0 + KT - 1 > pos_lo || (p.window > 0 && key0 <= pos_hi - p.window)) {  // (uniform in the warp)
-        const int over = pos - key0, under = p.window > 0 ? pos - p.window - key0 : -1;  // keys key0 + c with under < c <= over are seen
+      if (key0 + KT - 1 > pos_lo) {  // (uniform in the warp)
+        const int over = pos - key0;
 #pragma unroll
         for (int c = 0; c < KT; ++c)
-          if (c > over || c <= under) x[c] = -INFINITY;
+          if (c > over) x[c] = -INFINITY;
       }
       float mx0 = x[0], mx1 = x[1], mx2 = x[2], mx3 = x[3];
 #pragma unroll
@@ -259,44 +257,40 @@ prefill_flash_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         const float fix = m_new == -INFINITY ? 1.0f : flash_ex2(m - m_new);
         l *= fix;
         m = m_new;
-        if (i > 0) {  // the accumulator holds the tiles before: they are complete (NQ = 2: s_full came after them in order)
-          if (NQ == 1) {
-            mbar_wait(&tail->o_done[0], (i - 1) & 1);
-            tcgen05_fence_after();
-          }
+        if (j > 0) {  // the accumulator holds the tiles before: they are complete (s_full came after them in order)
 #pragma unroll 1
-          for (int c = 0; c < D; c += 32) {
-            uint32_t o[32];
-            tmem_ld_x32(acc + c, o);
-            tmem_wait_ld();
+          for (int c = 0; c < D; c += 16) {
+            float o[16];
+            tmem_ld_x16(acc + c, o);
+            uint32_t w[16];
 #pragma unroll
-            for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * fix);
-            tmem_st_x32(acc + c, o);
+            for (int e = 0; e < 16; ++e) w[e] = __float_as_uint(o[e] * fix);
+            tmem_st_x16(acc + c, w);
           }
         }
       }
       const float ms = m == -INFINITY ? 0.0f : m;
       float l0 = 0.0f, l1 = 0.0f;
 #pragma unroll
-      for (int c = 0; c < KT; c += 64) {
-        uint32_t pk[32];
+      for (int c = 0; c < KT; c += 32) {
+        uint32_t pk[16];
 #pragma unroll
-        for (int e = 0; e < 32; ++e) {
+        for (int e = 0; e < 16; ++e) {
           const float p0 = flash_ex2(fmaf(x[c + 2 * e], kPfLog2e, -ms)), p1 = flash_ex2(fmaf(x[c + 2 * e + 1], kPfLog2e, -ms));
           l0 += p0;
           l1 += p1;
           pk[e] = pack_bf16x2(p0, p1);
         }
-        tmem_st_x32(lanes + buf * KT + c / 2, pk);
+        tmem_st_x16(lanes + t * KT + c / 2, pk);
       }
       l += l0 + l1;
       tmem_wait_st();
       tcgen05_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&tail->p_ready[buf]);
+      if (lane == 0) mbar_arrive(&tail->p_ready[t]);
     }
-    if (la >= f) {
-      mbar_wait(&tail->o_done[t], NQ == 2 ? 0 : ((la - f) & 1));
+    if (la >= 0) {
+      mbar_wait(&tail->o_done[t], 0);
       tcgen05_fence_after();
       const float inv = 1.0f / l;
       bf16* out = p.out + (long long)row * p.hq * D + (long long)head * D;
@@ -320,7 +314,7 @@ prefill_flash_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
-  if (warp == 1) tmem_dealloc(tmem, 512);
+  if (warp == 1) tmem_dealloc(tmem, F::kTmemCols);
 }
 
 }  // namespace mtx

@@ -296,10 +296,7 @@ paged_flash_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       if constexpr (KT == 64) {
         tmem_st_x32(p_col, pk);
       } else {
-        asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};" ::"r"(pk[0]), "r"(pk[1]),
-                     "r"(pk[2]), "r"(pk[3]), "r"(pk[4]), "r"(pk[5]), "r"(pk[6]), "r"(pk[7]), "r"(pk[8]), "r"(pk[9]), "r"(pk[10]), "r"(pk[11]), "r"(pk[12]), "r"(pk[13]),
-                     "r"(pk[14]), "r"(pk[15]), "r"(p_col)
-                     : "memory");
+        tmem_st_x16(p_col, pk);
       }
       tmem_wait_st();
       tcgen05_fence_before();
