@@ -1813,7 +1813,7 @@ int mtx_sample_logits(mtx_engine* e, const float* logits, int rows, long long ld
   sa.out_raw = e->part_raw;
   sa.out_max = e->part_max;
   sa.out_sum = e->part_sum;
-  MTX_TRY(launch(sample_rows_kernel, dim3(rows), dim3(kSampleThreads), 0, st, sa));
+  MTX_TRY(launch(sa.mode < MTX_SAMPLE_NUCLEUS ? pick_rows_kernel : sample_rows_kernel, dim3(rows), dim3(kSampleThreads), 0, st, sa));
   FinalizeArgs fa;
   memset(&fa, 0, sizeof(fa));
   fa.part_score = e->part_score;
@@ -1858,7 +1858,7 @@ int mtx_sample_rows(const float* logits, int rows, long long ld, int vocab, int 
   sa.out_raw = f + 2 * size_t(rows);
   sa.out_max = f + 3 * size_t(rows);
   sa.out_sum = f + 4 * size_t(rows);
-  MTX_TRY(launch(sample_rows_kernel, dim3(rows), dim3(kSampleThreads), 0, st, sa));
+  MTX_TRY(launch(sa.mode < MTX_SAMPLE_NUCLEUS ? pick_rows_kernel : sample_rows_kernel, dim3(rows), dim3(kSampleThreads), 0, st, sa));
   FinalizeArgs fa;
   memset(&fa, 0, sizeof(fa));
   fa.part_score = sa.out_score;
