@@ -78,6 +78,18 @@ def design_module(config):
   raise ValueError(f"decoder_block={config.decoder_block!r} is not a layered design")
 
 
+def _token_array(tokens) -> np.ndarray:
+  """[n] int32 of a sequence of tokens (a list of 4096 Python integers through the descriptor's loops cost 1.2 ms before the first launch)."""
+  a = np.asarray(tokens)
+  if a.dtype.kind not in "iu" or a.ndim != 1:
+    a = np.array([int(t) for t in tokens], dtype=np.int64)
+  if a.dtype != np.int32:
+    if a.min() < -(2**31) or a.max() >= 2**31:
+      raise RuntimeError("a token cannot be converted to int32 without overflow")
+    a = a.astype(np.int32)
+  return a
+
+
 class LayeredParams:
   """Device-resident weights of a layered model: one entry per layer RUN of the plan (a layer that runs several times is listed
   once per run; the runs share the device copy of every tensor that is the same host tensor)."""
@@ -434,7 +446,8 @@ class LayeredEngine(MaxEngine):
     logits [n, vocab] (fp32, on the device) in the order of the entries.  Steps longer than max_step_rows run in slices."""
     self._require_params(None)
     B, V = self.max_concurrent_decodes, int(self.config.vocab_size)
-    tok, grp, pos, want, runs = [], [], [], [], []
+    tok, grp, pos, want, runs, rows = [], [], [], [], [], 0
+    slots, lengths = [], []
     ps = self.page_state
     seen = set()
     for slot, tokens, wanted in entries:
@@ -446,37 +459,36 @@ class LayeredEngine(MaxEngine):
       if n == 0:
         continue
       start = int(ps.sequence_lengths[slot])
-      new = self.page_manager.extend_pages(ps, slot, start + n)
-      if int(new.sequence_lengths[slot]) != start + n:
-        raise ValueError(f"slot {slot}: the page pool cannot hold {start + n} tokens")
-      ps = new
-      base = len(tok)
-      runs.append((base, base + n))
-      tok.extend(int(t) for t in tokens)
-      grp.extend([slot] * n)
-      pos.extend(range(start, start + n))
+      slots.append(slot)
+      lengths.append(start + n)
+      base = rows
+      rows += n
+      runs.append((base, rows))
+      tok.append(_token_array(tokens))
+      grp.append(np.full(n, slot, np.int32))
+      pos.append(np.arange(start, start + n, dtype=np.int32))
       for w in wanted:
         if not 0 <= int(w) < n:
           raise ValueError(f"slot {slot}: wanted index {w} outside its {n} tokens")
         want.append(base + int(w))
+    ps, failed = self.page_manager.extend_pages_of(ps, slots, lengths)
+    if failed >= 0:
+      raise ValueError(f"slot {slots[failed]}: the page pool cannot hold {lengths[failed]} tokens")
     self.page_state = ps
     self._upload_page_map()
-    rows = len(tok)
     out = torch.empty(len(want), V, dtype=torch.float32, device=self.device)
     if rows == 0:
       return out
     R = self._max_rows
+    desc = np.stack([np.concatenate(x) for x in (tok, grp, pos)])
+    host = self._desc_host.numpy()
     done_want = 0
     for lo in range(0, rows, R):
       hi = min(rows, lo + R)
       n = hi - lo
       w = [x - lo for x in want if lo <= x < hi]
-      host = self._desc_host
-      host[0:n] = torch.tensor(tok[lo:hi], dtype=torch.int32)
-      host[R : R + n] = torch.tensor(grp[lo:hi], dtype=torch.int32)
-      host[2 * R : 2 * R + n] = torch.tensor(pos[lo:hi], dtype=torch.int32)
-      if w:
-        host[3 * R : 3 * R + len(w)] = torch.tensor(w, dtype=torch.int32)
+      host[: 3 * R].reshape(3, R)[:, :n] = desc[:, lo:hi]
+      host[3 * R : 3 * R + len(w)] = w
       # query tiles: every run of consecutive positions (an entry, cut at the slice) in pieces of at most 16 rows
       # and the runs themselves (recurrent mixers walk a run in order from its group's state)
       tiles, cuts = [], []
@@ -487,11 +499,11 @@ class LayeredEngine(MaxEngine):
         tiles.extend(range(a - lo, b - lo, QUERY_TILE_ROWS))
       tiles.append(n)
       cuts.append(n)
-      host[4 * R : 4 * R + len(tiles)] = torch.tensor(tiles, dtype=torch.int32)
-      host[5 * R + 8 : 5 * R + 8 + len(cuts)] = torch.tensor(cuts, dtype=torch.int32)
+      host[4 * R : 4 * R + len(tiles)] = tiles
+      host[5 * R + 8 : 5 * R + 8 + len(cuts)] = cuts
       if lo:
         torch.cuda.current_stream(self.device).synchronize()  # the previous slice has read the staging buffer
-      self._desc_dev.copy_(host, non_blocking=True)
+      self._desc_dev.copy_(self._desc_host, non_blocking=True)
       p = self._desc_dev.data_ptr()
       dst = out[done_want : done_want + len(w)]
       self._run(n, p, p + 4 * R, p + 8 * R, len(w), p + 12 * R, dst, len(tiles) - 1, p + 16 * R, n_runs=len(cuts) - 1, runs_ptr=p + 4 * (5 * R + 8))
@@ -533,7 +545,7 @@ class LayeredEngine(MaxEngine):
       self.release_pages(slot)
     if start + true_length >= int(self.config.max_target_length):
       raise ValueError(f"{start + true_length} prompt tokens leave no room to decode (max_target_length={self.config.max_target_length})")
-    logits = self.step([(slot, toks[:true_length].tolist(), [true_length - 1])])
+    logits = self.step([(slot, toks[:true_length].cpu().numpy(), [true_length - 1])])
     self._sample(logits, 1, self._first_token, self._first_log_prob if self.config.return_log_prob else None, 0x40000000)
     first = self._first_token.clone().reshape(1, 1)
     n = start + true_length

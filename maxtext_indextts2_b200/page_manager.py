@@ -11,6 +11,7 @@ it with jitted loops; the state is a few hundred integers, so here it is numpy o
 from __future__ import annotations
 
 import dataclasses
+from typing import Sequence, Tuple
 
 import numpy as np
 
@@ -134,6 +135,42 @@ def _extend_pages_for_group(state: PageState, group: int, new_length: int, token
   )
 
 
+def _extend_pages_for_groups(state: PageState, groups: np.ndarray, new_lengths: np.ndarray, tokens_per_page: int, max_pages_per_group: int) -> Tuple[PageState, int]:
+  """`_extend_pages_for_group` for several different groups in turn, with one copy of the state.  Returns the new state and -1, or the state unchanged
+  and the index of the first group that the pool (or its row of the page map) cannot hold."""
+  needed = (new_lengths + tokens_per_page - 1) // tokens_per_page
+  used = state.num_pages_used[groups]
+  extra = np.maximum(needed - used, 0)
+  status, page_map, n_used = state.page_status, state.page_map, state.num_pages_used
+  ends = np.cumsum(extra)
+  free = np.flatnonzero(status[1:] == 0) + 1 if ends[-1] else ends[:0]
+  failed = (needed > max_pages_per_group) | ((extra > 0) & (ends > free.size))
+  if failed.any():
+    return state, int(np.argmax(failed))
+  if ends[-1]:
+    take = free[: ends[-1]].astype(np.int32)
+    status, page_map, n_used = status.copy(), page_map.copy(), n_used.copy()
+    status[take] = 1
+    for i in np.flatnonzero(extra):
+      page_map[groups[i], used[i] : needed[i]] = take[ends[i] - extra[i] : ends[i]]
+    n_used[groups] = np.maximum(used, needed)
+
+  def with_values(a, values):
+    a = a.copy()
+    a[groups] = values
+    return a
+
+  return state.replace(
+      page_status=status,
+      page_map=page_map,
+      num_pages_used=n_used,
+      sequence_lengths=with_values(state.sequence_lengths, new_lengths),
+      active_page=with_values(state.active_page, np.where(needed > 0, page_map[groups, needed - 1], 0)),
+      has_active_page=with_values(state.has_active_page, True),
+      active_page_position=with_values(state.active_page_position, new_lengths % tokens_per_page),
+  ), -1
+
+
 def _update_decode_pages_global(state: PageState, tokens_per_page: int, max_pages_per_group: int) -> PageState:
   """page_manager.py:332-412: one more token for every active group; groups that crossed a page boundary get the lowest
   free page, in group order, while free pages last."""
@@ -203,6 +240,18 @@ class PageManager:
     if new_length < int(page_state.sequence_lengths[page_group_id]) or new_length > self.max_target_length:
       raise ValueError(f"PageManager: new_length ({new_length}) out of range [{int(page_state.sequence_lengths[page_group_id])}, {self.max_target_length}]")
     return _extend_pages_for_group(page_state, page_group_id, int(new_length), self.tokens_per_page, self.max_pages_per_group)
+
+  def extend_pages_of(self, page_state: PageState, page_group_ids: Sequence[int], new_lengths: Sequence[int]) -> Tuple[PageState, int]:
+    """`extend_pages` for several different groups (one mixed batch).  Returns the new state and -1, or the state unchanged and the index of the first
+    group that does not fit."""
+    for g, n in zip(page_group_ids, new_lengths):
+      if g < 0 or g >= self.max_page_groups:
+        raise ValueError(f"PageManager: page_group_id ({g}) out of range [0, {self.max_page_groups})")
+      if n < int(page_state.sequence_lengths[g]) or n > self.max_target_length:
+        raise ValueError(f"PageManager: new_length ({n}) out of range [{int(page_state.sequence_lengths[g])}, {self.max_target_length}]")
+    if not len(page_group_ids):
+      return page_state, -1
+    return _extend_pages_for_groups(page_state, np.asarray(page_group_ids), np.asarray(new_lengths), self.tokens_per_page, self.max_pages_per_group)
 
   def update_decode_pages(self, page_state: PageState) -> PageState:
     """:538-563."""
