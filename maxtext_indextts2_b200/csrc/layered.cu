@@ -409,60 +409,87 @@ int launch_window_mma_t(const WindowAttnArgs<bf16>& wa, const WindowMmaExtra& x,
   return launch(window_attention_mma_kernel<HPW, DVT>, dim3(x.n_tiles, x.splits), dim3(kWmmaThreads), smem, st, wa, x);
 }
 
-// the tensor-core mixer: (query tile, key split) work items, then the sum over the splits
-int launch_window_mma(mtx_layered* e, const WindowAttnArgs<bf16>& wa, const WindowMmaPlan& plan, const mtx_ragged_batch& b, cudaStream_t st) {
-  WindowMmaExtra x;
-  x.tile_row0 = b.tile_row0;
-  x.partial = e->attn_part;
-  x.n_tiles = b.n_tiles;
-  x.bn = plan.bn;
-  x.hg = plan.hg;
+// key splits of the tensor-core mixer: enough work items to fill the SMs (one CTA each), at least two key tiles per split, and among the next few
+// counts the one whose last wave is fullest (256 tiles x 2 splits on 148 SMs leave the fourth wave half empty; x 4 fill seven waves)
+int window_mma_splits(const mtx_layered* e, const WindowAttnArgs<bf16>& wa, const WindowMmaPlan& plan, int tiles) {
   const int key_tiles = (wa.window + kWmmaRows - 1 + plan.bn - 1) / plan.bn;  // most key tiles a query tile can have
-  // key splits: enough work items to fill the SMs (one CTA each), at least two key tiles per split, and among the next few counts
-  // the one whose last wave is fullest (256 tiles x 2 splits on 148 SMs leave the fourth wave half empty; x 4 fill seven waves)
   int cap = key_tiles / 2;
   if (size_t(cap) * wa.rows > e->attn_part_rows) cap = int(e->attn_part_rows / wa.rows);
   if (cap < 1) cap = 1;
-  int lo = (e->num_sms + b.n_tiles - 1) / b.n_tiles;
+  int lo = (e->num_sms + tiles - 1) / tiles;
   if (lo > cap) lo = cap;
   int splits = lo;
   double best = 0.0;
   for (int sp = lo; sp <= cap && sp < lo + 8; ++sp) {
-    const double waves = double(b.n_tiles) * sp / e->num_sms, eff = waves / std::ceil(waves);
+    const double waves = double(tiles) * sp / e->num_sms, eff = waves / std::ceil(waves);
     if (eff > best + 0.02) {
       best = eff;
       splits = sp;
     }
   }
-  x.splits = splits;
-  int rc = MTX_ERR_UNSUPPORTED;
-  if (plan.hpw == 1 && plan.dvt == 8) rc = launch_window_mma_t<1, 8>(wa, x, plan.smem, st);
-  else if (plan.hpw == 1 && plan.dvt == 16) rc = launch_window_mma_t<1, 16>(wa, x, plan.smem, st);
-  else if (plan.hpw == 1 && plan.dvt == 32) rc = launch_window_mma_t<1, 32>(wa, x, plan.smem, st);
-  else if (plan.hpw == 2 && plan.dvt == 8) rc = launch_window_mma_t<2, 8>(wa, x, plan.smem, st);
-  else if (plan.hpw == 2 && plan.dvt == 16) rc = launch_window_mma_t<2, 16>(wa, x, plan.smem, st);
-  MTX_TRY(rc);
+  return splits;
+}
+
+int sum_window_partials(mtx_layered* e, const WindowAttnArgs<bf16>& wa, int splits, cudaStream_t st) {
   const long long per_split = (long long)wa.rows * wa.heads * wa.vdim;
   long long blocks = (per_split / 2 + 255) / 256;
   if (blocks > 148 * 8) blocks = 148 * 8;
   return launch(window_partial_sum_kernel, dim3(unsigned(blocks)), dim3(256), 0, st, (const float*)e->attn_part, wa.out, splits, per_split);
 }
 
+// the tensor-core mixer's partial results: (query tile, key split) work items
+int launch_window_mma_parts(mtx_layered* e, const WindowAttnArgs<bf16>& wa, const WindowMmaPlan& plan, const mtx_ragged_batch& b, int splits, int skip_single,
+                            cudaStream_t st) {
+  WindowMmaExtra x;
+  x.tile_row0 = b.tile_row0;
+  x.partial = e->attn_part;
+  x.n_tiles = b.n_tiles;
+  x.bn = plan.bn;
+  x.hg = plan.hg;
+  x.splits = splits;
+  x.skip_single = skip_single;
+  if (plan.hpw == 1 && plan.dvt == 8) return launch_window_mma_t<1, 8>(wa, x, plan.smem, st);
+  if (plan.hpw == 1 && plan.dvt == 16) return launch_window_mma_t<1, 16>(wa, x, plan.smem, st);
+  if (plan.hpw == 1 && plan.dvt == 32) return launch_window_mma_t<1, 32>(wa, x, plan.smem, st);
+  if (plan.hpw == 2 && plan.dvt == 8) return launch_window_mma_t<2, 8>(wa, x, plan.smem, st);
+  if (plan.hpw == 2 && plan.dvt == 16) return launch_window_mma_t<2, 16>(wa, x, plan.smem, st);
+  return MTX_ERR_UNSUPPORTED;
+}
+
+// ... then the sum over the splits
+int launch_window_mma(mtx_layered* e, const WindowAttnArgs<bf16>& wa, const WindowMmaPlan& plan, const mtx_ragged_batch& b, cudaStream_t st) {
+  const int splits = window_mma_splits(e, wa, plan, b.n_tiles);
+  MTX_TRY(launch_window_mma_parts(e, wa, plan, b, splits, 0, st));
+  return sum_window_partials(e, wa, splits, st);
+}
+
 template <int CPW, int DT>
-int launch_window_decode_t(const WindowAttnArgs<bf16>& wa, const WindowDecodeExtra& x, size_t smem, cudaStream_t st) {
+int launch_window_decode_t(const WindowAttnArgs<bf16>& wa, const WindowDecodeExtra& x, int items, size_t smem, cudaStream_t st) {
   static size_t have = 0;  // per instantiation
   if (smem > have) {
     MTX_CUDA(cudaFuncSetAttribute(window_attention_decode_kernel<CPW, DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     have = smem;
   }
-  return launch(window_attention_decode_kernel<CPW, DT>, dim3(wa.rows, x.splits), dim3(kWdecThreads), smem, st, wa, x);
+  return launch(window_attention_decode_kernel<CPW, DT>, dim3(items, x.splits), dim3(kWdecThreads), smem, st, wa, x);
 }
 
-// the decode mixer (every row a token of its own sequence): (row, key split) work items, then the sum over the splits
-int launch_window_decode(mtx_layered* e, const WindowAttnArgs<bf16>& wa, const WindowDecodePlan& plan, cudaStream_t st) {
+// the decode mixer's partial results: (row, key split) work items; tile_row0: of the single-row tiles only
+int launch_window_decode_parts(mtx_layered* e, const WindowAttnArgs<bf16>& wa, const WindowDecodePlan& plan, const int* tile_row0, int items, int splits, cudaStream_t st) {
   WindowDecodeExtra x;
   x.partial = e->attn_part;
   x.stages = plan.stages;
+  x.splits = splits;
+  x.tile_row0 = tile_row0;
+  if (plan.cpw == 1 && plan.dt == 4) return launch_window_decode_t<1, 4>(wa, x, items, plan.smem, st);
+  if (plan.cpw == 1 && plan.dt == 8) return launch_window_decode_t<1, 8>(wa, x, items, plan.smem, st);
+  if (plan.cpw == 1 && plan.dt == 16) return launch_window_decode_t<1, 16>(wa, x, items, plan.smem, st);
+  if (plan.cpw == 2 && plan.dt == 4) return launch_window_decode_t<2, 4>(wa, x, items, plan.smem, st);
+  if (plan.cpw == 2 && plan.dt == 8) return launch_window_decode_t<2, 8>(wa, x, items, plan.smem, st);
+  return MTX_ERR_UNSUPPORTED;
+}
+
+// the decode mixer (every row a token of its own sequence), then the sum over the splits
+int launch_window_decode(mtx_layered* e, const WindowAttnArgs<bf16>& wa, const WindowDecodePlan& plan, cudaStream_t st) {
   const int key_tiles = (wa.window + kWdecKeys - 1) / kWdecKeys;
   // one wave: as many work items as CTAs fit on the GPU at once (a split's start-up -- its first tile's latency, the staging of
   // the queries -- is worth several tiles, so more and shorter splits lose), at least four key tiles per split
@@ -472,18 +499,19 @@ int launch_window_decode(mtx_layered* e, const WindowAttnArgs<bf16>& wa, const W
   if (splits > key_tiles / 4) splits = key_tiles / 4;
   if (size_t(splits) * wa.rows > e->attn_part_rows) splits = int(e->attn_part_rows / wa.rows);
   if (splits < 1) splits = 1;
-  x.splits = splits;
-  int rc = MTX_ERR_UNSUPPORTED;
-  if (plan.cpw == 1 && plan.dt == 4) rc = launch_window_decode_t<1, 4>(wa, x, plan.smem, st);
-  else if (plan.cpw == 1 && plan.dt == 8) rc = launch_window_decode_t<1, 8>(wa, x, plan.smem, st);
-  else if (plan.cpw == 1 && plan.dt == 16) rc = launch_window_decode_t<1, 16>(wa, x, plan.smem, st);
-  else if (plan.cpw == 2 && plan.dt == 4) rc = launch_window_decode_t<2, 4>(wa, x, plan.smem, st);
-  else if (plan.cpw == 2 && plan.dt == 8) rc = launch_window_decode_t<2, 8>(wa, x, plan.smem, st);
-  MTX_TRY(rc);
-  const long long per_split = (long long)wa.rows * wa.heads * wa.vdim;
-  long long blocks = (per_split / 2 + 255) / 256;
-  if (blocks > 148 * 8) blocks = 148 * 8;
-  return launch(window_partial_sum_kernel, dim3(unsigned(blocks)), dim3(256), 0, st, (const float*)e->attn_part, wa.out, splits, per_split);
+  MTX_TRY(launch_window_decode_parts(e, wa, plan, nullptr, wa.rows, splits, st));
+  return sum_window_partials(e, wa, splits, st);
+}
+
+// A mixed batch: the single tokens on the decode mixer, the tiles of prompts on the other, one sum.  A tile of one row leaves 15 of the MMA's 16 rows,
+// and of the sigmoids and the mixing, to padding, over as many keys as its sequence has: 500 rows of one prompt and 31 single tokens with
+// contexts up to 1024 took 213 us, 130 so.
+int launch_window_mixed(mtx_layered* e, const WindowAttnArgs<bf16>& wa, const WindowMmaPlan& plan, const WindowDecodePlan& dplan, const mtx_ragged_batch& b, int prompt_tiles,
+                        cudaStream_t st) {
+  const int splits = window_mma_splits(e, wa, plan, prompt_tiles);
+  MTX_TRY(launch_window_decode_parts(e, wa, dplan, b.tile_row0, b.n_tiles, splits, st));
+  MTX_TRY(launch_window_mma_parts(e, wa, plan, b, splits, 1, st));
+  return sum_window_partials(e, wa, splits, st);
 }
 
 bool use_window_decode() {
@@ -564,7 +592,11 @@ int window_layer(mtx_layered* e, int li, const mtx_ragged_batch& b, cudaStream_t
       MTX_TRY(launch_window_decode(e, wa, dplan, st));
       done = true;
     } else if (plan.ok && b.n_tiles > 0 && b.tile_row0 != nullptr && use_window_mma()) {
-      MTX_TRY(launch_window_mma(e, wa, plan, b, st));
+      // tiles of several rows: at least this many (the host does not see the table), single tokens at most the rest.  From four of them on the second
+      // kernel's start-up is paid for.
+      const int prompt_tiles = (rows - b.n_tiles + kWmmaRows - 2) / (kWmmaRows - 1);
+      if (dplan.ok && use_window_decode() && prompt_tiles > 0 && b.n_tiles - prompt_tiles >= 4) MTX_TRY(launch_window_mixed(e, wa, plan, dplan, b, prompt_tiles, st));
+      else MTX_TRY(launch_window_mma(e, wa, plan, b, st));
       done = true;
     }
   }

@@ -23,6 +23,7 @@ constexpr int kWdecKeys = 16;
 struct WindowDecodeExtra {
   float* partial;  // [splits, rows, H * dv]
   int splits, stages;
+  const int* tile_row0;  // mixed batches: blockIdx.x is a query tile of this table, those of several rows are left out; null: blockIdx.x is a row
 };
 
 inline size_t window_decode_tile_bytes(int kv_heads, int dim, int vdim) {
@@ -59,7 +60,8 @@ __global__ void __launch_bounds__(kWdecThreads) window_attention_decode_kernel(c
   int* sSlot = reinterpret_cast<int*>(sPb + H);          // [H] row of sP that holds head h: (h / rep) * 8 + h % rep
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g4 = lane >> 2, t4 = lane & 3;
   griddep_wait();
-  const int r = blockIdx.x, split = blockIdx.y;
+  const int r = x.tile_row0 ? x.tile_row0[blockIdx.x] : int(blockIdx.x), split = blockIdx.y;
+  if (x.tile_row0 && x.tile_row0[blockIdx.x + 1] - r != 1) return;
   const int i = a.pos[r], grp = a.group[r];
   const int klo = i - a.window + 1 > 0 ? i - a.window + 1 : 0;
   const int n_kt = (i - klo + kWdecKeys) / kWdecKeys, per = (n_kt + x.splits - 1) / x.splits;

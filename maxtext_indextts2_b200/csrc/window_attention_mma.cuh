@@ -26,6 +26,7 @@ struct WindowMmaExtra {
   const int* tile_row0;  // [n_tiles + 1]
   float* partial;        // [splits, rows, H * dv]
   int n_tiles, splits, bn;
+  int skip_single;  // 1: tiles of one row are left to window_attention_decode_kernel
   int hg;  // head groups of the S phase: 2 = two warps share a key group (bn = 32), each with half the heads; else 1
 };
 
@@ -75,6 +76,7 @@ __global__ void __launch_bounds__(kWmmaThreads, 1) window_attention_mma_kernel(c
   griddep_wait();
   const int tile = blockIdx.x, split = blockIdx.y;
   const int r0 = x.tile_row0[tile], nrows = x.tile_row0[tile + 1] - r0;
+  if (x.skip_single && nrows == 1) return;
   const int grp = a.group[r0], p0 = a.pos[r0];
   const int klo = p0 - a.window + 1 > 0 ? p0 - a.window + 1 : 0, khi = p0 + nrows - 1;
   const int n_kt = (khi - klo + BN) / BN, per = (n_kt + x.splits - 1) / x.splits;
