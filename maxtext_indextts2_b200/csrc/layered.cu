@@ -14,6 +14,7 @@
 #include "layer_ops.cuh"
 #include "linear_any.cuh"
 #include "linear_wide.cuh"
+#include "linear_stream.cuh"
 #include "grouped_gemm.cuh"
 #include "window_attention.cuh"
 #include "window_attention_mma.cuh"
@@ -180,6 +181,30 @@ __global__ void __launch_bounds__(256) bf16_cols_to_f32_kernel(bf16* src, float*
   }
 }
 
+// Few rows per product (at most a tile's 32): linear_stream.cuh.  Above, its 32-row tiles read the weights twice where linear_mma_kernel's read them
+// once.
+bool takes_stream(const LinArgs<bf16>& p, int rows_per_product) {
+  static const int on = env_int("MTX_LINEAR_STREAM", 1);
+  auto aligned = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+  return on && rows_per_product <= kLsBM && p.k % kLsBK == 0 && p.lda % 8 == 0 && p.w_group_stride % 8 == 0 && p.batch_a % 8 == 0 && aligned(p.a) && aligned(p.w);
+}
+
+template <int EPI, int BN>
+int launch_stream_t(const LinArgs<bf16>& p, int row_tiles, int products, cudaStream_t st) {
+  static bool attr_set = false;  // per instantiation
+  if (!attr_set) {
+    MTX_CUDA(cudaFuncSetAttribute(linear_stream_kernel<EPI, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ls_smem_bytes<BN>())));
+    attr_set = true;
+  }
+  return launch(linear_stream_kernel<EPI, BN>, dim3((p.n + BN - 1) / BN, row_tiles, products), dim3(kLsThreads), ls_smem_bytes<BN>(), st, p);
+}
+// (64-column tiles need one per SM: 2048 x 2048 for one row gives 32 of them)
+template <int EPI>
+int launch_stream(const LinArgs<bf16>& p, int row_tiles, int products, cudaStream_t st) {
+  const long long weights = p.group_off ? p.groups : products;
+  return (p.n + 63) / 64 * weights >= 148 ? launch_stream_t<EPI, 64>(p, row_tiles, products, st) : launch_stream_t<EPI, 32>(p, row_tiles, products, st);
+}
+
 // out (fp32, or the gated activation) = EPI(a[rows, k] . w[n, k]^T)
 template <typename T, int EPI>
 int run_linear(mtx_layered* e, const void* a, const void* w, const float* bias, float* out, void* act, int rows, int n, int k, cudaStream_t st,
@@ -202,7 +227,7 @@ int run_linear(mtx_layered* e, const void* a, const void* w, const float* bias, 
   p.k = k;
   const dim3 grid((n + 63) / 64, (rows + 63) / 64);
   if constexpr (sizeof(T) == 4) return launch(linear_f32_kernel<EPI>, grid, dim3(kLinF32Threads), 0, st, p);
-  else return launch(linear_mma_kernel<EPI>, grid, dim3(kLinThreads), 0, st, p);
+  else return takes_stream(p, rows) ? launch_stream<EPI>(p, 1, 1, st) : launch(linear_mma_kernel<EPI>, grid, dim3(kLinThreads), 0, st, p);
 }
 
 // (kind LIN_RELU2: max(., 0)^2; LIN_GELU: gelu_tanh(.); act has the row pitch ldo)
@@ -325,7 +350,7 @@ int linear_batched(const void* a, long long lda, long long batch_a, const void* 
   p.batch_o = batch_o;
   const dim3 grid((n + 63) / 64, (rows + 63) / 64, batches);
   if constexpr (sizeof(T) == 4) return launch(linear_f32_kernel<LIN_ACT>, grid, dim3(kLinF32Threads), 0, st, p);
-  else return launch(linear_mma_kernel<LIN_ACT>, grid, dim3(kLinThreads), 0, st, p);
+  else return takes_stream(p, rows) ? launch_stream<LIN_ACT>(p, 1, batches, st) : launch(linear_mma_kernel<LIN_ACT>, grid, dim3(kLinThreads), 0, st, p);
 }
 
 // one matrix product per group of slots (linear_any.cuh, grouped mode): slot ranges group_off [groups + 1] on the device, at most
@@ -367,6 +392,8 @@ int linear_grouped(const void* a, const int* a_row, const void* w, long long w_s
       const dim3 pgrid((n + kGgBN - 1) / kGgBN, (slots + kGgBM - 1) / kGgBM + groups, 1);
       return launch(grouped_mma_pipe_kernel<EPI>, pgrid, dim3(kGgThreads), kGgSmemBytes, st, p);
     }
+    // few tokens per expert: 256 slots of 16 experts, 2048 -> 2 x 1024 -> 2048, take 61 + 30 us on linear_mma_kernel, 44 + 24 so
+    if (packed && takes_stream(p, (slots + groups - 1) / groups)) return launch_stream<EPI>(p, (slots + kLsBM - 1) / kLsBM + groups, 1, st);
   }
   const dim3 grid((n + 63) / 64, packed ? (slots + 63) / 64 + groups : (slots + 63) / 64, packed ? 1 : groups);
   if constexpr (sizeof(T) == 4) return launch(linear_f32_kernel<EPI>, grid, dim3(kLinF32Threads), 0, st, p);
