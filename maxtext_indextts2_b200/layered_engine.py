@@ -80,8 +80,11 @@ def design_module(config):
 
 def _token_array(tokens) -> np.ndarray:
   """[n] int32 of a sequence of tokens (a list of 4096 Python integers through the descriptor's loops cost 1.2 ms before the first launch)."""
-  a = np.asarray(tokens)
-  if a.dtype.kind not in "iu" or a.ndim != 1:
+  try:
+    a = np.asarray(tokens)
+  except (TypeError, ValueError):  # (tensors on the device, or of types that numpy has not)
+    a = None
+  if a is None or a.dtype.kind not in "iu" or a.ndim != 1:
     a = np.array([int(t) for t in tokens], dtype=np.int64)
   if a.dtype != np.int32:
     if a.min() < -(2**31) or a.max() >= 2**31:
@@ -545,7 +548,8 @@ class LayeredEngine(MaxEngine):
       self.release_pages(slot)
     if start + true_length >= int(self.config.max_target_length):
       raise ValueError(f"{start + true_length} prompt tokens leave no room to decode (max_target_length={self.config.max_target_length})")
-    logits = self.step([(slot, toks[:true_length].cpu().numpy(), [true_length - 1])])
+    prompt = toks[:true_length].cpu()
+    logits = self.step([(slot, prompt.tolist() if prompt.is_floating_point() else prompt.numpy(), [true_length - 1])])
     self._sample(logits, 1, self._first_token, self._first_log_prob if self.config.return_log_prob else None, 0x40000000)
     first = self._first_token.clone().reshape(1, 1)
     n = start + true_length

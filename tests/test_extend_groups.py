@@ -4,6 +4,7 @@ import dataclasses
 import random
 
 import numpy as np
+import torch
 
 from maxtext_indextts2_b200 import layered_engine
 from maxtext_indextts2_b200 import page_manager as pm
@@ -39,6 +40,7 @@ def test_groups_at_once_against_in_turn():
 
 
 def test_token_arrays():
-  for tokens in ([3, 4, 5], (3, 4, 5), np.array([3, 4, 5]), np.array([3, 4, 5], np.int16), [3.7, 4.0, 5.2], np.array([3.0, 4.0, 5.0]), [np.int64(3), 4, 5]):
+  for tokens in ([3, 4, 5], (3, 4, 5), np.array([3, 4, 5]), np.array([3, 4, 5], np.int16), [3.7, 4.0, 5.2], np.array([3.0, 4.0, 5.0]), [np.int64(3), 4, 5],
+                 torch.tensor([3, 4, 5]), torch.tensor([3.0, 4.0, 5.0], dtype=torch.bfloat16), [torch.tensor(3), 4, 5]):
     a = layered_engine._token_array(tokens)
     assert a.dtype == np.int32 and a.tolist() == [3, 4, 5]
