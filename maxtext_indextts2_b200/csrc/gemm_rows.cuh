@@ -274,11 +274,22 @@ __device__ __forceinline__ void rows_logits_frag(const EpiArgs& e, int V, int r,
     if (n0 + j < V) {
       const float sc = e.gumbel ? lg[j] * e.inv_temp + gumbel_noise(seed, step, uint32_t(e.row_offset + r), uint32_t(e.vocab_offset + n0 + j)) : lg[j];
       if (sc > s.best) { s.best = sc; s.raw = lg[j]; s.bi = n0 + j; }  // ascending scan: strict > keeps the lowest index
-      if (e.want_lse) {
-        const float mn = fmaxf(s.mx, lg[j]);
-        s.sum = s.sum * __expf(s.mx - mn) + __expf(lg[j] - mn);
-        s.mx = mn;
-      }
+    }
+  }
+  if (e.want_lse) {
+    // one maximum for the 16 columns, then sixteen independent exponentials: with a running maximum per column the two exponentials of each waited for
+    // those of the one before (48 rows x 2560 x 262144: 268 us so, 251 like this, of 202 for the weights)
+    float mn = s.mx;
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+      if (n0 + j < V) mn = fmaxf(mn, lg[j]);
+    if (mn > -INFINITY) {
+      float t[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        if (n0 + j < V) t[j & 3] += __expf(lg[j] - mn);
+      s.sum = s.sum * __expf(s.mx - mn) + ((t[0] + t[1]) + (t[2] + t[3]));
+      s.mx = mn;
     }
   }
 }
