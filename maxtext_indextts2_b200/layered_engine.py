@@ -82,15 +82,11 @@ def _token_array(tokens) -> np.ndarray:
   """[n] int32 of a sequence of tokens (a list of 4096 Python integers through the descriptor's loops cost 1.2 ms before the first launch)."""
   try:
     a = np.asarray(tokens)
-  except (TypeError, ValueError):  # (tensors on the device, or of types that numpy has not)
+  except (TypeError, ValueError, RuntimeError):  # (tensors on the device, of types that numpy has not, or that require a gradient)
     a = None
-  if a is None or a.dtype.kind not in "iu" or a.ndim != 1:
-    a = np.array([int(t) for t in tokens], dtype=np.int64)
-  if a.dtype != np.int32:
-    if a.min() < -(2**31) or a.max() >= 2**31:
-      raise RuntimeError("a token cannot be converted to int32 without overflow")
-    a = a.astype(np.int32)
-  return a
+  if a is None or a.dtype.kind not in "iu" or a.ndim != 1 or a.min() < -(2**31) or a.max() >= 2**31:
+    return torch.tensor([int(t) for t in tokens], dtype=torch.int32).numpy()  # (which refuses what is no token)
+  return a.astype(np.int32, copy=False)
 
 
 class LayeredParams:

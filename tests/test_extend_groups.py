@@ -4,6 +4,7 @@ import dataclasses
 import random
 
 import numpy as np
+import pytest
 import torch
 
 from maxtext_indextts2_b200 import layered_engine
@@ -44,3 +45,16 @@ def test_token_arrays():
                  torch.tensor([3, 4, 5]), torch.tensor([3.0, 4.0, 5.0], dtype=torch.bfloat16), [torch.tensor(3), 4, 5]):
     a = layered_engine._token_array(tokens)
     assert a.dtype == np.int32 and a.tolist() == [3, 4, 5]
+
+
+def test_token_arrays_of_odd_forms():
+  """Whatever a loop of int() over the tokens takes, and its refusals."""
+  for tokens in (torch.tensor([3.0, 4.0, 5.0], requires_grad=True), ["3", "4", "5"], np.array([3, 4, 5], np.uint64), np.array([3, 4, 5], np.int32)[::1],
+                 np.array([3, 0, 4, 0, 5])[::2], np.array([3, 4, 5], object)):
+    a = layered_engine._token_array(tokens)
+    assert a.dtype == np.int32 and a.tolist() == [3, 4, 5]
+  for tokens in ([2**40], [-(2**31) - 1], [2**63], [2**70], [2**70, 3], [1e30], [float("nan")], [[1], [2]], [None], np.array([2**31])):
+    with pytest.raises(Exception) as old:
+      torch.tensor([int(t) for t in tokens], dtype=torch.int32)
+    with pytest.raises(type(old.value)):
+      layered_engine._token_array(tokens)
