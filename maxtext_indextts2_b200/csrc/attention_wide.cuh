@@ -300,7 +300,9 @@ decode_attn_wide_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
 // same rows -- tiles begin at the position's first key, and the windows of positions 64 apart begin 64 apart.  A tile that a column's
 // position does not see leaves the column alone (probabilities 0, factor 1), and a column's warps are merged in the order in which its own
 // tiles went to them, so that a position gets the bits that decode_attn_wide_kernel gives it with one work item per (position, kv head).
-// Positions before and behind the window's length begin their tiles at other offsets: a group of both is walked position by position.
+// Positions before and behind the window's length begin their tiles at other offsets: a group of both is walked position by position.  So is, once
+// more, a group with a result that is no finite number: 0 times an infinite or NaN value is NaN, and the value may be one that only another
+// position of the group sees.
 //
 // Bound: the L2, from which decode_attn_wide_kernel reads 64 KB per tile for one position's two heads.  256 positions of 8 heads over 4
 // kv heads took 96 us there (a window of 1024); 2816 positions take 455 us here, 41 per 256.
@@ -365,7 +367,7 @@ prompt_attn_wide_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
     const int plane_row = p.plane_row0 + h * p.T;
     bool together = true;
     for (int i = 1; i < np; ++i) together &= ((first_key(row0 + 64 * i) - first_key(row0)) & 63) == 0;
-    for (int i_lo = 0; i_lo < np; i_lo = together ? np : i_lo + 1) {
+    for (int i_lo = 0; i_lo < np;) {
       const int i_hi = together ? np : i_lo + 1;
       const int key0 = first_key(row0 + 64 * i_lo);                 // tile u holds the keys key0 + 64 u ..
       const int last_key = p.start_pos + row0 + 64 * (i_hi - 1);    // of the last position
@@ -535,6 +537,7 @@ prompt_attn_wide_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
         sm_l[warp * 16 + c0 + 1] = l1;
       }
       aw_bar_sync();
+      bool finite = true;
       for (int e = tid; e < NP * G * D; e += kWideThreads) {
         const int c = e / D, d = e - c * D;
         int first, last;
@@ -553,9 +556,13 @@ prompt_attn_wide_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
             O += sm_o_all[(w * 8 + c) * D + d] * sc;
           }
         }
-        p.out[(long long)(row0 + 64 * (c / G)) * p.hq * D + (long long)(h * G + c % G) * D + d] = __float2bfloat16_rn(O / L);
+        const float y = O / L;
+        finite &= fabsf(y) < INFINITY;
+        p.out[(long long)(row0 + 64 * (c / G)) * p.hq * D + (long long)(h * G + c % G) * D + d] = __float2bfloat16_rn(y);
       }
-      aw_bar_sync();  // the merge buffer is rewritten by the next item
+      const bool all_finite = __syncthreads_and(finite);  // (the merge buffer is rewritten by the next item)
+      if (together && np > 1 && !all_finite) together = false;
+      else i_lo = i_hi;
     }
   }
 }
