@@ -190,7 +190,7 @@ class LayeredEngine(MaxEngine):
     # one pinned staging buffer per step: [token | group | pos | want | query tiles | runs] rows
     self._desc_host = torch.zeros(6 * self._max_rows + 16, dtype=i32).pin_memory()
     self._desc_dev = torch.zeros(6 * self._max_rows + 16, dtype=i32, device=dev)
-    self._desc_read = torch.cuda.Event()  # the last copy has read _desc_host (recorded by step after each copy)
+    self._desc_read = torch.cuda.Event()  # a slice's copy has read _desc_host (recorded by step before its next slice)
     self._decode_tiles = torch.arange(B + 1, dtype=i32, device=dev)  # a decode step: every row is its own query tile and run
     self._decode_groups = torch.arange(B, dtype=i32, device=dev)
     self._states: List[tuple] = []
@@ -487,7 +487,8 @@ class LayeredEngine(MaxEngine):
       hi = min(rows, lo + R)
       n = hi - lo
       w = [x - lo for x in want if lo <= x < hi]
-      self._desc_read.synchronize()  # (a copy waits for whatever its stream still holds: the buffer is its own until then)
+      if lo:
+        self._desc_read.synchronize()  # (a copy waits for whatever its stream still holds: the buffer is its own until then)
       host[: 3 * R].reshape(3, R)[:, :n] = desc[:, lo:hi]
       host[3 * R : 3 * R + len(w)] = w
       # query tiles: every run of consecutive positions (an entry, cut at the slice) in pieces of at most 16 rows
@@ -503,7 +504,8 @@ class LayeredEngine(MaxEngine):
       host[4 * R : 4 * R + len(tiles)] = tiles
       host[5 * R + 8 : 5 * R + 8 + len(cuts)] = cuts
       self._desc_dev.copy_(self._desc_host, non_blocking=True)
-      self._desc_read.record(torch.cuda.current_stream(self.device))
+      if hi < rows:
+        self._desc_read.record(torch.cuda.current_stream(self.device))
       p = self._desc_dev.data_ptr()
       dst = out[done_want : done_want + len(w)]
       self._run(n, p, p + 4 * R, p + 8 * R, len(w), p + 12 * R, dst, len(tiles) - 1, p + 16 * R, n_runs=len(cuts) - 1, runs_ptr=p + 4 * (5 * R + 8))
