@@ -410,6 +410,7 @@ int launch_prefill_flash(mtx_engine* e, int layer, int rows, int start_pos, int 
   PrefillFlashParams p;
   memset(&p, 0, sizeof(p));
   p.out = e->attn;
+  p.v = static_cast<const bf16*>(e->s.v_cache);
   p.rows = rows;
   p.start_pos = start_pos;
   p.hq = c.num_q_heads;

@@ -11,7 +11,7 @@
 // their relative rounding is the same), which after the first tiles is hardly ever: a rescale reads and writes D columns of TMEM.
 //
 //   D = 64:   NQ = 1, KT = 128, half of the TMEM: two CTAs per SM, each under the other's MMAs.  20 heads x 16 CTAs of 256 positions (NQ = 2, one CTA
-//             per SM) left SMs idle behind the longest ones: 87 us for 4000 positions, 72 so
+//             per SM) left SMs idle behind the longest ones: 87 us for 4000 positions, 74 so
 //   D = 128:  NQ = 2, KT = 128: the MMAs of one half of the positions run under the softmax of the other
 //
 // Bound: the special-function units at D = 64 (one exp2 per score: 16 per SM and clock), 4000 positions x 20 heads: 36 us at least.
@@ -28,6 +28,7 @@ constexpr float kPfLog2e = 1.4426950408889634f;
 
 struct PrefillFlashParams {
   bf16* out;       // [rows, hq * D]
+  const bf16* v;   // the cache rows of tm_v
   int rows;        // positions of the pass
   int start_pos;   // position of row 0
   int hq, hkv, T;
@@ -42,12 +43,15 @@ struct FlashShape {
   static constexpr int kThreads = 64 + NQ * 128, kCtas = D == 64 ? 2 : 1;  // CTAs per SM
   static constexpr int kQBytes = 128 * D * 2, kTileBytes = KT * D * 2;    // a Q tile; a K or a V tile
   static constexpr int kOCol = NQ * KT, kTmemCols = 512 / kCtas;           // first TMEM column of the accumulators; columns in all
+  static constexpr int kNoteWords = (NQ * 128 + KT) / 32;                  // keys of the tiles that reach beyond the first position: at most so many bits
 };
 
 struct FlashTail {
   uint64_t q_full;
   uint64_t k_full[4], v_full[4], empty[4];
   uint64_t s_full[2], p_ready[2], o_done[2];
+  uint64_t noted_all[2];  // the keys that a Q tile's rows see are searched
+  uint32_t noted[12];     // see flash_take_out_nonfinite
   uint32_t tmem_base;
   uint32_t pad;
 };
@@ -88,8 +92,11 @@ prefill_flash_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     last[t] = r1 >= r0 ? (p.start_pos + r1) / KT : -1;
     hi = last[t] > hi ? last[t] : hi;
   }
+  const int masked = (p.start_pos + q0 + 1) / KT;  // the first tile with keys beyond the CTA's first position
 
   griddep_launch_dependents();
+  static_assert(F::kNoteWords <= 12, "FlashTail::noted");
+  if (threadIdx.x < F::kNoteWords) tail->noted[threadIdx.x] = 0;
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&tm_q);
     tma_prefetch_desc(&tm_k);
@@ -104,6 +111,7 @@ prefill_flash_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       mbar_init(&tail->s_full[t], 1);
       mbar_init(&tail->p_ready[t], 4);  // one arrival per softmax warp
       mbar_init(&tail->o_done[t], 1);
+      mbar_init(&tail->noted_all[t], 1);
     }
     fence_barrier_init();
   }
@@ -183,12 +191,19 @@ prefill_flash_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       }
       mbar_wait(&tail->v_full[s], par);
       const int beyond = p.start_pos + p.rows - j * KT;  // the tile's first key that the prompt does not have
+      uint8_t* v = ring + s * 2 * F::kTileBytes + F::kTileBytes;
       if (beyond < KT) {                                 // rows of no key may hold anything, and 0 * NaN is not 0
-        uint8_t* v = ring + s * 2 * F::kTileBytes + F::kTileBytes;
         for (int c = 0; c < CH; ++c)
           for (int b = beyond * 128 + lane * 16; b < KT * 128; b += 512) *reinterpret_cast<uint4*>(v + c * KT * 128 + b) = make_uint4(0, 0, 0, 0);
         fence_proxy_async();
         __syncwarp();
+      }
+      if (j >= masked) {
+        flash_take_out_nonfinite<KT, CH>(v, tail->noted, (j - masked) * KT, lane);
+        __syncwarp();
+#pragma unroll
+        for (int t = 0; t < NQ; ++t)
+          if (j == last[t] && lane == 0) mbar_arrive(&tail->noted_all[t]);
       }
 #pragma unroll
       for (int t = 0; t < NQ; ++t) {
@@ -292,6 +307,12 @@ prefill_flash_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     if (la >= 0) {
       mbar_wait(&tail->o_done[t], 0);
       tcgen05_fence_after();
+      uint32_t noted = 0;
+      if (la >= masked) {
+        mbar_wait(&tail->noted_all[t], 0);
+#pragma unroll
+        for (int w = 0; w < F::kNoteWords; ++w) noted |= tail->noted[w];
+      }
       const float inv = 1.0f / l;
       bf16* out = p.out + (long long)row * p.hq * D + (long long)head * D;
 #pragma unroll 1
@@ -300,6 +321,8 @@ prefill_flash_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         tmem_ld_x32(acc + c, o);
         tmem_wait_ld();
         if (row < p.rows) {
+          if (noted != 0)
+            flash_add_noted<F::kNoteWords>(o, tail->noted, masked * KT, pos, c, [&](int key) { return p.v + (long long)(plane_row + key) * D; });
 #pragma unroll
           for (int e = 0; e < 32; e += 8) {
             uint32_t w[4];
