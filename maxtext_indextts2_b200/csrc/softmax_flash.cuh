@@ -11,7 +11,7 @@
 // tiles, CTAs without one leave.  As in prefill_flash.cuh a thread of the softmax warps owns a row; S is free as soon as it is in registers.
 //
 // Bound: tcgen05 (43 us at the sizes below); what it spends is the softmax warps' time, half of it for the rescales.  4096 rows, 16 heads of 128
-// over 4 key heads: 135 us.  softmax_attention_mma_kernel, where a warp reads all of a tile's K and V for 16 rows of one head, takes 700.
+// over 4 key heads: 140 us.  softmax_attention_mma_kernel, where a warp reads all of a tile's K and V for 16 rows of one head, takes 700.
 #pragma once
 
 #include "flash_tmem.cuh"
@@ -26,11 +26,14 @@ struct PagedFlashShape {
   static constexpr int kThreads = 64 + NQ * 128;
   static constexpr int kQBytes = 128 * D * 2, kTileBytes = KT * D * 2;
   static constexpr int kPCol = NQ * KT, kOCol = 256;  // TMEM columns: S, P, accumulators
+  static constexpr int kNoteWords = (NQ * 128 + KT) / 32;  // keys of the tiles that reach beyond the first position: at most so many bits
 };
 struct PagedFlashTail {
   uint64_t q_full;
   uint64_t k_full[4], v_full[4], empty[4];
   uint64_t s_full[2], s_free[2], p_ready[2], o_done[2];
+  uint64_t noted_all[2];  // the keys that a Q tile's rows see are searched
+  uint32_t noted[10];     // see flash_take_out_nonfinite
   uint32_t tmem_base;
   uint32_t pad;
 };
@@ -87,7 +90,10 @@ paged_flash_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     last[t] = q_hi >= q_lo ? q_hi / KT : -1;
     hi = last[t] > hi ? last[t] : hi;
   }
+  const int masked = (p0 + 1) / KT;  // the first tile with keys beyond the CTA's first position
 
+  static_assert(F::kNoteWords <= 10, "PagedFlashTail::noted");
+  if (threadIdx.x < F::kNoteWords) tail->noted[threadIdx.x] = 0;
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&tm_q);
     tma_prefetch_desc(&tm_k);
@@ -103,6 +109,7 @@ paged_flash_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       mbar_init(&tail->s_free[t], 4);
       mbar_init(&tail->p_ready[t], 4);
       mbar_init(&tail->o_done[t], 1);
+      mbar_init(&tail->noted_all[t], 1);
     }
     fence_barrier_init();
   }
@@ -187,12 +194,19 @@ paged_flash_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       if (j < 0) continue;
       mbar_wait(&tail->v_full[s], par);
       const int beyond = p_end + 1 - j * KT;  // the tile's first key that the sequence does not have
+      uint8_t* v = ring + s * 2 * F::kTileBytes + F::kTileBytes;
       if (beyond < KT) {                      // values of no key: 0 (their probabilities are 0, which a left-over NaN would not leave 0)
-        uint8_t* v = ring + s * 2 * F::kTileBytes + F::kTileBytes;
         for (int c = 0; c < CH; ++c)
           for (int b = beyond * 128 + lane * 16; b < KT * 128; b += 512) *reinterpret_cast<uint4*>(v + c * KT * 128 + b) = make_uint4(0, 0, 0, 0);
         fence_proxy_async();
         __syncwarp();
+      }
+      if (j >= masked) {
+        flash_take_out_nonfinite<KT, CH>(v, tail->noted, (j - masked) * KT, lane);
+        __syncwarp();
+#pragma unroll
+        for (int t = 0; t < NQ; ++t)
+          if (j == last[t] && lane == 0) mbar_arrive(&tail->noted_all[t]);
       }
 #pragma unroll
       for (int t = 0; t < NQ; ++t)
@@ -306,6 +320,12 @@ paged_flash_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     if (la >= 0) {
       mbar_wait(&tail->o_done[t], la & 1);
       tcgen05_fence_after();
+      uint32_t noted = 0;
+      if (la >= masked) {
+        mbar_wait(&tail->noted_all[t], 0);
+#pragma unroll
+        for (int w = 0; w < F::kNoteWords; ++w) noted |= tail->noted[w];
+      }
       const bool valid = row < r_end;
       const float total = (l[0] + l[1]) + (l[2] + l[3]), f = a.out_scale / total * (valid ? smax_gate(a, row, head) : 1.0f);
       bf16* out = a.out + size_t(valid ? row : r0) * a.ld_out + head * D;
@@ -315,6 +335,9 @@ paged_flash_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         tmem_ld_x32(acc + c, o);
         tmem_wait_ld();
         if (!valid) continue;
+        if (noted != 0)
+          flash_add_noted<F::kNoteWords>(o, tail->noted, masked * KT, pos, c,
+                                         [&](int key) { return a.v_pages + (size_t(kvh) * a.num_pages * tpp + size_t(pages[key / tpp]) * tpp + key % tpp) * D; });
 #pragma unroll
         for (int e = 0; e < 32; e += 2) {
           float v0 = __uint_as_float(o[e]), v1 = __uint_as_float(o[e + 1]);
