@@ -96,6 +96,8 @@ typedef struct {
                                         too) and every decode step begins with PageManager.update_decode_pages ON THE DEVICE
                                         (page_manager.py:332-412; in the step's first kernel), as the reference's jitted update does;
                                         0: the caller advances the page state and refreshes page_map etc. before the step */
+  int32_t max_prefill_rows;          /* most rows of a prompt that go through the layers together (and that the workspace has room for);
+                                        0: as many as run best, up to 4096 */
 } mtx_model_config;
 
 /* Weights, repacked once at load time for K-major streaming (see DESIGN.md "Data layout").
@@ -250,7 +252,8 @@ int mtx_profile_decode_step(mtx_engine* e, int rows, mtx_stream stream, float* c
 int mtx_prefill_chunk(mtx_engine* e, const int32_t* tokens, int count, int start_pos, int slot, int sample_last,
                       int32_t* first_token, float* logits_out, float* first_log_prob, mtx_stream stream);
 
-/* The same for any number of positions, up to max_prefill_len in all: long prompts run through the layers in passes of thousands of rows.
+/* The same for any number of positions, up to max_prefill_len in all: long prompts run through the layers in passes of thousands of rows, or
+ * of max_prefill_rows.
  * `draw_row` (0..255): which of the prefill's noise rows the draw of the first token uses; mtx_prefill_chunk uses its last row's index. */
 int mtx_prefill_rows(mtx_engine* e, const int32_t* tokens, int count, int start_pos, int slot, int sample_last, int draw_row, int32_t* first_token,
                      float* logits_out, float* first_log_prob, mtx_stream stream);

@@ -64,6 +64,7 @@ class ModelConfig(ctypes.Structure):
       ("paged_tokens_per_page", ctypes.c_int32),
       ("paged_max_pages_per_group", ctypes.c_int32),
       ("paged_device_state", ctypes.c_int32),
+      ("max_prefill_rows", ctypes.c_int32),
   ]
 
 

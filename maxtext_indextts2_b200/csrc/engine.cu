@@ -1427,6 +1427,7 @@ int mtx_engine_create(const mtx_model_config* cfg, mtx_engine** out) {
     return fail(MTX_ERR_UNSUPPORTED, "emb_dim, mlp_dim and Hq*D must be multiples of 64");
   if (c.mlp_dim % 16 != 0) return fail(MTX_ERR_UNSUPPORTED, "mlp_dim must be a multiple of 16");
   if (c.max_rows < 1 || c.max_rows > 256) return fail(MTX_ERR_ARG, "max_rows must be in [1, 256]");
+  if (c.max_prefill_rows < 0) return fail(MTX_ERR_ARG, "max_prefill_rows must not be negative");
   if (c.max_target_len <= c.max_prefill_len) return fail(MTX_ERR_ARG, "max_target_len must exceed max_prefill_len");
   if (c.num_layers < 1 || c.vocab_size < 1 || c.num_slots < 1) return fail(MTX_ERR_ARG, "bad layer / vocab / slot count");
   mtx_engine* e = new mtx_engine();
@@ -1458,8 +1459,8 @@ int mtx_engine_create(const mtx_model_config* cfg, mtx_engine** out) {
   if (c.kv_quant && e->max_r_tile < 128) e->max_r_tile = 128;  // every step of an int8 engine runs the 128-row-block GEMM
   if (c.decoder_block == 1 && e->max_r_tile < 128) e->max_r_tile = 128;  // and so does every step of the gemma3 block
   if (c.max_prefill_len > 256) {
-    const int rows = (c.max_prefill_len + 255) / 256 * 256;
-    e->pf_rows = rows < kPfMaxRows ? rows : kPfMaxRows;
+    const int rows = (c.max_prefill_len + 255) / 256 * 256, most = c.max_prefill_rows > 0 && c.max_prefill_rows < kPfMaxRows ? c.max_prefill_rows : kPfMaxRows;
+    e->pf_rows = most <= 256 ? 0 : (rows < most ? rows : most);
   }
   e->qkv_n = (c.num_q_heads + 2 * c.num_kv_heads) * c.head_dim;
   e->attn_max_chunks = attn_max_chunks(c.max_prefill_len, c.max_target_len);
@@ -2002,7 +2003,7 @@ int mtx_prefill_rows(mtx_engine* e, const int32_t* tokens, int count, int start_
   }
   const bf16* last = nullptr;
   for (int at = 0; at < count;) {
-    const int left = count - at, small = e->cfg.max_rows;
+    const int left = count - at, most = e->cfg.max_prefill_rows, small = most > 0 && most < e->cfg.max_rows ? most : e->cfg.max_rows;
     int n;
     const int wide = left < e->pf_rows ? left : e->pf_rows, take = e->cfg.decoder_block == 1 ? wide / 256 * 256 : wide;
     if (take > 256 && (e->cfg.head_dim != 256 || takes_prompt_wide(e, 256))) {

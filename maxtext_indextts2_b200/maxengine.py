@@ -271,6 +271,8 @@ class MaxEngine:
     B = self.max_concurrent_decodes
     if B < 1 or B > 256:
       raise ValueError(f"per_device_batch_size={config.per_device_batch_size}: this engine holds 1..256 slots per GPU")
+    # prefill_chunk_size below 256 (its default): a caller's bound on a prompt's share of the GPU, kept as it is.  From 256 on prompts go through the
+    # layers in passes of up to 4096 rows.
     self._chunk = max(1, min(256, int(config.prefill_chunk_size), config.max_prefill_predict_length))
     self._staging = B  # extra KV plane prefill writes into
     self._num_slots = B + 1
@@ -337,6 +339,7 @@ class MaxEngine:
         paged_tokens_per_page=int(config.pagedattn_tokens_per_page) if self._paged else 0,
         paged_max_pages_per_group=int(config.pagedattn_max_pages_per_group) if self._paged else 0,
         paged_device_state=1 if self._page_on_device else 0,
+        max_prefill_rows=self._chunk if int(config.prefill_chunk_size) < 256 else 0,
     )
     _lib.check(self.lib.mtx_engine_create(ctypes.byref(self._cfg_struct), ctypes.byref(self._handle)))
     ws = self.lib.mtx_engine_workspace_bytes(self._handle)

@@ -98,3 +98,21 @@ def test_xla_ffi_handlers_type_check_against_the_stub_header():
 
   for symbol in jax_ffi.TARGETS.values():  # every target jax_ffi.register() looks up is defined by the source
     assert f"XLA_FFI_DEFINE_HANDLER_SYMBOL({symbol}," in text
+
+
+def test_a_bound_on_prompt_rows_bounds_the_workspace(lib):
+  """max_prefill_rows: an engine whose prompts run in steps of at most 256 rows carries no workspace for longer passes."""
+  sizes = {}
+  for rows in (0, 4096, 1024, 256, 64):
+    cfg = _lib.ModelConfig(num_layers=2, emb_dim=1280, num_q_heads=20, num_kv_heads=4, head_dim=64, mlp_dim=5120, vocab_size=512, max_prefill_len=8192,
+                           max_target_len=8448, num_slots=2, max_rows=64, rms_eps=1e-5, rope_min_timescale=1, rope_max_timescale=10000, logits_scale=1.0,
+                           logits_round_bf16=1, max_prefill_rows=rows)
+    h = ctypes.c_void_p()
+    assert lib.mtx_engine_create(ctypes.byref(cfg), ctypes.byref(h)) == _lib.MTX_OK
+    sizes[rows] = lib.mtx_engine_workspace_bytes(h)
+    assert lib.mtx_engine_destroy(h) == _lib.MTX_OK
+  assert sizes[0] == sizes[4096] > sizes[1024] > sizes[256] == sizes[64]
+  activations = 2 * (5 * 1280 + 5120)  # bytes of a row's bf16 activations: x, h, n, q, attn, act
+  assert sizes[1024] - sizes[64] > 900 * activations and sizes[4096] - sizes[1024] >= 3072 * activations
+  cfg.max_prefill_rows = -1
+  assert lib.mtx_engine_create(ctypes.byref(cfg), ctypes.byref(h)) == _lib.MTX_ERR_ARG

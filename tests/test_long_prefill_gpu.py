@@ -68,3 +68,22 @@ def test_gemma3_pass_repeats_steps(dim, kw):
     prefix, _ = engine.prefill(params=params, padded_tokens=toks[at : at + m], true_length=m, existing_prefix=before, slot=0)
   for name in ("key", "value"):
     assert torch.equal(whole["cache"][name], prefix["cache"][name])
+
+
+@pytest.mark.parametrize("block,dim,chunk", [("llama2", 64, 64), ("llama2", 128, 200), ("gemma3", 256, 100)])
+def test_prefill_chunk_size_bounds_a_step(block, dim, chunk):
+  """A prefill_chunk_size below its default of 256 is the most rows of a prompt that a step takes: the bits of the prompt in portions of that size."""
+  cfg = _config(block, dim, prefill_chunk_size=chunk)
+  engine = maxengine.MaxEngine(cfg)
+  params = engine.load_params(on_device_init=True, norm_jitter=0.1)
+  engine.init_decode_state()
+  toks = torch.randint(0, cfg.vocab_size, (700,), generator=torch.Generator().manual_seed(3))
+  whole, _ = engine.prefill(params=params, padded_tokens=toks, true_length=700, slot=0)
+  prefix = None
+  for at in range(0, 700, chunk):
+    m = min(chunk, 700 - at)
+    before = maxengine.ExistingPrefix(cache=prefix["cache"], common_prefix_tokens=toks[:at]) if at else None
+    prefix, _ = engine.prefill(params=params, padded_tokens=toks[at : at + m], true_length=m, existing_prefix=before, slot=0)
+  for name in ("key", "value"):
+    assert torch.equal(whole["cache"][name], prefix["cache"][name])
+  assert torch.equal(whole["logits"], prefix["logits"])
