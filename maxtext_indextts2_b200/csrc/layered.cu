@@ -392,8 +392,12 @@ int linear_grouped(const void* a, const int* a_row, const void* w, long long w_s
       const dim3 pgrid((n + kGgBN - 1) / kGgBN, (slots + kGgBM - 1) / kGgBM + groups, 1);
       return launch(grouped_mma_pipe_kernel<EPI>, pgrid, dim3(kGgThreads), kGgSmemBytes, st, p);
     }
-    // few tokens per expert: 256 slots of 16 experts, 2048 -> 2 x 1024 -> 2048, take 61 + 30 us on linear_mma_kernel, 44 + 24 so
-    if (packed && takes_stream(p, (slots + groups - 1) / groups)) return launch_stream<EPI>(p, (slots + kLsBM - 1) / kLsBM + groups, 1, st);
+    // few tokens per expert.  Both products of 16 experts, 2048 -> 2 x 1024 -> 2048, with 8 / 16 / 24 / 32 rows each take 82 / 94 / 96 / 107 us on
+    // linear_mma_kernel, 66 / 68 / 94 / 98 so; of 32 experts, 1024 -> 2 x 512 -> 1024, with 16 / 24 / 32: 59 / 64 / 60 and 47 / 60 / 63; of 64, 2048 -> 2 x 512
+    // -> 2048: 169 / 194 / 218 and 157 / 193 / 225.  (An expert's 33rd row reads its weights once more, and with many experts linear_mma_kernel's tiles
+    // fill the chip.)
+    const int mean = (slots + groups - 1) / groups;
+    if (packed && mean <= (groups <= 16 ? kLsBM : 24) && takes_stream(p, mean)) return launch_stream<EPI>(p, (slots + kLsBM - 1) / kLsBM + groups, 1, st);
   }
   const dim3 grid((n + 63) / 64, packed ? (slots + 63) / 64 + groups : (slots + 63) / 64, packed ? 1 : groups);
   if constexpr (sizeof(T) == 4) return launch(linear_f32_kernel<EPI>, grid, dim3(kLinF32Threads), 0, st, p);
