@@ -248,7 +248,7 @@ int mtx_profile_decode_step(mtx_engine* e, int rows, mtx_stream stream, float* c
  * lengths.  If `sample_last`, the last position's logits are sampled into first_token[0]
  * (and copied to logits_out [V] fp32 when non-NULL); its log-probability goes to first_log_prob[0] when non-NULL
  * (return_log_prob, maxengine.py:503-520).  The sampler's noise for a prefill draw comes from its own row namespace (one per
- * prefill call), never from the rows of a decode step. */
+ * prefill call), never from the rows of a decode step.  (At most max_rows positions: a call of mtx_prefill_rows.) */
 int mtx_prefill_chunk(mtx_engine* e, const int32_t* tokens, int count, int start_pos, int slot, int sample_last,
                       int32_t* first_token, float* logits_out, float* first_log_prob, mtx_stream stream);
 

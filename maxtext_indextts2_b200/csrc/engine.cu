@@ -892,12 +892,12 @@ int enqueue_prefill_pass(mtx_engine* e, int rows, const int32_t* tokens, int sta
   return MTX_OK;
 }
 
-int enqueue_step(mtx_engine* e, int mode, int rows, const int32_t* chunk_tokens, int start_pos, int slot, int want_logits,
-                 int32_t* first_token, float* prefill_logits, cudaStream_t st, float* cand_out = nullptr, float* first_log_prob = nullptr) {
+// One step: a decode step of `rows` slots up to its tokens (mode 0), or the layers over `rows` prompt positions (mode 1; e->x holds the result).
+int enqueue_step(mtx_engine* e, int mode, int rows, const int32_t* chunk_tokens, int start_pos, int slot, cudaStream_t st, float* cand_out = nullptr) {
   const mtx_model_config& c = e->cfg;
   // (an int8 cache is appended to by the row-major GEMM's epilogue only: steps of any size run it, padded to 128 rows)
   const bool gemma3 = c.decoder_block == 1;
-  const bool mega = mode == 0 && want_logits && pk_usable(e, rows);  // the persistent step kernel (up to 64 rows)
+  const bool mega = mode == 0 && pk_usable(e, rows);  // the persistent step kernel (up to 64 rows)
   const int r_tile = (c.kv_quant || gemma3) && !mega && round_rows(rows) < 128 ? 128 : round_rows(rows);
   XMaps* xm;
   MTX_TRY(get_xmaps(e, r_tile, &xm));
@@ -1065,7 +1065,7 @@ int enqueue_step(mtx_engine* e, int mode, int rows, const int32_t* chunk_tokens,
       MTX_TRY(launch(post_norm_residual_kernel, dim3(rows), dim3(128), 0, st, (const bf16*)e->n, (const bf16*)e->h,
                      static_cast<const bf16*>(e->w.post_ffw_norm) + size_t(l) * E, e->x, e->rows_ss_x, e->max_r_tile, E, c.rms_eps));
     }
-    if (want_logits && mode == 0)
+    if (mode == 0)
       MTX_TRY(launch(rmsnorm_kernel<false>, dim3(rows), dim3(128), 0, st, (const bf16*)e->x, (const int*)nullptr, (const bf16*)nullptr,
                      static_cast<const bf16*>(e->w.final_norm), (bf16*)nullptr, e->n, E, c.rms_eps));
   } else if (!mega) {
@@ -1196,16 +1196,14 @@ int enqueue_step(mtx_engine* e, int mode, int rows, const int32_t* chunk_tokens,
 
     g_class = KC_RMSNORM;
     const bf16* next_scale = l + 1 < L ? attn_norm + size_t(l + 1) * E : static_cast<const bf16*>(e->w.final_norm);
-    if ((l + 1 < L && !fused_norm) || (l + 1 == L && want_logits && mode == 0))
+    if ((l + 1 < L && !fused_norm) || (l + 1 == L && mode == 0))
       MTX_TRY(launch(rmsnorm_kernel<false>, dim3(rows), dim3(128), 0, st, (const bf16*)e->x, (const int*)nullptr,
                      (const bf16*)nullptr, next_scale, (bf16*)nullptr, e->n, E, c.rms_eps));
   }
 
   }
 
-  if (want_logits && mode == 1)
-    return enqueue_last_logits(e, e->x + size_t(rows - 1) * E, rows - 1, first_token, prefill_logits, first_log_prob, st);
-  if (want_logits) {
+  if (mode == 0) {
     const bool two_pass = e->strategy == MTX_SAMPLE_NUCLEUS || e->strategy == MTX_SAMPLE_TOPK;
     if (two_pass && e->s.logits == nullptr) return fail(MTX_ERR_ARG, "%s", kTwoPassNeedsLogits);
     EpiArgs ea;
@@ -1692,7 +1690,7 @@ int mtx_engine_set_sampling(mtx_engine* e, int strategy, int top_k, float nucleu
 int mtx_decode_step(mtx_engine* e, int rows, mtx_stream stream) {
   if (!e || !e->bound) return fail(MTX_ERR_ARG, "engine is not bound");
   if (rows < 1 || rows > e->cfg.max_rows) return fail(MTX_ERR_ARG, "rows %d outside [1, %d]", rows, e->cfg.max_rows);
-  return enqueue_step(e, 0, rows, nullptr, 0, 0, 1, nullptr, nullptr, static_cast<cudaStream_t>(stream));
+  return enqueue_step(e, 0, rows, nullptr, 0, 0, static_cast<cudaStream_t>(stream));
 }
 
 int mtx_decode_step_graph(mtx_engine* e, int rows, mtx_stream stream) {
@@ -1703,7 +1701,7 @@ int mtx_decode_step_graph(mtx_engine* e, int rows, mtx_stream stream) {
     if (!e->cap_stream) MTX_CUDA(cudaStreamCreateWithFlags(&e->cap_stream, cudaStreamNonBlocking));
     cudaGraph_t graph = nullptr;
     MTX_CUDA(cudaStreamBeginCapture(e->cap_stream, cudaStreamCaptureModeThreadLocal));
-    const int rc = enqueue_step(e, 0, rows, nullptr, 0, 0, 1, nullptr, nullptr, e->cap_stream);
+    const int rc = enqueue_step(e, 0, rows, nullptr, 0, 0, e->cap_stream);
     const cudaError_t end = cudaStreamEndCapture(e->cap_stream, &graph);
     if (rc != MTX_OK) {
       if (graph) cudaGraphDestroy(graph);
@@ -1757,7 +1755,7 @@ int mtx_decode_step_host(mtx_engine* e, int rows, const int32_t* tokens_host, in
     cudaGraph_t graph = nullptr;
     MTX_CUDA(cudaStreamBeginCapture(e->cap_stream, cudaStreamCaptureModeThreadLocal));
     int rc = copies_in(e->cap_stream);
-    if (rc == MTX_OK) rc = enqueue_step(e, 0, rows, nullptr, 0, 0, 1, nullptr, nullptr, e->cap_stream);
+    if (rc == MTX_OK) rc = enqueue_step(e, 0, rows, nullptr, 0, 0, e->cap_stream);
     if (rc == MTX_OK) rc = copies_out(e->cap_stream);
     const cudaError_t end = cudaStreamEndCapture(e->cap_stream, &graph);
     if (rc != MTX_OK) {
@@ -1790,7 +1788,7 @@ int mtx_decode_step_candidates(mtx_engine* e, int rows, float* candidates, mtx_s
   if (rows < 1 || rows > e->cfg.max_rows) return fail(MTX_ERR_ARG, "rows %d outside [1, %d]", rows, e->cfg.max_rows);
   if (e->strategy == MTX_SAMPLE_TOPK && e->top_k > kCandK)
     return fail(MTX_ERR_UNSUPPORTED, "vocab-parallel top-k carries %d candidates per shard: decode_sampling_top_k must be <= %d", kCandK, kCandK);
-  return enqueue_step(e, 0, rows, nullptr, 0, 0, 1, nullptr, nullptr, static_cast<cudaStream_t>(stream), candidates);
+  return enqueue_step(e, 0, rows, nullptr, 0, 0, static_cast<cudaStream_t>(stream), candidates);
 }
 
 int mtx_sample_logits(mtx_engine* e, const float* logits, int rows, long long ld, int vocab, int row_offset, int32_t* token_out,
@@ -1956,7 +1954,7 @@ int mtx_profile_decode_step(mtx_engine* e, int rows, mtx_stream stream, float* c
   if (rows < 1 || rows > e->cfg.max_rows) return fail(MTX_ERR_ARG, "rows %d outside [1, %d]", rows, e->cfg.max_rows);
   ProfileSink sink;
   g_profile = &sink;
-  const int rc = enqueue_step(e, 0, rows, nullptr, 0, 0, 1, nullptr, nullptr, static_cast<cudaStream_t>(stream));
+  const int rc = enqueue_step(e, 0, rows, nullptr, 0, 0, static_cast<cudaStream_t>(stream));
   g_profile = nullptr;
   cudaError_t sync = cudaStreamSynchronize(static_cast<cudaStream_t>(stream));
   for (int i = 0; i < KC_COUNT; ++i) { class_ms[i] = 0.f; class_launches[i] = 0; }
@@ -1978,15 +1976,7 @@ int mtx_prefill_chunk(mtx_engine* e, const int32_t* tokens, int count, int start
                       int32_t* first_token, float* logits_out, float* first_log_prob, mtx_stream stream) {
   if (!e || !e->bound) return fail(MTX_ERR_ARG, "engine is not bound");
   if (count < 1 || count > e->cfg.max_rows) return fail(MTX_ERR_ARG, "count %d outside [1, %d]", count, e->cfg.max_rows);
-  if (start_pos < 0 || start_pos + count > e->cfg.max_prefill_len) return fail(MTX_ERR_ARG, "prompt positions exceed max_prefill_len");
-  if (slot < 0 || slot >= e->cfg.num_slots) return fail(MTX_ERR_ARG, "slot out of range");
-  if (sample_last && first_token == nullptr) return fail(MTX_ERR_ARG, "first_token is null");
-  if (sample_last) {
-    ++e->prefill_draws;
-    e->last_prefill_rows = count;
-  }
-  return enqueue_step(e, 1, count, tokens, start_pos, slot, sample_last, first_token, logits_out, static_cast<cudaStream_t>(stream), nullptr,
-                      first_log_prob);
+  return mtx_prefill_rows(e, tokens, count, start_pos, slot, sample_last, count - 1, first_token, logits_out, first_log_prob, stream);
 }
 
 int mtx_prefill_rows(mtx_engine* e, const int32_t* tokens, int count, int start_pos, int slot, int sample_last, int draw_row, int32_t* first_token,
@@ -2011,7 +2001,7 @@ int mtx_prefill_rows(mtx_engine* e, const int32_t* tokens, int count, int start_
       MTX_TRY(enqueue_prefill_pass(e, n, tokens + at, start_pos + at, slot, st));
     } else {
       n = left < small ? left : small;
-      MTX_TRY(enqueue_step(e, 1, n, tokens + at, start_pos + at, slot, 0, nullptr, nullptr, st));
+      MTX_TRY(enqueue_step(e, 1, n, tokens + at, start_pos + at, slot, st));
     }
     last = e->x + size_t(n - 1) * e->cfg.emb_dim;
     at += n;

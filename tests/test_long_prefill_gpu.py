@@ -5,7 +5,7 @@ that start and end inside a tile, unfolded norm scales, a paged and an 8-bit eng
 import pytest
 import torch
 
-from maxtext_indextts2_b200 import maxengine, pyconfig
+from maxtext_indextts2_b200 import _lib, maxengine, pyconfig
 
 pytestmark = pytest.mark.gpu
 
@@ -87,3 +87,23 @@ def test_prefill_chunk_size_bounds_a_step(block, dim, chunk):
   for name in ("key", "value"):
     assert torch.equal(whole["cache"][name], prefix["cache"][name])
   assert torch.equal(whole["logits"], prefix["logits"])
+
+
+def test_chunk_entry_is_the_same_prefill():
+  """mtx_prefill_chunk (at most max_rows positions) leaves what MaxEngine.prefill leaves of the same prompt, and refuses longer ones."""
+  cfg = _config("llama2", 64)
+  engine = maxengine.MaxEngine(cfg)
+  params = engine.load_params(on_device_init=True, norm_jitter=0.1)
+  engine.init_decode_state()
+  toks = torch.randint(0, cfg.vocab_size, (200,), generator=torch.Generator().manual_seed(3))
+  prefix, _ = engine.prefill(params=params, padded_tokens=toks, true_length=200)
+  plane = engine._staging
+  engine._k[:, plane].zero_()
+  dev = toks.to(device="cuda", dtype=torch.int32)
+  first, logits = torch.zeros(1, dtype=torch.int32, device="cuda"), torch.zeros(cfg.vocab_size, device="cuda")
+  call = lambda n, at, last: engine.lib.mtx_prefill_chunk(engine._handle, dev.data_ptr() + 4 * at, n, at, plane, last, first.data_ptr(), logits.data_ptr(), None, None)
+  assert call(120, 0, 0) == _lib.MTX_OK and call(80, 120, 1) == _lib.MTX_OK
+  torch.cuda.synchronize()
+  assert int(first) == int(prefix["tokens"])
+  torch.testing.assert_close(logits, prefix["logits"].reshape(-1), rtol=4e-2, atol=4e-2 * float(logits.abs().max()))  # (two steps against one)
+  assert call(257, 0, 0) == _lib.MTX_ERR_ARG and call(0, 0, 0) == _lib.MTX_ERR_ARG
