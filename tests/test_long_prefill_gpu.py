@@ -70,6 +70,37 @@ def test_gemma3_pass_repeats_steps(dim, kw):
     assert torch.equal(whole["cache"][name], prefix["cache"][name])
 
 
+@pytest.mark.parametrize("block,dim,kw", [("llama2", 64, {}), ("llama2", 128, {}), ("gemma3", 256, {}), ("llama2", 64, dict(quantize_kvcache=True, kv_quant_axis="dkv"))])
+def test_several_passes_and_a_prefix(block, dim, kw):
+  """A prompt of more rows than a pass takes (4096), and passes behind prefixes that end inside a tile, against portions of 200."""
+  cfg = _config(block, dim, max_prefill_predict_length=5000, max_target_length=5100, **kw)
+  engine = maxengine.MaxEngine(cfg)
+  params = engine.load_params(on_device_init=True, norm_jitter=0.1)
+  engine.init_decode_state()
+  n = 4096 + 401
+  toks = torch.randint(0, cfg.vocab_size, (n,), generator=torch.Generator().manual_seed(n))
+
+  def portions(*sizes):
+    prefix, done = None, 0
+    for m in sizes:
+      before = maxengine.ExistingPrefix(cache=prefix["cache"], common_prefix_tokens=toks[:done]) if done else None
+      prefix, _ = engine.prefill(params=params, padded_tokens=toks[done : done + m], true_length=m, existing_prefix=before, slot=0)
+      done += m
+    return prefix
+
+  want = portions(*[200] * 22, n - 4400)
+  for sizes in ((n,), (99, 4397 - 1000, 1001), (1300, n - 1300)):
+    assert sum(sizes) == n
+    got = portions(*sizes)
+    for name in ("key", "value"):
+      a, b = got["cache"][name].double(), want["cache"][name].double()  # [L, heads, n, D]
+      # bf16 activations through at most two layers: 2^-9 for each of about ten roundings
+      err = ((a - b).square().mean((0, 1, 3)) / b.square().mean()).sqrt()
+      assert float(err.max()) < 4e-2, (sizes, name, int(err.argmax()))
+    a, b = got["logits"].double(), want["logits"].double()
+    assert float((a - b).norm() / b.norm()) < 4e-2, sizes
+
+
 @pytest.mark.parametrize("block,dim,chunk", [("llama2", 64, 64), ("llama2", 128, 200), ("gemma3", 256, 100)])
 def test_prefill_chunk_size_bounds_a_step(block, dim, chunk):
   """A prefill_chunk_size below its default of 256 is the most rows of a prompt that a step takes: the bits of the prompt in portions of that size."""

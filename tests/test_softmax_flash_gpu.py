@@ -49,3 +49,40 @@ def test_long_runs_repeat_short_ones(name, dim, page):
     keys = state["cache"]["key_pages"][1][:, pages].flatten(1, 2)
     out.append(keys[:, :662].clone())
   assert torch.isfinite(out[0]).all() and torch.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("name,dim,page", [("gugidra", 64, 16), ("gugidra", 128, 24), ("gugidra", 256, 64), ("ginodra", 64, 8), ("ligidra", 128, 40), ("zakelorn", 64, 64)])
+@pytest.mark.parametrize("portions", [(700,), (257, 512), (512, 257, 129), (3, 690, 300)])
+def test_runs_of_several_tiles(name, dim, page, portions):
+  """Runs of one to three CTAs' rows, alone and side by side, at the start of a sequence and behind the 200 tokens that it holds, against runs of 85."""
+  design, model = _model(name, dim)
+  rng = np.random.Generator(np.random.PCG64(sum(portions)))
+  held = [0, 200, 37][: len(portions)]
+  toks = [rng.integers(0, model["vocab"], size=h + n).tolist() for h, n in zip(held, portions)]
+  out = []
+  for long_runs in (True, False):
+    cfg = pyconfig.from_model_dict(model, dtype="bfloat16", per_device_batch_size=7, max_target_length=960, pagedattn_tokens_per_page=page,
+                                   pagedattn_num_pages=7 * (960 // page + 1) + 2, max_step_rows=1024)
+    engine = maxengine.MaxEngine(cfg)
+    engine.load_params(design.random_tensors(cfg, seed=3))
+    state = engine.init_decode_state()
+    at = [0] * len(portions)
+    for end, most in ((held, 85), ([h + n for h, n in zip(held, portions)], 960 if long_runs else 85)):
+      while at != end:
+        part = [min(b - a, most) for a, b in zip(at, end)]
+        entries = [(s, toks[s][a : a + n], []) for s, (a, n) in enumerate(zip(at, part)) if n]
+        if sum(part) <= 256:  # (more rows in every step, in short runs: the products' plans are then the same)
+          for s in range(3, 7):
+            engine.release_pages(s)
+            entries.append((s, toks[0][:85] if len(toks[0]) >= 85 else toks[1][:85], []))
+        rows = sum(len(e[1]) for e in entries)
+        assert rows > 256 and (rows >= 128 * len(entries)) == (max(part) > 85)  # (takes_paged_flash)
+        engine.step(entries)
+        at = [a + n for a, n in zip(at, part)]
+    keys = []
+    for s, n in enumerate(at):
+      pages = torch.as_tensor(engine.page_state.page_map[s], device="cuda").long()
+      keys.append(state["cache"]["key_pages"][1][:, pages].flatten(1, 2)[:, :n].clone())
+    out.append(keys)
+  for a, b in zip(*out):
+    assert torch.isfinite(a).all() and torch.equal(a, b)

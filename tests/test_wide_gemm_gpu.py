@@ -21,15 +21,31 @@ def _model(name, width):
     layers = [ligidra.attention_layer(4, 2, 64, window=64, pool=16, mlp=ligidra.moe_ff(4, 4, 128, shared_ff=ff)),
               ligidra.delta_layer(4, 2, 32, 64, mlp=ligidra.moe_ff(4, 4, 128, shared_ff=ff))]
     return ligidra, ligidra.model_dict(width, 384, layers, side_dim=64)
-  ffs = [zakelorn.dense_ff(ff), zakelorn.moe_ff(5, 4, 96, identity=1, groups=2, keep=2)]  # unequal experts, slots beyond their ranges
+  ffs = [zakelorn.dense_ff(ff), zakelorn.moe_ff(5, 4, 128, identity=1, groups=2, keep=2)]  # unequal experts, slots beyond their ranges
   layers = [zakelorn.parallel_layer(zakelorn.attention_part(4, 2, 64, window=64, keep_first=4), zakelorn.lightning_part(4, 64), mlp=f) for f in ffs]
   return zakelorn, zakelorn.model_dict(width, 384, layers)
 
 
+def _repeating(name):
+  """Models whose every result is the same in steps of any length, but for kifusun's behind the first attention (its key splits go by the number
+  of query tiles).  zakelorn's windows are longer than the sequence and its decayed sums, whose chunks go by the run, are left out; 768 rows reach the grouped
+  pair GEMM with experts of their own number of rows each, 256 do not."""
+  if name == "kifusun":
+    return _model(name, 256)
+  if name == "gugidra":
+    ffs = [gugidra.dense_ff(384), gugidra.moe_ff(5, 1, 128, shared_ff=256)]
+    return gugidra, gugidra.model_dict(256, 384, [gugidra.parallel_layer(4, 2, 64, 2, 32, 64, mlp=ffs[0]), gugidra.gla_layer(4, 32, 64, mlp=ffs[1]),
+                                                  gugidra.parallel_layer(4, 2, 64, 2, 32, 64, mlp=ffs[1])])
+  ffs = [zakelorn.moe_ff(5, 1, 128, identity=1, shared_ff=256), zakelorn.dense_ff(384), zakelorn.moe_ff(3, 1, 64)]
+  layers = [zakelorn.parallel_layer(zakelorn.attention_part(4, 2, 64, window=1024, keep_first=4), zakelorn.lightning_part(4, 64), right_scale=0.0, mlp=f) for f in ffs]
+  return zakelorn, zakelorn.model_dict(256, 384, layers)
+
+
 @pytest.mark.parametrize("name", ["kifusun", "gugidra", "zakelorn"])
 def test_long_steps_repeat_short_ones(name):
-  """A row's bits do not depend on how many rows its step has: 768 rows at once against three steps of 256."""
-  design, model = _model(name, 256)
+  """A row's bits do not depend on how many rows its step has: 768 rows at once against three steps of 256.  Every layer's keys, and the logits of
+  every row."""
+  design, model = _repeating(name)
   toks = np.random.Generator(np.random.PCG64(1)).integers(0, model["vocab"], size=768).tolist()
   out = []
   for rows in (768, 256):
@@ -38,9 +54,44 @@ def test_long_steps_repeat_short_ones(name):
     engine = maxengine.MaxEngine(cfg)
     engine.load_params(design.random_tensors(cfg, seed=3))
     state = engine.init_decode_state()
-    engine.step([(0, toks, [])])
-    out.append([t.clone() for t in state["cache"]["key_pages"][:1]])
-  assert all(torch.equal(a, b) for a, b in zip(*out))
+    logits = engine.step([(0, toks, list(range(768)))])
+    pages = torch.as_tensor(engine.page_state.page_map[0][:48], device="cuda").long()
+    keys = [t[:, pages].clone() for t in state["cache"]["key_pages"]]
+    out.append(keys[:1] if name == "kifusun" else keys + [t.clone() for t in state["cache"]["recurrent_state"]] * (name == "gugidra") + [logits])
+  assert all(torch.isfinite(t).all() for t in out[0]) and all(torch.equal(a, b) for a, b in zip(*out))
+
+
+def test_unequal_experts_against_float32():
+  """Experts of 0, 1, 255, 256 and 257 rows on the grouped pair GEMM, and slots of an identity expert behind the last range: the token says which
+  expert its row takes."""
+  counts, ff, width = [0, 1, 255, 256, 257, 100], 128, 256  # (the last: the identity expert)
+  rows, experts = sum(counts), len(counts) - 1
+  assert rows >= 128 * experts and ff % 64 == 0 and width % 64 == 0  # (takes_wide_grouped)
+  layer = zakelorn.parallel_layer(zakelorn.attention_part(4, 2, 64, window=64, keep_first=4), zakelorn.lightning_part(4, 64),
+                                  mlp=zakelorn.moe_ff(experts, 1, ff, identity=1, shared_ff=64))
+  model = zakelorn.model_dict(width, 384, [layer] * 2)
+  toks = np.concatenate([np.full(n, e) + 6 * np.arange(n) % 384 // 6 * 6 for e, n in enumerate(counts)]) % 384
+  expert_of = toks % 6
+  assert np.bincount(expert_of, minlength=6).tolist() == counts
+  toks = np.random.Generator(np.random.PCG64(2)).permutation(toks).tolist()
+  out = {}
+  for dtype in ("float32", "bfloat16"):
+    cfg = pyconfig.from_model_dict(model, dtype=dtype, per_device_batch_size=2, max_target_length=rows + 8, pagedattn_tokens_per_page=16,
+                                   pagedattn_num_pages=rows // 16 + 4, max_step_rows=1024)
+    tensors = zakelorn.random_tensors(cfg, seed=3)
+    embed = next(t for n, t in tensors.items() if "embed" in n and t.shape == (384, width))
+    embed[:, :6] = 30.0 * torch.nn.functional.one_hot(torch.arange(384) % 6, 6)  # the stream's first channels name the token's expert
+    for n, t in tensors.items():
+      if n.endswith("mlp.router"):
+        t.zero_()
+        t[:, :6] = torch.eye(6)
+    engine = maxengine.MaxEngine(cfg)
+    engine.load_params(tensors)
+    engine.init_decode_state()
+    out[dtype] = engine.step([(0, toks, list(range(rows)))]).double()
+  # bf16 operands (2^-9 each) through two layers, no row's experts near a tie
+  off = (out["bfloat16"] - out["float32"]).square().mean(1).sqrt() / out["float32"].square().mean().sqrt()
+  assert float(off.max()) < 4e-2
 
 
 @pytest.mark.parametrize("name", ["kifusun", "gugidra", "ligidra", "zakelorn"])
