@@ -529,7 +529,7 @@ def run_vocab_parallel(args, world, rank, local_rank):
 
 def run_prefill(args):
   """--mode prefill: MaxEngine.prefill of one `--prompt-len`-token prompt (the 4k text + reference-audio prompt,
-  timed separately from the decode steps), chunks of prefill_chunk_size rows through the tcgen05 GEMMs and the causal attention
+  timed separately from the decode steps), in passes of up to 4096 rows through the tcgen05 GEMMs and the causal attention
   kernel, then MaxEngine.insert into slot 0.  Not the main metric: a second line for profiles/."""
   from maxtext_indextts2_b200 import maxengine
 

@@ -11,9 +11,9 @@
 //
 // BN is chosen per shape (wide_tile_columns) so that the tiles fill whole waves of pairs.
 //
-// Bound: the tensor pipe at BN = 256 (0.28 us per k block of a tile; 4096 x 2048 x 4096 in 47 us, 1.45 PFLOP/s, 0.91 of the 1.59 that
+// Bound: the tensor pipe at BN = 256 (0.32 us per k block of a tile with the grid full; 4096 x 2048 x 4096 in 47 us, 1.45 PFLOP/s, 0.91 of the 1.59 that
 // cuBLAS reaches in a burst; gemm_rows.cuh in sixteen launches: 257 us), below that the round of barrier, four MMAs and commit
-// (0.16 us per k block).  That round took 0.29 us as long as the issuing threads were picked by `lane == 0`.
+// (0.2 us per k block up to 128 columns).  That round took 0.29 us as long as the issuing threads were picked by `lane == 0`.
 //
 //   warp 0    TMA: its CTA's half of both operands into a ring of stages, both halves counted on the leader's barrier
 //   warp 1    the leader's issues tcgen05.mma and commits (multicast to both CTAs' barriers)

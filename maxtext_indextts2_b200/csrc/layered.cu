@@ -266,7 +266,7 @@ __global__ void act_bf16_kernel(const bf16* src, bf16* act, int n, long long ldo
 // steps of more than 256 rows run the pair GEMM, all rows in one launch (gemm_rows.cuh needs a launch per 256 rows: 257 rows of a
 // 1792 x 1280 projection take 12 us against 21)
 bool takes_wide(int rows) { return rows > 256; }
-// ... and accumulate as a full 256-row step does, so that a prompt's results do not change with the step's length
+// ... and accumulate as a full 256-row step does, so that a prompt's results do not change with the step's length (148: what single_gemm plans with)
 int wide_segments(int n, int k) { return plan_rows(n, k, 256, 148, EPI_STORE_BF16).splits; }
 
 // the same product on a tcgen05 GEMM: the bf16 result stays in e->obf

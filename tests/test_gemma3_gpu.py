@@ -38,7 +38,7 @@ def gemma_config(**kw):
 @pytest.mark.parametrize("head_dim,model", [(64, "gemma3-27b"), (128, "gemma3-27b"), (256, "gemma3-4b")])
 def test_gemma3_prefill_and_decode_match_oracle(head_dim, model):
   """head_dim 256 (gemma3-1b/4b/12b; query scalar head_dim ** -0.5) runs the transposed decode attention of
-  csrc/attention_wide.cuh, and its prompt positions go through the same kernel as decode rows."""
+  csrc/attention_wide.cuh; its prompt positions run the file's prompt kernel."""
   cfg = gemma_config(head_dim=head_dim, model_name=model)
   assert cfg.decoder_block == "gemma3" and cfg.logits_via_embedding
   params = make_params(cfg)
@@ -73,9 +73,10 @@ def test_gemma3_window_wider_than_the_cache_is_full_attention():
 
 @pytest.mark.parametrize("head_dim,model", [(64, "gemma3-27b"), (256, "gemma3-4b")])
 def test_gemma3_chunked_prefill_with_a_window_inside_the_chunks(head_dim, model):
-  """A 550-token prompt in three chunks of 256 positions with sliding_window_size 100: the position window
-  (attentions.py:624-631) cuts inside and across chunks, in prefill_attn_kernel (head_dim 64) and in the decode kernel
-  that runs prompt positions as rows (head_dim 256); then decode steps on the inserted prefix."""
+  """Prompts of 550 and 300 tokens with sliding_window_size 100: the position window (attentions.py:624-631) cuts inside and across the pass
+  of 512 positions, the remainder's step and two steps of up to 256, in prefill_attn_kernel (head_dim 64) and in
+  prompt_attn_wide_kernel or, where a step's keys are split, the decode kernel (head_dim 256); then decode steps on the inserted
+  prefix."""
   cfg = gemma_config(head_dim=head_dim, model_name=model, sliding_window_size=100, max_prefill_predict_length=600,
                      max_target_length=640, per_device_batch_size=2, base_num_decoder_layers=6, prefill_chunk_size=256)
   params = make_params(cfg)
