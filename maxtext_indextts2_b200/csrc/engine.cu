@@ -370,7 +370,7 @@ int launch_prompt_wide(mtx_engine* e, int layer, int rows, int start_pos, int sl
   const int planes = staged_prefill(c) ? 1 : c.num_slots;
   static bool attr_set = false;
   if (!attr_set) {
-    MTX_CUDA(cudaFuncSetAttribute(prompt_attn_wide_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(attn_wide_smem_bytes(256))));
+    MTX_CUDA(cudaFuncSetAttribute(prompt_attn_wide_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(prompt_wide_smem_bytes(256))));
     attr_set = true;
   }
   PromptWideParams p;
@@ -385,8 +385,8 @@ int launch_prompt_wide(mtx_engine* e, int layer, int rows, int start_pos, int sl
   p.plane_row0 = (layer * planes + slot) * c.num_kv_heads * c.max_target_len;
   p.softcap = c.attn_softcap;
   p.window = layer_is_local(e, layer) ? c.sliding_window : 0;
-  const int np = 8 / (p.hq / p.hkv), items = (rows + 64 * np - 1) / (64 * np) * 64 * p.hkv;
-  return launch(prompt_attn_wide_kernel<256>, dim3(items < e->num_sms ? items : e->num_sms), dim3(kWideThreads), attn_wide_smem_bytes(256), st, e->tm_k, e->tm_v, p);
+  const int block = 64 * kPromptGroups * (8 / (p.hq / p.hkv)), items = (rows + block - 1) / block * 64 * p.hkv;
+  return launch(prompt_attn_wide_kernel<256>, dim3(items < e->num_sms ? items : e->num_sms), dim3(kPromptThreads), prompt_wide_smem_bytes(256), st, e->tm_k, e->tm_v, p);
 }
 
 // The same for a pass of more than 256 rows of the llama block (prefill_flash.cuh).  The 16-position CTAs above keep more SMs busy when positions are few: 256 rows

@@ -70,6 +70,32 @@ def test_gemma3_pass_repeats_steps(dim, kw):
     assert torch.equal(whole["cache"][name], prefix["cache"][name])
 
 
+@pytest.mark.parametrize("heads,kv_heads,window,sizes", [(4, 4, 700, (2304,)), (4, 2, 1024, (2304,)), (8, 1, 300, (1280,)), (5, 1, 64, (768, 512)), (4, 2, 500, (512, 1536))])
+def test_gemma3_items_of_many_positions(heads, kv_heads, window, sizes):
+  """Wide heads: items of 4 to 32 positions (four groups of 8 columns), more positions than one item takes, windows that end inside an item, behind a
+  prefix that begins inside a group; the bits of the 256-token steps in every layer's keys and values, and in the logits."""
+  cfg = _config("gemma3", 256, base_num_query_heads=heads, base_num_kv_heads=kv_heads, sliding_window_size=window, max_prefill_predict_length=2400, max_target_length=2500,
+                base_num_decoder_layers=7)
+  engine = maxengine.MaxEngine(cfg)
+  params = engine.load_params(on_device_init=True, norm_jitter=0.1)
+  engine.init_decode_state()
+  n = sum(sizes)
+  toks = torch.randint(0, cfg.vocab_size, (n,), generator=torch.Generator().manual_seed(n))
+
+  def portions(sizes):
+    prefix, done = None, 0
+    for m in sizes:
+      before = maxengine.ExistingPrefix(cache=prefix["cache"], common_prefix_tokens=toks[:done]) if done else None
+      prefix, _ = engine.prefill(params=params, padded_tokens=toks[done : done + m], true_length=m, existing_prefix=before, slot=0)
+      done += m
+    return prefix
+
+  got, want = portions(sizes), portions([256] * (n // 256) + [n % 256] * (n % 256 > 0))
+  for name in ("key", "value"):
+    assert torch.equal(got["cache"][name], want["cache"][name])
+  assert torch.equal(got["logits"], want["logits"])
+
+
 @pytest.mark.parametrize("block,dim,kw", [("llama2", 64, {}), ("llama2", 128, {}), ("gemma3", 256, {}), ("llama2", 64, dict(quantize_kvcache=True, kv_quant_axis="dkv"))])
 def test_several_passes_and_a_prefix(block, dim, kw):
   """A prompt of more rows than a pass takes (4096), and passes behind prefixes that end inside a tile, against portions of 200."""
