@@ -751,7 +751,7 @@ int enqueue_last_logits(mtx_engine* e, const bf16* x, int draw_row, int32_t* fir
 // The layers over `rows` (more than 256, at most pf_rows) prompt positions from start_pos on, all rows in every launch: the projections
 // on the pair GEMM (gemm_wide.cuh), RMSNorm fused into them as in the 65..256-row steps when its scales are folded.  e->x holds the
 // result.
-// The gemma3 block's passes (a multiple of 256 rows) repeat the bits of its 256-row steps: the GEMMs add up K in the steps' segments, the attention
+// The gemma3 block's passes (pass_rows) repeat the bits of its 256-row steps: the GEMMs add up K in the steps' segments, the attention
 // kernels keep the steps' key tiles.  Its logits are products with the embedding table, the largest of them around 10 and rounded to bf16
 // (steps of 1/16), so that a last bit elsewhere moves the first token's log-probability by 6 %.
 int enqueue_prefill_pass(mtx_engine* e, int rows, const int32_t* tokens, int start_pos, int slot, cudaStream_t st) {
@@ -890,6 +890,16 @@ int enqueue_prefill_pass(mtx_engine* e, int rows, const int32_t* tokens, int sta
                      attn_norm + size_t(l + 1) * E, (bf16*)nullptr, e->n, E, c.rms_eps));
   }
   return MTX_OK;
+}
+
+// Rows of the next pass of a prompt with `left` rows to go; 256 or fewer: a step of the 256-row kernels takes them.  A gemma3 pass has the bits of the
+// steps, so the rows behind its last 256 come along only where their own step would cut K and the keys as the 256-row steps do: the plans
+// know rows rounded up to a power of two, so from 129 on.  (3001 positions through six layers, the last 185 as a step
+// of their own: 5.90 ms, in the pass 5.18.)
+int pass_rows(const mtx_engine* e, int left) {
+  const int wide = left < e->pf_rows ? left : e->pf_rows, rest = wide % 256;
+  if (e->cfg.decoder_block != 1 || rest == 0) return wide;
+  return rest > 128 && (e->cfg.head_dim != 256 || takes_prompt_wide(e, rest)) ? wide : wide - rest;
 }
 
 // One step: a decode step of `rows` slots up to its tokens (mode 0), or the layers over `rows` prompt positions (mode 1; e->x holds the result).
@@ -1995,7 +2005,7 @@ int mtx_prefill_rows(mtx_engine* e, const int32_t* tokens, int count, int start_
   for (int at = 0; at < count;) {
     const int left = count - at, most = e->cfg.max_prefill_rows, small = most > 0 && most < e->cfg.max_rows ? most : e->cfg.max_rows;
     int n;
-    const int wide = left < e->pf_rows ? left : e->pf_rows, take = e->cfg.decoder_block == 1 ? wide / 256 * 256 : wide;
+    const int take = pass_rows(e, left);
     if (take > 256 && (e->cfg.head_dim != 256 || takes_prompt_wide(e, 256))) {
       n = take;
       MTX_TRY(enqueue_prefill_pass(e, n, tokens + at, start_pos + at, slot, st));

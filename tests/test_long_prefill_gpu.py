@@ -70,6 +70,25 @@ def test_gemma3_pass_repeats_steps(dim, kw):
     assert torch.equal(whole["cache"][name], prefix["cache"][name])
 
 
+@pytest.mark.parametrize("dim,n", [(64, 641), (128, 767), (256, 640), (256, 641), (256, 767)])
+def test_gemma3_rows_behind_the_last_256(dim, n):
+  """129 to 255 rows behind the last multiple of 256 go with the pass, up to 128 are a step of their own: the bits of the 256-token steps either way."""
+  cfg = _config("gemma3", dim)
+  engine = maxengine.MaxEngine(cfg)
+  params = engine.load_params(on_device_init=True, norm_jitter=0.1)
+  engine.init_decode_state()
+  toks = torch.randint(0, cfg.vocab_size, (n,), generator=torch.Generator().manual_seed(n))
+  whole, _ = engine.prefill(params=params, padded_tokens=toks, true_length=n, slot=0)
+  prefix = None
+  for at in range(0, n, 256):
+    m = min(256, n - at)
+    before = maxengine.ExistingPrefix(cache=prefix["cache"], common_prefix_tokens=toks[:at]) if at else None
+    prefix, _ = engine.prefill(params=params, padded_tokens=toks[at : at + m], true_length=m, existing_prefix=before, slot=0)
+  for name in ("key", "value"):
+    assert torch.equal(whole["cache"][name], prefix["cache"][name])
+  assert torch.equal(whole["logits"], prefix["logits"])
+
+
 @pytest.mark.parametrize("heads,kv_heads,window,sizes", [(4, 4, 700, (2304,)), (4, 2, 1024, (2304,)), (8, 1, 300, (1280,)), (5, 1, 64, (768, 512)), (4, 2, 500, (512, 1536))])
 def test_gemma3_items_of_many_positions(heads, kv_heads, window, sizes):
   """Wide heads: items of 4 to 32 positions (four groups of 8 columns), more positions than one item takes, windows that end inside an item, behind a
