@@ -140,6 +140,11 @@ __global__ void attn_build_worklist_kernel(const int* len0, const int* ring_firs
   if (tid == 0) *work_count = s_off[rows];
 }
 
+// The item that CTA `first` of `stride` takes in turn `turn`: there and back through the list, so that of a list that is sorted by length (prepare_rows_kernel)
+// the CTA with the longest item of one turn gets the shortest of the next.  (200 rows x 4 kv heads of 200 to 2000 tokens, 8 bits, on 592 CTAs: 43.9 us
+// with an unsorted list walked forwards only, 36.9 so; 48 x 4 of 256-wide heads on 148 CTAs: 51.9, 46.0.)
+__device__ __forceinline__ int attn_item(int turn, int first, int stride) { return turn * stride + ((turn & 1) ? stride - 1 - first : first); }
+
 // One thread requests 64-row tile `t` (physical row `row` when the cache is contiguous) of kv head `h` for row `r`: the whole tile,
 // or -- paged with pages shorter than the tile -- the pages that hold its `cnt` valid rows (the rest of the tile keeps stale
 // bytes: the scores of those rows are masked by selection and the value rows are zeroed before the P V product).
@@ -208,7 +213,9 @@ __device__ __forceinline__ void attn_process_items(const CUtensorMap& tm_k, cons
   const long long t_start = clock64();
   int iter = 0;
 
-  for (int item = first_item; item < n_items; item += item_stride) {
+  for (int turn = 0; turn * item_stride < n_items; ++turn) {
+    const int item = attn_item(turn, first_item, item_stride);
+    if (item >= n_items) continue;
     const int packed = p.work_items[item / p.hkv];
     const int h = item % p.hkv;
     const int r = packed >> 16, chunk = packed & 0xffff;
@@ -697,7 +704,9 @@ __device__ __forceinline__ void attn_process_items_q8(const CUtensorMap& tm_k, c
   const uint32_t kb = smem_u32(k_tile), vb = smem_u32(v_tile);
 
   const int n_items = *p.work_count * p.hkv;
-  for (int item = first_item; item < n_items; item += item_stride) {
+  for (int turn = 0; turn * item_stride < n_items; ++turn) {
+    const int item = attn_item(turn, first_item, item_stride);
+    if (item >= n_items) continue;
     const int packed = p.work_items[item / p.hkv];
     const int h = item % p.hkv;
     const int r = packed >> 16, chunk = packed & 0xffff;

@@ -69,7 +69,9 @@ decode_attn_wide_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
   uint32_t phase = 0;
   const int n_items = *p.work_count * p.hkv;
 
-  for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
+  for (int turn = 0; turn * int(gridDim.x) < n_items; ++turn) {
+    const int item = attn_item(turn, blockIdx.x, gridDim.x);
+    if (item >= n_items) continue;
     const int packed = p.work_items[item / p.hkv];
     const int h = item % p.hkv;
     const int r = packed >> 16, chunk = packed & 0xffff;

@@ -968,7 +968,7 @@ int enqueue_step(mtx_engine* e, int mode, int rows, const int32_t* chunk_tokens,
     pa.pk_pair_mode_tiles = env_int("MTX_PK_PAIR_MODE_TILES", 8);
   }
   g_class = KC_PREPARE;
-  MTX_TRY(launch(prepare_rows_kernel, dim3(1), dim3(256), 0, st, pa, e->rd));
+  MTX_TRY(launch(prepare_rows_kernel, dim3(prepare_blocks(rows, c.head_dim)), dim3(256), 0, st, pa, e->rd));
   g_class = KC_RMSNORM;
 
   GemmParams gp;

@@ -72,21 +72,36 @@ struct PrepareArgs {
   int pk_pair_mode_tiles;  // longest pair (in 64-row tiles) for which a CTA takes a whole pair
 };
 
-// One block of 256 threads.  Fills the row descriptors, the RoPE table
-// (embeddings.py:304-307: sin/cos of position / timescale, cast to bf16) and the attention work list.
-__global__ void prepare_rows_kernel(const PrepareArgs a, const RowDesc rd) {
-  __shared__ int s_off[257];
-  __shared__ int s_pos[256];
-  __shared__ int s_nt[256];
+// Blocks of 256 threads.  Block 0 fills the row descriptors and the attention work list, longest rows first (attn_item walks it so that the CTAs' shares
+// come out even); the others fill the RoPE table (embeddings.py:304-307: sin/cos of position / timescale, cast to bf16), one (row, frequency) pair
+// per thread.  Bound: latency of one block.  With the table and running sums over 256 entries by one thread in a single block a step of 200 rows took
+// 13.2 us (9.8 so), a gemma3 step of 48 rows 18.6 (4.5).
+__host__ __device__ inline int prepare_blocks(int rows, int D) { return 1 + (rows * (D / 2) + 255) / 256; }
+__global__ void __launch_bounds__(256) prepare_rows_kernel(const PrepareArgs a, const RowDesc rd) {
+  __shared__ int4 s_rows[256];  // per row: tiles, work items; the same in the sliding-window layers
   const int tl = timeline_begin(0);
   griddep_launch_dependents();
   griddep_wait();
   const int tid = threadIdx.x;
+  if (blockIdx.x > 0) {
+    const int half = a.D / 2, idx = (int(blockIdx.x) - 1) * 256 + tid, r = idx / half, i = idx - r * half;
+    if (r < a.rows) {
+      const float pos = float(a.mode == 0 ? a.next_pos[r] : a.start_pos + r);
+      const float ang = pos / a.rope_timescale[i];
+      rd.rope_cs[idx] = make_float2(bf16r(cosf(ang)), bf16r(sinf(ang)));
+      if (a.window > 0) {
+        const float angw = pos / a.rope_timescale_w[i];
+        rd.rope_cs_w[idx] = make_float2(bf16r(cosf(angw)), bf16r(sinf(angw)));
+      }
+    }
+    timeline_end(tl);
+    return;
+  }
   const int R = a.T - a.P;
-  int chunks = 0, chunks_w = 0;
+  int4 mine = make_int4(0, 0, 0, 0);
   if (a.page_update) {  // (uniform)
-    __shared__ int s_free[256];
-    page_update_decode(a.page_state, s_off, s_free);  // (s_off: scratch until the work list below)
+    __shared__ int s_scan[9], s_free[256];
+    page_update_decode(a.page_state, s_scan, s_free);
     __syncthreads();
   }
   if (tid < a.rows) {
@@ -129,9 +144,8 @@ __global__ void prepare_rows_kernel(const PrepareArgs a, const RowDesc rd) {
       rd.iota[tid] = tid;
       rd.tmp_row[tid] = wr >= 0 ? 0 : -1;
     }
-    s_nt[tid] = attn_num_tiles(l0, rf, rl, R);
-    chunks = (s_nt[tid] + a.tiles_per_item - 1) / a.tiles_per_item;
-    s_pos[tid] = pos;
+    mine.x = attn_num_tiles(l0, rf, rl, R);
+    mine.y = (mine.x + a.tiles_per_item - 1) / a.tiles_per_item;
     if (a.window > 0) {
       // attentions.py:600-602,624-631 in AUTOREGRESSIVE mode: the window covers the last `window` CACHE INDICES of each segment
       // (next_pos = kv_seq_len - 1): prefill rows [s0, P) and ring indices [o, R).  The valid ring rows inside [o, R) are again a
@@ -150,62 +164,42 @@ __global__ void prepare_rows_kernel(const PrepareArgs a, const RowDesc rd) {
       rd.skip_w[tid] = a.mode == 0 ? 0 : l0 - l0p;
       rd.ring_first_w[tid] = rfw;
       rd.ring_len_w[tid] = rlw;
-      chunks_w = (attn_num_tiles(a.mode == 0 ? l0w : l0p, rfw, rlw, R - o) + a.tiles_per_item - 1) / a.tiles_per_item;
+      mine.z = attn_num_tiles(a.mode == 0 ? l0w : l0p, rfw, rlw, R - o);
+      mine.w = (mine.z + a.tiles_per_item - 1) / a.tiles_per_item;
     }
   }
-  s_off[tid + 1] = chunks;
-  if (tid == 0) s_off[0] = 0;
+  s_rows[tid] = mine;
   __syncthreads();
-  {  // RoPE table, all threads: (row, frequency) pairs
-    const int half = a.D / 2;
-    for (int idx = tid; idx < a.rows * half; idx += 256) {
-      const int r = idx / half, i = idx - r * half;
-      const float ang = float(s_pos[r]) / a.rope_timescale[i];
-      rd.rope_cs[idx] = make_float2(bf16r(cosf(ang)), bf16r(sinf(ang)));
-      if (a.window > 0) {
-        const float angw = float(s_pos[r]) / a.rope_timescale_w[i];
-        rd.rope_cs_w[idx] = make_float2(bf16r(cosf(angw)), bf16r(sinf(angw)));
-      }
-    }
+  // every thread for its own row: sums over the rows before it, in the row's order (tiles) and from the longest row down (work items)
+  int tiles_before = 0, tiles = 0, nt_max = 1, at = 0, count = 0, at_w = 0, count_w = 0;
+#pragma unroll 4
+  for (int r = 0; r < a.rows; ++r) {
+    const int4 o = s_rows[r];
+    tiles += o.x;
+    if (r < tid) tiles_before += o.x;
+    nt_max = max(nt_max, o.x);
+    count += o.y;
+    if (o.x > mine.x || (o.x == mine.x && r < tid)) at += o.y;
+    count_w += o.w;
+    if (o.z > mine.z || (o.z == mine.z && r < tid)) at_w += o.w;
   }
   if (a.grid_bar == nullptr) {  // the per-kernel path's attention work list (the persistent kernel cuts its own)
-    if (tid == 0)
-      for (int i = 1; i <= 256; ++i) s_off[i] += s_off[i - 1];
-    __syncthreads();
-    if (tid < a.rows) {
-      const int base = s_off[tid];
-      for (int c = 0; c < chunks; ++c) rd.work_items[base + c] = (tid << 16) | c;
-    }
-    if (tid == 0) *rd.work_count = s_off[a.rows];
+    for (int c = 0; c < mine.y; ++c) rd.work_items[at + c] = (tid << 16) | c;
+    if (tid == 0) *rd.work_count = count;
     if (a.window > 0) {  // the same list for the sliding-window layers
-      __syncthreads();
-      s_off[tid + 1] = chunks_w;
-      if (tid == 0) s_off[0] = 0;
-      __syncthreads();
-      if (tid == 0)
-        for (int i = 1; i <= 256; ++i) s_off[i] += s_off[i - 1];
-      __syncthreads();
-      if (tid < a.rows) {
-        const int base = s_off[tid];
-        for (int c = 0; c < chunks_w; ++c) rd.work_items_w[base + c] = (tid << 16) | c;
-      }
-      if (tid == 0) *rd.work_count_w = s_off[a.rows];
+      for (int c = 0; c < mine.w; ++c) rd.work_items_w[at_w + c] = (tid << 16) | c;
+      if (tid == 0) *rd.work_count_w = count_w;
     }
   }
   if (a.grid_bar != nullptr) {
+    if (tid < a.rows) a.tile_prefix[tid] = tiles_before;
     if (tid == 0) {
       *a.grid_bar = 0u;
-      int acc = 0, nt_max = 1;
-      for (int r = 0; r < a.rows; ++r) {
-        a.tile_prefix[r] = acc;
-        acc += s_nt[r];
-        nt_max = s_nt[r] > nt_max ? s_nt[r] : nt_max;
-      }
-      a.tile_prefix[a.rows] = acc;
+      a.tile_prefix[a.rows] = tiles;
       // Every active CTA gets q = total / nc tiles (rounded either way) and each of its pk_warps attention warps a
       // fifth of them.  The warps that hold the tiles of a pair outside the pair's first CTA each own one slot of
       // the pair's exchange workspace: at most nt - 1 of them, and at most (nt - 1) / floor(q / warps) + 2.
-      const int total = acc * a.hkv;
+      const int total = tiles * a.hkv;
       int nc = total < a.pk_ctas ? total : a.pk_ctas;
       if (nt_max - 1 > a.pk_max_parts) {
         const int f = (nt_max - 1 + a.pk_max_parts - 3) / (a.pk_max_parts - 2);  // tiles per warp needed
