@@ -89,7 +89,10 @@ __device__ __forceinline__ bool elect_one() {
 
 // Blocks until every kernel this one depends on has completed and its writes are visible.
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// Lets the next kernel in the stream start its prologue (weight prefetch) early.
+// Lets the next kernel in the stream start its prologue (weight prefetch) early.  Every kernel that calls it is followed by kernels that wait (griddep_wait)
+// before they touch memory.  The short row-wise kernels of the layered steps call it first of all (a decode step of 64 rows with 80 launches: 932 ->
+// 901 us); the long ones that a few CTAs per SM walk through do not, nor do the kernels right before a recurrence's walk: its CTAs would be
+// placed on the SMs that are free just then, two on some and none on others (a prompt of 4096: 4480 -> 5125 us).
 __device__ __forceinline__ void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Named barrier 1 over the 128 "worker" threads of a CTA (GEMM epilogue warps / attention warps).

@@ -42,6 +42,7 @@ struct LatentPrepareArgs {
 template <typename T>
 __global__ void __launch_bounds__(256) latent_prepare_kernel(const LatentPrepareArgs<T> a) {
   __shared__ float red[8];
+  griddep_launch_dependents();
   griddep_wait();
   const int r = blockIdx.x, tid = threadIdx.x;
   const float* rq = a.proj + size_t(r) * a.ld + a.q_col;
@@ -86,6 +87,7 @@ struct LatentQueryArgs {
 
 template <typename T>
 __global__ void __launch_bounds__(256) latent_query_kernel(const LatentQueryArgs<T> a) {
+  griddep_launch_dependents();
   griddep_wait();
   const int r = blockIdx.x, H = a.heads, d = a.dim, dr = a.rot_dim, rh = dr / 2, dq = d + dr, dl = a.kv_rank + dr;
   const float* q = a.q + size_t(r) * H * dq;

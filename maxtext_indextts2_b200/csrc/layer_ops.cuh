@@ -51,6 +51,7 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 // (x0: a second copy of the embedding output for layers that add it again, or null)
 template <typename T>
 __global__ void embed_rows_kernel(const int* token, const T* embedding, int vocab, float scale, float* x, T* xa, int width, float* x0) {
+  griddep_launch_dependents();
   griddep_wait();
   const int r = blockIdx.x;
   int tok = token[r];
@@ -83,6 +84,7 @@ template <typename T, int V>
 __global__ void __launch_bounds__(256) sandwich_step_kernel(const SandwichArgs a, T* xa) {
   __shared__ float red[8];
   constexpr int N = V == 4 ? kSandwichVec : kSandwichMax;  // register groups of V floats per thread
+  griddep_launch_dependents();
   griddep_wait();
   const int r = blockIdx.x, W = a.width;
   float* xr = a.x + size_t(r) * W;
@@ -169,6 +171,7 @@ __global__ void __launch_bounds__(256) sandwich_step_kernel(const SandwichArgs a
 template <typename T>
 __global__ void __launch_bounds__(256) weighted_norm_rows_kernel(const float* x, const int* rows, const float* w, float eps, T* out, int width) {
   __shared__ float red[8];
+  griddep_launch_dependents();
   griddep_wait();
   const int src = rows ? rows[blockIdx.x] : int(blockIdx.x);
   const float* xr = x + size_t(src) * width;
@@ -180,6 +183,7 @@ __global__ void __launch_bounds__(256) weighted_norm_rows_kernel(const float* x,
 }
 
 __global__ void softcap_kernel(float* z, float cap, long long total) {
+  griddep_launch_dependents();
   griddep_wait();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x)
     z[i] = cap * tanhf(z[i] / cap);
@@ -207,6 +211,7 @@ template <typename T, bool FUSED>
 __global__ void __launch_bounds__(256) group_norm_step_kernel(const float* y, float mult, float* x, const float* w, float eps, float* h, int width,
                                                               int groups, const InputConvArgs<T> cv) {
   __shared__ float red[8];
+  griddep_launch_dependents();
   griddep_wait();
   const int r = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gs = width / groups;
   float* xr = x + size_t(r) * width;
@@ -272,6 +277,7 @@ __global__ void __launch_bounds__(256) group_norm_step_kernel(const float* y, fl
 template <typename T>
 __global__ void __launch_bounds__(256) group_norm_rows_kernel(const float* x, const int* rows, const float* w, float eps, T* out, int width, int groups) {
   __shared__ float red[8];
+  griddep_launch_dependents();
   griddep_wait();
   const int src = rows ? rows[blockIdx.x] : int(blockIdx.x), warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gs = width / groups;
   const float* xr = x + size_t(src) * width;
@@ -293,6 +299,7 @@ __global__ void __launch_bounds__(256) group_norm_rows_kernel(const float* x, co
 }
 
 __global__ void logit_post_kernel(float* z, float scale, float cap, long long total) {
+  griddep_launch_dependents();
   griddep_wait();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const float v = z[i] * scale;
@@ -309,6 +316,7 @@ constexpr int kConvMaxBack = 16;
 template <typename T>
 __global__ void __launch_bounds__(256) input_conv_kernel(const InputConvArgs<T> a) {
   __shared__ const float* s_src[kConvMaxBack];
+  griddep_launch_dependents();
   griddep_wait();
   const int r = blockIdx.x, W = a.width, p = a.pos[r], grp = a.group[r], ring = a.taps - 1;
   const int n_back = ring < p ? ring : p;
@@ -350,6 +358,7 @@ __global__ void __launch_bounds__(256) input_conv_kernel(const InputConvArgs<T> 
 // grid (runs, taps - 1): CTA (run, i) keeps the run's i-th row from its end, if the run is that long (`ld`: row pitch of h)
 __global__ void __launch_bounds__(256) conv_state_update_kernel(const float* h, float* state, const int* run_row0, const int* group, const int* pos,
                                                                 int width, int taps, long long ld) {
+  griddep_launch_dependents();
   griddep_wait();
   const int r0 = run_row0[blockIdx.x], r1 = run_row0[blockIdx.x + 1], r = r1 - 1 - int(blockIdx.y), ring = taps - 1;
   if (r < r0) return;
@@ -374,6 +383,7 @@ struct PreNormArgs {
 template <typename T, bool FUSED>
 __global__ void __launch_bounds__(256) pre_norm_step_kernel(const PreNormArgs a, T* x_copy, T* out, const InputConvArgs<T> cv) {
   __shared__ float red[8];
+  griddep_launch_dependents();
   griddep_wait();
   const int r = blockIdx.x, W = a.width;
   float* xr = a.x + size_t(r) * W;
@@ -443,6 +453,7 @@ template <typename T, int V>
 __global__ void __launch_bounds__(256) out_layer_norm_kernel(const OutLayerNormArgs a, T* xa) {
   __shared__ float red[8];
   constexpr int N = kOutLnVec / V;
+  griddep_launch_dependents();
   griddep_wait();
   const int r = blockIdx.x, W = a.width;
   float* xr = a.x + size_t(r) * W;
@@ -530,6 +541,7 @@ __global__ void __launch_bounds__(256) out_layer_norm_kernel(const OutLayerNormA
 template <typename T>
 __global__ void __launch_bounds__(256) layer_norm_rows_kernel(const float* x, const int* rows, const float* w, const float* b, float eps, T* out, int width) {
   __shared__ float red[8];
+  griddep_launch_dependents();
   griddep_wait();
   const int src = rows ? rows[blockIdx.x] : int(blockIdx.x);
   const float* xr = x + size_t(src) * width;
@@ -546,6 +558,7 @@ __global__ void __launch_bounds__(256) layer_norm_rows_kernel(const float* x, co
 template <typename T>
 __global__ void __launch_bounds__(256) side_act_kernel(const float* gate, long long ld_gate, const int* token, const T* table, long long ld_table, int col,
                                                        int vocab, T* act, int dim, long long total) {
+  griddep_launch_dependents();
   griddep_wait();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const long long r = i / dim;
@@ -579,6 +592,7 @@ struct QkvPostArgs {
 // one CTA per row; a warp per head for the norms
 template <typename T>
 __global__ void __launch_bounds__(256) qkv_post_kernel(const QkvPostArgs<T> a) {
+  griddep_launch_dependents();
   griddep_wait();
   const int r = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
   const int H = a.heads, G = a.kv_heads, d = a.dim, dv = a.vdim;
@@ -617,6 +631,7 @@ __global__ void __launch_bounds__(256) qkv_post_kernel(const QkvPostArgs<T> a) {
 template <typename T>
 __global__ void __launch_bounds__(256) norm_residual_kernel(const float* y, const bf16* y_bf16, float gain, float eps, float* x, T* xa, int width) {
   __shared__ float red[8];
+  griddep_launch_dependents();
   griddep_wait();
   const int r = blockIdx.x;
   const float* yf = y ? y + size_t(r) * width : nullptr;
@@ -639,6 +654,7 @@ __global__ void __launch_bounds__(256) norm_residual_kernel(const float* y, cons
 template <typename T>
 __global__ void __launch_bounds__(256) scalar_norm_rows_kernel(const float* x, const int* rows, float gain, float eps, T* out, int width) {
   __shared__ float red[8];
+  griddep_launch_dependents();
   griddep_wait();
   const int src = rows ? rows[blockIdx.x] : int(blockIdx.x);
   const float* xr = x + size_t(src) * width;

@@ -137,6 +137,7 @@ bool fits_umma(const mtx_layered* e, int n, int k) {
 }
 
 __global__ void bf16_rows_to_f32_kernel(const bf16* src, const float* bias, float* dst, int n, long long total) {
+  griddep_launch_dependents();
   griddep_wait();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x)
     dst[i] = __bfloat162float(src[i]) + (bias ? bias[i % n] : 0.0f);
@@ -144,6 +145,7 @@ __global__ void bf16_rows_to_f32_kernel(const bf16* src, const float* bias, floa
 
 // (mode 0: gelu_tanh(g) u; 1: the clamped form g sigmoid(1.702 g) (u + 1); 2: silu(g) u)
 __global__ void gate_up_bf16_kernel(const bf16* src, bf16* act, int ff, long long total, float limit, int mode) {
+  griddep_launch_dependents();
   griddep_wait();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const long long r = i / ff, f = i % ff;
@@ -155,6 +157,7 @@ __global__ void gate_up_bf16_kernel(const bf16* src, bf16* act, int ff, long lon
 // eight columns per thread: fp32 values of a bf16 projection, the columns [silu0, silu1) through silu and rounded to bf16 again, or (in_place:
 // silu0 and silu1 multiples of 8) these columns through silu where they are, for a reader of bf16
 __global__ void __launch_bounds__(256) bf16_cols_to_f32_kernel(bf16* src, float* dst, int n, int silu0, int silu1, int in_place, long long groups) {
+  griddep_launch_dependents();
   griddep_wait();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < groups; i += (long long)gridDim.x * blockDim.x) {
     const uint4 q = *reinterpret_cast<const uint4*>(src + i * 8);
@@ -242,6 +245,7 @@ __device__ __forceinline__ float act_of_kind(float v, int kind) {
 
 // the same with eight columns per thread (n and ldo multiples of 8)
 __global__ void __launch_bounds__(256) act8_bf16_kernel(const bf16* src, bf16* act, int n, long long ldo, long long groups, int kind) {
+  griddep_launch_dependents();
   griddep_wait();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < groups; i += (long long)gridDim.x * blockDim.x) {
     const uint4 q = *reinterpret_cast<const uint4*>(src + i * 8);
@@ -257,6 +261,7 @@ __global__ void __launch_bounds__(256) act8_bf16_kernel(const bf16* src, bf16* a
 }
 
 __global__ void act_bf16_kernel(const bf16* src, bf16* act, int n, long long ldo, long long total, int kind) {
+  griddep_launch_dependents();
   griddep_wait();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     act[(i / n) * ldo + i % n] = __float2bfloat16_rn(act_of_kind(__bfloat162float(src[i]), kind));

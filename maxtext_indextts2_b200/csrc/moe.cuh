@@ -22,6 +22,7 @@ namespace mtx {
 // a matrix-product kernel would be mostly padding and its k loop one long chain)
 template <typename T>
 __global__ void __launch_bounds__(256) moe_router_kernel(const T* x, const T* w, const float* bias, float* logits, int experts, int width) {
+  griddep_launch_dependents();
   griddep_wait();
   const int r = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const T* xr = x + size_t(r) * width;
@@ -74,6 +75,7 @@ __global__ void __launch_bounds__(32) moe_route_kernel(const MoeRouteArgs a) {
   float* s = sm;                  // [E] scores
   float* c = s + a.experts;       // [E] choice scores
   float* gs = c + a.experts;      // [groups]
+  griddep_launch_dependents();
   griddep_wait();
   const int r = blockIdx.x, lane = threadIdx.x, E = a.experts, per = E / a.groups;
   float zmax = -INFINITY, zsum = 1.0f;
@@ -157,6 +159,7 @@ __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* chosen, int e
   extern __shared__ int si[];
   int* count = si;               // [E]
   int* start = count + experts;  // [E + 1]
+  griddep_launch_dependents();
   griddep_wait();
   for (int e = threadIdx.x; e < experts; e += blockDim.x) count[e] = 0;
   __syncthreads();
@@ -182,6 +185,7 @@ __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* chosen, int e
 
 // the rows that the slots read, side by side for the pair GEMM: dst[s] = src[a_row[s]], `pieces` 16-byte pieces per row, for the slots below *n
 __global__ void __launch_bounds__(256) moe_gather_kernel(const uint4* src, const int* a_row, const int* n, int pieces, uint4* dst) {
+  griddep_launch_dependents();
   griddep_wait();
   const int slots = *n;
   for (int s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); s < slots; s += gridDim.x * (blockDim.x >> 5)) {
@@ -192,6 +196,7 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const uint4* src, const
 }
 
 __global__ void __launch_bounds__(256) moe_combine_kernel(const float* ye, const int* slot_of, const float* weight, int top, int width, int add, float* y) {
+  griddep_launch_dependents();
   griddep_wait();
   const int r = blockIdx.x;
   for (int c = threadIdx.x; c < width; c += blockDim.x) {

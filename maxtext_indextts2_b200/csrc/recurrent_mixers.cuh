@@ -154,6 +154,7 @@ __device__ __forceinline__ float softplus_f(float z) { return fmaxf(z, 0.0f) + l
 template <typename T>
 __global__ void __launch_bounds__(256) lowrank_split_kernel(const float* proj, long long ld, int a_col, int rank, int g_col, int gate_rank, T* decay_in,
                                                             T* gate_in, long long rows) {
+  griddep_launch_dependents();
   griddep_wait();
   const long long per = rank + gate_rank, total = rows * per;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -848,6 +849,7 @@ struct RecOutArgs {
 // one CTA per row, a warp per head
 template <typename T>
 __global__ void __launch_bounds__(256) recurrent_out_kernel(const RecOutArgs<T> a) {
+  griddep_launch_dependents();
   griddep_wait();
   if (a.next_n && (blockIdx.x + 1 == gridDim.x || a.group[blockIdx.x + 1] != a.group[blockIdx.x])) {
     const size_t at = size_t(a.group[blockIdx.x]) * a.heads;
@@ -878,6 +880,7 @@ template <typename T, int V, int MAX>
 __global__ void __launch_bounds__(256) recurrent_out_whole_kernel(const RecOutArgs<T> a) {
   __shared__ float red[8];
   constexpr int N = MAX / V;
+  griddep_launch_dependents();
   griddep_wait();
   const int r = blockIdx.x, n = a.heads * a.vdim;
   const float* o = a.o + size_t(r) * n;

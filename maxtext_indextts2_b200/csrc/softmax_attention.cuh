@@ -81,6 +81,7 @@ struct RopeAppendArgs {
 
 template <typename T>
 __global__ void __launch_bounds__(256) rope_append_kernel(const RopeAppendArgs<T> a) {
+  griddep_launch_dependents();
   griddep_wait();
   const int r = blockIdx.x, tid = threadIdx.x;
   const int H = a.heads, G = a.kv_heads, d = a.dim, dv = a.vdim, half = d / 2, rh = a.rot_dims / 2;
@@ -157,6 +158,7 @@ __device__ __forceinline__ void rot_sincos(double p, double freq, float* sn, flo
 // one CTA per row, a warp per head (query heads, then key heads): norm, rotation, write; then the values
 template <typename T>
 __global__ void __launch_bounds__(256) qk_prepare_append_kernel(const QkPrepareArgs<T> a) {
+  griddep_launch_dependents();
   griddep_wait();
   const int r = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
   extern __shared__ float qkp_rows[];  // talk: the row's rotated queries
@@ -250,6 +252,7 @@ struct PoolAppendArgs {
 // position (fp32) and writes their means; every other CTA leaves at once
 template <typename T>
 __global__ void __launch_bounds__(256) pool_append_kernel(const PoolAppendArgs<T> a) {
+  griddep_launch_dependents();
   griddep_wait();
   const int r = blockIdx.x, p = a.pos[r], P = a.pool;
   if ((p + 1) % P != 0) return;
@@ -962,6 +965,7 @@ __global__ void __launch_bounds__(kSdecWarps * 32) softmax_attention_decode_kern
 
 // out[row, h] = out_scale * sum_z e^(m_z - M) o_z / sum_z e^(m_z - M) l_z, M = max_z m_z; one warp per (row, head)
 __global__ void __launch_bounds__(128) softmax_attention_merge_kernel(const SoftmaxAttnArgs<bf16> a) {
+  griddep_launch_dependents();
   griddep_wait();
   const int unit = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (unit >= a.rows * a.heads) return;
@@ -989,6 +993,7 @@ __global__ void __launch_bounds__(128) softmax_attention_merge_kernel(const Soft
 // (row, head)
 template <typename T>
 __global__ void __launch_bounds__(128) softmax_diff_merge_kernel(const SoftmaxAttnArgs<T> a) {
+  griddep_launch_dependents();
   griddep_wait();
   const int unit = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (unit >= a.rows * a.heads) return;

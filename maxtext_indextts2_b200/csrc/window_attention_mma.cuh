@@ -285,6 +285,7 @@ __global__ void __launch_bounds__(kWmmaThreads, 1) window_attention_mma_kernel(c
 
 // out[r, o] = bf16(sum over the splits, in order)
 __global__ void window_partial_sum_kernel(const float* partial, bf16* out, int splits, long long per_split) {
+  griddep_launch_dependents();
   griddep_wait();
   for (long long i = (blockIdx.x * (long long)blockDim.x + threadIdx.x) * 2; i < per_split; i += (long long)gridDim.x * blockDim.x * 2) {
     float2 s = *reinterpret_cast<const float2*>(partial + i);
