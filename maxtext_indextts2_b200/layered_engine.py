@@ -157,6 +157,8 @@ class LayeredEngine(MaxEngine):
   """``MaxEngine(config)`` returns this class when ``config.decoder_block`` is a layered design."""
 
   prompt_and_decode_share_pages = True  # no prefill segment + AR ring: a sequence is one page group that grows
+  _desc_pending = _map_pending = False  # _desc_read / _map_read stand for a copy that may not have run yet
+  _behind = None  # the stream that still holds a step of this engine, or None
 
   def __init__(self, config, devices: Any = None, use_cuda_graph: bool = True, vocab_shard: Optional[tuple] = None, gather: Any = None):
     if vocab_shard is not None or int(config.vocab_parallelism) != 1:
@@ -190,7 +192,12 @@ class LayeredEngine(MaxEngine):
     # one pinned staging buffer per step: [token | group | pos | want | query tiles | runs] rows
     self._desc_host = torch.zeros(6 * self._max_rows + 16, dtype=i32).pin_memory()
     self._desc_dev = torch.zeros(6 * self._max_rows + 16, dtype=i32, device=dev)
-    self._desc_read = torch.cuda.Event()  # a slice's copy has read _desc_host (recorded by step before its next slice)
+    self._desc_read = torch.cuda.Event()  # a copy has read _desc_host (recorded where the buffer is written again before the stream is waited for)
+    # the page map's staging buffer, and whether its last copy may still have to read it
+    self._map_host = torch.zeros(B, MP, dtype=i32).pin_memory()
+    self._map_read = torch.cuda.Event()
+    # a step that returned before its kernels were done: the event behind them and its stream (another stream waits for it)
+    self._step_done = torch.cuda.Event()
     self._decode_tiles = torch.arange(B + 1, dtype=i32, device=dev)  # a decode step: every row is its own query tile and run
     self._decode_groups = torch.arange(B, dtype=i32, device=dev)
     self._states: List[tuple] = []
@@ -389,6 +396,7 @@ class LayeredEngine(MaxEngine):
   # -- state --------------------------------------------------------------------------------------
 
   def init_decode_state(self, rng: Any = None) -> dict:
+    self._follow()
     for t in (self._tokens, self._next_pos, self._generated, self._active, self._result):
       t.zero_()
     self._rng_state[0:1].zero_()
@@ -410,8 +418,21 @@ class LayeredEngine(MaxEngine):
   def _upload_page_map(self) -> None:
     ps = self.page_state
     if ps.page_map is not self._uploaded_map:
-      self._page_map_dev[: ps.page_map.shape[0]].copy_(torch.from_numpy(ps.page_map))
+      if self._map_pending:
+        self._map_read.synchronize()
+      self._map_host.numpy()[:] = ps.page_map
+      self._page_map_dev[: ps.page_map.shape[0]].copy_(self._map_host, non_blocking=True)
+      self._map_read.record(torch.cuda.current_stream(self.device))
+      self._map_pending = True
       self._uploaded_map = ps.page_map
+
+  def _follow(self) -> None:
+    """The caller's stream behind a step that another stream may still hold (a step's pages, states and descriptors are the engine's)."""
+    if self._behind is not None:
+      stream = torch.cuda.current_stream(self.device)
+      if stream != self._behind:
+        stream.wait_event(self._step_done)
+        self._behind = None
 
   def _upload_page_state(self) -> None:  # (MaxEngine.release_pages calls it for device-resident page states; nothing to do here)
     return
@@ -420,15 +441,16 @@ class LayeredEngine(MaxEngine):
     """The slot's pages go back to the pool.  Its row of the page map is cleared too, so that the row an empty slot still
     contributes to a decode step lands on page 0 (never handed out) and not on a page somebody else owns by then."""
     slot = int(slot)
+    self._follow()
     ps = self.page_manager.release_pages(page_state=self.page_state, page_group_id=slot)
     page_map = ps.page_map.copy()
     page_map[slot] = 0
     self.page_state = ps.replace(page_map=page_map)
-    self._active[slot].zero_()
-    self._next_pos[slot].zero_()
-    for st in self._states:  # (a sequence that starts at position 0 starts from zero anyway; this keeps a freed slot clean)
-      for t in st:
-        t[slot].zero_()
+    # (a sequence that starts at position 0 starts from zero anyway; zeroing the states keeps a freed slot clean)
+    torch._foreach_zero_([t[slot] for t in (self._active, self._next_pos)])
+    states = [t[slot] for st in self._states for t in st]
+    if states:
+      torch._foreach_zero_(states)
 
   # -- the ragged step ----------------------------------------------------------------------------
 
@@ -444,11 +466,18 @@ class LayeredEngine(MaxEngine):
     """One mixed batch.  `entries`: (slot, the sequence's next tokens, indices among them whose logits are wanted).  Every
     sequence grows by its tokens (pages are reserved as needed; ValueError when the pool is exhausted); returns the wanted
     logits [n, vocab] (fp32, on the device) in the order of the entries.  Steps longer than max_step_rows run in slices."""
+    return self._step(entries, wait=True)
+
+  def _step(self, entries: Sequence[Tuple[int, Sequence[int], Sequence[int]]], wait: bool) -> torch.Tensor:
+    """`step`; wait=False returns as soon as the kernels are enqueued.
+
+    The host's part is bound by Python, about a microsecond per operation: the rows' arrays are made for all entries at once (31 single tokens beside a
+    portion of 500, with the slot's release: 403 us with an array or two per entry, 208 so)."""
     self._require_params(None)
+    self._follow()
     B, V = self.max_concurrent_decodes, int(self.config.vocab_size)
-    tok, grp, pos, want, runs, rows = [], [], [], [], [], 0
-    slots, lengths = [], []
     ps = self.page_state
+    slots, counts, want, pieces, flat, rows = [], [], [], [], [], 0
     seen = set()
     for slot, tokens, wanted in entries:
       slot = int(slot)
@@ -458,59 +487,79 @@ class LayeredEngine(MaxEngine):
       n = len(tokens)
       if n == 0:
         continue
-      start = int(ps.sequence_lengths[slot])
-      slots.append(slot)
-      lengths.append(start + n)
-      base = rows
-      rows += n
-      runs.append((base, rows))
-      tok.append(_token_array(tokens))
-      grp.append(np.full(n, slot, np.int32))
-      pos.append(np.arange(start, start + n, dtype=np.int32))
       for w in wanted:
-        if not 0 <= int(w) < n:
+        w = int(w)
+        if not 0 <= w < n:
           raise ValueError(f"slot {slot}: wanted index {w} outside its {n} tokens")
-        want.append(base + int(w))
-    ps, failed = self.page_manager.extend_pages_of(ps, slots, lengths)
+        want.append(rows + w)
+      slots.append(slot)
+      counts.append(n)
+      rows += n
+      if type(tokens) is list:  # (lists are converted together)
+        flat += tokens
+      else:
+        if flat:
+          pieces.append(_token_array(flat))
+          flat = []
+        pieces.append(_token_array(tokens))
+    if flat:
+      pieces.append(_token_array(flat))
+    groups, counts = np.array(slots, np.int64), np.array(counts, np.int64)
+    starts = ps.sequence_lengths[groups] if slots else groups
+    lengths = starts + counts
+    ps, failed = self.page_manager.extend_pages_of(ps, groups, lengths)
     if failed >= 0:
-      raise ValueError(f"slot {slots[failed]}: the page pool cannot hold {lengths[failed]} tokens")
+      raise ValueError(f"slot {slots[failed]}: the page pool cannot hold {int(lengths[failed])} tokens")
     self.page_state = ps
     self._upload_page_map()
     out = torch.empty(len(want), V, dtype=torch.float32, device=self.device)
     if rows == 0:
       return out
     R = self._max_rows
-    desc = np.stack([np.concatenate(x) for x in (tok, grp, pos)])
+    ends = np.cumsum(counts)
+    bases = ends - counts
+    desc = np.empty((3, rows), np.int32)
+    desc[0] = pieces[0] if len(pieces) == 1 else np.concatenate(pieces)
+    desc[1] = np.repeat(groups, counts)
+    desc[2] = np.arange(rows) + np.repeat(starts - bases, counts)
+    want_at = np.array(want, np.int64)
     host = self._desc_host.numpy()
     done_want = 0
     for lo in range(0, rows, R):
       hi = min(rows, lo + R)
       n = hi - lo
-      w = [x - lo for x in want if lo <= x < hi]
-      if lo:
+      w = want_at if rows <= R else want_at[(want_at >= lo) & (want_at < hi)] - lo
+      if lo or self._desc_pending:
         self._desc_read.synchronize()  # (a copy waits for whatever its stream still holds: the buffer is its own until then)
+        self._desc_pending = False
       host[: 3 * R].reshape(3, R)[:, :n] = desc[:, lo:hi]
       host[3 * R : 3 * R + len(w)] = w
       # query tiles: every run of consecutive positions (an entry, cut at the slice) in pieces of at most 16 rows
       # and the runs themselves (recurrent mixers walk a run in order from its group's state)
-      tiles, cuts = [], []
-      for a, b in runs:
-        a, b = max(a, lo), min(b, hi)
-        if a < b:
-          cuts.append(a - lo)
-        tiles.extend(range(a - lo, b - lo, QUERY_TILE_ROWS))
-      tiles.append(n)
-      cuts.append(n)
-      host[4 * R : 4 * R + len(tiles)] = tiles
-      host[5 * R + 8 : 5 * R + 8 + len(cuts)] = cuts
+      first, last = np.maximum(bases, lo) - lo, np.minimum(ends, hi) - lo
+      here = first < last
+      first, last = first[here], last[here]
+      pieces_of = (last - first + QUERY_TILE_ROWS - 1) // QUERY_TILE_ROWS
+      n_cuts, n_tiles = len(first), int(pieces_of.sum())
+      tiles = np.repeat(first - QUERY_TILE_ROWS * (np.cumsum(pieces_of) - pieces_of), pieces_of) + QUERY_TILE_ROWS * np.arange(n_tiles)
+      host[4 * R : 4 * R + n_tiles], host[4 * R + n_tiles] = tiles, n
+      host[5 * R + 8 : 5 * R + 8 + n_cuts], host[5 * R + 8 + n_cuts] = first, n
       self._desc_dev.copy_(self._desc_host, non_blocking=True)
-      if hi < rows:
+      if hi < rows or not wait:
         self._desc_read.record(torch.cuda.current_stream(self.device))
       p = self._desc_dev.data_ptr()
       dst = out[done_want : done_want + len(w)]
-      self._run(n, p, p + 4 * R, p + 8 * R, len(w), p + 12 * R, dst, len(tiles) - 1, p + 16 * R, n_runs=len(cuts) - 1, runs_ptr=p + 4 * (5 * R + 8))
+      self._run(n, p, p + 4 * R, p + 8 * R, len(w), p + 12 * R, dst, n_tiles, p + 16 * R, n_runs=n_cuts, runs_ptr=p + 4 * (5 * R + 8))
       done_want += len(w)
-    torch.cuda.current_stream(self.device).synchronize()  # the pinned staging buffer is free again when step returns
+    stream = torch.cuda.current_stream(self.device)
+    if wait:
+      stream.synchronize()  # the pinned staging buffers are free again when step returns
+      self._desc_pending = self._map_pending = False
+      self._behind = None
+    else:
+      self._desc_pending = True
+      self._step_done.record(stream)
+      self._behind = stream
     return out
 
   def _sample(self, logits: torch.Tensor, rows: int, token_out: torch.Tensor, log_prob_out: Optional[torch.Tensor], row_offset: int) -> None:
@@ -527,7 +576,8 @@ class LayeredEngine(MaxEngine):
   def prefill(self, *, params: Any = None, padded_tokens: Any, true_length: int, existing_prefix: Any = None, images: Any = None,
               sampler: Any = None, rng: Any = None, request_id: Any = None, slot: Optional[int] = None, return_prompt_logp: bool = False):
     """maxengine.py:533-574 for one sequence; the rows go straight into the pages of `slot` (required).  `existing_prefix`
-    (chunked prefill): the slot already holds that prefix and grows."""
+    (chunked prefill): the slot already holds that prefix and grows.  Returns once everything is enqueued, as ``generate`` does: the results are the
+    current stream's."""
     self._require_params(params)
     if slot is None:
       raise ValueError("a layered model prefills into the pages of a slot: pass slot=")
@@ -548,7 +598,7 @@ class LayeredEngine(MaxEngine):
     if start + true_length >= int(self.config.max_target_length):
       raise ValueError(f"{start + true_length} prompt tokens leave no room to decode (max_target_length={self.config.max_target_length})")
     prompt = toks[:true_length].cpu()
-    logits = self.step([(slot, prompt.tolist() if prompt.is_floating_point() else prompt.numpy(), [true_length - 1])])
+    logits = self._step([(slot, prompt.tolist() if prompt.is_floating_point() else prompt.numpy(), [true_length - 1])], wait=False)
     self._sample(logits, 1, self._first_token, self._first_log_prob if self.config.return_log_prob else None, 0x40000000)
     first = self._first_token.clone().reshape(1, 1)
     n = start + true_length
@@ -570,6 +620,7 @@ class LayeredEngine(MaxEngine):
     slot = int(slot)
     if int(prefix["cache"]["slot"]) != slot:
       raise ValueError(f"this prefix was prefilled into slot {prefix['cache']['slot']}, not {slot}")
+    self._follow()
     self._next_pos[slot].copy_(prefix["next_pos"][0])
     self._generated[slot].copy_(prefix["generated_tokens"][0])
     self._tokens[slot].copy_(prefix["tokens"][0])
@@ -609,6 +660,7 @@ class LayeredEngine(MaxEngine):
 
   def _decode_rows(self) -> None:
     """One row per slot: token and position from the device state, the slot's pages grown by one token on the host."""
+    self._follow()
     B = self.max_concurrent_decodes
     ps = self.page_manager.update_decode_pages(self.page_state)
     grew = ps.has_active_page & (ps.num_pages_used * self.page_manager.tokens_per_page < ps.sequence_lengths)

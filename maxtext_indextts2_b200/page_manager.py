@@ -244,14 +244,18 @@ class PageManager:
   def extend_pages_of(self, page_state: PageState, page_group_ids: Sequence[int], new_lengths: Sequence[int]) -> Tuple[PageState, int]:
     """`extend_pages` for several different groups (one mixed batch).  Returns the new state and -1, or the state unchanged and the index of the first
     group that does not fit."""
-    for g, n in zip(page_group_ids, new_lengths):
-      if g < 0 or g >= self.max_page_groups:
-        raise ValueError(f"PageManager: page_group_id ({g}) out of range [0, {self.max_page_groups})")
-      if n < int(page_state.sequence_lengths[g]) or n > self.max_target_length:
-        raise ValueError(f"PageManager: new_length ({n}) out of range [{int(page_state.sequence_lengths[g])}, {self.max_target_length}]")
     if not len(page_group_ids):
       return page_state, -1
-    return _extend_pages_for_groups(page_state, np.asarray(page_group_ids), np.asarray(new_lengths), self.tokens_per_page, self.max_pages_per_group)
+    groups, lengths = np.asarray(page_group_ids), np.asarray(new_lengths)
+    known = (groups >= 0) & (groups < self.max_page_groups)
+    held = page_state.sequence_lengths[np.where(known, groups, 0)]
+    ok = known & (lengths >= held) & (lengths <= self.max_target_length)
+    if not ok.all():
+      i = int(np.argmin(ok))  # the first that is not
+      if not known[i]:
+        raise ValueError(f"PageManager: page_group_id ({int(groups[i])}) out of range [0, {self.max_page_groups})")
+      raise ValueError(f"PageManager: new_length ({int(lengths[i])}) out of range [{int(held[i])}, {self.max_target_length}]")
+    return _extend_pages_for_groups(page_state, groups, lengths, self.tokens_per_page, self.max_pages_per_group)
 
   def update_decode_pages(self, page_state: PageState) -> PageState:
     """:538-563."""

@@ -1,0 +1,111 @@
+"""Steps that return before their kernels are done (a prompt of the layered engine): what the host writes for the next one reaches the device as it was
+written, and another stream does not run ahead of them.  The streams are queues here that run when somebody waits for them."""
+
+import types
+
+import numpy as np
+import pytest
+import torch
+
+from maxtext_indextts2_b200 import layered_engine
+from maxtext_indextts2_b200 import page_manager as pm
+
+
+class _Stream:
+  def __init__(self):
+    self.queue = []
+
+  def synchronize(self):
+    while self.queue:
+      self.queue.pop(0)()
+
+  def wait_event(self, event):
+    self.queue.append(event.synchronize)
+
+
+class _Event:
+  def __init__(self):
+    self.stream, self.left = None, None
+
+  def record(self, stream):
+    self.stream, self.left = stream, object()
+    mark = self.left
+    stream.queue.append(lambda: mark)
+    self.item = stream.queue[-1]
+
+  def synchronize(self):
+    while self.stream is not None and self.item in self.stream.queue:
+      self.stream.queue.pop(0)()
+
+
+class _DeviceBuffer:
+  def __init__(self, now, *shape):
+    self.now_stream, self.now = now, np.zeros(shape, np.int32)
+
+  def __getitem__(self, rows):
+    return self
+
+  def copy_(self, src, non_blocking=False):
+    assert non_blocking
+    self.now_stream[0].queue.append(lambda: self.now.__setitem__(slice(None), src.numpy()))
+
+  def data_ptr(self):
+    return 0
+
+
+def _engine(monkeypatch, rows=40):
+  now = [_Stream()]
+  monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: now[0])
+  e = object.__new__(layered_engine.LayeredEngine)
+  e.config = types.SimpleNamespace(vocab_size=7, per_device_batch_size=3, pagedattn_num_pages=40, pagedattn_tokens_per_page=4, max_target_length=60,
+                                   pagedattn_max_pages_per_group=16)
+  e.device, e._max_rows = torch.device("cpu"), rows
+  e.page_manager = pm.PageManager(e.config)
+  e.page_state = pm.initialize_page_state(40, 3, 16)
+  e._require_params = lambda params: None
+  e._desc_host, e._map_host = torch.zeros(6 * rows + 16, dtype=torch.int32), torch.zeros(3, 16, dtype=torch.int32)
+  e._desc_dev, e._page_map_dev = _DeviceBuffer(now, 6 * rows + 16), _DeviceBuffer(now, 3, 16)
+  e._desc_read, e._map_read, e._step_done = _Event(), _Event(), _Event()
+  e._uploaded_map = None
+  seen = []
+
+  def run(n, token_ptr, group_ptr, pos_ptr, n_want, want_ptr, logits, n_tiles, tiles_ptr, graph=False, n_runs=0, runs_ptr=None):
+    now[0].queue.append(lambda: seen.append((e._desc_dev.now[:n].tolist(), int(e._desc_dev.now[rows]), e._page_map_dev.now.copy())))
+
+  e._run = run
+  return e, now, seen
+
+
+@pytest.mark.parametrize("rows", [40, 8])
+def test_back_to_back_prompts(monkeypatch, rows):
+  e, now, seen = _engine(monkeypatch, rows)
+  maps = []
+  for slot, first in ((0, 100), (2, 200), (1, 300)):
+    e._step([(slot, np.arange(first, first + 8), [7])], wait=False)
+    maps.append(e.page_state.page_map.copy())
+  now[0].synchronize()
+  assert [s[0] for s in seen] == [list(range(f, f + 8)) for f in (100, 200, 300)] and [s[1] for s in seen] == [0, 2, 1]
+  assert all((s[2] == m).all() for s, m in zip(seen, maps))
+  e.step([(0, [5], [0]), (1, [6, 7], [])])  # (a step that waits, behind those)
+  assert seen[-1][0] == [5, 6, 7] and (seen[-1][2] == e.page_state.page_map).all()
+
+
+def test_another_stream_waits(monkeypatch):
+  e, now, seen = _engine(monkeypatch)
+  e._step([(0, [1, 2, 3], [2])], wait=False)
+  first, now[0] = now[0], _Stream()
+  e.step([(1, [4, 5], [1])])
+  assert [s[0] for s in seen] == [[1, 2, 3], [4, 5]] and not first.queue
+  e._step([(2, [6], [])], wait=False)
+  e._step([(0, [7], [])], wait=False)  # (the same stream: nothing to wait for but the buffers)
+  assert not any(getattr(q, "__func__", None) is _Event.synchronize for q in now[0].queue)
+  now[0].synchronize()
+  assert [s[0] for s in seen[2:]] == [[6], [7]]
+
+
+def test_tokens_of_mixed_forms(monkeypatch):
+  """Entries given as lists, arrays and tensors keep their order."""
+  e, now, seen = _engine(monkeypatch)
+  e.step([(0, [1, 2], [0]), (2, np.array([3, 4, 5], np.int64), []), (1, [6], [0])])
+  e.step([(0, torch.tensor([7, 8]), [1]), (1, (9,), [0]), (2, [True, 2.0], [])])
+  assert [s[0] for s in seen] == [[1, 2, 3, 4, 5, 6], [7, 8, 9, 1, 2]]
