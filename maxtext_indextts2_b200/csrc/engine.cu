@@ -357,6 +357,13 @@ int launch_prefill_attention(mtx_engine* e, int layer, int rows, int start_pos, 
   return launch(prefill_attn_kernel<128>, grid, block, smem, st, e->tm_k, e->tm_v, p);
 }
 
+int launch_qk_norm(const QkNormArgs& a, cudaStream_t st) {
+  const dim3 grid((a.rows * (a.hq + 2 * a.hkv) + kQkNormWarps - 1) / kQkNormWarps), block(kQkNormWarps * 32);
+  if (a.d == 64) return launch(qk_norm_rope_append_kernel<1>, grid, block, 0, st, a);
+  if (a.d == 128) return launch(qk_norm_rope_append_kernel<2>, grid, block, 0, st, a);
+  return launch(qk_norm_rope_append_kernel<4>, grid, block, 0, st, a);  // (head_dim 256: mtx_create takes no others)
+}
+
 // Prompt positions with heads of 256 (attention_wide.cuh): groups of positions share the K / V tiles.  Where the 256-row steps cut a position's keys
 // over several work items (fewer (position, kv head) pairs than CTAs are worth filling), they stay with decode_attn_wide_kernel.
 bool takes_prompt_wide(const mtx_engine* e, int rows) {
@@ -823,7 +830,8 @@ int enqueue_prefill_pass(mtx_engine* e, int rows, const int32_t* tokens, int sta
       qa.t_alloc = c.max_target_len;
       qa.eps = c.rms_eps;
       qa.q_scalar = c.query_scalar;
-      MTX_TRY(launch(qk_norm_rope_append_kernel, dim3(rows, c.num_q_heads + 2 * c.num_kv_heads), dim3(c.head_dim / 2), 0, st, qa));
+      qa.rows = rows;
+      MTX_TRY(launch_qk_norm(qa, st));
     } else {
       WideEpi<EPI_QKV_ROPE> qkv;
       memset(&qkv, 0, sizeof(qkv));
@@ -1029,7 +1037,8 @@ int enqueue_step(mtx_engine* e, int mode, int rows, const int32_t* chunk_tokens,
       qa.t_alloc = c.max_target_len;
       qa.eps = c.rms_eps;
       qa.q_scalar = c.query_scalar;
-      MTX_TRY(launch(qk_norm_rope_append_kernel, dim3(rows, c.num_q_heads + 2 * c.num_kv_heads), dim3(c.head_dim / 2), 0, st, qa));
+      qa.rows = rows;
+      MTX_TRY(launch_qk_norm(qa, st));
 
       g_class = KC_ATTENTION;
       // A row whose window holds no valid key (a prompt shorter than max_prefill_len - window while the ring's window is still

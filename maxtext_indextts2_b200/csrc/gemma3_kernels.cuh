@@ -21,58 +21,105 @@ struct QkNormArgs {
   bf16* q_out;           // [rows, Hq D]
   bf16* k_cache;         // this layer's [planes, Hkv, t_alloc, D]
   bf16* v_cache;
-  int hq, hkv, d, t_alloc;
+  int rows, hq, hkv, d, t_alloc;
   float eps, q_scalar;   // normalization_layer_epsilon; query_pre_attn_scalar (0 / 1: none)
 };
 
-// One CTA per (row, head), D / 2 threads: thread i owns dims i and i + D/2 (the RoPE pair, embeddings.py:304-315).
+// A warp per (row, head); lane l owns the RoPE pairs (i, i + D/2), i = E l .. E l + E - 1 (embeddings.py:304-315), E = D / 64.
 //   q, k:  y = bf16(x * rsqrt(mean(x^2) + eps)); y = bf16(y * scale)          normalizations.py:57-69 over head_dim
 //          RoPE with every product rounded to bf16 (bf16 arrays in the reference)
 //   q:     bf16(q * query_pre_attn_scalar)                                      attentions.py:2263-2265
 //   k, v:  appended to the cache row (kvcache.py:626-718)
-__global__ void __launch_bounds__(128) qk_norm_rope_append_kernel(const QkNormArgs a) {
-  __shared__ float s_part[4];
+// The squares of pairs i ^ 16, i ^ 8, .. i ^ 1 are added first and the sums of 32 pairs in order: the order of a block with a thread per pair.
+//
+// Bound: HBM / L2 traffic (4 D bytes per row and head).  3001 rows of 16 heads of 256: 53 us with a block of 128 threads per (row, head) that moved two
+// bytes per thread, 24 us so.
+constexpr int kQkNormWarps = 8;
+
+template <int E>
+__device__ __forceinline__ void qk_load(const bf16* src, float (&x)[E]) {
+  if constexpr (E == 1) {
+    x[0] = __bfloat162float(src[0]);
+  } else {
+    uint32_t w[E / 2];
+    if constexpr (E == 4) {
+      const uint2 raw = *reinterpret_cast<const uint2*>(src);
+      w[0] = raw.x, w[1] = raw.y;
+    } else {
+      w[0] = *reinterpret_cast<const uint32_t*>(src);
+    }
+#pragma unroll
+    for (int e = 0; e < E; e += 2) x[e] = bf16_lo(w[e / 2]), x[e + 1] = bf16_hi(w[e / 2]);
+  }
+}
+template <int E>
+__device__ __forceinline__ void qk_store(bf16* dst, const float (&x)[E]) {
+  if constexpr (E == 1) dst[0] = __float2bfloat16_rn(x[0]);
+  else if constexpr (E == 2) *reinterpret_cast<uint32_t*>(dst) = pack_bf16x2(x[0], x[1]);
+  else *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]));
+}
+
+template <int E>
+__global__ void __launch_bounds__(kQkNormWarps * 32) qk_norm_rope_append_kernel(const QkNormArgs a) {
   griddep_launch_dependents();
   griddep_wait();
-  const int r = blockIdx.x, head = blockIdx.y, i = threadIdx.x;
-  const int D = a.d, half = D >> 1;
+  constexpr int D = 64 * E, half = D / 2;
+  const int heads = a.hq + 2 * a.hkv, u = blockIdx.x * kQkNormWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int r = u / heads, head = u - r * heads, i0 = E * lane;
+  if (r >= a.rows) return;
   const bool is_q = head < a.hq, is_k = !is_q && head < a.hq + a.hkv;
-  const bf16* src = a.qkv + (long long)r * (a.hq + 2 * a.hkv) * D + (long long)head * D;
-  float x0 = __bfloat162float(src[i]), x1 = __bfloat162float(src[i + half]);
+  const bf16* src = a.qkv + (long long)u * D;
+  float x0[E], x1[E];
+  qk_load<E>(src + i0, x0);
+  qk_load<E>(src + half + i0, x1);
   if (is_q || is_k) {
-    float ss = x0 * x0 + x1 * x1;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    if ((i & 31) == 0) s_part[i >> 5] = ss;
-    __syncthreads();
-    float tot = 0.0f;
-    for (int w = 0; w < (half + 31) / 32; ++w) tot += s_part[w];
-    const float rstd = 1.0f / sqrtf(tot / float(D) + a.eps);
     const bf16* sc = is_q ? a.q_scale : a.k_scale;
-    x0 = bf16r(bf16r(x0 * rstd) * __bfloat162float(sc[i]));
-    x1 = bf16r(bf16r(x1 * rstd) * __bfloat162float(sc[i + half]));
-    const float2 c = a.rope_cs[(long long)r * half + i];
-    const float f = bf16r(bf16r(x0 * c.x) - bf16r(x1 * c.y));
-    const float s = bf16r(bf16r(x1 * c.x) + bf16r(x0 * c.y));
-    x0 = f;
-    x1 = s;
-    if (is_q && a.q_scalar != 0.0f && a.q_scalar != 1.0f) {
-      x0 = bf16r(x0 * a.q_scalar);
-      x1 = bf16r(x1 * a.q_scalar);
+    float s0[E], s1[E], ss[E];
+    float2 c[E];
+    qk_load<E>(sc + i0, s0);
+    qk_load<E>(sc + half + i0, s1);
+#pragma unroll
+    for (int e = 0; e < E; ++e) c[e] = a.rope_cs[(long long)r * half + i0 + e];
+#pragma unroll
+    for (int e = 0; e < E; ++e) ss[e] = x0[e] * x0[e] + x1[e] * x1[e];
+#pragma unroll
+    for (int o = 16; o >= E; o >>= 1)
+#pragma unroll
+      for (int e = 0; e < E; ++e) ss[e] += __shfl_xor_sync(0xffffffffu, ss[e], o / E);
+#pragma unroll
+    for (int o = E / 2; o > 0; o >>= 1) {
+      float t[E];
+#pragma unroll
+      for (int e = 0; e < E; ++e) t[e] = ss[e] + ss[e ^ o];
+#pragma unroll
+      for (int e = 0; e < E; ++e) ss[e] = t[e];
+    }
+    float tot = 0.0f;
+#pragma unroll
+    for (int w = 0; w < E; ++w) tot += __shfl_sync(0xffffffffu, ss[0], w * (32 / E));
+    const float rstd = 1.0f / sqrtf(tot / float(D) + a.eps);
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const float y0 = bf16r(bf16r(x0[e] * rstd) * s0[e]), y1 = bf16r(bf16r(x1[e] * rstd) * s1[e]);
+      x0[e] = bf16r(bf16r(y0 * c[e].x) - bf16r(y1 * c[e].y));
+      x1[e] = bf16r(bf16r(y1 * c[e].x) + bf16r(y0 * c[e].y));
+      if (is_q && a.q_scalar != 0.0f && a.q_scalar != 1.0f) {
+        x0[e] = bf16r(x0[e] * a.q_scalar);
+        x1[e] = bf16r(x1[e] * a.q_scalar);
+      }
     }
   }
+  bf16* dst;
   if (is_q) {
-    bf16* dst = a.q_out + (long long)r * a.hq * D + (long long)head * D;
-    dst[i] = __float2bfloat16_rn(x0);
-    dst[i + half] = __float2bfloat16_rn(x1);
+    dst = a.q_out + (long long)r * a.hq * D + (long long)head * D;
   } else {
     const int wr = a.write_row[r];
     if (wr < 0) return;
     const int kvh = is_k ? head - a.hq : head - a.hq - a.hkv;
-    bf16* dst = (is_k ? a.k_cache : a.v_cache) + (((long long)a.plane[r] * a.hkv + kvh) * a.t_alloc + wr) * D;
-    dst[i] = __float2bfloat16_rn(x0);
-    dst[i + half] = __float2bfloat16_rn(x1);
+    dst = (is_k ? a.k_cache : a.v_cache) + (((long long)a.plane[r] * a.hkv + kvh) * a.t_alloc + wr) * D;
   }
+  qk_store<E>(dst + i0, x0);
+  qk_store<E>(dst + half + i0, x1);
 }
 
 // out[r, :] = bf16(resid[r, :] + RMSNorm(y[r, :]; scale))   (gemma3.py:142-153 / 161-170), and the per-128-feature-tile sums of
