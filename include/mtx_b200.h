@@ -258,6 +258,10 @@ int mtx_prefill_chunk(mtx_engine* e, const int32_t* tokens, int count, int start
 int mtx_prefill_rows(mtx_engine* e, const int32_t* tokens, int count, int start_pos, int slot, int sample_last, int draw_row, int32_t* first_token,
                      float* logits_out, float* first_log_prob, mtx_stream stream);
 
+/* What a prefill left: the first n_rows cache rows of plane `slot` of every layer and head into k_out / v_out [L, Hkv, n_rows, D] bf16 (the prefix that
+ * MaxEngine.prefill returns). */
+int mtx_copy_prefix(mtx_engine* e, int n_rows, int slot, void* k_out, void* v_out, mtx_stream stream);
+
 /* MaxEngine.insert (maxengine.py:1166-1192, _insert_jit :1045-1164): the first n_rows cache rows of a prefix (k_src / v_src
  * [L, Hkv, n_src_rows, D] bf16, what prefill left) into the prefill segment of decode slot `slot`, every layer and head in one
  * launch, and the slot's bookkeeping: prefill_len = n_rows, ar_lengths = 0, next_pos / generated / tokens as given.  The AR ring

@@ -344,6 +344,8 @@ def _declare(lib) -> None:
   lib.mtx_prefill_chunk.argtypes = [vp, vp, i32, i32, i32, i32, vp, vp, vp, vp]
   lib.mtx_prefill_rows.restype = i32
   lib.mtx_prefill_rows.argtypes = [vp, vp, i32, i32, i32, i32, i32, vp, vp, vp, vp]
+  lib.mtx_copy_prefix.restype = i32
+  lib.mtx_copy_prefix.argtypes = [vp, i32, i32, vp, vp, vp]
   lib.mtx_insert_prefix.restype = i32
   lib.mtx_insert_prefix.argtypes = [vp, vp, vp, i32, i32, i32, i32, i32, i32, vp]
   lib.mtx_rmsnorm.restype = i32

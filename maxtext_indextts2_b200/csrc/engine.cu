@@ -2028,6 +2028,28 @@ int mtx_prefill_rows(mtx_engine* e, const int32_t* tokens, int count, int start_
   return sample_last ? enqueue_last_logits(e, last, draw_row, first_token, logits_out, first_log_prob, st) : MTX_OK;
 }
 
+int mtx_copy_prefix(mtx_engine* e, int n_rows, int slot, void* k_out, void* v_out, mtx_stream stream) {
+  if (!e || !e->bound || !k_out || !v_out) return fail(MTX_ERR_ARG, "engine is not bound / null prefix");
+  const mtx_model_config& c = e->cfg;
+  if (slot < 0 || slot >= c.num_slots) return fail(MTX_ERR_ARG, "slot out of range");
+  if (n_rows < 1 || n_rows > c.max_prefill_len) return fail(MTX_ERR_ARG, "prefix rows %d outside [1, %d]", n_rows, c.max_prefill_len);
+  if (((reinterpret_cast<uintptr_t>(k_out) | reinterpret_cast<uintptr_t>(v_out)) & 15) != 0) return fail(MTX_ERR_ARG, "a prefix starts on 16-byte boundaries");
+  PrefixCopyArgs a;
+  memset(&a, 0, sizeof(a));
+  a.k_cache = static_cast<const bf16*>(e->s.k_cache);
+  a.v_cache = static_cast<const bf16*>(e->s.v_cache);
+  a.k_out = static_cast<bf16*>(k_out);
+  a.v_out = static_cast<bf16*>(v_out);
+  a.planes = staged_prefill(c) ? 1 : c.num_slots;
+  a.slot = staged_prefill(c) ? 0 : slot;
+  a.hkv = c.num_kv_heads;
+  a.T = c.max_target_len;
+  a.D = c.head_dim;
+  a.n = n_rows;
+  const int per_cta = 256 * kPrefixVecs, pieces = (n_rows * (c.head_dim / 8) + per_cta - 1) / per_cta;
+  return launch(prefix_copy_kernel, dim3(pieces, c.num_layers * c.num_kv_heads, 2), dim3(256), 0, static_cast<cudaStream_t>(stream), a);
+}
+
 int mtx_insert_prefix(mtx_engine* e, const void* k_src, const void* v_src, int n_rows, int n_src_rows, int slot, int next_pos, int generated,
                       int token, mtx_stream stream) {
   if (!e || !e->bound || !k_src || !v_src) return fail(MTX_ERR_ARG, "engine is not bound / null prefix");

@@ -690,11 +690,13 @@ class MaxEngine:
                                             self._stream()))
     first = self._first_token.clone().reshape(1, 1)
     full_true_length = start_position + true_length  # maxengine.py:442
+    key, value = (torch.empty(t.shape[0], t.shape[2], full_true_length, t.shape[4], dtype=t.dtype, device=t.device) for t in (self._k, self._v))  # [L, Hkv, len, D]
+    _lib.check(self.lib.mtx_copy_prefix(self._handle, full_true_length, self._staging, ctypes.c_void_p(key.data_ptr()), ctypes.c_void_p(value.data_ptr()), self._stream()))
     prefix = {
         "logits": self._prefill_logits.clone().reshape(1, 1, -1) if want_logits else None,
         "cache": {
-            "key": self._k[:, self._staging, :, :full_true_length].clone(),  # [L, Hkv, len, D]
-            "value": self._v[:, self._staging, :, :full_true_length].clone(),
+            "key": key,
+            "value": value,
             "prefill_length": full_true_length,
         },
         "next_pos": torch.full((1, 1), full_true_length, dtype=torch.int32, device=self.device),
