@@ -419,61 +419,81 @@ __device__ __forceinline__ float4 pk_logit_transform(const EpiArgs& e, float4 a)
   return a;
 }
 
-// Sampling partials of one parked logits tile ([rows][kPkParkPitch] fp32 accumulators in shared memory).  Two
-// threads scan one row (alternating 4-wide chunks, so the 8 lanes of a shared-memory phase hit distinct banks):
-// the row's best candidate of this tile (lowest index wins ties, jnp.argmax), optionally Gumbel-perturbed
-// (jax.random.categorical), and the (max, sum exp) pair for log-softmax.  No cross-lane traffic but one shuffle.
+// Threads that scan one row of a parked logits tile: as many as 128 threads have for the step's rows, at most a warp.
+__device__ __forceinline__ int pk_scan_threads(int rows) { return rows > 32 ? 2 : rows > 16 ? 4 : rows > 8 ? 8 : rows > 4 ? 16 : 32; }
+
+// Sampling partials of one parked logits tile ([rows][kPkParkPitch] fp32 accumulators in shared memory).  A row's threads take its 4-wide chunks in turn (so
+// the 8 lanes of a shared-memory phase hit distinct banks): the row's best candidate of this tile (lowest index wins ties, jnp.argmax), optionally
+// Gumbel-perturbed (jax.random.categorical), and the (max, sum exp) pair for log-softmax, the maximum brought up once per 16 values.
+// Bound: latency -- the tile's epilogue has to be over when the next tile's weights are there.  With two threads per row whatever the rows and a
+// running maximum per value the logits of one row of 256 took 89 us (135 MB), of 64 rows of 1280 137 us (676 MB): 35 and 119 us so.
 __device__ __forceinline__ void pk_logits_scan(const float* park, int wtid, int rows, int tile, const EpiArgs& e, int V, uint32_t step, uint64_t seed) {
-  const int r = wtid >> 1, half = wtid & 1;
+  const int T = pk_scan_threads(rows), r = wtid / T, part = wtid % T;
   const bool active = r < rows;
   float best = -INFINITY, raw = -INFINITY, mx = -INFINITY, sum = 0.0f;
   int bi = 0x7fffffff;
   if (active) {
     const float* row = park + r * kPkParkPitch;
-#pragma unroll 4
-    for (int i = 0; i < 16; ++i) {
-      const int c = (2 * i + half) * 4;
-      const int n0 = tile * 128 + c;
-      const float4 lg4 = pk_logit_transform(e, *reinterpret_cast<const float4*>(row + c));
-      const float lg[4] = {lg4.x, lg4.y, lg4.z, lg4.w};
-      // the four ids of the chunk share one Philox block when the shard starts at a multiple of four
-      float gn[4] = {0.f, 0.f, 0.f, 0.f};
-      if (e.gumbel) {
-        if ((e.vocab_offset & 3) == 0) {
-          const float4 g4 = gumbel_noise4(seed, step, uint32_t(e.row_offset + r), uint32_t(e.vocab_offset + n0));
-          gn[0] = g4.x; gn[1] = g4.y; gn[2] = g4.z; gn[3] = g4.w;
-        } else {
+#pragma unroll 1
+    for (int c0 = part; c0 < 32; c0 += 4 * T) {  // four chunks of this thread
+      float lg[16], top = -INFINITY;
 #pragma unroll
-          for (int q = 0; q < 4; ++q) gn[q] = gumbel_noise(seed, step, uint32_t(e.row_offset + r), uint32_t(e.vocab_offset + n0 + q));
+      for (int i = 0; i < 4; ++i) {
+        const int c = (c0 + i * T) * 4, n0 = tile * 128 + c;
+        const float4 lg4 = c < 128 ? pk_logit_transform(e, *reinterpret_cast<const float4*>(row + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        lg[4 * i] = lg4.x, lg[4 * i + 1] = lg4.y, lg[4 * i + 2] = lg4.z, lg[4 * i + 3] = lg4.w;
+        // the four ids of the chunk share one Philox block when the shard starts at a multiple of four
+        float gn[4] = {0.f, 0.f, 0.f, 0.f};
+        if (e.gumbel && c < 128) {
+          if ((e.vocab_offset & 3) == 0) {
+            const float4 g4 = gumbel_noise4(seed, step, uint32_t(e.row_offset + r), uint32_t(e.vocab_offset + n0));
+            gn[0] = g4.x; gn[1] = g4.y; gn[2] = g4.z; gn[3] = g4.w;
+          } else {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) gn[q] = gumbel_noise(seed, step, uint32_t(e.row_offset + r), uint32_t(e.vocab_offset + n0 + q));
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float x = lg[4 * i + q];
+          if (c < 128 && n0 + q < V) {
+            const float sc = e.gumbel ? x * e.inv_temp + gn[q] : x;
+            if (sc > best) { best = sc; raw = x; bi = n0 + q; }  // ascending scan: strict > keeps the lowest index
+            top = fmaxf(top, x);
+          } else {
+            lg[4 * i + q] = -INFINITY;
+          }
         }
       }
+      if (e.want_lse) {
+        const float mn = fmaxf(mx, top);
+        if (mn > -INFINITY) {
+          float s[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        if (n0 + q < V) {
-          const float sc = e.gumbel ? lg[q] * e.inv_temp + gn[q] : lg[q];
-          if (sc > best) { best = sc; raw = lg[q]; bi = n0 + q; }  // ascending scan: strict > keeps the lowest index
-          if (e.want_lse) {
-            const float mn = fmaxf(mx, lg[q]);
-            sum = sum * __expf(mx - mn) + __expf(lg[q] - mn);
-            mx = mn;
-          }
+          for (int j = 0; j < 16; ++j) s[j & 3] += __expf(lg[j] - mn);
+          sum = sum * __expf(mx - mn) + ((s[0] + s[1]) + (s[2] + s[3]));
+          mx = mn;
+        } else {  // (nothing but values that compare with nothing)
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (lg[j] != lg[j]) sum = lg[j];
         }
       }
     }
   }
-  {  // combine the two halves of the row
-    const float b2 = __shfl_xor_sync(0xffffffffu, best, 1);
-    const float r2 = __shfl_xor_sync(0xffffffffu, raw, 1);
-    const int i2 = __shfl_xor_sync(0xffffffffu, bi, 1);
+  for (int o = 1; o < T; o <<= 1) {  // combine the row's threads
+    const float b2 = __shfl_xor_sync(0xffffffffu, best, o);
+    const float r2 = __shfl_xor_sync(0xffffffffu, raw, o);
+    const int i2 = __shfl_xor_sync(0xffffffffu, bi, o);
     if (b2 > best || (b2 == best && i2 < bi)) { best = b2; raw = r2; bi = i2; }
     if (e.want_lse) {
-      const float m2 = __shfl_xor_sync(0xffffffffu, mx, 1), s2 = __shfl_xor_sync(0xffffffffu, sum, 1);
+      const float m2 = __shfl_xor_sync(0xffffffffu, mx, o), s2 = __shfl_xor_sync(0xffffffffu, sum, o);
       const float mn = fmaxf(mx, m2);
       if (mn > -INFINITY) sum = sum * __expf(mx - mn) + s2 * __expf(m2 - mn);
       mx = mn;
     }
   }
-  if (active && half == 0) {
+  if (active && part == 0) {
     const long long o = (long long)r * e.n_tiles + tile;
     e.part_score[o] = best;
     e.part_idx[o] = e.vocab_offset + bi;
