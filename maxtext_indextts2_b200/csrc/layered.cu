@@ -69,6 +69,9 @@ struct mtx_layered {
   int max_rec_gate = 0, max_rec_z = 0;
   bool outlayer = false;  // MTX_NORM_OUT_LAYER layers
   float *rec_gate = nullptr, *rec_z = nullptr;
+  size_t max_before = 0;   // decayed sums: elements of the states before one chunk (decayed_before_elems)
+  int decay_chunks = 0;    // chunks whose states the workspace holds
+  bf16* rec_s = nullptr;
   float* rec_n = nullptr;  // mLSTM: new n [groups, heads, dim], then new m [groups, heads]
 };
 
@@ -79,7 +82,7 @@ size_t elem(const mtx_layered* e) { return e->cfg.float32 ? 4 : 2; }
 struct LWs {
   size_t x, y, qkv, v_shared, xa, q, attn, act, wanted, obf, attn_part, total;
   size_t smax_ml, x0, rec_o, rec_aux, moe_logits, moe_weight, moe_y, moe_chosen, moe_slot, moe_row, moe_off, moe_act;
-  size_t h, xb, lat_q, lat_o, rec_gate, rec_z, rec_n;
+  size_t h, xb, lat_q, lat_o, rec_gate, rec_z, rec_n, rec_s;
 };
 
 LWs layered_layout(const mtx_layered* e) {
@@ -123,6 +126,7 @@ LWs layered_layout(const mtx_layered* e) {
   L.rec_gate = take(R * size_t(e->max_rec_gate > 0 ? e->max_rec_gate : 1) * 4);
   L.rec_z = take(R * size_t(e->max_rec_z > 0 ? e->max_rec_z : 1) * 4);
   L.rec_n = take(size_t(c.num_groups > 0 ? c.num_groups : 1) * size_t(e->max_rec_n) * 2 * 4 + 4);
+  L.rec_s = take(size_t(e->decay_chunks) * e->max_before * 2 + 4);
   L.lat_q = take(R * size_t(e->max_lat_q > 0 ? e->max_lat_q : 1) * 4);
   L.lat_o = take(R * size_t(e->max_lat_o > 0 ? e->max_lat_o : 1) * es);
   L.total = off;
@@ -1931,6 +1935,34 @@ bool use_decayed_chunks(const mtx_layered* e, const mtx_ragged_batch& b) {
   return on != 0 && !e->cfg.float32 && b.rows >= 4 * b.n_runs;
 }
 
+// States and outputs in launches of their own: where a run has two chunks and more on average (one chunk of
+// decayed_chunks_kernel takes about two microseconds, which is what the second launch costs), the
+// copies are 16-byte ones and the workspace holds every chunk's state.
+bool use_decayed_split(const mtx_layered* e, const mtx_ragged_batch& b, const DecayedChunksArgs& da) {
+  static int on = env_int("MTX_DECAY_SPLIT", 1);
+  return on != 0 && da.vec8 && b.rows >= 2 * kDcTokens * b.n_runs && b.rows / kDcTokens + b.n_runs <= e->decay_chunks &&
+         decayed_states_smem_bytes(da.dim) <= 200 * 1024 && decayed_outputs_smem_bytes(da.dim, da.vdim) <= 200 * 1024;
+}
+int launch_decayed_split(mtx_layered* e, const DecayedChunksArgs& da, const mtx_ragged_batch& b, cudaStream_t st) {
+  DecayedSplitArgs sa;
+  memset(&sa, 0, sizeof(sa));
+  sa.a = da;
+  sa.before = e->rec_s;
+  sa.n_runs = b.n_runs;
+  const size_t s1 = decayed_states_smem_bytes(da.dim), s2 = decayed_outputs_smem_bytes(da.dim, da.vdim);
+  static size_t have1 = 48 * 1024, have2 = 48 * 1024;
+  if (s1 > have1) {
+    MTX_CUDA(cudaFuncSetAttribute(decayed_states_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(s1)));
+    have1 = s1;
+  }
+  if (s2 > have2) {
+    MTX_CUDA(cudaFuncSetAttribute(decayed_outputs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(s2)));
+    have2 = s2;
+  }
+  MTX_TRY(launch(decayed_states_kernel, dim3(b.n_runs, da.heads, (da.vdim + kDcCols - 1) / kDcCols), dim3(32 * (mat_pad16(da.dim) / 16)), s1, st, sa));
+  return launch(decayed_outputs_kernel, dim3(b.rows / kDcTokens + b.n_runs, da.heads), dim3(128), s2, st, sa);
+}
+
 // a MTX_NORM_OUT_LAYER layer: both sublayers read x itself (xa = x in the matmul dtype)
 template <typename T>
 int outlayer_layer(mtx_layered* e, int li, const mtx_ragged_batch& b, cudaStream_t st) {
@@ -2019,7 +2051,8 @@ int outlayer_layer(mtx_layered* e, int li, const mtx_ragged_batch& b, cudaStream
       da.vdim = r.vdim;
       da.q_scale = r.q_scale;
       da.vec8 = (n_in % 8 == 0 && cc.rq % 8 == 0 && r.dim % 8 == 0 && r.vdim % 8 == 0) ? 1 : 0;
-      if (chunks_bf16) MTX_TRY(launch_decayed_chunks<bf16>(da, b.n_runs, st));
+      if (chunks_bf16 && use_decayed_split(e, b, da)) MTX_TRY(launch_decayed_split(e, da, b, st));
+      else if (chunks_bf16) MTX_TRY(launch_decayed_chunks<bf16>(da, b.n_runs, st));
       else MTX_TRY(launch_decayed_chunks<float>(da, b.n_runs, st));
     } else {
       RecScanArgs ra;
@@ -2371,6 +2404,8 @@ int check_outlayer(mtx_layered* e, int i) {
     if (!r.state_s || !r.out_norm || !r.head_decay) return fail(MTX_ERR_ARG, "layer %d: the recurrence's state, output norm or decays are missing", i);
     if (r.norm_whole && r.heads * r.vdim > 256 * kRecOutVec) return fail(MTX_ERR_UNSUPPORTED, "layer %d: heads * vdim = %d exceeds %d", i, r.heads * r.vdim, 256 * kRecOutVec);
     if (r.heads * r.vdim > e->max_rec_o) e->max_rec_o = r.heads * r.vdim;
+    const size_t before = e->cfg.float32 ? 0 : decayed_before_elems(r.heads, r.dim, r.vdim);
+    if (before > e->max_before) e->max_before = before;
   }
   const CompositeCols cc = composite_cols(l);
   if (l.n_in < cc.n) return fail(MTX_ERR_ARG, "layer %d: n_in = %d, the sub-mixers need %d projection rows", i, l.n_in, cc.n);
@@ -2483,6 +2518,10 @@ int mtx_layered_create(const mtx_layered_config* cfg, const mtx_layer_desc* laye
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0) e->num_sms = sms;
   cudaGetLastError();
+  if (e->max_before > 0 && e->cfg.max_rows >= 2 * kDcTokens) {  // a step of max_rows in a few runs, or what 256 MB hold
+    const size_t most = (size_t(256) << 20) / (e->max_before * 2), want = size_t(e->cfg.max_rows / kDcTokens) + 8;
+    e->decay_chunks = int(want < most ? want : most);
+  }
   e->ws_bytes = layered_layout(e).total;
   *out = e;
   return MTX_OK;
@@ -2535,6 +2574,7 @@ int mtx_layered_bind(mtx_layered* e, void* workspace, size_t workspace_bytes) {
   e->rec_gate = reinterpret_cast<float*>(base + L.rec_gate);
   e->rec_z = reinterpret_cast<float*>(base + L.rec_z);
   e->rec_n = reinterpret_cast<float*>(base + L.rec_n);
+  e->rec_s = reinterpret_cast<bf16*>(base + L.rec_s);
   e->bound = true;
   return MTX_OK;
 }
