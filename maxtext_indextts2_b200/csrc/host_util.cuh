@@ -102,6 +102,21 @@ int make_map_u8(CUtensorMap* m, const void* base, uint64_t outer) {
   return MTX_OK;
 }
 
+// fp32 rows [rows, ld] that hold `heads` vectors of `dim` side by side from `base` on, box [box_inner, 1 head, box_rows]; elements beyond dim and rows are zero.
+int make_map_heads_f32(CUtensorMap* m, const float* base, uint64_t dim, uint64_t heads, uint64_t rows, uint64_t ld, uint32_t box_inner, uint32_t box_rows) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (fn == nullptr) return fail(MTX_ERR_CUDA, "cuTensorMapEncodeTiled is not available (no CUDA driver?)");
+  if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || dim % 4 != 0 || ld % 4 != 0) return fail(MTX_ERR_ARG, "TMA needs a 16-byte aligned base and row pitch");
+  const cuuint64_t dims[3] = {dim, heads, rows};
+  const cuuint64_t strides[2] = {dim * 4, ld * 4};
+  const cuuint32_t box[3] = {box_inner, 1, box_rows};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  CUresult rc = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (rc != CUDA_SUCCESS) return fail(MTX_ERR_CUDA, "cuTensorMapEncodeTiled (fp32 heads) failed with CUresult %d", int(rc));
+  return MTX_OK;
+}
+
 // ---- launch helper -------------------------------------------------------------------------
 
 // Optional per-kernel timing: when a sink is installed every launch is bracketed by CUDA

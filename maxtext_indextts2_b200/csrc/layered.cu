@@ -724,15 +724,28 @@ int launch_rec_scan_cb(const RecScanArgs& ra, int n_runs, cudaStream_t st) {
   return fail(MTX_ERR_UNSUPPORTED, "recurrence: dim %d", ra.dim);
 }
 
-template <int KIND, int RPT>
-int launch_rec_walk(const RecScanArgs& ra, int n_runs, cudaStream_t st) {
-  const size_t smem = rec_walk_smem_bytes(KIND, ra.dim);
-  static size_t have = 0;  // per instantiation
-  if (smem > 48 * 1024 && smem > have) {
-    MTX_CUDA(cudaFuncSetAttribute(recurrent_walk_kernel<KIND, RPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    have = smem;
+template <int KIND, int RPT, int C>
+int launch_rec_walk_t(const RecScanArgs& ra, int n_runs, cudaStream_t st) {
+  constexpr int CB = 2 * kWalkWarps * C, QP = kWalkSlices * RPT;
+  const size_t smem = rec_walk_smem_bytes(KIND, RPT, C);
+  static bool attr_set = false;  // per instantiation
+  if (!attr_set && smem > 48 * 1024) {
+    MTX_CUDA(cudaFuncSetAttribute(recurrent_walk_kernel<KIND, RPT, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    attr_set = true;
   }
-  return launch(recurrent_walk_kernel<KIND, RPT>, dim3(n_runs, ra.heads, (ra.vdim + kWalkCols - 1) / kWalkCols), dim3(kWalkCols * kWalkSlices), smem, st, ra);
+  CUtensorMap tm_q, tm_k, tm_a, tm_v;
+  MTX_TRY(make_map_heads_f32(&tm_q, ra.proj + ra.q_col, ra.dim, ra.heads, ra.rows, ra.ld, QP, kWalkTokens));
+  MTX_TRY(make_map_heads_f32(&tm_k, ra.proj + ra.k_col, ra.dim, ra.heads, ra.rows, ra.ld, QP, kWalkTokens));
+  if (KIND == REC_GLA) MTX_TRY(make_map_heads_f32(&tm_a, ra.aux, ra.dim, ra.heads, ra.rows, (long long)ra.heads * ra.dim, QP, kWalkTokens));
+  else tm_a = tm_k;
+  MTX_TRY(make_map_heads_f32(&tm_v, ra.proj + ra.v_col, ra.vdim, ra.heads, ra.rows, ra.ld, CB, kWalkTokens));
+  return launch(recurrent_walk_kernel<KIND, RPT, C>, dim3(n_runs, ra.heads, (ra.vdim + CB - 1) / CB), dim3(kWalkThreads), smem, st, tm_q, tm_k, tm_a, tm_v, ra);
+}
+template <int KIND, int RPT>
+int launch_rec_walk(const RecScanArgs& ra, int n_runs, int num_sms, cudaStream_t st) {
+  // one column per thread while that leaves every CTA an SM of its own
+  const bool single = (long long)n_runs * ra.heads * ((ra.vdim + 2 * kWalkWarps - 1) / (2 * kWalkWarps)) <= num_sms;
+  return single ? launch_rec_walk_t<KIND, RPT, 1>(ra, n_runs, st) : launch_rec_walk_t<KIND, RPT, 2>(ra, n_runs, st);
 }
 
 // A walk is bound by latency, so what counts is how many warps share an SM.  16 value columns per CTA when that still gives every
@@ -750,9 +763,10 @@ int launch_rec_scan(mtx_layered* e, RecScanArgs& ra, int n_runs, int rows, cudaS
     static const int walk = env_int("MTX_REC_WALK", 1);
     if (walk && fine && ra.vec4 && ra.dim <= 256 && rows >= kWalkTokens * n_runs) {
       const int rpt = rec_rpt(ra.dim, kWalkSlices);
-      if (rpt == 4) return launch_rec_walk<KIND, 4>(ra, n_runs, st);
-      if (rpt == 8) return launch_rec_walk<KIND, 8>(ra, n_runs, st);
-      return launch_rec_walk<KIND, 16>(ra, n_runs, st);
+      ra.rows = rows;
+      if (rpt == 4) return launch_rec_walk<KIND, 4>(ra, n_runs, e->num_sms, st);
+      if (rpt == 8) return launch_rec_walk<KIND, 8>(ra, n_runs, e->num_sms, st);
+      return launch_rec_walk<KIND, 16>(ra, n_runs, e->num_sms, st);
     }
   }
   if (fine && ra.dim >= 16) return launch_rec_scan_cb<KIND, 8, 16>(ra, n_runs, st);

@@ -256,7 +256,7 @@ struct RecScanArgs {
   const int* run_row0; // [n_runs + 1]
   const int* group;
   const int* pos;
-  int heads, dim, vdim, chunk;
+  int heads, dim, vdim, chunk, rows;
   int vec4;            // 1: every staged row starts on a 16-byte boundary and holds whole float4s (set by the host from the sizes)
   float q_scale, denom_eps;
   // REC_GDELTA: q / k head of head h is h / qk_rep (0 or 1: its own); the decays are the columns [dec_col + h * dim, ..) and the write
@@ -637,194 +637,272 @@ __global__ void __launch_bounds__(CB * SL) recurrent_scan_kernel(const RecScanAr
   if (write_n && tid == 0) a.next_m[size_t(slot) * H + h] = m;
 }
 
-// The walk of a long run without a reduction per token (GLA and mLSTM; a column cut into 16 slices, whole float4s): the same CTAs, threads and
-// state as recurrent_scan_kernel<KIND, RPT, 8, 16>, but a thread leaves its slice's part of a token's read-out in shared memory and the parts
-// of 16 tokens x 8 columns are added at the end of the chunk, one output per thread, in the order in which the shuffles added them
-// (pairs of slices, pairs of pairs, ..): the results are the same bits.  The walk is then loads and multiply-adds only: nothing waits
-// for a shuffle.  The mLSTM's running maximum is walked by every warp for itself (lane t keeps token t's factors), without a barrier.
-// One run of 4096 tokens: GLA (16 heads of 64 x 128) and mLSTM (8 heads of 64 x 128) took 486 and 568 us with four shuffles per token, 366 and 315 us so.
-constexpr int kWalkTokens = 16, kWalkCols = 8, kWalkSlices = 16, kWalkPitch = 20;  // (pitch of a column's 16 parts: conflict-free float4 reads)
-inline int rec_walk_parts(int kind) { return kWalkTokens * kWalkCols * kWalkPitch + (kind == REC_MLSTM ? kWalkTokens * kWalkPitch + 4 * kWalkTokens * 4 : 0); }
-inline size_t rec_walk_smem_bytes(int kind, int dim) {
-  return rec_scan_smem_bytes(dim, kWalkCols, kWalkSlices, kWalkTokens, rec_vectors(kind)) + sizeof(float) * rec_walk_parts(kind);
+// The walk of a long run without a reduction per token (GLA and mLSTM; a column cut into 16 slices, whole float4s): a thread leaves its slice's part of a
+// token's read-out in shared memory and the parts of 16 tokens are added at the end of the chunk in the order in which recurrent_scan_kernel's shuffles
+// add them (pairs of slices, pairs of pairs, ..): the results are the same bits.  The walk is then loads and multiply-adds only.
+//
+// Four warps walk, each on its own: a warp has C columns in each of its two halves of 16 slices and keeps its parts to itself, so that nothing but the
+// arrival of a chunk holds it up.  A fifth warp brings the chunks (one TMA box per vector, four stages) and walks the mLSTM's running maximum,
+// whose factors come with the chunk.  C = 2 (each q, k and decay read from shared memory serves two columns) where single columns would not fit on the SMs at once.
+//
+// Bound: the issue of one warp per scheduler, about 40 instructions per token (24 of them multiply-adds) at one in 2.5 clocks; more columns per thread on fewer
+// warps, more warps with fewer, operands read groups of tokens ahead and two-wide multiply-adds were all slower.  One run of 4096 tokens, GLA (16
+// heads of 64 x 128) and mLSTM (8 heads of 64 x 128): 366 and 315 us with eight columns per CTA of 128 threads that staged, walked and added up in turn,
+// 242 and 211 us so.
+constexpr int kWalkTokens = 16, kWalkSlices = 16, kWalkWarps = 4, kWalkStages = 4;
+constexpr int kWalkThreads = (kWalkWarps + 1) * 32;
+__host__ __device__ constexpr int walk_vectors(int kind) { return kind == REC_GLA ? 3 : 2; }  // q, k, GLA: decays
+__host__ __device__ constexpr int walk_token_floats(int kind, int rpt, int c) { return walk_vectors(kind) * kWalkSlices * rpt + 2 * kWalkWarps * c; }
+__host__ __device__ constexpr int walk_stages(int kind, int rpt, int c) {
+  return walk_token_floats(kind, rpt, c) * kWalkTokens * 4 * kWalkStages > 200 * 1024 ? kWalkStages - 1 : kWalkStages;
+}
+inline size_t rec_walk_smem_bytes(int kind, int rpt, int c) {
+  const int stages = walk_stages(kind, rpt, c);
+  return sizeof(float) * (size_t(stages) * kWalkTokens * (walk_token_floats(kind, rpt, c) + 4) + kWalkWarps * kWalkTokens * 16 * (2 * c + 1)) + 2 * stages * 8;
 }
 
-template <int KIND, int RPT>
-__global__ void __launch_bounds__(kWalkCols* kWalkSlices) recurrent_walk_kernel(const RecScanArgs a) {
-  extern __shared__ __align__(16) float rec_smem[];
-  constexpr int NV = rec_vectors(KIND), SL = kWalkSlices, CB = kWalkCols, TC = kWalkTokens;
-  constexpr int NT = CB * SL, QP = SL * RPT, TF = NV * QP + CB + 4, GS = 4 * SL;
-  float* const parts = rec_smem + kRecStages * TC * TF;  // [TC][CB][kWalkPitch]
-  float* const nparts = parts + TC * CB * kWalkPitch;    // mLSTM: [TC][kWalkPitch], column 0's
+// a vector of 16 tokens' heads: the box (channels, one head, tokens) of a plane of rows; what lies beyond a head's channels or the plane's rows is zero
+__device__ __forceinline__ void walk_load(void* dst, const CUtensorMap* tm, int c0, int head, int row, uint64_t* bar) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)),
+               "l"(reinterpret_cast<uint64_t>(tm)), "r"(smem_u32(bar)), "r"(c0), "r"(head), "r"(row)
+               : "memory");
+}
+
+template <int KIND, int RPT, int C>
+__global__ void __launch_bounds__(kWalkThreads) recurrent_walk_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                                                                      const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_v,
+                                                                      const RecScanArgs a) {
+  extern __shared__ __align__(128) float walk_smem[];
+  constexpr int NV = walk_vectors(KIND), SL = kWalkSlices, TC = kWalkTokens, CB = 2 * kWalkWarps * C;
+  constexpr int QP = SL * RPT, SF = TC * walk_token_floats(KIND, RPT, C), GS = 4 * SL, ST = walk_stages(KIND, RPT, C);
+  // a stage: [vector][TC][QP], then the values [TC][CB]
+  float* const factors = walk_smem + ST * SF;           // mLSTM: [stage][TC] keep, put, floor
+  float* const all_parts = factors + ST * TC * 4;       // [warp][TC][2 C + 1][16]: the columns', the normaliser's
+  uint64_t* const full = reinterpret_cast<uint64_t*>(all_parts + kWalkWarps * TC * 16 * (2 * C + 1));
+  uint64_t* const empty = full + ST;
   const int d = a.dim, dv = a.vdim, H = a.heads;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, jl = tid / SL, sl = tid % SL;
-  float* const factors = nparts + TC * kWalkPitch + warp * TC * 4;  // mLSTM, this warp's: [TC] keep, put, floor
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, jl = lane >> 4, sl = lane & 15;
+  if (tid == 0) {
+    for (int i = 0; i < ST; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], kWalkWarps);
+    }
+    fence_barrier_init();
+  }
+  const int col0 = blockIdx.z * CB;
+  __syncthreads();
   griddep_wait();
   const int r0 = a.run_row0[blockIdx.x], nr = a.run_row0[blockIdx.x + 1] - r0, h = blockIdx.y;
   if (nr <= 0) return;
-  const int col0 = blockIdx.z * CB, j = col0 + jl;
-  const bool col_ok = j < dv;
   const int slot = a.group[r0];
   const bool fresh = a.pos[r0] == 0;
+  const int n_chunks = (nr + TC - 1) / TC;
+
+  if (warp == kWalkWarps) {
+    float m = KIND == REC_MLSTM && !fresh ? a.state_m[size_t(slot) * H + h] : 0.0f;
+    // the log gates of 64 tokens, requested 64 tokens ahead: lane t % 32 holds token t's
+    float ig[2], fg[2], ig_next[2], fg_next[2];
+    auto request = [&](int t0) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int t = t0 + 32 * i + lane;
+        const float* g = a.aux + size_t(r0 + t) * 2 * H + h;
+        ig_next[i] = t < nr ? g[0] : -INFINITY;
+        fg_next[i] = t < nr ? g[H] : 0.0f;
+      }
+    };
+    if (KIND == REC_MLSTM) request(0);
+    const bool issuer = elect_one();
+    uint32_t phase = 1;
+    int s = 0;
+    for (int c = 0; c < n_chunks; ++c) {
+      mbar_wait(&empty[s], phase);
+      if (KIND == REC_MLSTM) {
+        if ((c & 3) == 0) {
+#pragma unroll
+          for (int i = 0; i < 2; ++i) ig[i] = ig_next[i], fg[i] = fg_next[i];
+          request((c + 4) * TC);
+        }
+        const float ic = (c & 2) ? ig[1] : ig[0], fc = (c & 2) ? fg[1] : fg[0];
+        const int at = (c & 1) * TC;
+        float m_old = 0.0f, m_new = 0.0f;
+#pragma unroll
+        for (int t = 0; t < TC; ++t) {
+          const float it = __shfl_sync(0xffffffffu, ic, at + t), ft = __shfl_sync(0xffffffffu, fc, at + t);
+          const float next = fmaxf(ft + m, it);
+          if (lane == at + t) {
+            m_old = m;
+            m_new = next;
+          }
+          m = next;
+        }
+        if (lane >= at && lane < at + TC)
+          *reinterpret_cast<float4*>(factors + (s * TC + lane - at) * 4) = make_float4(expf(fc + m_old - m_new), expf(ic - m_new), expf(-m_new), 0.0f);
+        __syncwarp();  // (the issuer's arrival stands for these stores too)
+      }
+      if (issuer) {  // (rows beyond the run are some other sequence's: nobody walks them)
+        float* dst = walk_smem + s * SF;
+        const int row = r0 + c * TC;
+        mbar_expect_tx(&full[s], uint32_t(SF) * 4);
+        walk_load(dst, &tm_q, 0, h, row, &full[s]);
+        walk_load(dst + TC * QP, &tm_k, 0, h, row, &full[s]);
+        if (KIND == REC_GLA) walk_load(dst + 2 * TC * QP, &tm_a, 0, h, row, &full[s]);
+        walk_load(dst + NV * TC * QP, &tm_v, col0, h, row, &full[s]);
+      }
+      if (++s == ST) s = 0, phase ^= 1;
+    }
+    if (KIND == REC_MLSTM && blockIdx.z == 0 && lane == 0) a.next_m[size_t(slot) * H + h] = m;
+    return;
+  }
+
   auto channel = [&](int i) { return (i >> 2) * GS + sl * 4 + (i & 3); };  // this thread's i-th key channel
-  float S[RPT], N[RPT];
-  float* gs = a.state_s + ((size_t(slot) * H + h) * dv + (col_ok ? j : 0)) * d;
+  const int col = warp * 2 * C + jl * C;                                   // its first column, of the CTA's
+  float S[C][RPT], N[RPT];
   float* gn = a.state_n + (size_t(slot) * H + h) * d;
 #pragma unroll
-  for (int i = 0; i < RPT; ++i) S[i] = N[i] = 0.0f;
-  float m = 0.0f;
+  for (int i = 0; i < RPT; ++i) {
+    N[i] = 0.0f;
+#pragma unroll
+    for (int x = 0; x < C; ++x) S[x][i] = 0.0f;
+  }
   if (!fresh) {
 #pragma unroll
     for (int i4 = 0; i4 < RPT; i4 += 4) {
       const int r = channel(i4);
-      if (r < d && col_ok) {
-        const float4 v4 = *reinterpret_cast<const float4*>(gs + r);
-        S[i4] = v4.x, S[i4 + 1] = v4.y, S[i4 + 2] = v4.z, S[i4 + 3] = v4.w;
-      }
+#pragma unroll
+      for (int x = 0; x < C; ++x)
+        if (r < d && col0 + col + x < dv) {
+          const float4 v4 = *reinterpret_cast<const float4*>(a.state_s + ((size_t(slot) * H + h) * dv + col0 + col + x) * d + r);
+          S[x][i4] = v4.x, S[x][i4 + 1] = v4.y, S[x][i4 + 2] = v4.z, S[x][i4 + 3] = v4.w;
+        }
       if (KIND == REC_MLSTM && r < d) {
         const float4 v4 = *reinterpret_cast<const float4*>(gn + r);
         N[i4] = v4.x, N[i4 + 1] = v4.y, N[i4 + 2] = v4.z, N[i4 + 3] = v4.w;
       }
     }
-    if (KIND == REC_MLSTM) m = a.state_m[size_t(slot) * H + h];
   }
-  const int n_chunks = (nr + TC - 1) / TC;
 
-  // stage <- chunk c; tokens beyond the run and channels beyond dim leave the state alone (k = v = q = 0, decay 1; gates 0 and -inf)
-  auto load_chunk = [&](int c, int stage) {
-    if (c < n_chunks) {
-      float* base = rec_smem + size_t(stage) * TC * TF;
-      const int t0 = c * TC;
-      constexpr int Q4 = QP / 4, C4 = CB / 4;
-      for (int e = tid; e < TC * Q4; e += NT) {
-        const int t = e / Q4, r = (e % Q4) * 4;
-        float* dst = base + t * TF + r;
-        if (t0 + t < nr && r < d) {
-          const float* row = a.proj + size_t(r0 + t0 + t) * a.ld;
-          rec_cp_async_16(dst, row + a.q_col + h * d + r);
-          rec_cp_async_16(dst + QP, row + a.k_col + h * d + r);
-          if (KIND == REC_GLA) rec_cp_async_16(dst + 2 * QP, a.aux + size_t(r0 + t0 + t) * H * d + h * d + r);
-        } else {
-          *reinterpret_cast<float4*>(dst) = *reinterpret_cast<float4*>(dst + QP) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          if (KIND == REC_GLA) *reinterpret_cast<float4*>(dst + 2 * QP) = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+  // one token: the state's step and this slice's parts of the read-out
+  auto step = [&](const float* stage, int t, const float* fac, float (&part)[C], float& npart) {
+    const float* q = stage + t * QP + sl * 4;
+    const float* k = q + TC * QP;
+    const float* vt = stage + NV * TC * QP + t * CB + col;
+    float v[C];
+    if constexpr (C == 2) {
+      const float2 v2 = *reinterpret_cast<const float2*>(vt);
+      v[0] = v2.x, v[1] = v2.y;
+    } else {
+      v[0] = *vt;
+    }
+#pragma unroll
+    for (int x = 0; x < C; ++x) part[x] = 0.0f;
+    npart = 0.0f;
+    if constexpr (KIND == REC_GLA) {
+      const float* al = k + TC * QP;
+#pragma unroll
+      for (int i4 = 0; i4 < RPT; i4 += 4) {
+        const float4 k4 = *reinterpret_cast<const float4*>(k + i4 * SL), q4 = *reinterpret_cast<const float4*>(q + i4 * SL),
+                     a4 = *reinterpret_cast<const float4*>(al + i4 * SL);
+        const float kk[4] = {k4.x, k4.y, k4.z, k4.w}, qq[4] = {q4.x, q4.y, q4.z, q4.w}, aa[4] = {a4.x, a4.y, a4.z, a4.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+          for (int x = 0; x < C; ++x) {
+            S[x][i4 + e] = fmaf(aa[e], S[x][i4 + e], kk[e] * v[x]);
+            part[x] = fmaf(S[x][i4 + e], qq[e], part[x]);
+          }
+      }
+    } else {
+      const float2 f = *reinterpret_cast<const float2*>(fac);  // keep, put
+#pragma unroll
+      for (int i4 = 0; i4 < RPT; i4 += 4) {
+        const float4 k4 = *reinterpret_cast<const float4*>(k + i4 * SL), q4 = *reinterpret_cast<const float4*>(q + i4 * SL);
+        const float pk[4] = {f.y * k4.x, f.y * k4.y, f.y * k4.z, f.y * k4.w}, qq[4] = {q4.x, q4.y, q4.z, q4.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+#pragma unroll
+          for (int x = 0; x < C; ++x) {
+            S[x][i4 + e] = fmaf(f.x, S[x][i4 + e], pk[e] * v[x]);
+            part[x] = fmaf(S[x][i4 + e], qq[e], part[x]);
+          }
+          N[i4 + e] = fmaf(f.x, N[i4 + e], pk[e]);
+          npart = fmaf(N[i4 + e], qq[e], npart);
         }
       }
-      for (int e = tid; e < TC * C4; e += NT) {
-        const int t = e / C4, c2 = (e % C4) * 4;
-        float* dst = base + t * TF + NV * QP + c2;
-        if (t0 + t < nr && col0 + c2 < dv) rec_cp_async_16(dst, a.proj + size_t(r0 + t0 + t) * a.ld + a.v_col + h * dv + col0 + c2);
-        else *reinterpret_cast<float4*>(dst) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      }
-      if (KIND == REC_MLSTM && tid < 2 * TC) {
-        const int t = tid >> 1, w = tid & 1;
-        float* dst = base + t * TF + 3 * QP + CB + w;
-        if (t0 + t < nr) rec_cp_async_4(dst, a.aux + size_t(r0 + t0 + t) * 2 * H + w * H + h);
-        else dst[0] = w ? 0.0f : -INFINITY;
-      }
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");  // (an empty group keeps the count of groups per iteration uniform)
+  };
+  // Row r of 16 parts lies at 16 r, its four float4s exchanged by (r >> 1) & 3: the two halves of a warp write two rows side by side, and eight
+  // lanes that read one float4 of eight rows find them in all 32 banks.  Column x of half jl of token t is row (t C + x) 2 + jl.
+  float* const parts = all_parts + warp * TC * 16 * (2 * C + 1);
+  float* const nparts = parts + TC * 16 * 2 * C;
+  auto spot = [&](int i) { return (((sl >> 2) ^ i) << 2) + (sl & 3); };
+  auto leave = [&](int t, int tc, const float (&part)[C], float npart) {  // (tc: t modulo 8, known to the compiler where the loop is unrolled)
+#pragma unroll
+    for (int x = 0; x < C; ++x) parts[(t * C + x) * 32 + jl * 16 + spot((tc * C + x) & 3)] = part[x];
+    if (KIND == REC_MLSTM && jl == 0) nparts[t * 16 + spot((tc >> 1) & 3)] = npart;  // (the same for every column)
+  };
+  auto add16 = [](const float* p, int i) {
+    const float4 x = *reinterpret_cast<const float4*>(p + ((0 ^ i) << 2)), y = *reinterpret_cast<const float4*>(p + ((1 ^ i) << 2)),
+                 z = *reinterpret_cast<const float4*>(p + ((2 ^ i) << 2)), w = *reinterpret_cast<const float4*>(p + ((3 ^ i) << 2));
+    return (((x.x + x.y) + (x.z + x.w)) + ((y.x + y.y) + (y.z + y.w))) + (((z.x + z.y) + (z.z + z.w)) + ((w.x + w.y) + (w.z + w.w)));
   };
 
-  for (int c = 0; c < kRecStages - 1; ++c) load_chunk(c, c);
+  uint32_t phase = 0;
+  int s = 0;
   for (int c = 0; c < n_chunks; ++c) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(kRecStages - 2) : "memory");
-    __syncthreads();  // chunk c is here; the parts of chunk c - 1 are added up, and its stage is walked
-    load_chunk(c + kRecStages - 1, (c + kRecStages - 1) % kRecStages);
-    const float* base = rec_smem + size_t(c % kRecStages) * TC * TF;
-    const int t0 = c * TC;
-    if (KIND == REC_MLSTM) {
-      const float* sc = base + (lane & (TC - 1)) * TF + 3 * QP + CB;
-      const float ig = sc[0], fg = sc[1];
-      float m_old = 0.0f, m_new = 0.0f;
-#pragma unroll
-      for (int t = 0; t < TC; ++t) {
-        const float it = __shfl_sync(0xffffffffu, ig, t), ft = __shfl_sync(0xffffffffu, fg, t);
-        const float next = fmaxf(ft + m, it);
-        if (lane == t) {
-          m_old = m;
-          m_new = next;
-        }
-        m = next;
-      }
-      if (lane < TC) *reinterpret_cast<float4*>(factors + lane * 4) = make_float4(expf(fg + m_old - m_new), expf(ig - m_new), expf(-m_new), 0.0f);
-      __syncwarp();
-    }
-    // (eight tokens' parts in registers before the first is stored: a store between them would hold back the next token's loads)
-    constexpr int U = RPT <= 8 ? 8 : 4;
+    const float* base = walk_smem + s * SF;
+    const float* fac = factors + s * TC * 4;
+    const int t0 = c * TC, tokens = min(TC, nr - t0);
+    mbar_wait(&full[s], phase);
+    if (tokens == TC) {
+      constexpr int U = RPT <= 8 ? 8 : 4;
 #pragma unroll 1
-    for (int tg = 0; tg < TC; tg += U) {
-      float part_of[U], npart_of[U];
+      for (int tg = 0; tg < TC; tg += U) {
+        // (the parts of U tokens in registers before the first is stored: a store between them would hold back the next token's loads)
+        float part[U][C], npart[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int t = tg + u;
-        const float* tok = base + t * TF;
-        const float* q = tok + sl * 4;
-        const float* k = q + QP;
-        const float v = tok[NV * QP + jl];
-        float part = 0.0f, npart = 0.0f;
-        if (KIND == REC_GLA) {
-          const float* al = k + QP;
+        for (int u = 0; u < U; ++u) step(base, tg + u, fac + (tg + u) * 4, part[u], npart[u]);
+        if constexpr (U == 8) {
 #pragma unroll
-          for (int i4 = 0; i4 < RPT; i4 += 4) {
-            const float4 k4 = *reinterpret_cast<const float4*>(k + i4 * SL), q4 = *reinterpret_cast<const float4*>(q + i4 * SL),
-                         a4 = *reinterpret_cast<const float4*>(al + i4 * SL);
-            S[i4] = fmaf(a4.x, S[i4], k4.x * v);
-            S[i4 + 1] = fmaf(a4.y, S[i4 + 1], k4.y * v);
-            S[i4 + 2] = fmaf(a4.z, S[i4 + 2], k4.z * v);
-            S[i4 + 3] = fmaf(a4.w, S[i4 + 3], k4.w * v);
-            part = fmaf(S[i4], q4.x, part);
-            part = fmaf(S[i4 + 1], q4.y, part);
-            part = fmaf(S[i4 + 2], q4.z, part);
-            part = fmaf(S[i4 + 3], q4.w, part);
-          }
+          for (int u = 0; u < U; ++u) leave(tg + u, u, part[u], npart[u]);
         } else {
-          const float2 f = *reinterpret_cast<const float2*>(factors + t * 4);  // keep, put
 #pragma unroll
-          for (int i4 = 0; i4 < RPT; i4 += 4) {
-            const float4 k4 = *reinterpret_cast<const float4*>(k + i4 * SL), q4 = *reinterpret_cast<const float4*>(q + i4 * SL);
-            const float pk[4] = {f.y * k4.x, f.y * k4.y, f.y * k4.z, f.y * k4.w}, qq[4] = {q4.x, q4.y, q4.z, q4.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              S[i4 + e] = fmaf(f.x, S[i4 + e], pk[e] * v);
-              N[i4 + e] = fmaf(f.x, N[i4 + e], pk[e]);
-              part = fmaf(S[i4 + e], qq[e], part);
-              npart = fmaf(N[i4 + e], qq[e], npart);
-            }
-          }
+          for (int u = 0; u < U; ++u) leave(tg + u, (tg & 4) + u, part[u], npart[u]);
         }
-        part_of[u] = part;
-        npart_of[u] = npart;
       }
+    } else {
+#pragma unroll 1
+      for (int t = 0; t < tokens; ++t) {
+        float part[C], npart;
+        step(base, t, fac + t * 4, part, npart);
+        leave(t, t & 7, part, npart);
+      }
+    }
+    __syncwarp();
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        parts[((tg + u) * CB + jl) * kWalkPitch + sl] = part_of[u];
-        if (KIND == REC_MLSTM && jl == 0) nparts[(tg + u) * kWalkPitch + sl] = npart_of[u];  // (the same for every column)
+    for (int i = 0; i < C; ++i) {
+      const int row = lane + 32 * i, t = row / (2 * C), out_col = col0 + warp * 2 * C + (row & 1) * C + (row >> 1) % C;
+      if (t < tokens && out_col < dv) {
+        float out = add16(parts + row * 16, (row >> 1) & 3) * a.q_scale;
+        if (KIND == REC_MLSTM) out = out / (fmaxf(fabsf(add16(nparts + t * 16, (t >> 1) & 3) * a.q_scale), fac[t * 4 + 2]) + a.denom_eps);
+        a.o[size_t(r0 + t0 + t) * H * dv + h * dv + out_col] = out;
       }
     }
-    __syncthreads();
-    {  // token tid / 8, column tid % 8
-      auto add16 = [](const float* p) {
-        const float4 x = *reinterpret_cast<const float4*>(p), y = *reinterpret_cast<const float4*>(p + 4), z = *reinterpret_cast<const float4*>(p + 8),
-                     w = *reinterpret_cast<const float4*>(p + 12);
-        return (((x.x + x.y) + (x.z + x.w)) + ((y.x + y.y) + (y.z + y.w))) + (((z.x + z.y) + (z.z + z.w)) + ((w.x + w.y) + (w.z + w.w)));
-      };
-      const int t = tid / CB, col = tid % CB;
-      if (t0 + t < nr && col0 + col < dv) {
-        float out = add16(parts + tid * kWalkPitch) * a.q_scale;
-        if (KIND == REC_MLSTM) out = out / (fmaxf(fabsf(add16(nparts + t * kWalkPitch) * a.q_scale), factors[t * 4 + 2]) + a.denom_eps);
-        a.o[size_t(r0 + t0 + t) * H * dv + h * dv + col0 + col] = out;
-      }
-    }
+    __syncwarp();  // the parts are read, the stage is walked
+    if (lane == 0) mbar_arrive(&empty[s]);
+    if (++s == ST) s = 0, phase ^= 1;
   }
-  const bool write_n = KIND == REC_MLSTM && blockIdx.z == 0 && jl == 0;
   float* gn_next = KIND == REC_MLSTM ? a.next_n + (size_t(slot) * H + h) * d : nullptr;
 #pragma unroll
   for (int i4 = 0; i4 < RPT; i4 += 4) {
     const int r = channel(i4);
-    if (r < d && col_ok) *reinterpret_cast<float4*>(gs + r) = make_float4(S[i4], S[i4 + 1], S[i4 + 2], S[i4 + 3]);
-    if (write_n && r < d) *reinterpret_cast<float4*>(gn_next + r) = make_float4(N[i4], N[i4 + 1], N[i4 + 2], N[i4 + 3]);
+    if (r >= d) continue;
+#pragma unroll
+    for (int x = 0; x < C; ++x)
+      if (col0 + col + x < dv)
+        *reinterpret_cast<float4*>(a.state_s + ((size_t(slot) * H + h) * dv + col0 + col + x) * d + r) = make_float4(S[x][i4], S[x][i4 + 1], S[x][i4 + 2], S[x][i4 + 3]);
+    if (KIND == REC_MLSTM && blockIdx.z == 0 && warp == 0 && jl == 0) *reinterpret_cast<float4*>(gn_next + r) = make_float4(N[i4], N[i4 + 1], N[i4 + 2], N[i4 + 3]);
   }
-  if (write_n && tid == 0) a.next_m[size_t(slot) * H + h] = m;
 }
 
 template <typename T>

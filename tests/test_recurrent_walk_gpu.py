@@ -50,3 +50,22 @@ def test_long_walk_repeats_short_portions():
         logits = engine.step([(0, toks[at : at + portion], [portion - 1])])
       states.append([t.clone() for t in state["cache"]["recurrent_state"]] + [logits])
     assert all(torch.equal(a, b) for a, b in zip(*states))
+
+
+@pytest.mark.parametrize("kind,heads,dim,vdim", [("gla", 24, 64, 128), ("gla", 2, 256, 40), ("gla", 3, 100, 72), ("mlstm", 20, 128, 128), ("mlstm", 2, 200, 20), ("mlstm", 1, 64, 8)])
+def test_walk_of_two_long_runs(kind, heads, dim, vdim):
+  """Two runs of a step, ends before, at and behind a chunk of 16 tokens, one and two columns per thread, channels and columns that fill neither slices nor
+  CTAs: the bits of portions of ten tokens, which are walked token by token."""
+  layer = g.gla_layer(heads, dim, vdim) if kind == "gla" else g.parallel_layer(4, 2, 32, heads, dim, vdim)
+  cfg = g.model_dict(256, 320, [layer])
+  config = pyconfig.from_model_dict(cfg, dtype="float32", per_device_batch_size=2, max_target_length=128, pagedattn_tokens_per_page=16, pagedattn_num_pages=20)
+  tensors, toks, states = g.random_tensors(config, seed=4), [tokens(n, 5) for n in (79, 64)], []
+  for portion in (47, 10):  # 47 + 32, 47 + 17 against tens
+    engine = maxengine.MaxEngine(config)
+    engine.load_params(tensors)
+    state = engine.init_decode_state()
+    for at in range(0, 79, portion):
+      parts = [(slot, t[at : at + portion], [len(t[at : at + portion]) - 1]) for slot, t in enumerate(toks) if t[at : at + portion]]
+      engine.step(parts)
+    states.append([t[:2].clone() for t in state["cache"]["recurrent_state"]])
+  assert all(torch.equal(a, b) for a, b in zip(*states))
