@@ -991,7 +991,7 @@ def main():
             "ms_per_step": e2e_ms / args.steps,
             "h2d_bytes_per_step": B * 4,
             "d2h_bytes_per_step": B * 3 * 4,
-            "api": "MaxEngine.generate_to_host(sync=True) (mtx_decode_step_host_sync): pinned host token buffer in, ResultTokens.data to a pinned host buffer, the copies are nodes of the step's CUDA graph, one stream sync per step",
+            "api": "MaxEngine.generate_to_host(sync=True) (mtx_decode_step_host_sync): pinned host token buffer in, ResultTokens.data to a pinned host buffer, read and written by the step's own kernels in its CUDA graph, one stream sync per step",
         },
         "gpu_launches": launches_per_step * args.steps,
         "launches_per_step": launches_per_step,

@@ -910,8 +910,15 @@ int pass_rows(const mtx_engine* e, int left) {
   return rest > 128 && (e->cfg.head_dim != 256 || takes_prompt_wide(e, rest)) ? wide : wide - rest;
 }
 
+// A decode step that takes its tokens from, and leaves its result in, pinned host memory (device addresses of it, or null).
+struct HostIo {
+  const int32_t* tokens = nullptr;
+  int32_t* result = nullptr;
+  float* log_prob = nullptr;
+};
 // One step: a decode step of `rows` slots up to its tokens (mode 0), or the layers over `rows` prompt positions (mode 1; e->x holds the result).
-int enqueue_step(mtx_engine* e, int mode, int rows, const int32_t* chunk_tokens, int start_pos, int slot, cudaStream_t st, float* cand_out = nullptr) {
+int enqueue_step(mtx_engine* e, int mode, int rows, const int32_t* chunk_tokens, int start_pos, int slot, cudaStream_t st, float* cand_out = nullptr,
+                 HostIo io = HostIo()) {
   const mtx_model_config& c = e->cfg;
   // (an int8 cache is appended to by the row-major GEMM's epilogue only: steps of any size run it, padded to 128 rows)
   const bool gemma3 = c.decoder_block == 1;
@@ -929,7 +936,7 @@ int enqueue_step(mtx_engine* e, int mode, int rows, const int32_t* chunk_tokens,
 
   PrepareArgs pa;
   memset(&pa, 0, sizeof(pa));
-  pa.tokens = e->s.tokens;
+  pa.tokens = io.tokens != nullptr ? io.tokens : e->s.tokens;
   pa.next_pos = e->s.next_pos;
   pa.prefill_len = e->s.prefill_len;
   pa.ar_lengths = e->s.ar_lengths;
@@ -1405,6 +1412,8 @@ int enqueue_step(mtx_engine* e, int mode, int rows, const int32_t* chunk_tokens,
     fa.rng_state = e->s.rng_state;
     fa.num_slots = c.num_slots;
     fa.R = c.max_target_len - c.max_prefill_len;
+    fa.result_host = io.result;
+    fa.log_prob_host = io.log_prob;
     MTX_TRY(launch(finalize_kernel, dim3(rows), dim3(kFinalizeThreads), 0, st, fa));
   }
   return MTX_OK;
@@ -1751,31 +1760,39 @@ int mtx_decode_step_host(mtx_engine* e, int rows, const int32_t* tokens_host, in
     if (want_lp) MTX_CUDA(cudaMemcpyAsync(log_prob_host, e->s.log_prob, size_t(rows) * 4, cudaMemcpyDeviceToHost, s2));
     return MTX_OK;
   };
-  // Pinned buffers (what a serving loop reuses every step): ONE graph holds the copy in, the step's kernels and the copies
-  // out, so a step is one driver call.  Pageable buffers cannot be captured: three calls.
-  auto pinned = [](const void* ptr) {
+  // Pinned buffers (what a serving loop reuses every step): ONE graph whose first kernel reads the tokens and whose last writes the result where the
+  // host has them, so a step is one driver call and no copies: a copy as a node of its own between the kernels cost about 3 us, three of them with log_prob.
+  // One slot, 4 layers of 256: 159 us with the copies, 145 so; 64 slots of the 24-layer model 1300 and 1283.  The graphs are kept by what the kernels are given,
+  // the device addresses of this call's buffers, so that memory that is no longer pinned never meets one.  Other buffers (pageable, unaligned): three calls.
+  auto pinned = [](const void* ptr, const void** dev) {
+    *dev = nullptr;
     if (ptr == nullptr) return true;
     cudaPointerAttributes at;
     if (cudaPointerGetAttributes(&at, ptr) != cudaSuccess) {
       cudaGetLastError();
       return false;
     }
-    return at.type == cudaMemoryTypeHost;
+    *dev = at.devicePointer;
+    return at.type == cudaMemoryTypeHost && at.devicePointer != nullptr && (reinterpret_cast<uintptr_t>(at.devicePointer) & 3) == 0;
   };
-  const mtx_engine::HostKey key{rows, tokens_host, result_host, want_lp ? log_prob_host : nullptr};
+  const void *tokens_dev, *result_dev, *log_prob_dev;
+  if (!(pinned(tokens_host, &tokens_dev) && pinned(result_host, &result_dev) && pinned(want_lp ? log_prob_host : nullptr, &log_prob_dev)) ||
+      env_int("MTX_HOST_GRAPH", 1) == 0) {
+    MTX_TRY(copies_in(st));
+    MTX_TRY(mtx_decode_step_graph(e, rows, stream));
+    return copies_out(st);
+  }
+  const mtx_engine::HostKey key{rows, tokens_dev, result_dev, log_prob_dev};
   auto it = e->host_graphs.find(key);
   if (it == e->host_graphs.end()) {
-    if (!(pinned(tokens_host) && pinned(result_host) && (!want_lp || pinned(log_prob_host))) || env_int("MTX_HOST_GRAPH", 1) == 0) {
-      MTX_TRY(copies_in(st));
-      MTX_TRY(mtx_decode_step_graph(e, rows, stream));
-      return copies_out(st);
-    }
     if (!e->cap_stream) MTX_CUDA(cudaStreamCreateWithFlags(&e->cap_stream, cudaStreamNonBlocking));
     cudaGraph_t graph = nullptr;
     MTX_CUDA(cudaStreamBeginCapture(e->cap_stream, cudaStreamCaptureModeThreadLocal));
-    int rc = copies_in(e->cap_stream);
-    if (rc == MTX_OK) rc = enqueue_step(e, 0, rows, nullptr, 0, 0, e->cap_stream);
-    if (rc == MTX_OK) rc = copies_out(e->cap_stream);
+    HostIo io;
+    io.tokens = static_cast<const int32_t*>(tokens_dev);
+    io.result = static_cast<int32_t*>(const_cast<void*>(result_dev));
+    io.log_prob = static_cast<float*>(const_cast<void*>(log_prob_dev));
+    const int rc = enqueue_step(e, 0, rows, nullptr, 0, 0, e->cap_stream, nullptr, io);
     const cudaError_t end = cudaStreamEndCapture(e->cap_stream, &graph);
     if (rc != MTX_OK) {
       if (graph) cudaGraphDestroy(graph);

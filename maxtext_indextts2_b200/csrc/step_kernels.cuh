@@ -530,6 +530,9 @@ struct FinalizeArgs {
   float* log_prob;    // [rows] or null
   uint32_t* rng_state;
   int num_slots, R;
+  // the result once more, in pinned host memory (or null): a copy behind the step would be a node of its own in its graph, about 3 us each
+  int* result_host;
+  float* log_prob_host;
   // prefill
   int* first_token;
 };
@@ -612,6 +615,12 @@ __global__ void __launch_bounds__(kFinalizeThreads) finalize_kernel(const Finali
       a.result[r * 3 + 1] = 1;
       a.result[r * 3 + 2] = gen;
       if (a.log_prob != nullptr) a.log_prob[r] = logp;
+      if (a.result_host != nullptr) {
+        a.result_host[r * 3 + 0] = idx;
+        a.result_host[r * 3 + 1] = 1;
+        a.result_host[r * 3 + 2] = gen;
+        if (a.log_prob_host != nullptr) a.log_prob_host[r] = logp;
+      }
     } else if (a.mode == 3) {
       a.first_token[r] = idx;
       if (a.log_prob != nullptr) a.log_prob[r] = logp;

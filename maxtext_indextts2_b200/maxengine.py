@@ -774,7 +774,7 @@ class MaxEngine:
   def generate_to_host(self, params: DeviceParams, decode_state: dict, host_result: torch.Tensor, host_tokens: Optional[torch.Tensor] = None,
                        host_log_prob: Optional[torch.Tensor] = None, sync: bool = False):
     """``generate`` for a serving loop that holds its tokens on the host (JetStream / OfflineEngine copy every step's
-    ResultTokens to the host: offline_engine.py:612-614): one C call -- with pinned buffers one graph launch -- does the host ->
+    ResultTokens to the host: offline_engine.py:612-614): one C call -- with pinned buffers one graph launch, whose kernels read and write them -- does the host ->
     device copy of this step's input tokens (`host_tokens` [B,1] int32 pinned, or None to continue from decode_state["tokens"]),
     the step, and the device -> host copy of ResultTokens.data into `host_result` [B,3] int32 pinned.  `sync=True` also waits
     for the stream inside that call (`host_result` is valid on return); otherwise the caller waits on the current stream.
