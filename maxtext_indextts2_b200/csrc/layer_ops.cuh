@@ -56,6 +56,25 @@ __global__ void embed_rows_kernel(const int* token, const T* embedding, int voca
   const int r = blockIdx.x;
   int tok = token[r];
   tok = tok < 0 ? 0 : (tok >= vocab ? vocab - 1 : tok);
+  if (sizeof(T) == 2 && (width & 7) == 0 && (reinterpret_cast<uintptr_t>(embedding) & 15) == 0) {  // eight channels at a time
+    for (int c = threadIdx.x * 8; c < width; c += blockDim.x * 8) {
+      const uint4 q = *reinterpret_cast<const uint4*>(embedding + size_t(tok) * width + c);
+      const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+      float v[8];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[2 * i] = bf16_lo(w[i]) * scale, v[2 * i + 1] = bf16_hi(w[i]) * scale;
+      const size_t at = size_t(r) * width + c;
+      const float4 lo = make_float4(v[0], v[1], v[2], v[3]), hi = make_float4(v[4], v[5], v[6], v[7]);
+      *reinterpret_cast<float4*>(x + at) = lo;
+      *reinterpret_cast<float4*>(x + at + 4) = hi;
+      *reinterpret_cast<uint4*>(xa + at) = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+      if (x0) {
+        *reinterpret_cast<float4*>(x0 + at) = lo;
+        *reinterpret_cast<float4*>(x0 + at + 4) = hi;
+      }
+    }
+    return;
+  }
   for (int c = threadIdx.x; c < width; c += blockDim.x) {
     const float v = act_f32(embedding[size_t(tok) * width + c]) * scale;
     x[size_t(r) * width + c] = v;
@@ -77,13 +96,15 @@ struct SandwichArgs {
 };
 
 // one CTA per row; the row of x stays in registers between the two reductions.  V = 4: the row moves as float4s (width a
-// multiple of 4, <= 256 * 4 * kSandwichVec); V = 1: any width <= 256 * kSandwichMax.
+// multiple of 4, <= 256 * 4 * kSandwichVec); V = 1: any width <= 256 * kSandwichMax.  N: groups of V floats per thread, as few as the row needs (row_groups).
+// Bound: latency -- two reductions per row -- so what counts is rows in flight: with eight groups for every width, three CTAs per SM, and x read
+// after the first reduction, 4096 rows of 2048 took 38.8 us, 25.5 us with two groups and every plane requested at the start.
 constexpr int kSandwichMax = 32, kSandwichVec = 8;
 
-template <typename T, int V>
+template <typename T, int V, int N>
 __global__ void __launch_bounds__(256) sandwich_step_kernel(const SandwichArgs a, T* xa) {
   __shared__ float red[8];
-  constexpr int N = V == 4 ? kSandwichVec : kSandwichMax;  // register groups of V floats per thread
+  constexpr bool kAhead = V == 4 && N <= 2;  // (registers for x and x0 beside y)
   griddep_launch_dependents();
   griddep_wait();
   const int r = blockIdx.x, W = a.width;
@@ -98,7 +119,17 @@ __global__ void __launch_bounds__(256) sandwich_step_kernel(const SandwichArgs a
       v[0] = p[c];
     }
   };
-  float yv[N][V];
+  float yv[N][V], xv[kAhead ? N : 1][V], x0v[kAhead ? N : 1][V];
+  if (kAhead) {
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+      const int c = (threadIdx.x + u * 256) * V;
+      if (c < W) {
+        load(xr, c, xv[u]);
+        if (x0r) load(x0r, c, x0v[u]);
+      }
+    }
+  }
   float f = 0.0f;
   if (yr) {
     float ss = 0.0f;
@@ -126,16 +157,21 @@ __global__ void __launch_bounds__(256) sandwich_step_kernel(const SandwichArgs a
     const int c = (threadIdx.x + u * 256) * V;
     if (c < W) {
       float v[V], w[V];
-      load(xr, c, v);
+      if (kAhead) {
+#pragma unroll
+        for (int e = 0; e < V; ++e) v[e] = xv[u][e];
+      } else {
+        load(xr, c, v);
+      }
       if (yr) {
         load(a.post, c, w);
 #pragma unroll
         for (int e = 0; e < V; ++e) v[e] += yv[u][e] * f * (1.0f + w[e]);
       }
       if (x0r) {
-        load(x0r, c, w);
+        if (!kAhead) load(x0r, c, w);
 #pragma unroll
-        for (int e = 0; e < V; ++e) v[e] += w[e];
+        for (int e = 0; e < V; ++e) v[e] += kAhead ? x0v[u][e] : w[e];
       }
       if (a.add_vec) {
         load(a.add_vec, c, w);
@@ -162,11 +198,20 @@ __global__ void __launch_bounds__(256) sandwich_step_kernel(const SandwichArgs a
     if (c < W) {
       float w[V];
       load(a.pre, c, w);
+      float v[V];
 #pragma unroll
-      for (int e = 0; e < V; ++e) xa[size_t(r) * W + c + e] = to_act<T>(yv[u][e] * f2 * (1.0f + w[e]));
+      for (int e = 0; e < V; ++e) v[e] = yv[u][e] * f2 * (1.0f + w[e]);
+      if constexpr (V == 4 && sizeof(T) == 2) {
+        *reinterpret_cast<uint2*>(xa + size_t(r) * W + c) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
+      } else {
+#pragma unroll
+        for (int e = 0; e < V; ++e) xa[size_t(r) * W + c + e] = to_act<T>(v[e]);
+      }
     }
   }
 }
+// Groups of 1024 channels that a row kernel's thread keeps: 1, 2, 4 or 8
+inline int row_groups(int width) { return width <= 1024 ? 1 : width <= 2048 ? 2 : width <= 4096 ? 4 : 8; }
 
 template <typename T>
 __global__ void __launch_bounds__(256) weighted_norm_rows_kernel(const float* x, const int* rows, const float* w, float eps, T* out, int width) {
@@ -448,11 +493,12 @@ struct OutLayerNormArgs {
 constexpr int kOutLnVec = 32;  // registers of a thread for its part of the row: width <= 256 * kOutLnVec
 
 // one CTA per row; the row stays in registers between the reductions (mean, then the squared deviations).  V = 4: the row moves in
-// groups of four channels (width a multiple of 4), V = 1: any width
-template <typename T, int V>
+// groups of four channels (width a multiple of 4), V = 1: any width; N groups per thread, as few as the row needs (row_groups).  1777 rows of 1024: 12.3 us with
+// eight groups for every width, 7.5 us so.
+template <typename T, int V, int N>
 __global__ void __launch_bounds__(256) out_layer_norm_kernel(const OutLayerNormArgs a, T* xa) {
   __shared__ float red[8];
-  constexpr int N = kOutLnVec / V;
+  constexpr bool kAhead = V == 4 && N <= 2;  // (registers for x beside y)
   griddep_launch_dependents();
   griddep_wait();
   const int r = blockIdx.x, W = a.width;
@@ -465,6 +511,12 @@ __global__ void __launch_bounds__(256) out_layer_norm_kernel(const OutLayerNormA
       v[0] = p[c];
     }
   };
+  float xv[kAhead ? N : 1][V];
+  if (kAhead) {
+#pragma unroll
+    for (int u = 0; u < N; ++u)
+      if ((threadIdx.x + u * 256) * V < W) load(xr, (threadIdx.x + u * 256) * V, xv[u]);
+  }
   const float sg = a.shared_gate ? 1.0f / (1.0f + expf(-a.shared_gate[size_t(r) * a.ld_gate])) : 1.0f;
   float yv[N][V];
   float sum = 0.0f;
@@ -517,7 +569,12 @@ __global__ void __launch_bounds__(256) out_layer_norm_kernel(const OutLayerNormA
     const int c = (threadIdx.x + u * 256) * V;
     if (c < W) {
       float v[V], w[V], b[V];
-      load(xr, c, v);
+      if (kAhead) {
+#pragma unroll
+        for (int e = 0; e < V; ++e) v[e] = xv[u][e];
+      } else {
+        load(xr, c, v);
+      }
       load(a.w, c, w);
       load(a.b, c, b);
 #pragma unroll

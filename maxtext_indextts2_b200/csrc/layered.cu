@@ -748,6 +748,12 @@ int launch_rec_walk(const RecScanArgs& ra, int n_runs, int num_sms, cudaStream_t
   return single ? launch_rec_walk_t<KIND, RPT, 1>(ra, n_runs, st) : launch_rec_walk_t<KIND, RPT, 2>(ra, n_runs, st);
 }
 
+template <typename T>
+int launch_rec_out(const RecOutArgs<T>& oa, int rows, cudaStream_t st) {
+  auto kern = oa.vdim <= 64 ? recurrent_out_kernel<T, 2> : oa.vdim <= 128 ? recurrent_out_kernel<T, 4> : oa.vdim <= 256 ? recurrent_out_kernel<T, 8> : recurrent_out_kernel<T, 0>;
+  return launch(kern, dim3(rows), dim3(256), 0, st, oa);
+}
+
 // A walk is bound by latency, so what counts is how many warps share an SM.  16 value columns per CTA when that still gives every
 // SM two CTAs, else 8; and when even 8-column CTAs with 8 slices per column leave the thread slots of the GPU mostly empty (one
 // prompt: heads x vdim columns in all), a column is cut into 16 slices.
@@ -794,8 +800,12 @@ int sandwich_step(mtx_layered* e, const float* y, const float* bias, const float
     sa.pre = nl.norm1;
   }
   if (!sa.y && !sa.x0 && !sa.add_vec && !sa.pre) return MTX_OK;
-  if (sa.width % 4 == 0 && sa.width <= 256 * 4 * kSandwichVec) return launch(sandwich_step_kernel<T, 4>, dim3(rows), dim3(256), 0, st, sa, static_cast<T*>(e->xa));
-  return launch(sandwich_step_kernel<T, 1>, dim3(rows), dim3(256), 0, st, sa, static_cast<T*>(e->xa));
+  if (sa.width % 4 == 0 && sa.width <= 256 * 4 * kSandwichVec) {
+    const int n = row_groups(sa.width);
+    return launch(n == 1 ? sandwich_step_kernel<T, 4, 1> : n == 2 ? sandwich_step_kernel<T, 4, 2> : n == 4 ? sandwich_step_kernel<T, 4, 4> : sandwich_step_kernel<T, 4, 8>,
+                  dim3(rows), dim3(256), 0, st, sa, static_cast<T*>(e->xa));
+  }
+  return launch(sandwich_step_kernel<T, 1, kSandwichMax>, dim3(rows), dim3(256), 0, st, sa, static_cast<T*>(e->xa));
 }
 
 bool use_softmax_mma() {
@@ -1258,7 +1268,7 @@ int composite_layer(mtx_layered* e, int li, const mtx_ragged_batch& b, cudaStrea
     oa.state_n = r.state_n;
     oa.state_m = r.state_m;
     oa.dim = r.dim;
-    MTX_TRY(launch(recurrent_out_kernel<T>, dim3(rows), dim3(256), 0, st, oa));
+    MTX_TRY(launch_rec_out<T>(oa, rows, st));
   }
   MTX_TRY((linear<T, LIN_PLAIN>(e, mix, l.wo, nullptr, e->y, nullptr, rows, E, cc.k_out, st)));
   const bool has_ff = l.ff_kind == MTX_FF_MOE ? l.moe.experts > 0 : l.ff > 0;
@@ -1585,7 +1595,7 @@ int parallel_layer(mtx_layered* e, int li, const mtx_ragged_batch& b, cudaStream
     oa.gate_silu = r.gate_silu;
     oa.eps = c.eps;
     oa.out_scale = r.out_scale;
-    MTX_TRY(launch(recurrent_out_kernel<T>, dim3(rows), dim3(256), 0, st, oa));
+    MTX_TRY(launch_rec_out<T>(oa, rows, st));
   }
   if (l.ff > 0) MTX_TRY((linear<T, LIN_RELU2>(e, xb, l.w_gate_up, nullptr, nullptr, cat + pc.k_mix, rows, l.ff, E, st, 0.0f, k_cat)));
   MTX_TRY((linear<T, LIN_PLAIN>(e, cat, l.wo, nullptr, e->y, nullptr, rows, E, k_cat, st)));
@@ -1873,7 +1883,7 @@ int prenorm_layer(mtx_layered* e, int li, const mtx_ragged_batch& b, cudaStream_
     oa.gate_silu = r.gate_silu;
     oa.eps = c.eps;
     oa.out_scale = r.out_scale != 0.0f ? r.out_scale : 1.0f;
-    MTX_TRY(launch(recurrent_out_kernel<T>, dim3(rows), dim3(256), 0, st, oa));
+    MTX_TRY(launch_rec_out<T>(oa, rows, st));
   }
   if (l.bo) MTX_TRY((linear<T, LIN_BIAS>(e, mix, l.wo, l.bo, e->y, nullptr, rows, E, pc.k_mix, st)));
   else MTX_TRY((linear<T, LIN_PLAIN>(e, mix, l.wo, nullptr, e->y, nullptr, rows, E, pc.k_mix, st)));
@@ -1906,8 +1916,12 @@ int out_layer_norm(mtx_layered* e, OutLayerNormArgs a, const float* w, const flo
   a.x = e->x;
   a.eps = e->cfg.eps;
   a.width = e->cfg.width;
-  if (a.width % 4 == 0) return launch(out_layer_norm_kernel<T, 4>, dim3(rows), dim3(256), 0, st, a, static_cast<T*>(e->xa));
-  return launch(out_layer_norm_kernel<T, 1>, dim3(rows), dim3(256), 0, st, a, static_cast<T*>(e->xa));
+  if (a.width % 4 == 0) {
+    const int n = row_groups(a.width);
+    return launch(n == 1 ? out_layer_norm_kernel<T, 4, 1> : n == 2 ? out_layer_norm_kernel<T, 4, 2> : n == 4 ? out_layer_norm_kernel<T, 4, 4> : out_layer_norm_kernel<T, 4, 8>,
+                  dim3(rows), dim3(256), 0, st, a, static_cast<T*>(e->xa));
+  }
+  return launch(out_layer_norm_kernel<T, 1, kOutLnVec>, dim3(rows), dim3(256), 0, st, a, static_cast<T*>(e->xa));
 }
 
 // ... of the projection a . w^T
@@ -2105,7 +2119,7 @@ int outlayer_layer(mtx_layered* e, int li, const mtx_ragged_batch& b, cudaStream
     oa.eps = c.eps;
     oa.out_scale = r.out_scale;
     const bool vec = (r.heads * r.vdim) % 4 == 0 && n_in % 4 == 0 && cc.rg % 4 == 0 && cc.k_out % 4 == 0 && cc.out_rec % 4 == 0;
-    if (!r.norm_whole) MTX_TRY(launch(recurrent_out_kernel<T>, dim3(rows), dim3(256), 0, st, oa));
+    if (!r.norm_whole) MTX_TRY(launch_rec_out<T>(oa, rows, st));
     else if (vec && r.heads * r.vdim <= 256 * 8) MTX_TRY(launch(recurrent_out_whole_kernel<T, 4, 8>, dim3(rows), dim3(256), 0, st, oa));
     else if (vec) MTX_TRY(launch(recurrent_out_whole_kernel<T, 4, kRecOutVec>, dim3(rows), dim3(256), 0, st, oa));
     else MTX_TRY(launch(recurrent_out_whole_kernel<T, 1, kRecOutVec>, dim3(rows), dim3(256), 0, st, oa));

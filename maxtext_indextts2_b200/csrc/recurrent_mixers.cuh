@@ -925,7 +925,9 @@ struct RecOutArgs {
 };
 
 // one CTA per row, a warp per head
-template <typename T>
+// K: channels of a head that a lane keeps (vdim <= 32 K), requested with the gates before the first is used; 0: any vdim, read twice.  4096 rows of 16
+// heads of 128: 41.5 us with two passes over o, 16.9 us so.
+template <typename T, int K>
 __global__ void __launch_bounds__(256) recurrent_out_kernel(const RecOutArgs<T> a) {
   griddep_launch_dependents();
   griddep_wait();
@@ -935,17 +937,36 @@ __global__ void __launch_bounds__(256) recurrent_out_kernel(const RecOutArgs<T> 
     for (int i = threadIdx.x; i < a.heads; i += blockDim.x) a.state_m[at + i] = a.next_m[at + i];
   }
   const int r = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5, dv = a.vdim;
+  auto gated = [&](float o, float inv, float w, float g) {
+    const float sig = 1.0f / (1.0f + expf(-g));
+    const float gate = a.gate_silu ? g * sig : sig;
+    return to_act<T>(o * inv * w * gate * a.out_scale);
+  };
+#pragma unroll 2
   for (int h = warp; h < a.heads; h += nw) {
     const float* o = a.o + size_t(r) * a.heads * dv + h * dv;
+    const float* g = a.proj + size_t(r) * a.ld + a.g_col + h * dv;
+    const float* w = a.weight + h * dv;
+    T* out = a.out + size_t(r) * a.ld_out + a.out_col + h * dv;
     float ss = 0.0f;
-    for (int c = lane; c < dv; c += 32) ss = fmaf(o[c], o[c], ss);
-    ss = warp_sum(ss);
-    const float inv = 1.0f / sqrtf(ss / float(dv) + a.eps);
-    for (int c = lane; c < dv; c += 32) {
-      const float g = a.proj[size_t(r) * a.ld + a.g_col + h * dv + c];
-      const float sig = 1.0f / (1.0f + expf(-g));
-      const float gate = a.gate_silu ? g * sig : sig;
-      a.out[size_t(r) * a.ld_out + a.out_col + h * dv + c] = to_act<T>(o[c] * inv * a.weight[h * dv + c] * gate * a.out_scale);
+    if constexpr (K > 0) {
+      float ov[K], gv[K], wv[K];
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if (lane + 32 * k < dv) ov[k] = o[lane + 32 * k], gv[k] = g[lane + 32 * k], wv[k] = w[lane + 32 * k];
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if (lane + 32 * k < dv) ss = fmaf(ov[k], ov[k], ss);
+      ss = warp_sum(ss);
+      const float inv = 1.0f / sqrtf(ss / float(dv) + a.eps);
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if (lane + 32 * k < dv) out[lane + 32 * k] = gated(ov[k], inv, wv[k], gv[k]);
+    } else {
+      for (int c = lane; c < dv; c += 32) ss = fmaf(o[c], o[c], ss);
+      ss = warp_sum(ss);
+      const float inv = 1.0f / sqrtf(ss / float(dv) + a.eps);
+      for (int c = lane; c < dv; c += 32) out[c] = gated(o[c], inv, w[c], g[c]);
     }
   }
 }
