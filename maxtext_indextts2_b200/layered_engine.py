@@ -427,12 +427,12 @@ class LayeredEngine(MaxEngine):
       self._uploaded_map = ps.page_map
 
   def _follow(self) -> None:
-    """The caller's stream behind a step that another stream may still hold (a step's pages, states and descriptors are the engine's)."""
+    """The caller's stream behind a step that another stream may still hold (a step's pages, states and descriptors are the engine's).  That one stream waits
+    says nothing about the next one: the step is pending for all of them until the host has waited for it."""
     if self._behind is not None:
       stream = torch.cuda.current_stream(self.device)
       if stream != self._behind:
         stream.wait_event(self._step_done)
-        self._behind = None
 
   def _upload_page_state(self) -> None:  # (MaxEngine.release_pages calls it for device-resident page states; nothing to do here)
     return

@@ -103,6 +103,18 @@ def test_another_stream_waits(monkeypatch):
   assert [s[0] for s in seen[2:]] == [[6], [7]]
 
 
+def test_a_third_stream_waits_too(monkeypatch):
+  """A stream that has waited for a prompt (here to free a slot) does not stand for the others."""
+  e, now, seen = _engine(monkeypatch)
+  e._states, e._active, e._next_pos = [], torch.ones(3, 1, dtype=torch.int32), torch.ones(3, 1, dtype=torch.int32)
+  e._step([(0, [1, 2, 3], [2])], wait=False)
+  first, now[0] = now[0], _Stream()
+  e.release_pages(1)
+  now[0] = _Stream()
+  e.step([(2, [4, 5], [1])])
+  assert [s[0] for s in seen] == [[1, 2, 3], [4, 5]] and not first.queue
+
+
 def test_tokens_of_mixed_forms(monkeypatch):
   """Entries given as lists, arrays and tensors keep their order."""
   e, now, seen = _engine(monkeypatch)
