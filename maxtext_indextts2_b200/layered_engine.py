@@ -158,7 +158,7 @@ class LayeredEngine(MaxEngine):
 
   prompt_and_decode_share_pages = True  # no prefill segment + AR ring: a sequence is one page group that grows
   _desc_pending = _map_pending = False  # _desc_read / _map_read stand for a copy that may not have run yet
-  _behind = None  # the stream that still holds a step of this engine, or None
+  _behind = None  # the stream that _step_done was recorded on, or None: the host has waited for it
 
   def __init__(self, config, devices: Any = None, use_cuda_graph: bool = True, vocab_shard: Optional[tuple] = None, gather: Any = None):
     if vocab_shard is not None or int(config.vocab_parallelism) != 1:
@@ -196,7 +196,7 @@ class LayeredEngine(MaxEngine):
     # the page map's staging buffer, and whether its last copy may still have to read it
     self._map_host = torch.zeros(B, MP, dtype=i32).pin_memory()
     self._map_read = torch.cuda.Event()
-    # a step that returned before its kernels were done: the event behind them and its stream (another stream waits for it)
+    # a call that returned before its kernels were done: the event behind the last of them (another stream waits for it)
     self._step_done = torch.cuda.Event()
     self._decode_tiles = torch.arange(B + 1, dtype=i32, device=dev)  # a decode step: every row is its own query tile and run
     self._decode_groups = torch.arange(B, dtype=i32, device=dev)
@@ -434,6 +434,11 @@ class LayeredEngine(MaxEngine):
       if stream != self._behind:
         stream.wait_event(self._step_done)
 
+  def _enqueued(self) -> None:
+    """The current stream holds work of this engine up to here, and the host does not wait for it: `_follow` of another stream does."""
+    self._behind = torch.cuda.current_stream(self.device)
+    self._step_done.record(self._behind)
+
   def _upload_page_state(self) -> None:  # (MaxEngine.release_pages calls it for device-resident page states; nothing to do here)
     return
 
@@ -558,8 +563,7 @@ class LayeredEngine(MaxEngine):
       self._behind = None
     else:
       self._desc_pending = True
-      self._step_done.record(stream)
-      self._behind = stream
+      self._enqueued()
     return out
 
   def _sample(self, logits: torch.Tensor, rows: int, token_out: torch.Tensor, log_prob_out: Optional[torch.Tensor], row_offset: int) -> None:
@@ -611,6 +615,7 @@ class LayeredEngine(MaxEngine):
     }
     data = torch.cat((first, torch.ones_like(first), torch.zeros_like(first)), dim=1)
     lp = self._first_log_prob.clone().reshape(1, 1) if self.config.return_log_prob else None
+    self._enqueued()  # (the draw and its copies included)
     return prefix, ResultTokens(data=data, log_prob=lp)
 
   def insert(self, prefix: dict, decode_state: dict, slot: int, request_id: Any = None) -> dict:

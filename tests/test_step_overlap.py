@@ -115,6 +115,46 @@ def test_a_third_stream_waits_too(monkeypatch):
   assert [s[0] for s in seen] == [[1, 2, 3], [4, 5]] and not first.queue
 
 
+class _OrderedStream(_Stream):
+  """Waits for what an event stood for when it was called, as a stream of the device does (the event may be recorded again before the wait is reached)."""
+
+  def wait_event(self, event):
+    stream, item = event.stream, event.item
+
+    def wait():
+      while item in stream.queue:
+        stream.queue.pop(0)()
+
+    self.queue.append(wait)
+
+
+def _serving(monkeypatch):
+  """An engine whose keys and draws leave a mark when their stream runs them."""
+  e, now, seen = _engine(monkeypatch)
+  now[0] = _OrderedStream()
+  i32 = torch.int32
+  e._params = e._state = {}
+  e.config.return_log_prob = True
+  e._states, e._uploaded_map = [], None
+  e._active, e._next_pos, e._generated, e._tokens = (torch.zeros(3, 1, dtype=i32) for _ in range(4))
+  e._first_token, e._first_log_prob, e._log_prob = torch.zeros(1, dtype=i32), torch.zeros(1), torch.zeros(3, 1)
+  e._result, e._logits, e._slot_ids = torch.zeros(3, 3, dtype=i32), torch.zeros(3, 1, 7), torch.arange(3, dtype=i32)
+  e._decode_groups, e._decode_tiles, e.use_cuda_graph = torch.zeros(3, dtype=i32), torch.arange(4, dtype=i32), False
+  marks = []
+  e._seed = lambda rng: rng is not None and now[0].queue.append(lambda: marks.append(("key", rng)))
+  e._sample = lambda logits, rows, *rest: now[0].queue.append(lambda: marks.append(("draw", rows)))
+  return e, now, marks
+
+
+def test_insert_on_another_stream_follows_the_draw(monkeypatch):
+  e, now, marks = _serving(monkeypatch)
+  prefix, _ = e.prefill(padded_tokens=[1, 2, 3], true_length=3, slot=1)
+  now[0] = _OrderedStream()
+  e.insert(prefix, e._state, 1)
+  now[0].synchronize()
+  assert marks == [("draw", 1)]
+
+
 def test_tokens_of_mixed_forms(monkeypatch):
   """Entries given as lists, arrays and tensors keep their order."""
   e, now, seen = _engine(monkeypatch)
