@@ -587,6 +587,7 @@ class LayeredEngine(MaxEngine):
       raise ValueError("a layered model prefills into the pages of a slot: pass slot=")
     if return_prompt_logp:
       raise NotImplementedError("return_prompt_logp is outside the decode path")
+    self._follow()  # (before the key: the draw in front has its own)
     self._seed(rng)
     slot, true_length = int(slot), int(true_length)
     toks = torch.as_tensor(padded_tokens).reshape(-1)
@@ -665,7 +666,6 @@ class LayeredEngine(MaxEngine):
 
   def _decode_rows(self) -> None:
     """One row per slot: token and position from the device state, the slot's pages grown by one token on the host."""
-    self._follow()
     B = self.max_concurrent_decodes
     ps = self.page_manager.update_decode_pages(self.page_state)
     grew = ps.has_active_page & (ps.num_pages_used * self.page_manager.tokens_per_page < ps.sequence_lengths)
@@ -689,6 +689,7 @@ class LayeredEngine(MaxEngine):
     if decode_state is not self._state:
       raise ValueError("decode_state must be the dict returned by this engine's init_decode_state (it is donated)")
     self._require_params(params)
+    self._follow()
     self._seed(rng)
     self._decode_rows()
     return decode_state, ResultTokens(data=self._result.clone(), log_prob=self._log_prob.clone() if self._log_prob is not None else None)
@@ -698,6 +699,7 @@ class LayeredEngine(MaxEngine):
     if decode_state is not self._state:
       raise ValueError("decode_state must be the dict returned by this engine's init_decode_state (it is donated)")
     self._require_params(params)
+    self._follow()
     if host_tokens is not None:
       self._tokens.copy_(host_tokens.reshape(self._tokens.shape), non_blocking=True)
     self._decode_rows()

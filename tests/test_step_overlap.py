@@ -155,6 +155,19 @@ def test_insert_on_another_stream_follows_the_draw(monkeypatch):
   assert marks == [("draw", 1)]
 
 
+@pytest.mark.parametrize("call", ["prefill", "generate"])
+def test_keys_follow_the_draws_before_them(monkeypatch, call):
+  e, now, marks = _serving(monkeypatch)
+  e.prefill(padded_tokens=[1, 2, 3], true_length=3, slot=1, rng=5)
+  now[0] = _OrderedStream()
+  if call == "prefill":
+    e.prefill(padded_tokens=[4], true_length=1, slot=2, rng=6)
+  else:
+    e.generate(e._params, e._state, rng=6)
+  now[0].synchronize()
+  assert marks == [("key", 5), ("draw", 1), ("key", 6), ("draw", 1 if call == "prefill" else 3)]
+
+
 def test_tokens_of_mixed_forms(monkeypatch):
   """Entries given as lists, arrays and tensors keep their order."""
   e, now, seen = _engine(monkeypatch)
