@@ -413,6 +413,7 @@ class LayeredEngine(MaxEngine):
         "generated_tokens": self._generated,
         "tokens": self._tokens,
     }
+    self._enqueued()
     return self._state
 
   def _upload_page_map(self) -> None:
@@ -427,15 +428,20 @@ class LayeredEngine(MaxEngine):
       self._uploaded_map = ps.page_map
 
   def _follow(self) -> None:
-    """The caller's stream behind a step that another stream may still hold (a step's pages, states and descriptors are the engine's).  That one stream waits
-    says nothing about the next one: the step is pending for all of them until the host has waited for it."""
+    """The caller's stream behind a call that another stream may still hold (pages, states and descriptors are the engine's).  Every call that enqueues something
+    starts with this and ends with `_enqueued`, so that the last event stands for all before it; it is pending for every other stream until the host has waited."""
     if self._behind is not None:
       stream = torch.cuda.current_stream(self.device)
-      if stream != self._behind:
+      if stream != self._behind and not self._capturing():  # (a graph's replays are ordered by who launches them)
         stream.wait_event(self._step_done)
+
+  def _capturing(self) -> bool:
+    return self.device.type == "cuda" and torch.cuda.is_current_stream_capturing()
 
   def _enqueued(self) -> None:
     """The current stream holds work of this engine up to here, and the host does not wait for it: `_follow` of another stream does."""
+    if self._capturing():  # (nothing is enqueued yet)
+      return
     self._behind = torch.cuda.current_stream(self.device)
     self._step_done.record(self._behind)
 
@@ -445,8 +451,11 @@ class LayeredEngine(MaxEngine):
   def release_pages(self, slot: int) -> None:
     """The slot's pages go back to the pool.  Its row of the page map is cleared too, so that the row an empty slot still
     contributes to a decode step lands on page 0 (never handed out) and not on a page somebody else owns by then."""
-    slot = int(slot)
     self._follow()
+    self._release(int(slot))
+    self._enqueued()
+
+  def _release(self, slot: int) -> None:
     ps = self.page_manager.release_pages(page_state=self.page_state, page_group_id=slot)
     page_map = ps.page_map.copy()
     page_map[slot] = 0
@@ -599,7 +608,7 @@ class LayeredEngine(MaxEngine):
       if int(self.page_state.sequence_lengths[slot]) != start:
         raise ValueError(f"slot {slot} holds {int(self.page_state.sequence_lengths[slot])} tokens, the prefix has {start}")
     else:
-      self.release_pages(slot)
+      self._release(slot)
     if start + true_length >= int(self.config.max_target_length):
       raise ValueError(f"{start + true_length} prompt tokens leave no room to decode (max_target_length={self.config.max_target_length})")
     prompt = toks[:true_length].cpu()
@@ -632,6 +641,7 @@ class LayeredEngine(MaxEngine):
     self._tokens[slot].copy_(prefix["tokens"][0])
     self._active[slot].fill_(1)
     self._logits[slot].copy_(prefix["logits"][0])
+    self._enqueued()
     return decode_state
 
   def fill_synthetic_context(self, prefill_lengths, ar_lengths=None, seed: int = 7) -> dict:
@@ -659,6 +669,7 @@ class LayeredEngine(MaxEngine):
         t.copy_(torch.randn(t.shape, device=self.device, generator=g) * 0.1)
     self._active.fill_(1)
     self._tokens.copy_(torch.randint(0, int(self.config.vocab_size), self._tokens.shape, device=self.device, generator=g, dtype=torch.int32))
+    self._enqueued()
     return state
 
   def bulk_insert(self, prefix: dict, decode_state: dict, slots: list) -> dict:
@@ -692,7 +703,9 @@ class LayeredEngine(MaxEngine):
     self._follow()
     self._seed(rng)
     self._decode_rows()
-    return decode_state, ResultTokens(data=self._result.clone(), log_prob=self._log_prob.clone() if self._log_prob is not None else None)
+    result = ResultTokens(data=self._result.clone(), log_prob=self._log_prob.clone() if self._log_prob is not None else None)
+    self._enqueued()
+    return decode_state, result
 
   def generate_to_host(self, params: Any, decode_state: dict, host_result: torch.Tensor, host_tokens: Optional[torch.Tensor] = None,
                        host_log_prob: Optional[torch.Tensor] = None, sync: bool = False):
@@ -708,4 +721,7 @@ class LayeredEngine(MaxEngine):
       host_log_prob.copy_(self._log_prob, non_blocking=True)
     if sync:
       torch.cuda.current_stream(self.device).synchronize()
+      self._behind = None
+    else:
+      self._enqueued()
     return decode_state, ResultTokens(data=host_result, log_prob=host_log_prob)

@@ -23,6 +23,19 @@ class _Stream:
     self.queue.append(event.synchronize)
 
 
+class _OrderedStream(_Stream):
+  """Waits for what an event stood for when it was called, as a stream of the device does (the event may be recorded again before the wait is reached)."""
+
+  def wait_event(self, event):
+    stream, item = event.stream, event.item
+
+    def wait():
+      while item in stream.queue:
+        stream.queue.pop(0)()
+
+    self.queue.append(wait)
+
+
 class _Event:
   def __init__(self):
     self.stream, self.left = None, None
@@ -106,26 +119,14 @@ def test_another_stream_waits(monkeypatch):
 def test_a_third_stream_waits_too(monkeypatch):
   """A stream that has waited for a prompt (here to free a slot) does not stand for the others."""
   e, now, seen = _engine(monkeypatch)
+  now[0] = _OrderedStream()
   e._states, e._active, e._next_pos = [], torch.ones(3, 1, dtype=torch.int32), torch.ones(3, 1, dtype=torch.int32)
   e._step([(0, [1, 2, 3], [2])], wait=False)
-  first, now[0] = now[0], _Stream()
+  first, now[0] = now[0], _OrderedStream()
   e.release_pages(1)
-  now[0] = _Stream()
+  now[0] = _OrderedStream()
   e.step([(2, [4, 5], [1])])
   assert [s[0] for s in seen] == [[1, 2, 3], [4, 5]] and not first.queue
-
-
-class _OrderedStream(_Stream):
-  """Waits for what an event stood for when it was called, as a stream of the device does (the event may be recorded again before the wait is reached)."""
-
-  def wait_event(self, event):
-    stream, item = event.stream, event.item
-
-    def wait():
-      while item in stream.queue:
-        stream.queue.pop(0)()
-
-    self.queue.append(wait)
 
 
 def _serving(monkeypatch):
@@ -166,6 +167,41 @@ def test_keys_follow_the_draws_before_them(monkeypatch, call):
     e.generate(e._params, e._state, rng=6)
   now[0].synchronize()
   assert marks == [("key", 5), ("draw", 1), ("key", 6), ("draw", 1 if call == "prefill" else 3)]
+
+
+def test_a_step_follows_a_decode_step(monkeypatch):
+  """A decode step whose page map is still on its way, a step on another stream (which uploads none), and a decode step that grows a page."""
+  e, now, marks = _serving(monkeypatch)
+  maps, run = [], e._run
+  e._run = lambda *args, **kw: now[0].queue.append(lambda: maps.append(e._page_map_dev.now.copy()))
+  e.step([(0, [1, 2, 3], []), (1, [4], [])])
+  first, want = now[0], [e.page_state.page_map]
+  e.generate(e._params, e._state)
+  e.generate(e._params, e._state)  # (slot 0 grows a page)
+  want += [maps[0], e.page_state.page_map]
+  now[0] = _OrderedStream()
+  e.step([(1, [5], [])])
+  want.append(e.page_state.page_map)
+  now[0] = first
+  for _ in range(4):
+    e.generate(e._params, e._state)
+    want.append(e.page_state.page_map)
+  first.synchronize()
+  assert len(maps) == len(want) and all((a == b).all() for a, b in zip(maps, want))
+
+
+def test_a_prompt_follows_its_slot_s_release(monkeypatch):
+  e, now, marks = _serving(monkeypatch)
+  e.step([(1, [1, 2], [])])
+  e._states = [(torch.zeros(3, 2),)]
+  monkeypatch.setattr(torch, "_foreach_zero_", lambda ts: now[0].queue.append(lambda: marks.append("zero")))
+  e.prefill(padded_tokens=[1, 2, 3], true_length=3, slot=1)
+  first, now[0] = now[0], _OrderedStream()
+  e.release_pages(1)
+  now[0] = first
+  e.prefill(padded_tokens=[4, 5], true_length=2, slot=1)
+  first.synchronize()
+  assert marks == ["zero", "zero", ("draw", 1), "zero", "zero", "zero", "zero", ("draw", 1)]
 
 
 def test_tokens_of_mixed_forms(monkeypatch):
