@@ -211,6 +211,8 @@ class LayeredEngine(MaxEngine):
 
   def __del__(self):
     try:
+      if not self._capturing():
+        self._settle()
       if self._handle:
         self.lib.mtx_layered_destroy(self._handle)
     except Exception:  # pragma: no cover - interpreter shutdown
@@ -240,6 +242,7 @@ class LayeredEngine(MaxEngine):
 
   def _create(self, lp: LayeredParams) -> None:
     cfg, dev = self.config, self.device
+    self._settle()
     if self._handle:
       self.lib.mtx_layered_destroy(self._handle)
       self._handle = ctypes.c_void_p()
@@ -444,6 +447,14 @@ class LayeredEngine(MaxEngine):
       return
     self._behind = torch.cuda.current_stream(self.device)
     self._step_done.record(self._behind)
+
+  def _settle(self) -> None:
+    """The host behind every call: pages, states and workspace that are given up go to whatever their own stream allocates next, which knows nothing of the
+    stream that may still use them."""
+    if self._behind is not None:
+      self._step_done.synchronize()
+      self._behind = None
+      self._desc_pending = self._map_pending = False
 
   def _upload_page_state(self) -> None:  # (MaxEngine.release_pages calls it for device-resident page states; nothing to do here)
     return

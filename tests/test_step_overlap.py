@@ -204,6 +204,19 @@ def test_a_prompt_follows_its_slot_s_release(monkeypatch):
   assert marks == ["zero", "zero", ("draw", 1), "zero", "zero", "zero", "zero", ("draw", 1)]
 
 
+def test_an_engine_gives_nothing_up_under_a_prompt(monkeypatch):
+  """Dropped engines and replaced weights: the buffers of a prompt that returned early are in use until its stream is done."""
+  e, now, seen = _engine(monkeypatch)
+  e._handle, first = None, now[0]
+  e._step([(0, [1, 2, 3], [2])], wait=False)
+  with pytest.raises(AttributeError):  # (no weights here: what comes after the wait)
+    e._create(types.SimpleNamespace(float32=False))
+  assert not first.queue and len(seen) == 1
+  e._step([(1, [4], [])], wait=False)
+  e.__del__()
+  assert not first.queue and len(seen) == 2
+
+
 def test_tokens_of_mixed_forms(monkeypatch):
   """Entries given as lists, arrays and tensors keep their order."""
   e, now, seen = _engine(monkeypatch)
