@@ -52,10 +52,21 @@ def test_long_walk_repeats_short_portions():
     assert all(torch.equal(a, b) for a, b in zip(*states))
 
 
-@pytest.mark.parametrize("kind,heads,dim,vdim", [("gla", 24, 64, 128), ("gla", 2, 256, 40), ("gla", 3, 100, 72), ("mlstm", 20, 128, 128), ("mlstm", 2, 200, 20), ("mlstm", 1, 64, 8)])
-def test_walk_of_two_long_runs(kind, heads, dim, vdim):
+def columns_per_thread(runs, heads, dim, vdim):
+  """What csrc/layered.cu (launch_rec_scan, launch_rec_walk) takes on this GPU for runs of 16 tokens and more; 0: the walk token by token."""
+  sms, ctas = torch.cuda.get_device_properties(0).multi_processor_count, lambda cols: runs * heads * -(-vdim // cols)
+  if ctas(16) >= 2 * sms or dim < 64 or runs * heads * vdim * 8 >= 512 * sms:
+    return 0
+  return 1 if ctas(8) <= sms else 2
+
+
+@pytest.mark.parametrize("kind,heads,dim,vdim,columns", [
+    ("gla", 24, 64, 128, 0), ("gla", 2, 256, 40, 1), ("gla", 3, 100, 72, 1), ("mlstm", 20, 128, 128, 0), ("mlstm", 2, 200, 20, 1), ("mlstm", 1, 64, 8, 1),
+    ("gla", 12, 64, 128, 2), ("gla", 16, 128, 40, 2), ("gla", 12, 256, 72, 2), ("mlstm", 16, 64, 40, 2), ("mlstm", 12, 128, 128, 2), ("mlstm", 12, 200, 72, 2)])
+def test_walk_of_two_long_runs(kind, heads, dim, vdim, columns):
   """Two runs of a step, ends before, at and behind a chunk of 16 tokens, one and two columns per thread, channels and columns that fill neither slices nor
-  CTAs: the bits of portions of ten tokens, which are walked token by token."""
+  CTAs: the bits of portions of ten tokens, which are walked token by token -- the states' and, by the logits of every position, the read-outs'."""
+  assert columns_per_thread(2, heads, dim, vdim) == columns
   layer = g.gla_layer(heads, dim, vdim) if kind == "gla" else g.parallel_layer(4, 2, 32, heads, dim, vdim)
   cfg = g.model_dict(256, 320, [layer])
   config = pyconfig.from_model_dict(cfg, dtype="float32", per_device_batch_size=2, max_target_length=128, pagedattn_tokens_per_page=16, pagedattn_num_pages=20)
@@ -64,8 +75,13 @@ def test_walk_of_two_long_runs(kind, heads, dim, vdim):
     engine = maxengine.MaxEngine(config)
     engine.load_params(tensors)
     state = engine.init_decode_state()
+    logits = ([], [])
     for at in range(0, 79, portion):
-      parts = [(slot, t[at : at + portion], [len(t[at : at + portion]) - 1]) for slot, t in enumerate(toks) if t[at : at + portion]]
-      engine.step(parts)
-    states.append([t[:2].clone() for t in state["cache"]["recurrent_state"]])
+      parts = [(slot, t[at : at + portion], list(range(len(t[at : at + portion])))) for slot, t in enumerate(toks) if t[at : at + portion]]
+      out = engine.step(parts).split([len(p[1]) for p in parts])
+      for (slot, _, _), rows in zip(parts, out):
+        logits[slot].append(rows)
+    if not columns:  # (the tens behind 70 are one run, for which the walk token by token cuts a column into more slices: read-outs added up in another order)
+      logits[0][-1] = logits[0][-1][: 23 if portion == 47 else 0]
+    states.append([t[:2].clone() for t in state["cache"]["recurrent_state"]] + [torch.cat(rows) for rows in logits])
   assert all(torch.equal(a, b) for a, b in zip(*states))

@@ -1,0 +1,53 @@
+"""The layered engine's row-wise kernels by the size of a row (csrc/layer_ops.cuh, recurrent_out_kernel): norms with 1, 2, 4 and 8 groups of 1024 channels per
+thread, the recurrences' output with 2, 4 and 8 channels of a head per lane and with any number of them, against the oracles."""
+
+import numpy as np
+import pytest
+import torch
+
+from maxtext_indextts2_b200 import gugidra, maxengine, pyconfig, zakelorn
+from oracle import gugidra_ref, zakelorn_ref
+
+pytestmark = pytest.mark.gpu
+
+# float32: sums of up to 8192 products of one sign at random, 2^-24 sqrt(8192) = 5e-6 of their size each, a few of them one after the other; bfloat16: the
+# bound of the designs' own tests (some ten roundings of 2^-9 along a row)
+TOL = {"float32": 3e-5, "bfloat16": 3e-2}
+TOKENS = [5, 0, 60, 7, 33]
+
+
+def error(dtype, got, want):
+  got, want = got.cpu().numpy().astype(np.float64), np.asarray(want)
+  if dtype == "float32":
+    return np.abs(got - want).max() / np.abs(want).max()
+  return np.sqrt(((got - want) ** 2).mean() / (want**2).mean())
+
+
+def logits(model, tensors, dtype):
+  cfg = pyconfig.from_model_dict(model, dtype=dtype, per_device_batch_size=2, max_target_length=32, pagedattn_tokens_per_page=8, pagedattn_num_pages=12)
+  engine = maxengine.MaxEngine(cfg)
+  engine.load_params({k: torch.from_numpy(np.asarray(v)).to(torch.bfloat16) for k, v in tensors.items()})
+  engine.init_decode_state()
+  return torch.cat([engine.step([(0, TOKENS[:4], [0, 1, 2, 3])]), engine.step([(0, TOKENS[4:], [0])])])
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("width", [1024, 1028, 2048, 2052, 4096, 4100, 8192])
+def test_norms_of_a_row(width, dtype):
+  """Widths at both ends of each number of groups; the loop adds the embedding and a vector to the row in front of its second time."""
+  layers = [gugidra.gla_layer(1, 8, 8, mlp=gugidra.dense_ff(16, 2.0)), gugidra.gla_layer(1, 8, 8)]
+  model = gugidra.model_dict(width, 61, layers, eps=1e-5, embed_scale=1.7, loop={"start": 0, "stop": 1, "times": 2})
+  t = gugidra_ref.random_model(model, seed=width)
+  assert error(dtype, logits(model, t, dtype), gugidra_ref.logits_of(model, t, TOKENS)) < TOL[dtype]
+  layer = zakelorn.parallel_layer(zakelorn.attention_part(1, 1, 8, window=4, keep_first=1), zakelorn.lightning_part(1, 8, 8), 0.9, 1.2, zakelorn.dense_ff(16))
+  model = zakelorn.model_dict(width, 61, [layer], eps=1e-5, embed_scale=3.0)
+  t = zakelorn_ref.random_model(model, seed=width)
+  assert error(dtype, logits(model, t, dtype), zakelorn_ref.forward(model, t, TOKENS)) < TOL[dtype]
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("vdim", [30, 64, 65, 128, 129, 250, 256, 257, 320])
+def test_output_of_a_recurrence(vdim, dtype):
+  model = gugidra.model_dict(64, 61, [gugidra.gla_layer(9, 8, vdim)], eps=1e-5, embed_scale=1.7)  # (nine heads: one more than warps)
+  t = gugidra_ref.random_model(model, seed=vdim)
+  assert error(dtype, logits(model, t, dtype), gugidra_ref.logits_of(model, t, TOKENS)) < TOL[dtype]
