@@ -198,14 +198,16 @@ int mtx_decode_step(mtx_engine* e, int rows, mtx_stream stream);
 /* Same step, replayed from a CUDA graph captured on first use (one graph per `rows`). */
 int mtx_decode_step_graph(mtx_engine* e, int rows, mtx_stream stream);
 
-/* The step as a serving loop calls it, with HOST buffers (pinned memory for the copies to be asynchronous): optionally copies this
- * step's input tokens host -> device (tokens_host [rows] or NULL to keep decode_state.tokens), replays the step's CUDA graph, and
- * copies ResultTokens.data [rows, 3] (and the log-probs [rows] when log_prob_host is non-NULL and return_log_prob is on) device ->
- * host, all enqueued on `stream`: the caller synchronises the stream once and reads result_host (offline_engine.py:612-614 copies
- * the result tokens to the host the same way). */
+/* The step as a serving loop calls it, with HOST buffers (pinned memory for the call to be asynchronous): takes this step's input
+ * tokens from tokens_host [rows] (NULL: decode_state.tokens), replays the step's CUDA graph, and leaves ResultTokens.data [rows, 3]
+ * in result_host (and the log-probs [rows] in log_prob_host when that is non-NULL and return_log_prob is on), all enqueued on
+ * `stream`: the caller synchronises the stream once and reads result_host (offline_engine.py:612-614 copies the result tokens to
+ * the host the same way). */
 int mtx_decode_step_host(mtx_engine* e, int rows, const int32_t* tokens_host, int32_t* result_host, float* log_prob_host, mtx_stream stream);
-/* With pinned buffers the copies are nodes of the step's graph (one graph per set of buffers: reuse them), so the call above is ONE
- * driver call.  This variant also waits for the stream: result_host is valid on return. */
+/* With pinned, 4-byte aligned buffers the step's own kernels read the tokens and write the result in host memory (one graph per set
+ * of buffers, 16 sets kept: reuse them), so the call above is ONE launch without copies; until the step has run, tokens_host stays
+ * as it is and result_host is the step's.  Other buffers are copied before and behind the step.  This variant also waits for the
+ * stream: result_host is valid on return. */
 int mtx_decode_step_host_sync(mtx_engine* e, int rows, const int32_t* tokens_host, int32_t* result_host, float* log_prob_host, mtx_stream stream);
 
 /* Vocab-parallel logits: this process holds `vocab_size` rows of the logits matrix starting
@@ -678,6 +680,9 @@ typedef struct mtx_layered mtx_layered; /* opaque */
 
 int mtx_layered_create(const mtx_layered_config* cfg, const mtx_layer_desc* layers, mtx_layered** out);
 int mtx_layered_destroy(mtx_layered* e);
+/* Activations of max_rows rows, and -- bfloat16 models with MTX_REC_DECAY layers, max_rows >= 128 -- the recurrence's state before every
+ * 64 tokens of a step: max_rows / 64 + 8 states of the widest layer (heads * vdim * dim * 4 bytes each, vdim and dim rounded up to 16),
+ * at most 256 MB. */
 size_t mtx_layered_workspace_bytes(const mtx_layered* e);
 int mtx_layered_bind(mtx_layered* e, void* workspace, size_t workspace_bytes);
 /* All layers for the rows of `b` (appending their keys / values to the pages), then the logits of the wanted rows. */

@@ -312,8 +312,8 @@ decode_attn_wide_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
 // its warps to be done with them.
 //
 // Bound: what an SM takes in from the L2 (64 KB per tile at about 64 B per ns), and the wait for it where the tiles are not yet used up.  3001 positions, 8 heads
-// over 4 kv heads, five layers with a window of 1024 and a global one: 492 us per layer with one group of columns per tile (the last 185
-// positions a step of their own), 290 us with four (and all in one launch).
+// over 4 kv heads, the mean of five layers with a window of 1024 and a global one: 492 us with one group of columns per tile, 336 us with four (the last
+// 185 positions a step of their own in both), 289 us with all of them in one launch (a windowed layer 280, the global one 351).
 struct PromptWideParams {
   const bf16* q;   // [rows, hq * D]
   bf16* out;       // [rows, hq * D]

@@ -902,8 +902,8 @@ int enqueue_prefill_pass(mtx_engine* e, int rows, const int32_t* tokens, int sta
 
 // Rows of the next pass of a prompt with `left` rows to go; 256 or fewer: a step of the 256-row kernels takes them.  A gemma3 pass has the bits of the
 // steps, so the rows behind its last 256 come along only where their own step would cut K and the keys as the 256-row steps do: the plans
-// know rows rounded up to a power of two, so from 129 on.  (3001 positions through six layers, the last 185 as a step
-// of their own: 5.90 ms, in the pass 5.18.)
+// know rows rounded up to a power of two, so from 129 on.  (3001 positions through six layers, this step alone: 5.90 ms with the last 185 as a step
+// of their own, 5.18 in the pass.)
 int pass_rows(const mtx_engine* e, int left) {
   const int wide = left < e->pf_rows ? left : e->pf_rows, rest = wide % 256;
   if (e->cfg.decoder_block != 1 || rest == 0) return wide;

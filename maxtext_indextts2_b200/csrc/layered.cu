@@ -743,7 +743,10 @@ int launch_rec_walk_t(const RecScanArgs& ra, int n_runs, cudaStream_t st) {
 }
 template <int KIND, int RPT>
 int launch_rec_walk(const RecScanArgs& ra, int n_runs, int num_sms, cudaStream_t st) {
-  // one column per thread while that leaves every CTA an SM of its own
+  // One column per thread while that leaves every CTA an SM of its own; two beyond, where a second CTA on an SM costs more than columns that share their
+  // operands.  2048 tokens, heads of 64 / 128 / 256 channels and 128 columns on 148 SMs, one column per thread against two: nine heads (144 CTAs of single
+  // columns) GLA 112 / 150 / 276 us against 124 / 181 / 291, mLSTM 109 / 172 / 309 against 175 / 214 / 347; ten heads (160) GLA 151 / 257 / 544 against
+  // 124 / 181 / 292, mLSTM 154 / 241 / 603 against 175 / 214 / 348.  (The mLSTM's heads of 64 channels are the one size that loses by the line.)
   const bool single = (long long)n_runs * ra.heads * ((ra.vdim + 2 * kWalkWarps - 1) / (2 * kWalkWarps)) <= num_sms;
   return single ? launch_rec_walk_t<KIND, RPT, 1>(ra, n_runs, st) : launch_rec_walk_t<KIND, RPT, 2>(ra, n_runs, st);
 }
