@@ -539,6 +539,7 @@ class LayeredEngine(MaxEngine):
     self._upload_page_map()
     out = torch.empty(len(want), V, dtype=torch.float32, device=self.device)
     if rows == 0:
+      self._enqueued()  # (the page map may be on its way)
       return out
     R = self._max_rows
     ends = np.cumsum(counts)

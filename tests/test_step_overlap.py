@@ -190,6 +190,21 @@ def test_a_step_follows_a_decode_step(monkeypatch):
   assert len(maps) == len(want) and all((a == b).all() for a, b in zip(maps, want))
 
 
+def test_a_step_of_no_rows_uploads_for_the_next_stream(monkeypatch):
+  e, now, marks = _serving(monkeypatch)
+  maps = []
+  e._run = lambda *args, **kw: now[0].queue.append(lambda: maps.append(e._page_map_dev.now.copy()))
+  first = now[0]
+  e.prefill(padded_tokens=[1, 2, 3], true_length=3, slot=1)
+  e.release_pages(1)
+  now[0] = _OrderedStream()
+  assert e.step([]).shape == (0, 7)
+  now[0] = first
+  e.generate(e._params, e._state)
+  first.synchronize()
+  assert (maps[-1] == e.page_state.page_map).all() and maps[-1].sum() == 0
+
+
 def test_a_prompt_follows_its_slot_s_release(monkeypatch):
   e, now, marks = _serving(monkeypatch)
   e.step([(1, [1, 2], [])])
