@@ -138,9 +138,7 @@ __device__ __forceinline__ void rows_scale16(float (&v)[16], float s) {
 
 // linears.py:425-476, mlp_activations [silu, linear]; w01 rows are interleaved 16 at a time (gate, value), so the
 // fragment at n0 (a multiple of 32) is the gate and the one at n0 + 16 the value of MLP features n0/2 .. n0/2+15.
-__device__ __forceinline__ void rows_epi_swiglu(const EpiArgs& e, int N2, int r, int n0, const float (&g)[16], const float (&u)[16]) {
-  if (n0 >= N2) return;
-  float o[16];
+__device__ __forceinline__ void rows_swiglu(const EpiArgs& e, const float (&g)[16], const float (&u)[16], float (&o)[16]) {
 #pragma unroll
   for (int j = 0; j < 16; j += 2) {
     const uint32_t ga = pack_bf16x2(g[j], g[j + 1]), ub = pack_bf16x2(u[j], u[j + 1]);
@@ -153,6 +151,11 @@ __device__ __forceinline__ void rows_epi_swiglu(const EpiArgs& e, int N2, int r,
     o[j] = bf16_lo(act) * bf16_lo(ub);
     o[j + 1] = bf16_hi(act) * bf16_hi(ub);
   }
+}
+__device__ __forceinline__ void rows_epi_swiglu(const EpiArgs& e, int N2, int r, int n0, const float (&g)[16], const float (&u)[16]) {
+  if (n0 >= N2) return;
+  float o[16];
+  rows_swiglu(e, g, u, o);
   frag_store_bf16(e.out + (long long)r * e.ld_out + (n0 >> 1), o);
 }
 

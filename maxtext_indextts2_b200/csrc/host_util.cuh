@@ -347,12 +347,19 @@ int wide_tile_columns(int rows, int n, int unit, int pairs) {
   return best;
 }
 
+// K blocks of a stage: two where the tile is narrow, since up to 128 columns a round of barrier, loads, MMAs and commit takes longer than its four MMAs
+// (389 x 1280 x 5120, tiles of 64 columns: 20.0 us with one, 13.6 with two).  From 160 on two such stages are too few in flight (4000 x 1280 x
+// 5120, 160 columns: 41.6 us with one, 44.9 with two).  Every segment has to be whole stages.
+int wide_group(int bn, int k, int segments) { return bn <= 128 && (k / kBlockK) % (2 * segments) == 0 ? 2 : 1; }
+
 // epi(x[rows, k] . w[n, k]^T), n a multiple of 32 (and of unit), k of 64, 16-byte aligned operands
-template <class EPI>
+template <class EPI, int MODE = kWideRows>
 int launch_wide(const void* x, const void* w, int rows, int n, int k, int unit, const EPI& epi, int num_sms, cudaStream_t st, int segments = 1) {
+  if constexpr (EPI::kFragments && MODE == kWideRows)
+    if (segments > 1) return launch_wide<EPI, kWideParts>(x, w, rows, n, k, unit, epi, num_sms, st, segments);
   static bool attr_set = false;  // per template instance
   if (!attr_set) {
-    MTX_CUDA(cudaFuncSetAttribute(gemm_wide_kernel<EPI, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    MTX_CUDA(cudaFuncSetAttribute(gemm_wide_kernel<EPI, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     attr_set = true;
   }
   const int pairs = num_sms / 2;
@@ -362,7 +369,8 @@ int launch_wide(const void* x, const void* w, int rows, int n, int k, int unit, 
   p.n = n;
   p.k = k;
   p.bn = wide_tile_columns(rows, n, unit, pairs);
-  p.stages = wide_stages(p.bn);
+  p.group = wide_group(p.bn, k, segments);
+  p.stages = wide_stages(p.bn, p.group, EPI::kRowBytes);
   p.segments = segments;
   p.first = (p.bn / unit + 1) / 2 * unit;
   CUtensorMap tw, tx;
@@ -370,7 +378,7 @@ int launch_wide(const void* x, const void* w, int rows, int n, int k, int unit, 
   MTX_TRY(make_map(&tx, x, k, rows, 128));
   const int tiles = ((rows + kPairRows - 1) / kPairRows) * ((n + p.bn - 1) / p.bn);
   g_cluster_x = 2;
-  const int rc = launch(gemm_wide_kernel<EPI, false>, dim3(2 * (tiles < pairs ? tiles : pairs)), dim3(kPairThreads), wide_smem_bytes(p.bn, p.stages), st, tw, tx, p, epi);
+  const int rc = launch(gemm_wide_kernel<EPI, MODE>, dim3(2 * (tiles < pairs ? tiles : pairs)), dim3(kPairThreads), wide_smem_bytes(p.bn, p.stages, p.group, EPI::kRowBytes), st, tw, tx, p, epi);
   g_cluster_x = 1;
   return rc;
 }
@@ -380,7 +388,7 @@ template <class EPI>
 int launch_wide_grouped(const void* x, const void* w, const int* group_off, int groups, int slots, int n, int k, const EPI& epi, int num_sms, cudaStream_t st) {
   static bool attr_set = false;  // per template instance
   if (!attr_set) {
-    MTX_CUDA(cudaFuncSetAttribute(gemm_wide_kernel<EPI, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    MTX_CUDA(cudaFuncSetAttribute(gemm_wide_kernel<EPI, kWideGrouped>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     attr_set = true;
   }
   const int pairs = num_sms / 2;
@@ -390,7 +398,8 @@ int launch_wide_grouped(const void* x, const void* w, const int* group_off, int 
   p.n = n;
   p.k = k;
   p.bn = wide_tile_columns(slots + groups * (kPairRows / 2), n, 32, pairs);  // (a group's last tile is half empty on average)
-  p.stages = wide_stages(p.bn);
+  p.group = wide_group(p.bn, k, 1);
+  p.stages = wide_stages(p.bn, p.group, EPI::kRowBytes);
   p.segments = 1;
   p.group_off = group_off;
   p.groups = groups;
@@ -399,7 +408,7 @@ int launch_wide_grouped(const void* x, const void* w, const int* group_off, int 
   MTX_TRY(make_map(&tw, w, k, uint64_t(groups) * n, uint32_t(p.bn / 2)));
   MTX_TRY(make_map(&tx, x, k, slots, 128));
   g_cluster_x = 2;
-  const int rc = launch(gemm_wide_kernel<EPI, true>, dim3(2 * pairs), dim3(kPairThreads), wide_smem_bytes(p.bn, p.stages), st, tw, tx, p, epi);
+  const int rc = launch(gemm_wide_kernel<EPI, kWideGrouped>, dim3(2 * pairs), dim3(kPairThreads), wide_smem_bytes(p.bn, p.stages, p.group, EPI::kRowBytes), st, tw, tx, p, epi);
   g_cluster_x = 1;
   return rc;
 }

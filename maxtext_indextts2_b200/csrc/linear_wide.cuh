@@ -19,33 +19,41 @@ struct WideLinEpi {
   float limit;
   int silu0, silu1;
 
-  __device__ __forceinline__ int prepare(const WideTile&) const { return 0; }
+  static constexpr bool kGated = EPI == LIN_GATED || EPI == LIN_GATED_CLAMP, kNarrow = kGated || EPI == LIN_ACT || EPI == LIN_RELU2 || EPI == LIN_GELU;
+  static constexpr int kChunks = kGated ? 2 : kNarrow ? 4 : 8;  // 16-byte chunks that 32 columns become
+  static constexpr int kRowBytes = kNarrow ? 64 : 128;
+  typedef WideStage<kRowBytes> Stage;
+
+  __device__ __forceinline__ int prepare(const WideTile&, const Stage&) const { return 0; }
 
   // 32 columns of a row
-  __device__ __forceinline__ void fragment(const WideTile& w, int n, int, int c, float (&a)[16], float (&b)[16]) const {
-    columns(w, n, c, a);
-    columns(w, n, c + 16, b);
+  __device__ __forceinline__ void fragment(const WideTile& w, int, int c, float (&a)[16], float (&b)[16], const Stage& st) const {
+    const int chunk = st.template chunk<kChunks>(w, c);
+    if (w.valid) {  // (a row that is not there is zeros: 0 / x takes the quotient's slow way, alone in its warp)
+      columns(w.n0 + c, a, chunk, st);
+      columns(w.n0 + c + 16, b, chunk + kChunks / 2, st);
+    }
+    const long long row0 = (long long)(w.row - st.lane) * ldo;
+    if constexpr (kNarrow) st.template done<kChunks>(w, c, act + row0 + ((w.n0 + w.c0) >> (kGated ? 1 : 0)), size_t(ldo) * 2);
+    else st.template done<kChunks>(w, c, out + row0 + w.n0 + w.c0, size_t(ldo) * 4);
   }
-  // 16 of them
-  __device__ __forceinline__ void columns(const WideTile& w, int n, int c, float (&v)[16]) const {
-    constexpr bool gated = EPI == LIN_GATED || EPI == LIN_GATED_CLAMP, narrow = gated || EPI == LIN_ACT || EPI == LIN_RELU2 || EPI == LIN_GELU;
+  // 16 of them, from column col of the output on, into the chunks from `chunk` on
+  __device__ __forceinline__ void columns(int col, float (&v)[16], int chunk, const Stage& st) const {
 #pragma unroll
     for (int j = 0; ROUND && j < 16; j += 2) {
       const uint32_t b = pack_bf16x2(v[j], v[j + 1]);
       v[j] = bf16_lo(b);
       v[j + 1] = bf16_hi(b);
     }
-    const int col = w.n0 + c;
-    if (gated) {  // (gate, up) of eight features
+    if constexpr (kGated) {  // (gate, up) of eight features
       float g[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const float a = v[2 * j], u = v[2 * j + 1];
         g[j] = EPI == LIN_GATED ? gelu_tanh_f(a) * u : (limit > 0.0f ? clamped_gate_f(a, u, limit) : silu_gate_f(a, u));
       }
-      *reinterpret_cast<uint4*>(act + (long long)w.row * ldo + (col >> 1)) =
-          make_uint4(pack_bf16x2(g[0], g[1]), pack_bf16x2(g[2], g[3]), pack_bf16x2(g[4], g[5]), pack_bf16x2(g[6], g[7]));
-    } else if (narrow) {
+      st.put(chunk, wide_pack8(g));
+    } else if constexpr (kNarrow) {
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         if (EPI == LIN_GELU) v[j] = gelu_tanh_f(v[j]);
@@ -54,12 +62,15 @@ struct WideLinEpi {
           v[j] *= v[j];
         }
       }
-      frag_store_bf16(act + (long long)w.row * ldo + col, v);
+      st.put(chunk, wide_pack8(v));
+      st.put(chunk + 1, wide_pack8(v + 8));
     } else {
       if (EPI == LIN_SILU_COLS && col + 16 > silu0 && col < silu1) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j)
-          if (col + j >= silu0 && col + j < silu1) v[j] = bf16r(silu_gate_f(v[j], 1.0f));
+        for (int j = 0; j < 16; ++j) {
+          const float g = bf16r(silu_gate_f(v[j], 1.0f));
+          v[j] = col + j >= silu0 && col + j < silu1 ? g : v[j];
+        }
       }
       if (EPI == LIN_BIAS) {
 #pragma unroll
@@ -71,18 +82,9 @@ struct WideLinEpi {
           v[j + 3] += b.w;
         }
       }
-      float4* o = reinterpret_cast<float4*>(out + (long long)w.row * ldo + col);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) o[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-    }
-  }
-
-  template <class LD>
-  __device__ __forceinline__ void operator()(const WideTile& w, int n, int, LD&& ld16) const {
-    for (int c = w.c0; c < w.c1; c += 16) {
-      float v[16];
-      ld16(c, v);
-      if (w.valid) columns(w, n, c, v);
+      for (int j = 0; j < 4; ++j)
+        st.put(chunk + j, make_uint4(__float_as_uint(v[4 * j]), __float_as_uint(v[4 * j + 1]), __float_as_uint(v[4 * j + 2]), __float_as_uint(v[4 * j + 3])));
     }
   }
 };

@@ -61,6 +61,25 @@ def test_long_steps_repeat_short_ones(name):
   assert all(torch.isfinite(t).all() for t in out[0]) and all(torch.equal(a, b) for a, b in zip(*out))
 
 
+@pytest.mark.parametrize("rows", [257, 288, 545, 767])
+@pytest.mark.parametrize("ff", [448, 256])
+def test_part_empty_row_tile_repeats_a_whole_one(rows, ff):
+  """The last row tile's warps with 32, some and no rows, and feed-forwards of an odd (7, one k block per stage) and an even number of k blocks
+  (two per stage on narrow tiles): bit for bit what the same rows are among 768."""
+  layers = [gugidra.parallel_layer(4, 2, 64, 2, 32, 64, mlp=gugidra.dense_ff(ff)), gugidra.gla_layer(4, 32, 64, mlp=gugidra.dense_ff(ff))]
+  model = gugidra.model_dict(256, 384, layers)
+  toks = np.random.Generator(np.random.PCG64(4)).integers(0, model["vocab"], size=768).tolist()
+  out = []
+  for n in (rows, 768):
+    cfg = pyconfig.from_model_dict(model, dtype="bfloat16", per_device_batch_size=2, max_target_length=800, pagedattn_tokens_per_page=16,
+                                   pagedattn_num_pages=60, max_step_rows=768)
+    engine = maxengine.MaxEngine(cfg)
+    engine.load_params(gugidra.random_tensors(cfg, seed=3))
+    engine.init_decode_state()
+    out.append(engine.step([(0, toks[:n], list(range(rows)))]).clone())
+  assert torch.isfinite(out[0]).all() and torch.equal(out[0], out[1])
+
+
 def test_unequal_experts_against_float32():
   """Experts of 0, 1, 255, 256 and 257 rows on the grouped pair GEMM, and slots of an identity expert behind the last range: the token says which
   expert its row takes."""
