@@ -975,6 +975,50 @@ int launch_multi_decode(mtx_layered* e, SoftmaxAttnArgs<bf16>& sa, const MultiDe
   return MTX_OK;
 }
 
+// q, k and v of the step's rows: rotated, to q_out and the pages
+template <typename T>
+int launch_qk_prepare(const QkPrepareArgs<T>& qa, int rows, size_t smem, cudaStream_t st) {
+  if constexpr (sizeof(T) == 2)
+    if (QkRotatePlan::ok(qa)) {
+      const int dn = qa.q_norm ? qa.dim : 0;
+      return launch(dn == 0     ? qk_rotate_append_kernel<0, false>
+                    : dn == 64  ? qk_rotate_append_kernel<64, false>
+                    : dn == 128 ? qk_rotate_append_kernel<128, false>
+                                : qk_rotate_append_kernel<256, false>,
+                    dim3(rows), dim3(256), 0, st, qa);
+    }
+  return launch(qk_prepare_append_kernel<T>, dim3(rows), dim3(256), smem, st, qa);
+}
+template <typename T>
+int launch_rope_append(const RopeAppendArgs<T>& ra, int rows, cudaStream_t st) {
+  if constexpr (sizeof(T) == 2) {
+    QkPrepareArgs<T> qa;
+    memset(&qa, 0, sizeof(qa));
+    qa.proj = ra.proj;
+    qa.ld = ra.ld;
+    qa.q_col = ra.q_col;
+    qa.k_col = ra.k_col;
+    qa.v_col = ra.v_col < 0 ? ra.k_col : ra.v_col;
+    qa.rot_freq = ra.rot_freq;
+    qa.q_out = ra.q_out;
+    qa.k_pages = ra.k_pages;
+    qa.v_pages = ra.v_pages;
+    qa.group = ra.group;
+    qa.pos = ra.pos;
+    qa.page_map = ra.page_map;
+    qa.heads = ra.heads;
+    qa.kv_heads = ra.kv_heads;
+    qa.dim = ra.dim;
+    qa.vdim = ra.vdim;
+    qa.rot_dims = ra.rot_dims;
+    qa.num_pages = ra.num_pages;
+    qa.tokens_per_page = ra.tokens_per_page;
+    qa.max_pages = ra.max_pages;
+    if (QkRotatePlan::ok(qa)) return launch(qk_rotate_append_kernel<0, true>, dim3(rows), dim3(256), 0, st, qa);
+  }
+  return launch(rope_append_kernel<T>, dim3(rows), dim3(256), 0, st, ra);
+}
+
 // rows of a page that one copy of a key tile takes: a page or the largest part of it that cuts the tile evenly (8 rows: the swizzle's period)
 int paged_flash_box(int tokens_per_page, int key_tile) {
   int box = key_tile;
@@ -1180,7 +1224,7 @@ int composite_layer(mtx_layered* e, int li, const mtx_ragged_batch& b, cudaStrea
     ra.num_pages = c.num_pages;
     ra.tokens_per_page = c.tokens_per_page;
     ra.max_pages = c.max_pages_per_group;
-    MTX_TRY(launch(rope_append_kernel<T>, dim3(rows), dim3(256), 0, st, ra));
+    MTX_TRY(launch_rope_append(ra, rows, st));
     SoftmaxAttnArgs<T> sa;
     memset(&sa, 0, sizeof(sa));
     sa.q = static_cast<const T*>(e->q);
@@ -1527,7 +1571,7 @@ int parallel_layer(mtx_layered* e, int li, const mtx_ragged_batch& b, cudaStream
     qa.tokens_per_page = c.tokens_per_page;
     qa.max_pages = c.max_pages_per_group;
     qa.eps = c.eps;
-    MTX_TRY(launch(qk_prepare_append_kernel<T>, dim3(rows), dim3(256), 0, st, qa));
+    MTX_TRY(launch_qk_prepare(qa, rows, 0, st));
     sa.q = static_cast<const T*>(e->q);
     sa.out = cat;
     sa.ld_out = k_cat;
@@ -1749,7 +1793,7 @@ int prenorm_layer(mtx_layered* e, int li, const mtx_ragged_batch& b, cudaStream_
     qa.talk = a.talk;
     const size_t qsmem = a.talk ? sizeof(float) * a.heads * a.dim : 0;
     if (qsmem > 48 * 1024) MTX_CUDA(cudaFuncSetAttribute(qk_prepare_append_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(qsmem)));
-    MTX_TRY(launch(qk_prepare_append_kernel<T>, dim3(rows), dim3(256), qsmem, st, qa));
+    MTX_TRY(launch_qk_prepare(qa, rows, qsmem, st));
     if (a.pool > 0 && !a.pool_shared) {  // the blocks that this step's rows complete
       PoolAppendArgs<T> pa;
       memset(&pa, 0, sizeof(pa));
@@ -2041,7 +2085,7 @@ int outlayer_layer(mtx_layered* e, int li, const mtx_ragged_batch& b, cudaStream
     qa.tokens_per_page = c.tokens_per_page;
     qa.max_pages = c.max_pages_per_group;
     qa.eps = c.eps;
-    MTX_TRY(launch(qk_prepare_append_kernel<T>, dim3(rows), dim3(256), 0, st, qa));
+    MTX_TRY(launch_qk_prepare(qa, rows, 0, st));
     SoftmaxAttnArgs<T> sa = attention_args<T>(c, b);
     sa.q = static_cast<const T*>(e->q);
     sa.out = mix;

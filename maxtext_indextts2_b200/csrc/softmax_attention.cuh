@@ -39,6 +39,7 @@
 //
 //   rope_append_kernel         per row: bias already in the projection; rotates q and k, writes q, appends k and v to the pages
 //   qk_prepare_append_kernel   the same with the optional head norms, either pairing, and layers that append nothing
+//   qk_rotate_append_kernel    both for bf16 heads without norms, eight channels per thread
 //   pool_append_kernel         per row that completes a block: the means of the block's cached keys and values into the pooled pools
 //   softmax_attention_rows_kernel<T>   one CTA per (query tile of <= 16 rows of one sequence, query head); keys walked in tiles
 //                              staged as fp32 in shared memory; running maximum and sum per row; everything fp32 (T is only the
@@ -232,6 +233,122 @@ __global__ void __launch_bounds__(256) qk_prepare_append_kernel(const QkPrepareA
   for (int e = tid; e < a.kv_heads * dv; e += blockDim.x) {
     const int kv = e / dv, c = e % dv;
     a.v_pages[(size_t(kv) * a.num_pages * a.tokens_per_page + slot) * dv + c] = to_act<T>(row[a.v_col + e]);
+  }
+}
+
+// The same in bf16 for heads whose channels come in eights: a thread takes eight channels of one head (or eight values), a CTA a row, 512 such pieces at a time, all of
+// them requested before the row's angles are worked out.  The angles go by the position alone and are the row's, not its heads'.  Sums of squares are added up in
+// the order of qk_prepare_append_kernel, so that the bits are its own.
+// DN > 0: heads of DN = 64, 128 or 256 channels are brought to unit RMS first.  ROPE: the sums of a turned pair as rope_append_kernel has them (the other product is
+// rounded first).
+// Bound: the way of a row from its position over its page to its stores, so what counts is rows in flight: with a warp walking the heads one after the other, a channel per
+// lane, and the angles in every head, 1777 rows of 16 + 8 normed heads of 64 took 23.3 us, 4096 rows of 16 + 4 turned heads of 128 31.6; so 8.9 and 14.3 (their bytes: 3.4 and 11.6).
+struct QkRotatePlan {
+  static bool ok(const QkPrepareArgs<bf16>& a) {
+    const auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+    const bool norms = a.q_norm || a.k_norm;
+    return !a.temp && !a.talk && !a.rot_half && !a.norm_whole && a.maps <= 1 && a.dim % 8 == 0 && a.dim <= 256 && a.vdim % 8 == 0 && a.rot_dims % 8 == 0 && a.rot_dims <= a.dim &&
+           (!norms || (a.q_norm && a.k_norm && (a.dim == 64 || a.dim == 128 || a.dim == 256) && aligned(a.q_norm) && aligned(a.k_norm))) && a.ld % 4 == 0 && a.q_col % 4 == 0 &&
+           a.k_col % 4 == 0 && a.v_col % 4 == 0 && aligned(a.proj) && aligned(a.q_out) && aligned(a.k_pages) && aligned(a.v_pages);
+  }
+};
+
+template <int DN, bool ROPE>
+__global__ void __launch_bounds__(256) qk_rotate_append_kernel(const QkPrepareArgs<bf16> a) {
+  constexpr int kPieces = 2;
+  __shared__ float2 turns[128];  // (cosine, sine) of the row's pairs
+  __shared__ __align__(16) float channels[DN > 0 ? 8 : 1][DN > 0 ? 256 : 1];  // a warp's pieces: 256 / DN heads
+  griddep_launch_dependents();
+  const int r = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rh = a.rot_dims / 2;
+  const double freq = tid < rh ? a.rot_freq[tid] : 0.0;
+  const int per = a.dim / 8, nq = a.heads * per, nk = a.shared_kv ? 0 : a.kv_heads * per, nv = a.shared_kv ? 0 : a.kv_heads * a.vdim / 8, n = nq + nk + nv;
+  griddep_wait();
+  const float* row = a.proj + size_t(r) * a.ld;
+  const int p = a.pos[r], grp = a.group[r];
+  const size_t slot = size_t(a.page_map[size_t(grp) * a.max_pages + p / a.tokens_per_page]) * a.tokens_per_page + p % a.tokens_per_page;
+  const size_t pool_rows = size_t(a.num_pages) * a.tokens_per_page;
+  for (int e0 = tid; e0 - tid < n; e0 += kPieces * 256) {
+    float x[kPieces][8];
+#pragma unroll
+    for (int i = 0; i < kPieces; ++i) {
+      const int e = e0 + i * 256;
+      if (e < n) {
+        const float* src = row + (e < nq ? a.q_col + e * 8 : e < nq + nk ? a.k_col + (e - nq) * 8 : a.v_col + (e - nq - nk) * 8);
+        const float4 lo = *reinterpret_cast<const float4*>(src), hi = *reinterpret_cast<const float4*>(src + 4);
+        x[i][0] = lo.x, x[i][1] = lo.y, x[i][2] = lo.z, x[i][3] = lo.w, x[i][4] = hi.x, x[i][5] = hi.y, x[i][6] = hi.z, x[i][7] = hi.w;
+      } else {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) x[i][q] = 0.0f;
+      }
+    }
+    if (e0 == tid) {
+      if (tid < rh) {
+        float sn, cs;
+        rot_sincos(double(p), freq, &sn, &cs);
+        turns[tid] = make_float2(cs, sn);
+      }
+      __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < kPieces; ++i) {
+      const int e = e0 + i * 256, u = e < nq ? e : e - nq, c = u % per * 8;  // c: the piece's first channel of its head
+      if (DN > 0 && e - lane < nq + nk) {  // (uniform in the warp; a head's pieces are neighbours in one)
+        constexpr int HW = DN > 0 ? 256 / DN : 1;
+        float* ch = channels[DN > 0 ? warp : 0];
+        *reinterpret_cast<float4*>(ch + lane * 8) = make_float4(x[i][0], x[i][1], x[i][2], x[i][3]);
+        *reinterpret_cast<float4*>(ch + lane * 8 + 4) = make_float4(x[i][4], x[i][5], x[i][6], x[i][7]);
+        __syncwarp();
+        float s[HW];  // lane c: the squares of the channels c, c + 32, .. of each head, then the warp's tree, in which a half keeps half of the heads
+#pragma unroll
+        for (int h = 0; h < HW; ++h) {
+          s[h] = 0.0f;
+#pragma unroll
+          for (int k = 0; k < DN / 32; ++k) {
+            const float y = ch[h * DN + 32 * k + lane];
+            s[h] = fmaf(y, y, s[h]);
+          }
+        }
+        __syncwarp();
+        int o = 16;
+#pragma unroll
+        for (int left = HW; left > 1; left >>= 1, o >>= 1)
+#pragma unroll
+          for (int h = 0; h < left / 2; ++h) {
+            const bool up = (lane & o) != 0;
+            const float keep = up ? s[h + left / 2] : s[h], send = up ? s[h] : s[h + left / 2];
+            s[h] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+          }
+        for (; o > 0; o >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], o);  // (of the head that this lane's piece belongs to)
+        const float inv = 1.0f / sqrtf(s[0] / float(a.dim) + a.eps);
+        if (e < nq + nk) {
+          const float* w = (e < nq ? a.q_norm : a.k_norm) + c;
+          const float4 lo = *reinterpret_cast<const float4*>(w), hi = *reinterpret_cast<const float4*>(w + 4);
+          const float ww[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+          for (int q = 0; q < 8; ++q) x[i][q] = x[i][q] * inv * ww[q];
+        }
+      }
+      if (e >= n) continue;
+      if (e < nq + nk && c < 2 * rh) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float2 t = turns[c / 2 + q];
+          const float x0 = x[i][2 * q], x1 = x[i][2 * q + 1];
+          x[i][2 * q] = fmaf(x0, t.x, -__fmul_rn(x1, t.y));
+          x[i][2 * q + 1] = ROPE ? fmaf(x1, t.x, __fmul_rn(x0, t.y)) : fmaf(x0, t.y, __fmul_rn(x1, t.x));
+        }
+      }
+      bf16* dst;
+      if (e < nq) {
+        dst = a.q_out + size_t(r) * a.heads * a.dim + size_t(e) * 8;
+      } else if (e < nq + nk) {
+        dst = a.k_pages + (size_t(u / per) * pool_rows + slot) * a.dim + c;
+      } else {
+        const int v = (e - nq - nk) * 8;
+        dst = a.v_pages + (size_t(v / a.vdim) * pool_rows + slot) * a.vdim + v % a.vdim;
+      }
+      *reinterpret_cast<uint4*>(dst) = make_uint4(pack_bf16x2(x[i][0], x[i][1]), pack_bf16x2(x[i][2], x[i][3]), pack_bf16x2(x[i][4], x[i][5]), pack_bf16x2(x[i][6], x[i][7]));
+    }
   }
 }
 

@@ -51,3 +51,37 @@ def test_output_of_a_recurrence(vdim, dtype):
   model = gugidra.model_dict(64, 61, [gugidra.gla_layer(9, 8, vdim)], eps=1e-5, embed_scale=1.7)  # (nine heads: one more than warps)
   t = gugidra_ref.random_model(model, seed=vdim)
   assert error(dtype, logits(model, t, dtype), gugidra_ref.logits_of(model, t, TOKENS)) < TOL[dtype]
+
+
+@pytest.mark.parametrize("heads,kv,dim,rot", [(4, 2, 64, 32), (2, 1, 16, 16), (8, 4, 256, 256), (16, 4, 128, 0), (16, 16, 64, 64), (3, 1, 96, 48), (4, 2, 64, 12), (2, 2, 48, 24)])
+@pytest.mark.parametrize("rows", [1, 300])
+def test_rotated_keys_and_values(heads, kv, dim, rot, rows):
+  """Keys (of unit RMS, then rotated) and values of a first layer, appended behind 37 tokens: heads of 64, 128 and 256 channels eight channels per thread, in one
+  and in several rounds of the CTA, the others, and where fewer channels turn than that, channel by channel."""
+  part = zakelorn.attention_part(heads, kv, dim, rot_dims=rot)
+  model = zakelorn.model_dict(256, 320, [zakelorn.parallel_layer(part, zakelorn.lightning_part(2, 64), mlp=zakelorn.dense_ff(256))])
+  cfg = pyconfig.from_model_dict(model, dtype="bfloat16", per_device_batch_size=2, max_target_length=400, pagedattn_tokens_per_page=24, pagedattn_num_pages=40, max_step_rows=400)
+  tensors = zakelorn.random_tensors(cfg, seed=3)
+  engine = maxengine.MaxEngine(cfg)
+  engine.load_params(tensors)
+  state = engine.init_decode_state()
+  toks = np.random.Generator(np.random.PCG64(5)).integers(0, 320, size=37 + rows).tolist()
+  engine.step([(1, toks[:37], [])])
+  engine.step([(1, toks[37:], [])])
+  pages = torch.as_tensor(engine.page_state.page_map[1], device="cuda").long()
+  f64 = lambda t: t.to("cuda", torch.float64)
+  x = f64(tensors["embed"].cuda()[toks])
+  pos = torch.arange(37 + rows, device="cuda", dtype=torch.float64)
+  for name, pool in (("k", "key_pages"), ("v", "value_pages")):
+    got = f64(state["cache"][pool][0][:, pages].flatten(1, 2)[:, : 37 + rows]).permute(1, 0, 2)
+    want = (x @ f64(tensors["l0.mix.left." + name]).T).reshape(37 + rows, kv, dim)
+    if name == "k":
+      want = want / torch.sqrt(want.square().mean(-1, keepdim=True) + cfg.normalization_layer_epsilon)
+    if name == "k" and rot:
+      ang = pos[:, None] * 10000.0 ** (-torch.arange(0, rot, 2, device="cuda", dtype=torch.float64) / rot)[None]
+      a, b = want[..., 0:rot:2].clone(), want[..., 1:rot:2].clone()
+      co, si = torch.cos(ang)[:, None], torch.sin(ang)[:, None]
+      want[..., 0:rot:2], want[..., 1:rot:2] = a * co - b * si, b * co + a * si
+    # the projection rounded to bf16 and its rotation again: at most 2^-8 (bf16's unit roundoff) of each value or turned pair, twice
+    off = (got - want).square().sum((1, 2)).sqrt() / want.square().sum((1, 2)).sqrt()
+    assert float(off.max()) < 2.0**-7
