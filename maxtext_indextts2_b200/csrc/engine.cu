@@ -53,7 +53,7 @@ struct mtx_engine {
   mtx_model_config cfg;
   int num_sms = 148;
   int max_r_tile = 16;
-  int pf_rows = 0;  // rows that one pass over a long prompt takes (0: prompts fit the steps)
+  int pf_rows = 0;  // rows that one pass over a long prompt takes (0: prompts fit the 256-row steps)
   int qkv_n = 0;
   int attn_max_chunks = 0;
   bool bound = false;
@@ -137,10 +137,6 @@ bool staged_prefill(const mtx_model_config& c) { return c.kv_quant != 0 || is_pa
 // A long prompt's rows go through the layers together, at most kPfMaxRows of them (a 4096-row pass of a 10240-wide feed-forward holds 84 MB of
 // activations and leaves no wave of the GEMMs short; longer prompts take several passes).
 constexpr int kPfMaxRows = 4096;
-// ... in steps up to so many rows, in passes above: the pair GEMM's half-empty row tiles and tcgen05's attention take less than the 64- and 256-row kernels, which cut K over
-// clusters (24 layers of width 1280 and the logits, us: 33 rows 1553 in a step, 1516 in a pass; 65: 1408, 1303; 129: 1544, 1334; 256: 1677, 1352), the 32-row kernels less again (20 rows:
-// 1294, 1402).  The gemma3 block's passes repeat its steps: from the largest step on.
-int pass_over(const mtx_model_config& c) { return c.decoder_block == 1 ? 256 : 32; }
 // most slices of a row that the residual epilogues of such a pass leave sums of squares of: two per tile of at least 64 columns
 size_t pf_slices(int emb_dim) { return 2 * size_t((emb_dim + 63) / 64); }
 
@@ -759,7 +755,7 @@ int enqueue_last_logits(mtx_engine* e, const bf16* x, int draw_row, int32_t* fir
   return launch(finalize_kernel, dim3(1), dim3(kFinalizeThreads), 0, st, fa);
 }
 
-// The layers over `rows` (more than pass_over, at most pf_rows) prompt positions from start_pos on, all rows in every launch: the projections
+// The layers over `rows` (more than 256, at most pf_rows) prompt positions from start_pos on, all rows in every launch: the projections
 // on the pair GEMM (gemm_wide.cuh), RMSNorm fused into them as in the 65..256-row steps when its scales are folded.  e->x holds the
 // result.
 // The gemma3 block's passes (pass_rows) repeat the bits of its 256-row steps: the GEMMs add up K in the steps' segments, the attention
@@ -904,7 +900,7 @@ int enqueue_prefill_pass(mtx_engine* e, int rows, const int32_t* tokens, int sta
   return MTX_OK;
 }
 
-// Rows of the next pass of a prompt with `left` rows to go; pass_over or fewer: a step takes them.  A gemma3 pass has the bits of the
+// Rows of the next pass of a prompt with `left` rows to go; 256 or fewer: a step of the 256-row kernels takes them.  A gemma3 pass has the bits of the
 // steps, so the rows behind its last 256 come along only where their own step would cut K and the keys as the 256-row steps do: the plans
 // know rows rounded up to a power of two, so from 129 on.  (3001 positions through six layers, this step alone: 5.90 ms with the last 185 as a step
 // of their own, 5.18 in the pass.)
@@ -1488,9 +1484,9 @@ int mtx_engine_create(const mtx_model_config* cfg, mtx_engine** out) {
   e->max_r_tile = round_rows(c.max_rows);
   if (c.kv_quant && e->max_r_tile < 128) e->max_r_tile = 128;  // every step of an int8 engine runs the 128-row-block GEMM
   if (c.decoder_block == 1 && e->max_r_tile < 128) e->max_r_tile = 128;  // and so does every step of the gemma3 block
-  if (c.max_prefill_len > pass_over(c)) {
+  if (c.max_prefill_len > 256) {
     const int rows = (c.max_prefill_len + 255) / 256 * 256, most = c.max_prefill_rows > 0 && c.max_prefill_rows < kPfMaxRows ? c.max_prefill_rows : kPfMaxRows;
-    e->pf_rows = most < 256 ? 0 : (rows < most ? rows : most);
+    e->pf_rows = most <= 256 ? 0 : (rows < most ? rows : most);
   }
   e->qkv_n = (c.num_q_heads + 2 * c.num_kv_heads) * c.head_dim;
   e->attn_max_chunks = attn_max_chunks(c.max_prefill_len, c.max_target_len);
@@ -2036,7 +2032,7 @@ int mtx_prefill_rows(mtx_engine* e, const int32_t* tokens, int count, int start_
     const int left = count - at, most = e->cfg.max_prefill_rows, small = most > 0 && most < e->cfg.max_rows ? most : e->cfg.max_rows;
     int n;
     const int take = pass_rows(e, left);
-    if (take > pass_over(e->cfg) && (e->cfg.head_dim != 256 || takes_prompt_wide(e, 256))) {
+    if (take > 256 && (e->cfg.head_dim != 256 || takes_prompt_wide(e, 256))) {
       n = take;
       MTX_TRY(enqueue_prefill_pass(e, n, tokens + at, start_pos + at, slot, st));
     } else {
