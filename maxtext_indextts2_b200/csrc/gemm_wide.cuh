@@ -332,12 +332,14 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       uint32_t phase = 0, acc_phase = 1;
       auto tiles_of = [&](auto group) {  // (the k blocks of a stage in straight code: the issue of four MMAs costs as much as they take up to 128 columns)
         constexpr int G = decltype(group)::value;
-        for (int j = 0, seg = 0; j < my_tiles * segments; ++j) {  // (tile, segment)
+        const int whole = nkb / segments, over = nkb % segments;  // segment s ends at (s + 1) nkb / segments: counted, no division in the loop
+        for (int j = 0, seg = 0, rest = 0; j < my_tiles * segments; ++j) {  // (tile, segment)
           mbar_wait(&tail->tmem_empty[buf], acc_phase);
           tcgen05_fence_after();
           const uint32_t acc = tmem_base + uint32_t(buf * p.bn);
-          const int n_seg = (seg + 1) * nkb / segments - seg * nkb / segments;
-          if (++seg == segments) seg = 0;
+          int n_seg = whole;
+          if ((rest += over) >= segments) rest -= segments, ++n_seg;
+          if (++seg == segments) seg = rest = 0;
           for (int i = 0; i < n_seg; ++i) {
             mbar_wait(&tail->full[s], phase);
             tcgen05_fence_after();
@@ -391,6 +393,8 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       auto pre = epi.prepare(w, stage);
       if constexpr (MODE == kWideParts) {
         float acc[kPairMaxCols / 32][16];
+#pragma unroll
+        for (int x = 0; x < kPairMaxCols / 2; ++x) acc[x >> 4][x & 15] = -0.0f;  // (-0 + y is y, its sign of zero too; a choice between y and the sum cost 3 us of 13 over eight parts)
         for (int seg = 0; seg < segments; ++seg) {
           const uint32_t taddr = lanes + uint32_t(buf * p.bn + w.c0);
           mbar_wait(&tail->tmem_full[buf], acc_phase);
@@ -403,10 +407,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
               tmem_ld_x16_issue(taddr + uint32_t(16 * i + 16), v[1]);
               tmem_ld_wait();
 #pragma unroll
-              for (int x = 0; x < 32; ++x) {
-                const float y = __uint_as_float(v[x >> 4][x & 15]);
-                acc[i + (x >> 4)][x & 15] = seg == 0 ? y : acc[i + (x >> 4)][x & 15] + y;
-              }
+              for (int x = 0; x < 32; ++x) acc[i + (x >> 4)][x & 15] += __uint_as_float(v[x >> 4][x & 15]);
             }
           release();
         }
