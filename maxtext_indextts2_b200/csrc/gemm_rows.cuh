@@ -93,11 +93,18 @@ __device__ __forceinline__ void rows_epi_store(const EpiArgs& e, int N, int r, i
 
 // out[r, n] = bf16(resid[r, n] + bf16(acc))      (llama2.py:139-165 residual adds on bf16 arrays)
 // Returns the sum of squares of the 16 stored (bf16) values: the next RMSNorm's statistic.
-__device__ __forceinline__ float rows_epi_residual(const EpiArgs& e, int N, int r, int n0, const float (&v)[16]) {
+__device__ __forceinline__ bool rows_residual_whole(const EpiArgs& e, int N, int n0) { return n0 + 16 <= N && (e.ld_out & 7) == 0; }
+__device__ __forceinline__ void rows_residual_load(const EpiArgs& e, int r, int n0, uint4 (&v)[2]) {
+  const uint4* p = reinterpret_cast<const uint4*>(e.resid + (long long)r * e.ld_out + n0);
+  v[0] = p[0];
+  v[1] = p[1];
+}
+// (have: the 16 of resid, where rows_residual_whole)
+__device__ __forceinline__ float rows_epi_residual(const EpiArgs& e, int N, int r, int n0, const float (&v)[16], const uint4 (&have)[2]) {
   const long long o = (long long)r * e.ld_out + n0;
   float sq = 0.0f;
-  if (n0 + 16 <= N && (e.ld_out & 7) == 0) {
-    const uint4 ra = reinterpret_cast<const uint4*>(e.resid + o)[0], rb = reinterpret_cast<const uint4*>(e.resid + o)[1];
+  if (rows_residual_whole(e, N, n0)) {
+    const uint4 ra = have[0], rb = have[1];
     const uint32_t rw[8] = {ra.x, ra.y, ra.z, ra.w, rb.x, rb.y, rb.z, rb.w};
     float s[16];
 #pragma unroll
@@ -124,10 +131,17 @@ __device__ __forceinline__ float rows_epi_residual(const EpiArgs& e, int N, int 
   return sq;
 }
 
+__device__ __forceinline__ float rows_epi_residual(const EpiArgs& e, int N, int r, int n0, const float (&v)[16]) {
+  uint4 have[2];
+  if (rows_residual_whole(e, N, n0)) rows_residual_load(e, r, n0, have);
+  return rows_epi_residual(e, N, r, n0, v, have);
+}
+
 // rstd of row r from the per-tile partial sums of squares a residual epilogue left (normalizations.py:57-69).
 __device__ __forceinline__ float rows_rstd(const EpiArgs& e, int r) {
   if (e.ss_in == nullptr) return 1.0f;
   float tot = 0.0f;
+#pragma unroll 8
   for (int t = 0; t < e.ss_tiles; ++t) tot += __ldcg(e.ss_in + t * e.ss_pitch + r);
   return 1.0f / sqrtf(tot / float(e.ss_dim) + e.ss_eps);
 }
@@ -161,7 +175,22 @@ __device__ __forceinline__ void rows_epi_swiglu(const EpiArgs& e, int N2, int r,
 
 // embeddings.py:304-315 + kvcache.py:626-718: `lo` = features d0 .. d0+15 of a head's first half, `hi` = the same
 // dims of its second half (d0 + D/2).  Query / key heads are rotated, value heads stored as they are.
-__device__ __forceinline__ void rows_epi_qkv(const EpiArgs& e, int N, int r, int head, int d0, const float (&lo)[16], const float (&hi)[16]) {
+struct RowsQkvIn {  // what the fragment reads of the step besides the accumulator
+  float4 cs[8];     // cosines and sines of the dims d0 .. d0 + 15
+  int wr, plane;    // the row's cache row and plane
+};
+__device__ __forceinline__ void rows_qkv_load(const EpiArgs& e, int r, int head, int d0, RowsQkvIn& in) {
+  if (head < e.hq + e.hkv) {
+    const float4* cs = reinterpret_cast<const float4*>(e.rope_cs + (long long)r * (e.d >> 1) + d0);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) in.cs[j] = cs[j];
+  }
+  if (head >= e.hq) {
+    in.wr = e.write_row[r];
+    in.plane = e.plane[r];
+  }
+}
+__device__ __forceinline__ void rows_epi_qkv(const EpiArgs& e, int N, int r, int head, int d0, const float (&lo)[16], const float (&hi)[16], const RowsQkvIn& in) {
   const int D = e.d, half = D >> 1;
   if (head * D >= N) return;
   const bool is_q = head < e.hq, is_k = !is_q && head < e.hq + e.hkv;
@@ -173,10 +202,9 @@ __device__ __forceinline__ void rows_epi_qkv(const EpiArgs& e, int N, int r, int
     b[j] = bf16_lo(pb); b[j + 1] = bf16_hi(pb);
   }
   if (is_q || is_k) {
-    const float2* cs = e.rope_cs + (long long)r * half + d0;
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
-      const float2 c = cs[j];
+      const float2 c = j & 1 ? make_float2(in.cs[j >> 1].z, in.cs[j >> 1].w) : make_float2(in.cs[j >> 1].x, in.cs[j >> 1].y);
       // first half: a cos - b sin ; second half: b cos + a sin, every product rounded to bf16 (bf16 arrays in the reference)
       const float ac = bf16r(a[j] * c.x), bs = bf16r(b[j] * c.y), bc = bf16r(b[j] * c.x), as = bf16r(a[j] * c.y);
       a[j] = ac - bs;
@@ -188,13 +216,19 @@ __device__ __forceinline__ void rows_epi_qkv(const EpiArgs& e, int N, int r, int
     frag_store_bf16(dst, a);
     frag_store_bf16(dst + half, b);
   } else {
-    const int wr = e.write_row[r];
-    if (wr < 0) return;
+    if (in.wr < 0) return;
     const int kvh = is_k ? head - e.hq : head - e.hq - e.hkv;
-    bf16* dst = (is_k ? e.k_cache : e.v_cache) + (((long long)e.plane[r] * e.hkv + kvh) * e.t_alloc + wr) * D + d0;
+    bf16* dst = (is_k ? e.k_cache : e.v_cache) + (((long long)in.plane * e.hkv + kvh) * e.t_alloc + in.wr) * D + d0;
     frag_store_bf16(dst, a);
     frag_store_bf16(dst + half, b);
   }
+}
+
+__device__ __forceinline__ void rows_epi_qkv(const EpiArgs& e, int N, int r, int head, int d0, const float (&lo)[16], const float (&hi)[16]) {
+  if (head * e.d >= N) return;
+  RowsQkvIn in;
+  rows_qkv_load(e, r, head, d0, in);
+  rows_epi_qkv(e, N, r, head, d0, lo, hi, in);
 }
 
 // One head (64 dims) of one row for the int8 cache: RoPE (key heads), then KVQuant.quantize over the head's dims.
@@ -245,6 +279,44 @@ __device__ __forceinline__ void rows_epi_qkv_q8(const EpiArgs& e, int N, int r, 
     *reinterpret_cast<uint4*>(dst + 16 * q) = make_uint4(w[0], w[1], w[2], w[3]);
   }
   (is_k ? e.k_scale : e.v_scale)[row] = mx;
+}
+
+// The same for an eighth of the head per thread (dims d0 .. d0 + 7 and d0 + 32 .. d0 + 39, d0 = 0, 8, 16, 24 in four neighbouring lanes, all of them here): the
+// split-K units have 32 rows or fewer to finish, and a thread per head left three quarters of the threads idle.
+__device__ __forceinline__ void rows_epi_qkv_q8_eighth(const EpiArgs& e, int N, int r, bool valid, int head, int d0, float (&lo)[8], float (&hi)[8], const RowsQkvIn& in) {
+  const bool is_q = head < e.hq, is_k = !is_q && head < e.hq + e.hkv;
+  valid = valid && head * 64 < N;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float a = bf16r(lo[j]), b = bf16r(hi[j]);
+    lo[j] = a;
+    hi[j] = b;
+    if (is_q || is_k) {
+      const float co = j & 1 ? in.cs[j >> 1].z : in.cs[j >> 1].x, si = j & 1 ? in.cs[j >> 1].w : in.cs[j >> 1].y;
+      lo[j] = bf16r(bf16r(a * co) - bf16r(b * si));
+      hi[j] = bf16r(bf16r(b * co) + bf16r(a * si));
+    }
+  }
+  if (valid && is_q) {
+    bf16* dst = e.q_out + (long long)r * (e.hq * 64) + head * 64 + d0;
+    *reinterpret_cast<uint4*>(dst) = make_uint4(pack_bf16x2(lo[0], lo[1]), pack_bf16x2(lo[2], lo[3]), pack_bf16x2(lo[4], lo[5]), pack_bf16x2(lo[6], lo[7]));
+    *reinterpret_cast<uint4*>(dst + 32) = make_uint4(pack_bf16x2(hi[0], hi[1]), pack_bf16x2(hi[2], hi[3]), pack_bf16x2(hi[4], hi[5]), pack_bf16x2(hi[6], hi[7]));
+  }
+  float mx = 0.0f;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) mx = fmaxf(mx, fmaxf(fabsf(lo[j]), fabsf(hi[j])));
+  mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+  mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+  if (!valid || is_q || in.wr < 0) return;
+  const bool fp8 = e.kv_fp8 != 0;
+  const float inv = mx > 0.0f ? kv_quant_max(fp8) / mx : 0.0f;
+  const int kvh = is_k ? head - e.hq : head - e.hq - e.hkv;
+  const long long row = ((long long)in.plane * e.hkv + kvh) * e.t_alloc + in.wr;
+  uint8_t* dst = (is_k ? e.kq_cache : e.vq_cache) + row * 64 + d0;
+  auto four = [&](const float* v) { return kv_quant_pair(v[0], v[1], inv, fp8) | (kv_quant_pair(v[2], v[3], inv, fp8) << 16); };
+  *reinterpret_cast<uint2*>(dst) = make_uint2(four(lo), four(lo + 4));
+  *reinterpret_cast<uint2*>(dst + 32) = make_uint2(four(hi), four(hi + 4));
+  if (d0 == 0) (is_k ? e.k_scale : e.v_scale)[row] = mx;
 }
 
 // Running sampling partials of one row over the columns of one weight tile (decoders.py:537-589 transform, then
@@ -353,6 +425,32 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   const uint32_t tmem_base = tail->tmem_base;
   if (trace && threadIdx.x == 0) trace[0] = clock64() - t_start;
 
+  // split-K: unit u of the rows that this CTA finishes is the 16 columns (u & 7) of row u >> 3 (an 8-bit cache: the quarter u & 3 of the two heads (u >> 2) & 1)
+  const int rpc = p.r_tile / p.splits, r_begin = int(blockIdx.y) * rpc;  // rows reduced and finished by this CTA, the first of them in the row block
+  const bool q8 = EPI == EPI_QKV_ROPE && e.kq_cache != nullptr;
+  float rs_in = 1.0f;
+  uint4 resid_in[2];
+  RowsQkvIn qkv_in;
+  auto fetch = [&](int u) {
+    const int row = row_base + r_begin + (u >> 3), n0 = first_tile * kTileN + (u & 7) * 16;
+    if (u >= rpc * 8 || row >= p.rows || first_tile >= n_tiles) return;
+    if (EPI == EPI_SWIGLU || EPI == EPI_QKV_ROPE || EPI == EPI_STORE_BF16) rs_in = rows_rstd(e, row);
+    if (EPI == EPI_RESIDUAL && n0 < p.n && rows_residual_whole(e, p.n, n0)) rows_residual_load(e, row, n0, resid_in);
+    if (EPI == EPI_QKV_ROPE && q8) {
+      const int head = first_tile * 2 + ((u >> 2) & 1);
+      const float4* cs = reinterpret_cast<const float4*>(e.rope_cs + (long long)row * 32 + (u & 3) * 8);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) qkv_in.cs[j] = cs[j];
+      if (head >= e.hq) {
+        qkv_in.wr = e.write_row[row];
+        qkv_in.plane = e.plane[row];
+      }
+    } else if (EPI == EPI_QKV_ROPE) {
+      const int d = n0 % e.d;
+      if (d < (e.d >> 1) && n0 < p.n) rows_qkv_load(e, row, n0 / e.d, d, qkv_in);
+    }
+  };
+
   const int F = my_tiles * nkb;  // ring fills of this CTA: fill f = (tile f / nkb, k-block kb0 + f % nkb)
 
   if (warp == 0) {
@@ -435,6 +533,13 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     if (EPI == EPI_LOGITS && e.gumbel) {
       step = e.rng_state[0];
       seed = (uint64_t(e.rng_state[2]) << 32) | e.rng_state[1];
+    }
+
+    // split-K: what this thread's part of the finished rows needs of the step, requested before the sums are there (behind the cluster's barrier and the
+    // reduction these loads stood one after the other at the kernel's end: 12 layers and the logits of 128 rows over an 8-bit cache 1042 us so, 1000 like this)
+    if (split) {
+      griddep_wait();
+      fetch(int(threadIdx.x) - 64);
     }
 
     // One tile of this thread's row, columns read through `ld16(col, dst)` (TMEM or the reduced slice in shared memory).
@@ -559,8 +664,6 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       float* partial = reinterpret_cast<float*>(smem);
       float* reduced = partial + p.r_tile * kRowsPitch;
       const int epi_tid = threadIdx.x - 64;
-      const int rpc = p.r_tile / p.splits;  // rows reduced and finished by this CTA
-      const int r_begin = int(blockIdx.y) * rpc;  // within the row block
       const uint32_t my = smem_u32(partial);
       // pull: one float4 column group of one row per thread and peer, all peers in flight; summed in split order
       for (int u = epi_tid; u < rpc * 32; u += kRowsEpiWarps * 32) {
@@ -579,25 +682,10 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       }
       asm volatile("bar.sync 1, 256;" ::: "memory");
       if (trace && threadIdx.x == 64) trace[7] = clock64() - t_start;
-      griddep_wait();
-      // epilogue: thread -> (row of the slice, 16-column chunk); RoPE / SwiGLU partners are read from the same row
+      // epilogue: thread -> unit; RoPE / SwiGLU partners are read from the same row
       const int tile = first_tile;
-      if (EPI == EPI_QKV_ROPE && e.kq_cache != nullptr) {  // int8 cache: thread -> (row of the slice, one of the tile's two heads)
-        for (int u = epi_tid; u < rpc * 2; u += kRowsEpiWarps * 32) {
-          const int rr = u >> 1, c0 = (u & 1) * 64;
-          const int row = row_base + r_begin + rr;
-          if (row >= p.rows) continue;
-          const float* src = reduced + rr * kRowsPitch + c0;
-          const float rs = rows_rstd(e, row);
-          float x[4][16];
-#pragma unroll
-          for (int q = 0; q < 4; ++q)
-#pragma unroll
-            for (int j = 0; j < 16; ++j) x[q][j] = src[16 * q + j] * rs;
-          rows_epi_qkv_q8(e, p.n, row, (tile * kTileN + c0) / 64, x[0], x[1], x[2], x[3]);
-        }
-      } else
       for (int u = epi_tid; u < rpc * 8; u += kRowsEpiWarps * 32) {
+        if (u != epi_tid) fetch(u);  // (the first is there: see above)
         const int rr = u >> 3, c0 = (u & 7) * 16;
         const int row = row_base + r_begin + rr;
         const float* src = reduced + rr * kRowsPitch;
@@ -609,7 +697,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
           }
         };
         const bool valid = row < p.rows;
-        const float rs = (valid && (EPI == EPI_SWIGLU || EPI == EPI_QKV_ROPE || EPI == EPI_STORE_BF16)) ? rows_rstd(e, row) : 1.0f;
+        const float rs = valid ? rs_in : 1.0f;
         if (EPI == EPI_SWIGLU) {
           if ((c0 & 16) == 0) {
             float g[16], uu[16];
@@ -619,6 +707,15 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
             rows_scale16(uu, rs);
             if (valid) rows_epi_swiglu(e, p.n, row, tile * kTileN + c0, g, uu);
           }
+        } else if (EPI == EPI_QKV_ROPE && q8) {
+          const int hd = (u >> 2) & 1, d0 = (u & 3) * 8;
+          float lo[8], hi[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            lo[j] = src[hd * 64 + d0 + j] * rs;
+            hi[j] = src[hd * 64 + 32 + d0 + j] * rs;
+          }
+          rows_epi_qkv_q8_eighth(e, p.n, row, valid, tile * 2 + hd, d0, lo, hi, qkv_in);
         } else if (EPI == EPI_QKV_ROPE) {
           const int D = e.d, half = D >> 1;
           const int d = (tile * kTileN + c0) % D;
@@ -628,7 +725,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
             ld16(c0 + half, hi);
             rows_scale16(lo, rs);
             rows_scale16(hi, rs);
-            if (valid) rows_epi_qkv(e, p.n, row, (tile * kTileN + c0) / D, d, lo, hi);
+            if (valid) rows_epi_qkv(e, p.n, row, (tile * kTileN + c0) / D, d, lo, hi, qkv_in);
           }
         } else if (EPI == EPI_STORE_BF16 || EPI == EPI_RESIDUAL) {
           float v[16];
@@ -639,7 +736,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
               rows_scale16(v, rs);
               rows_epi_store(e, p.n, row, tile * kTileN + c0, v);
             } else {
-              sq = rows_epi_residual(e, p.n, row, tile * kTileN + c0, v);
+              sq = rows_epi_residual(e, p.n, row, tile * kTileN + c0, v, resid_in);
             }
           }
           if (EPI == EPI_RESIDUAL && e.ss_out != nullptr) {
