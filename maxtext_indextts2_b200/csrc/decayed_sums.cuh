@@ -304,7 +304,9 @@ __device__ __forceinline__ uint32_t dc_movmatrix_trans(uint32_t a) {
   return d;
 }
 
-// grid (runs, heads, ceil(vdim / 16)), a warp per 16 channels
+// grid (runs, heads, ceil(vdim / (8 NT))), a warp per 16 channels.  NT: 8-column blocks of a CTA, two, or one where two leave SMs idle: the chunks are a serial chain, and a
+// warp that decays, splits and adds half of the values is through it sooner (one run of 1777 tokens, 16 heads of 64 x 64: 64 CTAs 20.4 us, 128 CTAs 15.9).
+template <int NT>
 __global__ void __launch_bounds__(512) decayed_states_kernel(const DecayedSplitArgs b) {
   extern __shared__ __align__(16) unsigned char dc_raw[];
   const DecayedChunksArgs& a = b.a;
@@ -314,7 +316,7 @@ __global__ void __launch_bounds__(512) decayed_states_kernel(const DecayedSplitA
   bf16* const stage0 = reinterpret_cast<bf16*>(dc_raw);
   float* const pw = reinterpret_cast<float*>(stage0 + kDsStages * stage_elems);  // c^0 .. c^64
   griddep_wait();
-  const int r0 = a.run_row0[blockIdx.x], nr = a.run_row0[blockIdx.x + 1] - r0, h = blockIdx.y, col0 = int(blockIdx.z) * kDcCols;
+  const int r0 = a.run_row0[blockIdx.x], nr = a.run_row0[blockIdx.x + 1] - r0, h = blockIdx.y, col0 = int(blockIdx.z) * (8 * NT);
   if (nr <= 0) return;
   int chunk0 = 0;  // the run's first chunk
   for (int r = 0; r < int(blockIdx.x); ++r) chunk0 += (a.run_row0[r + 1] - a.run_row0[r] + kDcTokens - 1) / kDcTokens;
@@ -338,8 +340,8 @@ __global__ void __launch_bounds__(512) decayed_states_kernel(const DecayedSplitA
         dc_cp_async_16(sk + (ki + i) * DP + kx, ok ? kp : src, ok);
         kp += 16 * a.ld;
       }
-      for (int e = tid; e < kDcTokens * 2; e += blockDim.x) {
-        const int i = e >> 1, x = (e & 1) * 8;
+      for (int e = tid; e < kDcTokens * NT; e += blockDim.x) {
+        const int i = e / NT, x = e % NT * 8;
         const bool ok = i < left && col0 + x < dv;
         dc_cp_async_16(sv + i * kDcVPitch + x, src + size_t(ok ? loaded * kDcTokens + i : 0) * a.ld + a.v_col + h * dv + (ok ? col0 + x : 0), ok);
       }
@@ -350,14 +352,14 @@ __global__ void __launch_bounds__(512) decayed_states_kernel(const DecayedSplitA
   // S[nt]: channels 16 m + g / + 8, columns col0 + 8 nt + 2 t / + 1
   float* const gs = a.state + (size_t(a.group[r0]) * H + h) * dv * d;
   const bool fresh = a.pos[r0] == 0;
-  float S[2][4];
+  float S[NT][4];
   auto state_at = [&](int nt, int e, int& ch, int& col) {
     ch = m * 16 + g + (e & 2) * 4;
     col = col0 + nt * 8 + 2 * t + (e & 1);
     return ch < d && col < dv;
   };
 #pragma unroll
-  for (int nt = 0; nt < 2; ++nt)
+  for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       int ch, col;
@@ -380,7 +382,7 @@ __global__ void __launch_bounds__(512) decayed_states_kernel(const DecayedSplitA
     {  // the state before the chunk, a column's channels side by side
       bf16* out = b.before + (size_t(chunk0 + c) * H + h) * 2 * dvp * dp + size_t(col0 + g) * dp + m * 16 + 2 * t;
 #pragma unroll
-      for (int nt = 0; nt < 2; ++nt)
+      for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
         for (int e = 0; e < 4; e += 2) {
           uint32_t hi, lo;
@@ -392,42 +394,51 @@ __global__ void __launch_bounds__(512) decayed_states_kernel(const DecayedSplitA
     }
     const float keep = pw[n];
 #pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
+    for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
       for (int e = 0; e < 4; ++e) S[nt][e] *= keep;
     // the values, each decayed to the end of the chunk (rows beyond the run: zero), as two bf16 parts: the rows 16 kt + 2 t, + 1 and those + 8
-    auto add = [&](int kt, const float (&w)[4]) {
-      uint32_t kf[4], vf[4], wh[4], wl[4];
-      mat_ldsm_x4_trans(kf, sk + (kt * 16 + (lane & 7) + (lane >> 4) * 8) * DP + m * 16 + ((lane >> 3) & 1) * 8);
-      mat_ldsm_x4_trans(vf, sv + (kt * 16 + (lane & 15)) * kDcVPitch + (lane >> 4) * 8);
+    // (NT 1: of two row tiles at once, the second's decays in w1)
+    auto add = [&](int kt, const float (&w)[4], const float (&w1)[4]) {
+      uint32_t vf[4], wh[4], wl[4];
+      mat_ldsm_x4_trans(vf, sv + (kt * 16 + (lane & 15) + (NT == 1 ? (lane >> 4) * 16 : 0)) * kDcVPitch + (NT == 1 ? 0 : (lane >> 4) * 8));
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&vf[j]));
-        dc_split(w[(j & 1) * 2] * v.x, w[(j & 1) * 2 + 1] * v.y, wh[j], wl[j]);
+        const float w0 = NT == 1 && j > 1 ? w1[(j & 1) * 2] : w[(j & 1) * 2], wx = NT == 1 && j > 1 ? w1[(j & 1) * 2 + 1] : w[(j & 1) * 2 + 1];
+        dc_split(w0 * v.x, wx * v.y, wh[j], wl[j]);
       }
-      mma_bf16_16816(S[0], kf, wh[0], wh[1]);
-      mma_bf16_16816(S[1], kf, wh[2], wh[3]);
-      mma_bf16_16816(S[0], kf, wl[0], wl[1]);
-      mma_bf16_16816(S[1], kf, wl[2], wl[3]);
+#pragma unroll
+      for (int k = 0; k < (NT == 1 ? 2 : 1); ++k) {
+        uint32_t kf[4];
+        mat_ldsm_x4_trans(kf, sk + ((kt + k) * 16 + (lane & 7) + (lane >> 4) * 8) * DP + m * 16 + ((lane >> 3) & 1) * 8);
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) mma_bf16_16816(S[nt], kf, wh[2 * (nt + k)], wh[2 * (nt + k) + 1]);
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) mma_bf16_16816(S[nt], kf, wl[2 * (nt + k)], wl[2 * (nt + k) + 1]);
+      }
     };
+    constexpr int kStep = NT == 1 ? 2 : 1;
     if (n == kDcTokens) {
 #pragma unroll
-      for (int kt = 0; kt < kDcTokens / 16; ++kt) add(kt, whole[kt]);
+      for (int kt = 0; kt < kDcTokens / 16; kt += kStep) add(kt, whole[kt], whole[kt + kStep - 1]);
     } else {
 #pragma unroll 1
-      for (int kt = 0; kt < (n + 15) >> 4; ++kt) {
-        float w[4];
+      for (int kt = 0; kt < (n + 15) >> 4; kt += kStep) {
+        float w[2][4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int i = kt * 16 + 2 * t + (j & 1) + (j >> 1) * 8;
-          w[j] = i < n ? pw[n - 1 - i] : 0.0f;
-        }
-        add(kt, w);
+        for (int k = 0; k < kStep; ++k)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int i = (kt + k) * 16 + 2 * t + (j & 1) + (j >> 1) * 8;
+            w[k][j] = i < n ? pw[n - 1 - i] : 0.0f;
+          }
+        add(kt, w[0], w[kStep - 1]);
       }
     }
   }
 #pragma unroll
-  for (int nt = 0; nt < 2; ++nt)
+  for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       int ch, col;

@@ -2027,14 +2027,16 @@ int launch_decayed_split(mtx_layered* e, const DecayedChunksArgs& da, const mtx_
   const size_t s1 = decayed_states_smem_bytes(da.dim), s2 = decayed_outputs_smem_bytes(da.dim, da.vdim);
   static size_t have1 = 48 * 1024, have2 = 48 * 1024;
   if (s1 > have1) {
-    MTX_CUDA(cudaFuncSetAttribute(decayed_states_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(s1)));
+    MTX_CUDA(cudaFuncSetAttribute(decayed_states_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(s1)));
+    MTX_CUDA(cudaFuncSetAttribute(decayed_states_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(s1)));
     have1 = s1;
   }
   if (s2 > have2) {
     MTX_CUDA(cudaFuncSetAttribute(decayed_outputs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(s2)));
     have2 = s2;
   }
-  MTX_TRY(launch(decayed_states_kernel, dim3(b.n_runs, da.heads, (da.vdim + kDcCols - 1) / kDcCols), dim3(32 * (mat_pad16(da.dim) / 16)), s1, st, sa));
+  const int columns = mat_pad16(da.vdim), nt = b.n_runs * da.heads * columns / 16 < e->num_sms ? 1 : 2;  // (8-column blocks per CTA: one where two leave SMs idle)
+  MTX_TRY(launch(nt == 1 ? decayed_states_kernel<1> : decayed_states_kernel<2>, dim3(b.n_runs, da.heads, columns / (8 * nt)), dim3(32 * (mat_pad16(da.dim) / 16)), s1, st, sa));
   return launch(decayed_outputs_kernel, dim3(b.rows / kDcTokens + b.n_runs, da.heads), dim3(128), s2, st, sa);
 }
 

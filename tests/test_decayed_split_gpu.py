@@ -29,3 +29,8 @@ def test_split_repeats_the_walk_of_chunks(heads, dim, vdim, n):
     logits = [engine.step([(0, toks, list(range(n)))] + beside).clone() for toks in (first, second)]
     got.append(logits + [t[0].clone() for t in state["cache"]["recurrent_state"]])
   assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
+def test_split_of_many_heads():
+  """Heads enough for 16 value columns per CTA."""
+  test_split_repeats_the_walk_of_chunks(40, 16, 64, 300)
