@@ -57,6 +57,55 @@ __device__ __forceinline__ float tanh_f32(float x) {
   return 1.0f - __fdividef(2.0f, __expf(2.0f * x) + 1.0f);
 }
 
+// s[i] = Q_h K^T of the heads g0 + i, i < n, for a warp's eight keys.  From eight heads per warp on 16 channels of every head at a time, so that the heads' chains of products run
+// side by side (one head after the other waits for each product) and heads of one key head share its fragment: 500 rows of one prompt, 16 heads of 128 over 4 key heads
+// 85 us one by one, 72 so; 16 heads of 64 over 8, 300 rows 101, 72.  Four heads (of 256) have too few chains for what the fragments' loads take: 72 one by one, 77 so.
+// qa, ka: this lane's ldmatrix addresses in head 0 / key head 0, qp and kp rows' pitches; kv_step: elements between key heads.
+template <int N>
+__device__ __forceinline__ void window_scores(float (&s)[N][4], const bf16* qa, const bf16* ka, int qp, int kp, int kv_step, int g0, int n, int rep, int d) {
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) s[i][e] = 0.0f;
+  if (n < 8) {
+    const int lane = threadIdx.x & 31, g4 = lane >> 2, t4 = lane & 3;
+    const bf16* q_row = qa - (lane & 15) * qp - (lane >> 4) * 8 + g4 * qp + 2 * t4;
+    const bf16* k_row = ka - (lane & 7) * kp - ((lane >> 3) & 1) * 8 + g4 * kp + 2 * t4;
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      if (i < n) {
+        const bf16 *qb = q_row + (g0 + i) * d, *kb = k_row + ((g0 + i) / rep) * kv_step;
+        for (int ks = 0; ks < d; ks += 16) {
+          uint32_t af[4];
+          af[0] = *reinterpret_cast<const uint32_t*>(qb + ks);
+          af[1] = *reinterpret_cast<const uint32_t*>(qb + ks + 8 * qp);
+          af[2] = *reinterpret_cast<const uint32_t*>(qb + ks + 8);
+          af[3] = *reinterpret_cast<const uint32_t*>(qb + ks + 8 * qp + 8);
+          mma_bf16_16816(s[i], af, *reinterpret_cast<const uint32_t*>(kb + ks), *reinterpret_cast<const uint32_t*>(kb + ks + 8));
+        }
+      }
+    return;
+  }
+  uint32_t begins = 0;  // bit i: head g0 + i is the first here of its key head
+  for (int i = 0; i < n; ++i) begins |= uint32_t(i == 0 || (g0 + i) % rep == 0) << i;
+  const uint32_t q0 = smem_u32(qa + g0 * d), k0 = smem_u32(ka + (g0 / rep) * kv_step);
+#pragma unroll 1
+  for (int ks = 0; ks < d; ks += 16) {
+    uint32_t k_at = k0 + ks * 2, b0 = 0, b1 = 0;
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      if (i < n) {
+        if (begins >> i & 1) {
+          asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(b0), "=r"(b1) : "r"(k_at));
+          k_at += kv_step * 2;
+        }
+        uint32_t af[4];
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(af[0]), "=r"(af[1]), "=r"(af[2]), "=r"(af[3]) : "r"(q0 + (i * d + ks) * 2));
+        mma_bf16_16816(s[i], af, b0, b1);
+      }
+  }
+}
+
 template <int HPW, int DVT>
 __global__ void __launch_bounds__(kWmmaThreads, 1) window_attention_mma_kernel(const WindowAttnArgs<bf16> a, const WindowMmaExtra x) {
   constexpr int HMAX = 8 * HPW;
@@ -160,19 +209,8 @@ __global__ void __launch_bounds__(kWmmaThreads, 1) window_attention_mma_kernel(c
     const int hpg = H / x.hg, h_lo = hg * hpg, h_hi = h_lo + hpg;
     if (hg < x.hg) {
       float w[HMAX][4];
-      // the four weights of head g that this thread's accumulator elements hold: (rows g4, g4 + 8) x (keys 2 t4, 2 t4 + 1)
-      auto head_weights = [&](int g, float (&out)[4]) {
-        float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        const bf16* qb = sQ + g4 * QP + g * d + 2 * t4;
-        const bf16* kb = sK + ((g / rep) * BN + kg * 8 + g4) * KP + 2 * t4;
-        for (int ks = 0; ks < d; ks += 16) {
-          uint32_t af[4];
-          af[0] = *reinterpret_cast<const uint32_t*>(qb + ks);
-          af[1] = *reinterpret_cast<const uint32_t*>(qb + ks + 8 * QP);
-          af[2] = *reinterpret_cast<const uint32_t*>(qb + ks + 8);
-          af[3] = *reinterpret_cast<const uint32_t*>(qb + ks + 8 * QP + 8);
-          mma_bf16_16816(s, af, *reinterpret_cast<const uint32_t*>(kb + ks), *reinterpret_cast<const uint32_t*>(kb + ks + 8));
-        }
+      // scores of head g to the weights of the four elements that this thread holds: (rows g4, g4 + 8) x (keys 2 t4, 2 t4 + 1)
+      auto weights = [&](int g, float (&s)[4]) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const int ir = g4 + (e >> 1) * 8, jj = kg * 8 + 2 * t4 + (e & 1), dist = p0 + ir - j0 - jj;
@@ -183,34 +221,37 @@ __global__ void __launch_bounds__(kWmmaThreads, 1) window_attention_mma_kernel(c
             sc += sBias[(ir + BN - 1 - jj) * H + g] + sPb[g];
             wv = __fdividef(1.0f, 1.0f + __expf(-sc));
           }
-          out[e] = wv;
+          s[e] = wv;
         }
       };
+      const bf16* qa = sQ + (lane & 15) * QP + (lane >> 4) * 8;
+      const bf16* ka = sK + (kg * 8 + (lane & 7)) * KP + ((lane >> 3) & 1) * 8;
       if (x.hg == 2) {
         // two warps share a key group: each computes the weights of half the heads, they meet in shared memory ([head][element]
         // [thread of the key group]: conflict-free), and each mixes for its own half of the output heads
         float* xw = sX + kg * 32 + lane;
+        {
+          float s[HMAX / 2][4];
+          window_scores(s, qa, ka, QP, KP, BN * KP, h_lo, hpg, rep, d);
 #pragma unroll
-        for (int gl = 0; gl < HMAX / 2; ++gl) {
-          if (gl < hpg) {
-            float o[4];
-            head_weights(h_lo + gl, o);
+          for (int gl = 0; gl < HMAX / 2; ++gl) {
+            if (gl < hpg) {
+              weights(h_lo + gl, s[gl]);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) xw[((h_lo + gl) * 4 + e) * (KG * 32)] = o[e];
+              for (int e = 0; e < 4; ++e) xw[((h_lo + gl) * 4 + e) * (KG * 32)] = s[gl][e];
+            }
           }
         }
         __syncthreads();  // (every warp is here: x.hg == 2 means KG * 2 == 8 warps)
 #pragma unroll
-        for (int g = 0; g < HMAX; ++g) {
-          if (g < H) {
+        for (int g = 0; g < HMAX; ++g)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) w[g][e] = xw[(g * 4 + e) * (KG * 32)];
-          }
-        }
+          for (int e = 0; e < 4; ++e) w[g][e] = g < H ? xw[(g * 4 + e) * (KG * 32)] : 0.0f;
       } else {
+        window_scores(w, qa, ka, QP, KP, BN * KP, 0, H, rep, d);
 #pragma unroll
         for (int g = 0; g < HMAX; ++g) {
-          if (g < H) head_weights(g, w[g]);
+          if (g < H) weights(g, w[g]);
         }
       }
       // mix the heads' weights; P_h as bf16
@@ -220,15 +261,13 @@ __global__ void __launch_bounds__(kWmmaThreads, 1) window_attention_mma_kernel(c
         const float* tr = sTalk + h * HMAX;  // (rows padded to HMAX floats: 16-byte reads, zeros beyond H)
 #pragma unroll
         for (int g = 0; g < HMAX; g += 4) {
-          if (g < H) {
-            const float4 tv = *reinterpret_cast<const float4*>(tr + g);
+          const float4 tv = *reinterpret_cast<const float4*>(tr + g);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              m[e] = fmaf(tv.x, w[g][e], m[e]);
-              if (g + 1 < H) m[e] = fmaf(tv.y, w[g + 1][e], m[e]);
-              if (g + 2 < H) m[e] = fmaf(tv.z, w[g + 2][e], m[e]);
-              if (g + 3 < H) m[e] = fmaf(tv.w, w[g + 3][e], m[e]);
-            }
+          for (int e = 0; e < 4; ++e) {  // (weights beyond H are zero too)
+            m[e] = fmaf(tv.x, w[g][e], m[e]);
+            m[e] = fmaf(tv.y, w[g + 1][e], m[e]);
+            m[e] = fmaf(tv.z, w[g + 2][e], m[e]);
+            m[e] = fmaf(tv.w, w[g + 3][e], m[e]);
           }
         }
         bf16* pb = sP + (h * kWmmaRows + g4) * PP + kg * 8 + 2 * t4;
