@@ -181,9 +181,12 @@ struct RowsQkvIn {  // what the fragment reads of the step besides the accumulat
 };
 __device__ __forceinline__ void rows_qkv_load(const EpiArgs& e, int r, int head, int d0, RowsQkvIn& in) {
   if (head < e.hq + e.hkv) {
-    const float4* cs = reinterpret_cast<const float4*>(e.rope_cs + (long long)r * (e.d >> 1) + d0);
+    const float2* cs = e.rope_cs + (long long)r * (e.d >> 1) + d0;  // (a caller's scratch: eight bytes is all that its alignment has to be)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) in.cs[j] = cs[j];
+    for (int j = 0; j < 8; ++j) {
+      const float2 even = cs[2 * j], odd = cs[2 * j + 1];
+      in.cs[j] = make_float4(even.x, even.y, odd.x, odd.y);
+    }
   }
   if (head >= e.hq) {
     in.wr = e.write_row[r];
