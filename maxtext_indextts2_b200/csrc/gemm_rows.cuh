@@ -175,25 +175,13 @@ __device__ __forceinline__ void rows_epi_swiglu(const EpiArgs& e, int N2, int r,
 
 // embeddings.py:304-315 + kvcache.py:626-718: `lo` = features d0 .. d0+15 of a head's first half, `hi` = the same
 // dims of its second half (d0 + D/2).  Query / key heads are rotated, value heads stored as they are.
-struct RowsQkvIn {  // what the fragment reads of the step besides the accumulator
-  float4 cs[8];     // cosines and sines of the dims d0 .. d0 + 15
-  int wr, plane;    // the row's cache row and plane
-};
-__device__ __forceinline__ void rows_qkv_load(const EpiArgs& e, int r, int head, int d0, RowsQkvIn& in) {
-  if (head < e.hq + e.hkv) {
-    const float2* cs = e.rope_cs + (long long)r * (e.d >> 1) + d0;  // (a caller's scratch: eight bytes is all that its alignment has to be)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float2 even = cs[2 * j], odd = cs[2 * j + 1];
-      in.cs[j] = make_float4(even.x, even.y, odd.x, odd.y);
-    }
-  }
-  if (head >= e.hq) {
-    in.wr = e.write_row[r];
-    in.plane = e.plane[r];
-  }
+// first half: a cos - b sin ; second half: b cos + a sin, every product rounded to bf16 (bf16 arrays in the reference)
+__device__ __forceinline__ void rows_turn(float& a, float& b, float2 c) {
+  const float ac = bf16r(a * c.x), bs = bf16r(b * c.y), bc = bf16r(b * c.x), as = bf16r(a * c.y);
+  a = ac - bs;
+  b = bc + as;
 }
-__device__ __forceinline__ void rows_epi_qkv(const EpiArgs& e, int N, int r, int head, int d0, const float (&lo)[16], const float (&hi)[16], const RowsQkvIn& in) {
+__device__ __forceinline__ void rows_epi_qkv(const EpiArgs& e, int N, int r, int head, int d0, const float (&lo)[16], const float (&hi)[16]) {
   const int D = e.d, half = D >> 1;
   if (head * D >= N) return;
   const bool is_q = head < e.hq, is_k = !is_q && head < e.hq + e.hkv;
@@ -205,33 +193,22 @@ __device__ __forceinline__ void rows_epi_qkv(const EpiArgs& e, int N, int r, int
     b[j] = bf16_lo(pb); b[j + 1] = bf16_hi(pb);
   }
   if (is_q || is_k) {
+    const float2* cs = e.rope_cs + (long long)r * half + d0;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const float2 c = j & 1 ? make_float2(in.cs[j >> 1].z, in.cs[j >> 1].w) : make_float2(in.cs[j >> 1].x, in.cs[j >> 1].y);
-      // first half: a cos - b sin ; second half: b cos + a sin, every product rounded to bf16 (bf16 arrays in the reference)
-      const float ac = bf16r(a[j] * c.x), bs = bf16r(b[j] * c.y), bc = bf16r(b[j] * c.x), as = bf16r(a[j] * c.y);
-      a[j] = ac - bs;
-      b[j] = bc + as;
-    }
+    for (int j = 0; j < 16; ++j) rows_turn(a[j], b[j], cs[j]);
   }
   if (is_q) {
     bf16* dst = e.q_out + (long long)r * (e.hq * D) + head * D + d0;
     frag_store_bf16(dst, a);
     frag_store_bf16(dst + half, b);
   } else {
-    if (in.wr < 0) return;
+    const int wr = e.write_row[r];
+    if (wr < 0) return;
     const int kvh = is_k ? head - e.hq : head - e.hq - e.hkv;
-    bf16* dst = (is_k ? e.k_cache : e.v_cache) + (((long long)in.plane * e.hkv + kvh) * e.t_alloc + in.wr) * D + d0;
+    bf16* dst = (is_k ? e.k_cache : e.v_cache) + (((long long)e.plane[r] * e.hkv + kvh) * e.t_alloc + wr) * D + d0;
     frag_store_bf16(dst, a);
     frag_store_bf16(dst + half, b);
   }
-}
-
-__device__ __forceinline__ void rows_epi_qkv(const EpiArgs& e, int N, int r, int head, int d0, const float (&lo)[16], const float (&hi)[16]) {
-  if (head * e.d >= N) return;
-  RowsQkvIn in;
-  rows_qkv_load(e, r, head, d0, in);
-  rows_epi_qkv(e, N, r, head, d0, lo, hi, in);
 }
 
 // One head (64 dims) of one row for the int8 cache: RoPE (key heads), then KVQuant.quantize over the head's dims.
@@ -284,37 +261,67 @@ __device__ __forceinline__ void rows_epi_qkv_q8(const EpiArgs& e, int N, int r, 
   (is_k ? e.k_scale : e.v_scale)[row] = mx;
 }
 
-// The same for an eighth of the head per thread (dims d0 .. d0 + 7 and d0 + 32 .. d0 + 39, d0 = 0, 8, 16, 24 in four neighbouring lanes, all of them here): the
-// split-K units have 32 rows or fewer to finish, and a thread per head left three quarters of the threads idle.
-__device__ __forceinline__ void rows_epi_qkv_q8_eighth(const EpiArgs& e, int N, int r, bool valid, int head, int d0, float (&lo)[8], float (&hi)[8], const RowsQkvIn& in) {
+// Both caches for eight dims of either half per thread (d0 .. d0 + 7 and d0 + D/2 .. d0 + D/2 + 7): the split-K units have 64 rows or fewer to finish, and neighbouring
+// lanes write neighbouring dims.  Bound: the chain of loads, sums and stores of a thread behind the cluster's barrier.  128 rows x 1280 x 768, bf16 cache: 9.8 us with 16 dims
+// of either half per thread and their angles loaded at the end, 11.3 with these requested early (704 bytes of spilled registers), 8.9 so; 200 rows x 1792 x 1280 11.6, 11.9, 8.9.
+// An 8-bit cache (heads of 64): the four lanes of a head are all here and share its scale.
+struct RowsQkvIn {  // what the dims need of the step besides the accumulator
+  float2 cs[8];     // cosines and sines of the dims d0 .. d0 + 7 (a caller's scratch: eight bytes is all that its alignment has to be)
+  int wr, plane;    // the row's cache row and plane
+};
+__device__ __forceinline__ void rows_qkv_load(const EpiArgs& e, int r, int head, int d0, RowsQkvIn& in) {
+  if (head < e.hq + e.hkv) {
+    const float2* cs = e.rope_cs + (long long)r * (e.d >> 1) + d0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) in.cs[j] = cs[j];
+  }
+  if (head >= e.hq) {
+    in.wr = e.write_row[r];
+    in.plane = e.plane[r];
+  }
+}
+__device__ __forceinline__ uint4 rows_pack8(const float (&v)[8]) {
+  return make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+}
+__device__ __forceinline__ void rows_epi_qkv_unit(const EpiArgs& e, int N, int r, bool valid, int head, int d0, float (&lo)[8], float (&hi)[8], const RowsQkvIn& in) {
+  const int D = e.d, half = D >> 1;
   const bool is_q = head < e.hq, is_k = !is_q && head < e.hq + e.hkv;
-  valid = valid && head * 64 < N;
+  valid = valid && head * D < N;
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    const float a = bf16r(lo[j]), b = bf16r(hi[j]);
-    lo[j] = a;
-    hi[j] = b;
-    if (is_q || is_k) {
-      const float co = j & 1 ? in.cs[j >> 1].z : in.cs[j >> 1].x, si = j & 1 ? in.cs[j >> 1].w : in.cs[j >> 1].y;
-      lo[j] = bf16r(bf16r(a * co) - bf16r(b * si));
-      hi[j] = bf16r(bf16r(b * co) + bf16r(a * si));
-    }
+    lo[j] = bf16r(lo[j]);
+    hi[j] = bf16r(hi[j]);
+    if (is_q || is_k) rows_turn(lo[j], hi[j], in.cs[j]);
   }
-  if (valid && is_q) {
-    bf16* dst = e.q_out + (long long)r * (e.hq * 64) + head * 64 + d0;
-    *reinterpret_cast<uint4*>(dst) = make_uint4(pack_bf16x2(lo[0], lo[1]), pack_bf16x2(lo[2], lo[3]), pack_bf16x2(lo[4], lo[5]), pack_bf16x2(lo[6], lo[7]));
-    *reinterpret_cast<uint4*>(dst + 32) = make_uint4(pack_bf16x2(hi[0], hi[1]), pack_bf16x2(hi[2], hi[3]), pack_bf16x2(hi[4], hi[5]), pack_bf16x2(hi[6], hi[7]));
+  if (is_q) {
+    if (!valid) return;
+    bf16* dst = e.q_out + (long long)r * (e.hq * D) + head * D + d0;
+    *reinterpret_cast<uint4*>(dst) = rows_pack8(lo);
+    *reinterpret_cast<uint4*>(dst + half) = rows_pack8(hi);
+    return;
+  }
+  const int kvh = is_k ? head - e.hq : head - e.hq - e.hkv;
+  const long long row = ((long long)in.plane * e.hkv + kvh) * e.t_alloc + in.wr;
+  if (e.kq_cache == nullptr) {
+    if (!valid || in.wr < 0) return;
+    bf16* dst = (is_k ? e.k_cache : e.v_cache) + row * D + d0;
+    *reinterpret_cast<uint4*>(dst) = rows_pack8(lo);
+    *reinterpret_cast<uint4*>(dst + half) = rows_pack8(hi);
+    return;
   }
   float mx = 0.0f;
 #pragma unroll
-  for (int j = 0; j < 8; ++j) mx = fmaxf(mx, fmaxf(fabsf(lo[j]), fabsf(hi[j])));
-  mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-  mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-  if (!valid || is_q || in.wr < 0) return;
+  for (int j = 0; j < 8; ++j) {
+    lo[j] = bf16r(lo[j]);
+    hi[j] = bf16r(hi[j]);
+    mx = fmaxf(mx, fmaxf(fabsf(lo[j]), fabsf(hi[j])));
+  }
+  const uint32_t head_lanes = 0xfu << (threadIdx.x & 28);
+  mx = fmaxf(mx, __shfl_xor_sync(head_lanes, mx, 1));
+  mx = fmaxf(mx, __shfl_xor_sync(head_lanes, mx, 2));
+  if (!valid || in.wr < 0) return;
   const bool fp8 = e.kv_fp8 != 0;
   const float inv = mx > 0.0f ? kv_quant_max(fp8) / mx : 0.0f;
-  const int kvh = is_k ? head - e.hq : head - e.hq - e.hkv;
-  const long long row = ((long long)in.plane * e.hkv + kvh) * e.t_alloc + in.wr;
   uint8_t* dst = (is_k ? e.kq_cache : e.vq_cache) + row * 64 + d0;
   auto four = [&](const float* v) { return kv_quant_pair(v[0], v[1], inv, fp8) | (kv_quant_pair(v[2], v[3], inv, fp8) << 16); };
   *reinterpret_cast<uint2*>(dst) = make_uint2(four(lo), four(lo + 4));
@@ -428,29 +435,25 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   const uint32_t tmem_base = tail->tmem_base;
   if (trace && threadIdx.x == 0) trace[0] = clock64() - t_start;
 
-  // split-K: unit u of the rows that this CTA finishes is the 16 columns (u & 7) of row u >> 3 (an 8-bit cache: the quarter u & 3 of the two heads (u >> 2) & 1)
+  // split-K: unit u of the rows that this CTA finishes is the 16 columns (u & 7) of row u >> 3 (rotated heads: eight of either half of a head)
   const int rpc = p.r_tile / p.splits, r_begin = int(blockIdx.y) * rpc;  // rows reduced and finished by this CTA, the first of them in the row block
-  const bool q8 = EPI == EPI_QKV_ROPE && e.kq_cache != nullptr;
   float rs_in = 1.0f;
   uint4 resid_in[2];
   RowsQkvIn qkv_in;
+  auto qkv_unit = [&](int u, int& hd, int& d0) {  // the unit's head in the tile, and its first dim
+    const int per = e.d >> 4;
+    hd = (u & 7) / per;
+    d0 = (u & 7) % per * 8;
+  };
   auto fetch = [&](int u) {
     const int row = row_base + r_begin + (u >> 3), n0 = first_tile * kTileN + (u & 7) * 16;
     if (u >= rpc * 8 || row >= p.rows || first_tile >= n_tiles) return;
     if (EPI == EPI_SWIGLU || EPI == EPI_QKV_ROPE || EPI == EPI_STORE_BF16) rs_in = rows_rstd(e, row);
     if (EPI == EPI_RESIDUAL && n0 < p.n && rows_residual_whole(e, p.n, n0)) rows_residual_load(e, row, n0, resid_in);
-    if (EPI == EPI_QKV_ROPE && q8) {
-      const int head = first_tile * 2 + ((u >> 2) & 1);
-      const float4* cs = reinterpret_cast<const float4*>(e.rope_cs + (long long)row * 32 + (u & 3) * 8);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) qkv_in.cs[j] = cs[j];
-      if (head >= e.hq) {
-        qkv_in.wr = e.write_row[row];
-        qkv_in.plane = e.plane[row];
-      }
-    } else if (EPI == EPI_QKV_ROPE) {
-      const int d = n0 % e.d;
-      if (d < (e.d >> 1) && n0 < p.n) rows_qkv_load(e, row, n0 / e.d, d, qkv_in);
+    if (EPI == EPI_QKV_ROPE) {
+      int hd, d0;
+      qkv_unit(u, hd, d0);
+      rows_qkv_load(e, row, first_tile * kTileN / e.d + hd, d0, qkv_in);
     }
   };
 
@@ -710,26 +713,17 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
             rows_scale16(uu, rs);
             if (valid) rows_epi_swiglu(e, p.n, row, tile * kTileN + c0, g, uu);
           }
-        } else if (EPI == EPI_QKV_ROPE && q8) {
-          const int hd = (u >> 2) & 1, d0 = (u & 3) * 8;
+        } else if (EPI == EPI_QKV_ROPE) {
+          int hd, d0;
+          qkv_unit(u, hd, d0);
           float lo[8], hi[8];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            lo[j] = src[hd * 64 + d0 + j] * rs;
-            hi[j] = src[hd * 64 + 32 + d0 + j] * rs;
+          for (int q = 0; q < 8; q += 4) {
+            const float4 x = *reinterpret_cast<const float4*>(src + hd * e.d + d0 + q), y = *reinterpret_cast<const float4*>(src + hd * e.d + (e.d >> 1) + d0 + q);
+            lo[q] = x.x * rs; lo[q + 1] = x.y * rs; lo[q + 2] = x.z * rs; lo[q + 3] = x.w * rs;
+            hi[q] = y.x * rs; hi[q + 1] = y.y * rs; hi[q + 2] = y.z * rs; hi[q + 3] = y.w * rs;
           }
-          rows_epi_qkv_q8_eighth(e, p.n, row, valid, tile * 2 + hd, d0, lo, hi, qkv_in);
-        } else if (EPI == EPI_QKV_ROPE) {
-          const int D = e.d, half = D >> 1;
-          const int d = (tile * kTileN + c0) % D;
-          if (d < half) {
-            float lo[16], hi[16];
-            ld16(c0, lo);
-            ld16(c0 + half, hi);
-            rows_scale16(lo, rs);
-            rows_scale16(hi, rs);
-            if (valid) rows_epi_qkv(e, p.n, row, (tile * kTileN + c0) / D, d, lo, hi, qkv_in);
-          }
+          rows_epi_qkv_unit(e, p.n, row, valid, tile * kTileN / e.d + hd, d0, lo, hi, qkv_in);
         } else if (EPI == EPI_STORE_BF16 || EPI == EPI_RESIDUAL) {
           float v[16];
           ld16(c0, v);
