@@ -272,6 +272,9 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     uint32_t phase = 1;
     const int m_step = pairs % m_div, n_step = pairs / m_div;
     Rows at = rows_of(m_tiles > 0 ? m : 0);
+    // Weights are read once per row tile: with one alone (a decode step's) nobody comes back for them, and what they would push out of L2 is what the step's next kernels
+    // read.  Kept like several row tiles', they made a layer's kernels wait: 128 rows of a model of 2048 x 8192 108 us per layer, 103 so; 200 rows of 1280 x 5120 70 and 67.
+    const uint64_t w_hint = !GROUPED && p.rows <= kPairRows ? kEvictFirst : kEvictLast;
     // the first tile's weights do not depend on the previous kernel
     const int pre = my_tiles == 0 ? 0 : (nkb < p.stages ? nkb : p.stages);
     auto fills = [&](auto group) {  // (as the MMAs below: in straight code, the issue of two loads takes as long as they do up to 128 columns)
@@ -281,7 +284,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
 #pragma unroll
         for (int g = 0; g < G; ++g)
           tma_load_2d_pair(smem + stage * stage_bytes + g * block_bytes + kPairABytes, &tm_w, (k * G + g) * kBlockK, at.w0 + nt * p.bn + rank * half_n, &tail->full[stage],
-                           kEvictLast);
+                           w_hint);
       };
       auto a_load = [&](int stage, int k) {
 #pragma unroll
