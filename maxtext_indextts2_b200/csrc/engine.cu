@@ -998,9 +998,8 @@ int enqueue_step(mtx_engine* e, int mode, int rows, const int32_t* chunk_tokens,
   // 65..256 rows with the norm scales folded into the weights: RMSNorm is fused into the GEMMs around it (the residual
   // epilogues leave the row statistics, the consuming epilogues apply rstd; the per-kernel rmsnorm launches disappear)
   const bool fused_norm = rows_k && c.norm_scales_folded && (gemma3 || env_int("MTX_ROWS_FUSED_NORM", 1) != 0);
-  // Products whose K the row-major GEMM leaves whole take the pair GEMM with the steps' roundings, the same bits: 200 rows x 10240 x 1280 15.3 -> 12.6 us.  (In parts the pair GEMM
-  // takes longer than a cluster with a part in each CTA: 200 x 1792 x 1280 in four, 4 us more.)
-  const bool wide_up = fused_norm && !gemma3 && plan_rows(2 * M, E, r_tile, e->num_sms, EPI_SWIGLU).splits == 1;
+  // (gemma3's steps stay on the row-major GEMM: not timed on the other one)
+  const bool wide_up = fused_norm && !gemma3 && takes_wide_up(rows, plan_rows(2 * M, E, r_tile, e->num_sms, EPI_SWIGLU), e->num_sms) && env_int("MTX_ROWS_WIDE_UP", 1) != 0;
   const int ss_tiles = (E + 127) / 128;
   auto ss_args = [&](EpiArgs& ea, const float* in, float* out) {
     ea.ss_in = fused_norm ? in : nullptr;

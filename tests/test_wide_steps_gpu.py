@@ -1,10 +1,11 @@
-"""Decode steps of 65 to 256 slots whose gated up-projection has columns enough for the pair GEMM (norm scales folded into the weights) against the same steps on
-the row-major GEMM (norm scales left alone): row counts at the edges of the 32-row warps and the 128-row halves of its tile, and the caches whose rows the
-split-K projections finish."""
+"""Decode steps whose gated up-projection may take the pair GEMM (takes_wide_up in csrc/host_util.cuh; norm scales folded into the weights): bit for bit what the
+row-major GEMM gives, and close to the steps with the norm scales left alone.  Row counts at the edges of the 32-row warps and the 128-row halves of its tile, and the
+caches whose rows the split-K projections finish."""
 
 import numpy as np
 import pytest
 import torch
+from torch.profiler import ProfilerActivity, profile
 
 from maxtext_indextts2_b200 import maxengine, pyconfig
 
@@ -14,27 +15,48 @@ CACHES = {"bf16": {}, "int8": dict(quantize_kvcache=True, kv_quant_axis="dkv"), 
           "tokens": dict(quantize_kvcache=True, kv_quant_axis="heads_and_dkv"), "paged": dict(attention="paged", pagedattn_tokens_per_page=16)}
 
 
+def _step(cache, dim, rows, mlp=4864, fold=True, graph=True):
+  """The state behind one generated token per slot, and the names of the kernels that ran."""
+  kw = dict(attention="dot_product")
+  kw.update(CACHES[cache])
+  if cache == "paged":
+    kw["pagedattn_num_pages"] = 6 * rows + 1
+  cfg = pyconfig.initialize(None, base_num_decoder_layers=2, base_emb_dim=320, base_num_query_heads=6, base_num_kv_heads=2, head_dim=dim, base_mlp_dim=mlp, vocab_size=640,
+                            per_device_batch_size=rows, max_prefill_predict_length=48, max_target_length=80, weight_dtype="bfloat16", scan_layers=False,
+                            materialize_logits=True, return_log_prob=True, decode_sampling_strategy="greedy", fold_norm_scales=fold, **kw)
+  engine = maxengine.MaxEngine(cfg, use_cuda_graph=graph)
+  params = engine.load_params(on_device_init=True, norm_jitter=0.1)
+  lengths = np.random.Generator(np.random.PCG64(rows)).integers(1, 49, size=rows)
+  state = engine.fill_synthetic_context(lengths, np.full(rows, 7), seed=3)
+  state["tokens"].copy_(torch.randint(0, 640, (rows, 1), generator=torch.Generator().manual_seed(4), dtype=torch.int32))
+  with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as p:
+    state, _ = engine.generate(params, state)
+    torch.cuda.synchronize()
+  got = {k: v.clone() for k, v in state["cache"].items() if torch.is_tensor(v)}
+  return dict(got, logits=state["logits"].clone()), {e.name for e in p.events()}
+
+
+@pytest.mark.parametrize("cache,dim,rows,mlp,wide", [
+    ("bf16", 64, 65, 4864, True), ("bf16", 128, 97, 4864, True), ("bf16", 64, 256, 4864, True), ("int8", 64, 129, 4864, True), ("int8", 64, 200, 4864, True),
+    ("fp8", 64, 255, 4864, True), ("tokens", 64, 161, 4864, True), ("paged", 64, 66, 4864, True), ("paged", 128, 224, 4864, True),
+    ("bf16", 64, 200, 9472, True),  # 148 tiles of 128 columns, more than 128 rows
+    ("bf16", 64, 70, 9472, False), ("tokens", 64, 64, 4864, False), ("tokens", 64, 1, 4864, False)])  # (a full wave; rows that fill a quarter of a tile)
+def test_up_projection_has_the_same_bits_on_either_gemm(cache, dim, rows, mlp, wide, monkeypatch):
+  """Logits and caches of a step on the GEMM that the rule picks and on the row-major one (MTX_ROWS_WIDE_UP=0)."""
+  got, names = _step(cache, dim, rows, mlp, graph=False)
+  monkeypatch.setenv("MTX_ROWS_WIDE_UP", "0")
+  want, plain = _step(cache, dim, rows, mlp, graph=False)
+  is_wide = lambda names: any("gemm_wide_kernel" in n for n in names)
+  assert any("gemm_rows_kernel" in n for n in plain) and is_wide(names) == wide and not is_wide(plain)
+  assert got.keys() == want.keys() and torch.isfinite(got["logits"]).all()
+  assert all(torch.equal(got[k], want[k]) for k in want)
+
+
 @pytest.mark.parametrize("cache,dim,rows", [("bf16", 64, 65), ("bf16", 128, 97), ("bf16", 64, 256), ("int8", 64, 128), ("int8", 64, 129), ("int8", 64, 200), ("fp8", 64, 255),
                                             ("tokens", 64, 40), ("tokens", 64, 161), ("paged", 64, 66), ("paged", 128, 224)])
 def test_step_against_row_major_gemm(cache, dim, rows):
-  out = []
-  for fold in (True, False):
-    kw = dict(attention="dot_product")
-    kw.update(CACHES[cache])
-    if cache == "paged":
-      kw["pagedattn_num_pages"] = 6 * rows + 1
-    cfg = pyconfig.initialize(None, base_num_decoder_layers=2, base_emb_dim=320, base_num_query_heads=6, base_num_kv_heads=2, head_dim=dim, base_mlp_dim=4864, vocab_size=640,
-                              per_device_batch_size=rows, max_prefill_predict_length=48, max_target_length=80, weight_dtype="bfloat16", scan_layers=False,
-                              materialize_logits=True, return_log_prob=True, decode_sampling_strategy="greedy", fold_norm_scales=fold, **kw)
-    assert 2 * (2 * cfg.mlp_dim // 128) > 148  # (its K stays whole: enqueue_step's wide_up)
-    engine = maxengine.MaxEngine(cfg)
-    params = engine.load_params(on_device_init=True, norm_jitter=0.1)
-    lengths = np.random.Generator(np.random.PCG64(rows)).integers(1, 49, size=rows)
-    state = engine.fill_synthetic_context(lengths, np.full(rows, 7), seed=3)
-    state["tokens"].copy_(torch.randint(0, 640, (rows, 1), generator=torch.Generator().manual_seed(4), dtype=torch.int32))
-    state, _ = engine.generate(params, state)
-    out.append(state["logits"].double().clone())
-  got, want = out
+  """Norm scales folded into the weights (fused into the products around them) against norm scales left alone (the row-major GEMM, norms of their own)."""
+  got, want = (_step(cache, dim, rows, fold=fold)[0]["logits"].double() for fold in (True, False))
   assert got.shape[0] == rows and torch.isfinite(got).all()
   # bf16 activations through two layers, 2^-9 for each of about ten roundings (and one step of an 8-bit cache's scale in the step's own keys); a row of its own is
   # off by its whole size
