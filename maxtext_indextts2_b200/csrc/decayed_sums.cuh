@@ -304,8 +304,9 @@ __device__ __forceinline__ uint32_t dc_movmatrix_trans(uint32_t a) {
   return d;
 }
 
-// grid (runs, heads, ceil(vdim / (8 NT))), a warp per 16 channels.  NT: 8-column blocks of a CTA, two, or one where two leave SMs idle: the chunks are a serial chain, and a
-// warp that decays, splits and adds half of the values is through it sooner (one run of 1777 tokens, 16 heads of 64 x 64: 64 CTAs 20.4 us, 128 CTAs 15.9).
+// grid (runs, heads, ceil(vdim / (8 NT))), a warp per 16 channels.  NT: 8-column blocks of a CTA, two, or one where every CTA of eight columns has an SM to itself: the chunks are
+// a serial chain, and a warp that decays, splits and adds half of the values is through it sooner (one run of 1777 tokens, 16 heads of 64 x 64: 64 CTAs 20.2 us, 128 CTAs 15.6).
+// Two such CTAs on an SM are slower than one of 16 columns, which loads the keys once for both halves.
 template <int NT>
 __global__ void __launch_bounds__(512) decayed_states_kernel(const DecayedSplitArgs b) {
   extern __shared__ __align__(16) unsigned char dc_raw[];

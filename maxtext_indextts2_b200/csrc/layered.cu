@@ -2035,7 +2035,9 @@ int launch_decayed_split(mtx_layered* e, const DecayedChunksArgs& da, const mtx_
     MTX_CUDA(cudaFuncSetAttribute(decayed_outputs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(s2)));
     have2 = s2;
   }
-  const int columns = mat_pad16(da.vdim), nt = b.n_runs * da.heads * columns / 16 < e->num_sms ? 1 : 2;  // (8-column blocks per CTA: one where two leave SMs idle)
+  // 8-column blocks per CTA: one as long as every CTA then still has an SM to itself.  Us, one / two blocks, 1777 tokens, heads of 64 x 64: 64 CTAs of 16 columns 15.6 / 20.2, 120 22.9 /
+  // 21.0, 144 23.2 / 21.2; heads of 128 x 64: 80 33.6 / 29.6; 2048 tokens, heads of 256 x 64: 76 84.1 / 62.5
+  const int columns = mat_pad16(da.vdim), nt = (long long)b.n_runs * da.heads * columns / 8 <= e->num_sms ? 1 : 2;
   MTX_TRY(launch(nt == 1 ? decayed_states_kernel<1> : decayed_states_kernel<2>, dim3(b.n_runs, da.heads, columns / (8 * nt)), dim3(32 * (mat_pad16(da.dim) / 16)), s1, st, sa));
   return launch(decayed_outputs_kernel, dim3(b.rows / kDcTokens + b.n_runs, da.heads), dim3(128), s2, st, sa);
 }

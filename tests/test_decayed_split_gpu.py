@@ -34,3 +34,9 @@ def test_split_repeats_the_walk_of_chunks(heads, dim, vdim, n):
 def test_split_of_many_heads():
   """Heads enough for 16 value columns per CTA."""
   test_split_repeats_the_walk_of_chunks(40, 16, 64, 300)
+
+
+@pytest.mark.parametrize("heads", [37, 38])
+def test_split_at_the_edge_of_the_rule_on_columns(heads):
+  """148 and 152 CTAs of eight value columns on 148 SMs: eight columns per CTA, then sixteen."""
+  test_split_repeats_the_walk_of_chunks(heads, 16, 32, 300)
