@@ -58,16 +58,18 @@ __device__ __forceinline__ float tanh_f32(float x) {
 }
 
 // s[i] = Q_h K^T of the heads g0 + i, i < n, for a warp's eight keys.  From eight heads per warp on 16 channels of every head at a time, so that the heads' chains of products run
-// side by side (one head after the other waits for each product) and heads of one key head share its fragment: 500 rows of one prompt, 16 heads of 128 over 4 key heads
-// 85 us one by one, 72 so; 16 heads of 64 over 8, 300 rows 101, 72.  Four heads (of 256) have too few chains for what the fragments' loads take: 72 one by one, 77 so.
+// side by side (one head after the other waits for each product) and heads of one key head share its fragment: 500 rows of one prompt beside 30 single tokens, 16 heads of 128 over 4
+// key heads 84 us one by one, 67 so; 300 rows beside 7, 16 heads of 64 over 8, 87 and 59.  Four heads (of 256) have too few chains for what the fragments' loads take:
+// 72 one by one, 77 so.
 // qa, ka: this lane's ldmatrix addresses in head 0 / key head 0, qp and kp rows' pitches; kv_step: elements between key heads.
-template <int N>
-__device__ __forceinline__ void window_scores(float (&s)[N][4], const bf16* qa, const bf16* ka, int qp, int kp, int kv_step, int g0, int n, int rep, int d) {
+// finish(i, s[i]): what becomes of a head's scores, right behind its products.  All sigmoids after all products: 2 heads of 64, 300 rows, 21 us for 19, 16 heads of 128 73 for 67.
+template <int N, class F>
+__device__ __forceinline__ void window_scores(float (&s)[N][4], const bf16* qa, const bf16* ka, int qp, int kp, int kv_step, int g0, int n, int rep, int d, F&& finish) {
 #pragma unroll
   for (int i = 0; i < N; ++i)
 #pragma unroll
     for (int e = 0; e < 4; ++e) s[i][e] = 0.0f;
-  if (n < 8) {
+  if (N < 8 || n < 8) {
     const int lane = threadIdx.x & 31, g4 = lane >> 2, t4 = lane & 3;
     const bf16* q_row = qa - (lane & 15) * qp - (lane >> 4) * 8 + g4 * qp + 2 * t4;
     const bf16* k_row = ka - (lane & 7) * kp - ((lane >> 3) & 1) * 8 + g4 * kp + 2 * t4;
@@ -83,6 +85,7 @@ __device__ __forceinline__ void window_scores(float (&s)[N][4], const bf16* qa, 
           af[3] = *reinterpret_cast<const uint32_t*>(qb + ks + 8 * qp + 8);
           mma_bf16_16816(s[i], af, *reinterpret_cast<const uint32_t*>(kb + ks), *reinterpret_cast<const uint32_t*>(kb + ks + 8));
         }
+        finish(i, s[i]);
       }
     return;
   }
@@ -104,6 +107,9 @@ __device__ __forceinline__ void window_scores(float (&s)[N][4], const bf16* qa, 
         mma_bf16_16816(s[i], af, b0, b1);
       }
   }
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+    if (i < n) finish(i, s[i]);
 }
 
 template <int HPW, int DVT>
@@ -232,15 +238,13 @@ __global__ void __launch_bounds__(kWmmaThreads, 1) window_attention_mma_kernel(c
         float* xw = sX + kg * 32 + lane;
         {
           float s[HMAX / 2][4];
-          window_scores(s, qa, ka, QP, KP, BN * KP, h_lo, hpg, rep, d);
+          window_scores(s, qa, ka, QP, KP, BN * KP, h_lo, hpg, rep, d, [&](int gl, float (&v)[4]) { weights(h_lo + gl, v); });
 #pragma unroll
-          for (int gl = 0; gl < HMAX / 2; ++gl) {
+          for (int gl = 0; gl < HMAX / 2; ++gl)  // (behind all products: a store between two heads' keeps the second's operands from being read ahead)
             if (gl < hpg) {
-              weights(h_lo + gl, s[gl]);
 #pragma unroll
               for (int e = 0; e < 4; ++e) xw[((h_lo + gl) * 4 + e) * (KG * 32)] = s[gl][e];
             }
-          }
         }
         __syncthreads();  // (every warp is here: x.hg == 2 means KG * 2 == 8 warps)
 #pragma unroll
@@ -248,11 +252,7 @@ __global__ void __launch_bounds__(kWmmaThreads, 1) window_attention_mma_kernel(c
 #pragma unroll
           for (int e = 0; e < 4; ++e) w[g][e] = g < H ? xw[(g * 4 + e) * (KG * 32)] : 0.0f;
       } else {
-        window_scores(w, qa, ka, QP, KP, BN * KP, 0, H, rep, d);
-#pragma unroll
-        for (int g = 0; g < HMAX; ++g) {
-          if (g < H) weights(g, w[g]);
-        }
+        window_scores(w, qa, ka, QP, KP, BN * KP, 0, H, rep, d, weights);
       }
       // mix the heads' weights; P_h as bf16
 #pragma unroll 1
