@@ -61,13 +61,26 @@ def test_long_steps_repeat_short_ones(name):
   assert all(torch.isfinite(t).all() for t in out[0]) and all(torch.equal(a, b) for a, b in zip(*out))
 
 
+def _blocks_per_stage(rows, n, k):
+  """K blocks of a stage for this product of a layered design: plan_rows, wide_tile_columns and wide_group (csrc/host_util.cuh) over again."""
+  tiles, kb, parts = -(-n // 128), k // 64, 1
+  if 2 * tiles <= 148:
+    while parts * 2 <= min(8, kb) and tiles * 2 * parts * 2 <= 148 + 148 // 4:
+      parts *= 2
+  pairs, row_tiles = torch.cuda.get_device_properties(0).multi_processor_count // 2, -(-rows // 256)
+  cost = lambda bn: -(-row_tiles * -(-n // bn) // pairs) * (128 + bn)
+  columns = min(range(256, 32, -32), key=cost)  # (of equal costs the widest)
+  return 2 if columns <= 128 and kb % (2 * parts) == 0 else 1
+
+
 @pytest.mark.parametrize("rows", [257, 288, 545, 767])
-@pytest.mark.parametrize("ff", [448, 256])
-def test_part_empty_row_tile_repeats_a_whole_one(rows, ff):
-  """The last row tile's warps with 32, some and no rows, and feed-forwards of an odd (7, one k block per stage) and an even number of k blocks
-  (two per stage on narrow tiles): bit for bit what the same rows are among 768."""
+@pytest.mark.parametrize("width,ff,blocks", [(256, 448, 1), (256, 256, 1), (1024, 1024, 2)])
+def test_part_empty_row_tile_repeats_a_whole_one(rows, width, ff, blocks):
+  """The last row tile's warps with 32, some and no rows, and feed-forwards with one k block per stage, of an odd number of them (7) and of four, and with two
+  (four and eight parts of two blocks and more): bit for bit what the same rows are among 768."""
+  assert all(_blocks_per_stage(r, n, k) == blocks for r in (rows, 768) for n, k in ((2 * ff, width), (width, ff)))
   layers = [gugidra.parallel_layer(4, 2, 64, 2, 32, 64, mlp=gugidra.dense_ff(ff)), gugidra.gla_layer(4, 32, 64, mlp=gugidra.dense_ff(ff))]
-  model = gugidra.model_dict(256, 384, layers)
+  model = gugidra.model_dict(width, 384, layers)
   toks = np.random.Generator(np.random.PCG64(4)).integers(0, model["vocab"], size=768).tolist()
   out = []
   for n in (rows, 768):
@@ -114,8 +127,10 @@ def test_unequal_experts_against_float32():
 
 
 @pytest.mark.parametrize("name", ["kifusun", "gugidra", "ligidra", "zakelorn"])
-@pytest.mark.parametrize("width,rows", [(256, 257), (384, 512), (256, 769)])
+@pytest.mark.parametrize("width,rows", [(256, 257), (384, 512), (256, 769), (1024, 389)])
 def test_long_steps_against_float32(name, width, rows):
+  """(1024 wide: the up-projection, for one, has two k blocks per stage.)"""
+  assert _blocks_per_stage(rows, 3 * width, width) == (2 if width == 1024 else 1)
   design, model = _model(name, width)
   toks = np.random.Generator(np.random.PCG64(rows)).integers(0, model["vocab"], size=rows).tolist()
   out = {}
