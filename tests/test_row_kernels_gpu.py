@@ -53,11 +53,12 @@ def test_output_of_a_recurrence(vdim, dtype):
   assert error(dtype, logits(model, t, dtype), gugidra_ref.logits_of(model, t, TOKENS)) < TOL[dtype]
 
 
-@pytest.mark.parametrize("heads,kv,dim,rot", [(4, 2, 64, 32), (2, 1, 16, 16), (8, 4, 256, 256), (16, 4, 128, 0), (16, 16, 64, 64), (3, 1, 96, 48), (4, 2, 64, 12), (2, 2, 48, 24)])
+@pytest.mark.parametrize("heads,kv,dim,rot", [(4, 2, 64, 32), (2, 1, 16, 16), (8, 4, 256, 256), (16, 4, 128, 0), (16, 16, 64, 64), (3, 1, 96, 48), (4, 2, 64, 12), (2, 2, 48, 24), (32, 8, 128, 64),
+                                                (16, 8, 256, 256), (33, 11, 64, 64)])
 @pytest.mark.parametrize("rows", [1, 300])
 def test_rotated_keys_and_values(heads, kv, dim, rot, rows):
   """Keys (of unit RMS, then rotated) and values of a first layer, appended behind 37 tokens: heads of 64, 128 and 256 channels eight channels per thread, in one
-  and in several rounds of the CTA, the others, and where fewer channels turn than that, channel by channel."""
+  round of the CTA (512 pieces of eight channels) and in two (768, 1024; 440 leave a warp with queries, keys and values), the others, and where fewer channels turn than that, channel by channel."""
   part = zakelorn.attention_part(heads, kv, dim, rot_dims=rot)
   model = zakelorn.model_dict(256, 320, [zakelorn.parallel_layer(part, zakelorn.lightning_part(2, 64), mlp=zakelorn.dense_ff(256))])
   cfg = pyconfig.from_model_dict(model, dtype="bfloat16", per_device_batch_size=2, max_target_length=400, pagedattn_tokens_per_page=24, pagedattn_num_pages=40, max_step_rows=400)
@@ -85,3 +86,29 @@ def test_rotated_keys_and_values(heads, kv, dim, rot, rows):
     # the projection rounded to bf16 and its rotation again: at most 2^-8 (bf16's unit roundoff) of each value or turned pair, twice
     off = (got - want).square().sum((1, 2)).sqrt() / want.square().sum((1, 2)).sqrt()
     assert float(off.max()) < 2.0**-7
+
+
+@pytest.mark.parametrize("rows", [1, 70])
+@pytest.mark.parametrize("design,heads,kv,dim,rot", [("zakelorn", 4, 2, 64, 32), ("zakelorn", 48, 8, 128, 64), ("zakelorn", 20, 4, 256, 256), ("gugidra", 4, 2, 64, 64), ("gugidra", 8, 2, 96, 32),
+                                                     ("gugidra", 48, 8, 128, 128)])
+def test_rotated_queries(design, heads, kv, dim, rot, rows):
+  """Logits behind 37 tokens against the float32 engine, whose queries come from the kernels of a channel per lane: with norms (zakelorn) and without (gugidra, whose layers call the other
+  kernel's instance), in one round of the CTA and in two (queries of more than 4096 channels).  The attention alone feeds the layer, so that a head's query of its own shows in every row."""
+  if design == "zakelorn":
+    mod, layer = zakelorn, zakelorn.parallel_layer(zakelorn.attention_part(heads, kv, dim, rot_dims=rot), zakelorn.lightning_part(2, 64), 1.0, 0.0, mlp=zakelorn.dense_ff(256))
+    model = zakelorn.model_dict(256, 320, [layer])
+  else:
+    mod, layer = gugidra, gugidra.parallel_layer(heads, kv, dim, 2, 32, 64, mlp=gugidra.dense_ff(256), rot_dims=rot, right_scale=0.0)
+    model = gugidra.model_dict(256, 320, [layer])
+  toks = np.random.Generator(np.random.PCG64(6)).integers(0, 320, size=37 + rows).tolist()
+  out = {}
+  for dtype in ("float32", "bfloat16"):
+    cfg = pyconfig.from_model_dict(model, dtype=dtype, per_device_batch_size=2, max_target_length=128, pagedattn_tokens_per_page=16, pagedattn_num_pages=20, max_step_rows=80)
+    engine = maxengine.MaxEngine(cfg)
+    engine.load_params(mod.random_tensors(cfg, seed=3))
+    engine.init_decode_state()
+    engine.step([(0, toks[:37], [])])
+    out[dtype] = engine.step([(0, toks[37:], list(range(rows)))]).double()
+  # the designs' own bound, over all logits and (twice) in each row
+  off = (out["bfloat16"] - out["float32"]).square().mean(1).sqrt() / out["float32"].square().mean().sqrt()
+  assert float(off.square().mean().sqrt()) < TOL["bfloat16"] and float(off.max()) < 2 * TOL["bfloat16"]
