@@ -1,4 +1,5 @@
-// GEMM of steps with more than 256 rows (prompts and long portions of prompts): all rows of the step in one launch.
+// GEMM of steps with more than 256 rows (prompts and long portions of prompts), all rows of the step in one launch, and of some decode steps' gated up-projections
+// (65 to 256 rows: takes_wide_up).
 //
 //   acc[r, n] = sum_k A[r, k] * W[n, k]        both operands K-major bf16, fp32 accumulation in TMEM
 //
@@ -26,9 +27,8 @@
 //
 // Segments: gemm_rows.cuh cuts the k blocks of a narrow projection over a cluster and adds the parts in order.  With `segments` set to that
 // number a tile's k range is accumulated in the same parts, which the epilogue threads add in registers, so that a row's result is bit
-// for bit what the 256-row steps give it, however many rows its step has.  Such an epilogue works on one fragment of 16 columns at a
-// time (kFragments; fragment(tile, n, column, values)).
-// Grouped (GROUPED; the experts of a routed feed-forward): the rows are slots, group g's are [group_off[g], group_off[g + 1]) (known on the
+// for bit what the 256-row steps give it, however many rows its step has (MODE kWideParts, epilogues with kFragments).
+// Grouped (MODE kWideGrouped; the experts of a routed feed-forward): the rows are slots, group g's are [group_off[g], group_off[g + 1]) (known on the
 // device only) and its weight the rows g * n .. of W.  The pairs walk the groups' row tiles one group after the other; a group's last tile
 // reads the next group's rows and drops their results.
 #pragma once
@@ -87,8 +87,8 @@ struct WideTile {
   int slice;  // index of this run of columns among all the runs of a row: 2 * tile + half
 };
 
-// A warp's 32 rows x 128 bytes between the arithmetic, where a thread owns a row, and global memory, where eight lanes share 128 bytes of a
-// row.  Chunk j (16 bytes) of row r lies at j ^ (r & 7): neither side has bank conflicts.  A thread that stored its own row wrote half sectors
+// A warp's 32 rows x 64 or 128 bytes between the arithmetic, where a thread owns a row, and global memory, where neighbouring lanes share a row's
+// bytes.  Chunk j (16 bytes) of row r lies at j ^ (r & 7), at j ^ (r >> 1 & 3) in rows of 64 bytes: neither side has bank conflicts.  A thread that stored its own row wrote half sectors
 // of 32 rows per instruction, and the next tile's operands waited behind them: 4000 x 1792 x 1280 (rotated q, k, v) took 12 us for
 // the second of its tiles, 5 without an epilogue beside it.
 template <int ROW>  // bytes of a row: 64 or 128

@@ -338,12 +338,11 @@ int single_gemm(const void* x, const void* w, int rows, int n, int k, EpiArgs ea
   return launch_gemm<EPI>(tw, tx, p, ea, plan_gemm(n, k, r_tile, 148, EPI), st);
 }
 
-// ---- steps of more than 256 rows: gemm_wide.cuh ------------------------------------------------
-// Columns of a pair's tile.  A k block is taken to cost a pair 128 + bn parts of time (measured with one wave of 72 pairs: 0.20 us up to 128 columns,
-// 0.22 / 0.24 / 0.26 / 0.32 at 160 / 192 / 224 / 256: narrow tiles cost a little more than that, and less since they carry two k blocks per stage; of 71 shapes of 257 to
-// 4096 rows the rule then still picks the best width or one within 4 %), so the best bn is the one whose waves of tiles over the pairs cost least in all: 4000 x 1280 x 5120
-// takes 38.7 us on tiles of 160 columns (two waves of 74 pairs, 64 tiles each) and 55.8 us on 256 (80 tiles).  `unit`: columns that
-// one epilogue thread has to hold together (a head of a rotated projection, else 32).
+// ---- steps of more than 256 rows, and what takes_wide_up sends here: gemm_wide.cuh -----------------
+// Columns of a pair's tile.  A k block is taken to cost a pair 128 + bn parts of time (measured with one wave of 72 pairs: 0.20 us up to 128 columns, 0.22 / 0.24 / 0.26 / 0.32 at
+// 160 / 192 / 224 / 256, one k block per stage; tiles of up to 128 columns with two cost a third less, which the rule does not know), so the best bn is the one
+// whose waves of tiles over the pairs cost least in all: 4000 x 1280 x 5120 takes 38.7 us on tiles of 160 columns (two waves of 74 pairs, 64 tiles each) and
+// 55.8 us on 256 (80 tiles).  `unit`: columns that one epilogue thread has to hold together (a head of a rotated projection, else 32).
 int wide_tile_columns(int rows, int n, int unit, int pairs) {
   const int m_tiles = (rows + kPairRows - 1) / kPairRows;
   int best = 0;

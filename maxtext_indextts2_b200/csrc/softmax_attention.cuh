@@ -39,7 +39,7 @@
 //
 //   rope_append_kernel         per row: bias already in the projection; rotates q and k, writes q, appends k and v to the pages
 //   qk_prepare_append_kernel   the same with the optional head norms, either pairing, and layers that append nothing
-//   qk_rotate_append_kernel    both for bf16 heads without norms, eight channels per thread
+//   qk_rotate_append_kernel    both for bf16 rows that QkRotatePlan takes (pairs of neighbours; heads of 64, 128 or 256 channels where they have norms), eight channels per thread
 //   pool_append_kernel         per row that completes a block: the means of the block's cached keys and values into the pooled pools
 //   softmax_attention_rows_kernel<T>   one CTA per (query tile of <= 16 rows of one sequence, query head); keys walked in tiles
 //                              staged as fp32 in shared memory; running maximum and sum per row; everything fp32 (T is only the
