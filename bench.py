@@ -1,5 +1,5 @@
 #!/usr/bin/env python3
-"""Decode-step benchmark: audio tokens/s at batch 64 on the IndexTTS2-scale model (BASELINE.json).
+"""Decode-step benchmark: audio tokens/s at batch 64 on the IndexTTS2-scale model.
 
   python bench.py --gpus N --steps K --warmup W            # this repo's CUDA path
   python bench.py --impl reference --gpus N --steps K ...   # the reference decode arithmetic on the host CPU
@@ -8,7 +8,7 @@ One "step" = one autoregressive decode step (MaxEngine.generate) for `batch` slo
 `batch` audio tokens per GPU.  Work is partitioned by request batch: every rank owns `batch` slots
 and a full weight replica; there is no data-path collective (weak scaling).
 
-Workload (SURVEY 8d, config C2): 24 layers, emb 1280, 20/4 heads x 64, mlp 5120, vocabulary 264,192
+Workload: 24 layers, emb 1280, 20/4 heads x 64, mlp 5120, vocabulary 264,192
 (text + audio codec tokens), bf16, P = 1024, T = 3072, contexts uniform in [512, 1536] (seed 7),
 random-init weights, random-normal KV fill (synthetic).
 """
@@ -50,13 +50,13 @@ def parse_args():
   ap.add_argument("--layers", type=int, default=0, help="override base_num_decoder_layers (e.g. gemma3-27b geometry with 12 of its 62 layers)")
   ap.add_argument("--context-min", type=int, default=512)
   ap.add_argument("--context-max", type=int, default=1536)
-  ap.add_argument("--prefill-len", type=int, default=0, help="override max_prefill_predict_length (BASELINE configs[3]: 4096)")
-  ap.add_argument("--target-len", type=int, default=0, help="override max_target_length (BASELINE configs[3]: 5632)")
+  ap.add_argument("--prefill-len", type=int, default=0, help="override max_prefill_predict_length (long prompts: 4096)")
+  ap.add_argument("--target-len", type=int, default=0, help="override max_target_length (long prompts: 5632)")
   ap.add_argument("--no-graph", action="store_true")
-  ap.add_argument("--kv-int8", action="store_true", help="quantize_kvcache=True, kv_quant_dtype=int8, kv_quant_axis=dkv (SURVEY 8f-2; not the judged line)")
+  ap.add_argument("--kv-int8", action="store_true", help="quantize_kvcache=True, kv_quant_dtype=int8, kv_quant_axis=dkv (not the headline)")
   ap.add_argument("--kv-fp8", action="store_true", help="quantize_kvcache=True, kv_quant_dtype=fp8 (float8_e4m3fn bytes)")
   ap.add_argument("--kv-axis", default="dkv", choices=["dkv", "heads_and_dkv"], help="kv_quant_axis of --kv-int8 / --kv-fp8")
-  ap.add_argument("--paged", type=int, default=0, help="attention=paged with this many tokens per page (SURVEY 8f-4; not the judged line): "
+  ap.add_argument("--paged", type=int, default=0, help="attention=paged with this many tokens per page (not the headline): "
                   "the page manager runs on the host before every step and its state is uploaded, inside the timed region")
   ap.add_argument("--no-fold", action="store_true", help="keep the RMSNorm scales out of the weights (fold_norm_scales=False)")
   ap.add_argument("--skip-cpu-baseline", action="store_true")
@@ -64,7 +64,7 @@ def parse_args():
   ap.add_argument("--cpu-steps", type=int, default=8, help="timed steps of the cpu_baseline leg of the GPU arm (after 2 warm-ups)")
   ap.add_argument("--cpu-budget-s", type=float, default=150.0, help="wall-clock bound of a CPU leg; steps are cut (and reported) past it")
   ap.add_argument("--no-verify", action="store_true", help="skip the oracle check of one step of the timed state")
-  ap.add_argument("--prompt-len", type=int, default=4000, help="--mode prefill: prompt tokens (BASELINE configs[3]: 4000 of P = 4096)")
+  ap.add_argument("--prompt-len", type=int, default=4000, help="--mode prefill: prompt tokens (4000 of P = 4096)")
   ap.add_argument("--size", default="all", help="--mode layered: one of the sizes of LAYERED_SIZES, or all")
   ap.add_argument("--design", default="kifusun", choices=["kifusun", "gugidra", "ginodra", "ligidra", "fibelix", "zakelorn"], help="--mode layered: the layered design that is measured beside gemma3")
   ap.add_argument("--mode", default="batch", choices=["batch", "vocab-parallel", "prefill", "layered"],
@@ -72,7 +72,7 @@ def parse_args():
                        "the logits projection is sharded over the GPUs and one NCCL all-gather carries the per-shard candidates")
   ap.add_argument("--sampling", default="greedy", choices=["greedy", "weighted", "topk", "nucleus"], help="decode_sampling_strategy")
   ap.add_argument("--scaling", default="weak", choices=["weak", "strong"],
-                  help="weak: --batch slots per GPU (default, the judged line); strong: --batch slots in total, split over the GPUs")
+                  help="weak: --batch slots per GPU (default, the headline); strong: --batch slots in total, split over the GPUs")
   return ap.parse_args()
 
 
@@ -113,7 +113,7 @@ def context_lengths(args, cfg, rank=0):
 
 
 def algorithmic_bytes(cfg, batch, ctx_sum, ctx_sum_local=None):
-  """weights once + valid KV rows + KV append + embedding rows + outputs.  `ctx_sum_local`: rows a sliding-window
+  """Weights once + valid KV rows + KV append + embedding rows + outputs.  `ctx_sum_local`: rows a sliding-window
   layer reads (gemma3: five layers of six); the global layers read `ctx_sum`."""
   E, Hq, Hkv, D = cfg.emb_dim, cfg.num_query_heads, cfg.num_kv_heads, cfg.head_dim
   M, V, L = cfg.mlp_dim, cfg.vocab_size, cfg.num_decoder_layers
@@ -211,7 +211,7 @@ class ClockSampler:
 def cpu_reference_run(args, cfg, slots, steps, warmup, budget_s):
   """Times oracle/decode_ref.py (dtype-faithful restatement of MaxEngine.generate) on `slots` slots of the workload.
 
-  The reference's own JAX path cannot run here (no jax in the image); BASELINE.md section 4.  Weights and cache are
+  The reference's own JAX path cannot run here (no jax here).  Weights and cache are
   random (one random layer repeated: the values do not matter for the time, only shapes and dtypes do)."""
   from oracle import decode_ref as ref
   from oracle import mirror
@@ -317,8 +317,8 @@ def workload_config(args, cfg, world=None):
   world = world or args.gpus
   per_gpu = args.batch // world if args.scaling == "strong" else args.batch
   return {
-      "workload": (f"IndexTTS2-scale text-to-semantic GPT decode step (BASELINE configs[1])" if cfg.decoder_block == "llama2" else
-                   f"{cfg.model_name} geometry, gemma3 block (not a BASELINE config), decode step") +
+      "workload": (f"IndexTTS2-scale text-to-semantic GPT decode step" if cfg.decoder_block == "llama2" else
+                   f"{cfg.model_name} geometry, gemma3 block, decode step") +
                   f": L={cfg.num_decoder_layers} E={cfg.emb_dim} "
                   f"Hq={cfg.num_query_heads} Hkv={cfg.num_kv_heads} D={cfg.head_dim} M={cfg.mlp_dim} V={cfg.vocab_size}, greedy",
       "batch_per_gpu": per_gpu,
@@ -391,7 +391,7 @@ def verify_step(engine, dparams, cfg, B):
   """Correctness gate of the timed run: ONE more decode step of the state the benchmark just timed, replayed for four slots
   through the CPU oracle (as the reference; weights downloaded from the device, KV rows of those slots mirrored).  The GPU's
   greedy token must be the dtype-faithful oracle's argmax, or differ from it only at a near-tie (fp32-oracle margin between the
-  two candidates in bf16 ulps of the top logit is reported; SURVEY 8c)."""
+  two candidates in bf16 ulps of the top logit is reported)."""
   from oracle import mirror
 
   slots = sorted({0, B // 3, (2 * B) // 3, B - 1})
@@ -424,8 +424,8 @@ def verify_step(engine, dparams, cfg, B):
 
 def run_vocab_parallel(args, world, rank, local_rank):
   """--mode vocab-parallel: every rank decodes the same `batch` slots (weights of the layers and the KV cache replicated), rank r
-  scores vocabulary rows [r V/N, (r+1) V/N) and ONE NCCL all-gather per step carries the candidates (BASELINE
-  configs[4]).  Strong scaling of the logits projection only: the whole-job throughput is `batch` tokens per step."""
+  scores vocabulary rows [r V/N, (r+1) V/N) and ONE NCCL all-gather per step carries the candidates.
+  Strong scaling of the logits projection only: the whole-job throughput is `batch` tokens per step."""
   import torch.distributed as dist
 
   from maxtext_indextts2_b200 import maxengine
@@ -528,9 +528,9 @@ def run_vocab_parallel(args, world, rank, local_rank):
 
 
 def run_prefill(args):
-  """--mode prefill: MaxEngine.prefill of one `--prompt-len`-token prompt (BASELINE configs[3]: the 4k text + reference-audio prompt,
+  """--mode prefill: MaxEngine.prefill of one `--prompt-len`-token prompt (the 4k text + reference-audio prompt,
   timed separately from the decode steps), in passes of up to 4096 rows through the tcgen05 GEMMs and the causal attention
-  kernel, then MaxEngine.insert into slot 0.  Not the main metric: a second line for profiles/."""
+  kernel, then MaxEngine.insert into slot 0.  Not the headline: a second line for profiles/."""
   from maxtext_indextts2_b200 import maxengine
 
   if not args.prefill_len:
@@ -564,7 +564,7 @@ def run_prefill(args):
   gemm_flops = 2.0 * n * L * (E * Hq * D + 2 * E * Hkv * D + Hq * D * E + 3 * E * M)
   attn_flops = 4.0 * (n * (n + 1) / 2) * L * Hq * D
   line = {
-      "metric": "prefill ms for one prompt (BASELINE configs[3], timed separately from decode)",
+      "metric": "prefill ms for one prompt (timed separately from decode)",
       "mode": "prefill",
       "value": pre_ms / steps,
       "unit": "ms",
@@ -584,7 +584,7 @@ def run_prefill(args):
 
 
 # --mode layered: layer geometries that resemble real models (width, heads, kv heads, head size, ff, window, layers, vocab, prompt,
-# decode batch, decode context).  Random weights; a second line for DESIGN.md, not the main metric.
+# decode batch, decode context).  Random weights; a second line beside the headline.
 LAYERED_SIZES = {
     "1b": dict(width=2048, heads=16, kv_heads=4, dim=128, ff=8192, window=1024, layers=4, vocab=32768, prompt=4096, batch=64, context=2048),
     "4b": dict(width=2560, heads=8, kv_heads=4, dim=256, ff=10240, window=1024, layers=4, vocab=32768, prompt=4096, batch=64, context=2048),

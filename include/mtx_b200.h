@@ -14,7 +14,7 @@
  *   - `stream` is a cudaStream_t; all work is enqueued on it, nothing synchronises;
  *   - return value: 0 = ok, otherwise an MTX_ERR_* code; mtx_last_error() gives the text;
  *   - no exceptions cross the ABI; functions are re-entrant per engine, an engine is
- *     used from one host thread at a time (as MaxEngine is, SURVEY 8b "Threading");
+ *     used from one host thread at a time (as MaxEngine is);
  *   - there is no CPU fallback: without a CUDA device every compute call fails.
  *
  * "rows": the independent sequences one call advances by one token -- the decode slots
@@ -100,8 +100,8 @@ typedef struct {
                                         0: as many as run best, up to 4096 */
 } mtx_model_config;
 
-/* Weights, repacked once at load time for K-major streaming (see DESIGN.md "Data layout").
- * All bfloat16.  Relation to the reference parameter tree ("Checkpoint / resume"):
+/* Weights, repacked once at load time for K-major streaming.
+ * All bfloat16.  Relation to the reference parameter tree:
  *   wqkv[l]  [ (Hq+2Hkv)*D, E ]  rows = query|key|value kernels transposed (attentions.py:1894-2030)
  *   wo[l]    [ E, Hq*D ]         out kernel transposed
  *   w01[l]   [ 2*M, E ]          wi_0 / wi_1 transposed and interleaved in groups of 16 rows:
@@ -210,7 +210,7 @@ int mtx_decode_step_host(mtx_engine* e, int rows, const int32_t* tokens_host, in
  * stream: result_host is valid on return. */
 int mtx_decode_step_host_sync(mtx_engine* e, int rows, const int32_t* tokens_host, int32_t* result_host, float* log_prob_host, mtx_stream stream);
 
-/* Vocab-parallel logits (SURVEY 8e): this process holds `vocab_size` rows of the logits matrix starting
+/* Vocab-parallel logits: this process holds `vocab_size` rows of the logits matrix starting
  * at `vocab_offset`.  mtx_decode_step_candidates runs the whole step but, instead of committing a token,
  * writes this shard's winner per row to candidates[5][rows] (fp32: score, vocab id as int bits, its
  * logit, shard max, shard sum exp) -- the payload of ONE all-gather.  mtx_commit_candidates takes the
@@ -282,7 +282,7 @@ int mtx_rmsnorm(const void* x, const void* scale, void* out, int rows, int emb_d
  * weight tile; the partial tiles are reduced over distributed shared memory. */
 int mtx_linear(const void* x, const void* w, void* out, int rows, int n, int k, int splits, mtx_stream stream);
 
-/* The two remaining fused blocks of a decoder layer as single ops (SURVEY 8b), on the GEMM kernels of the per-kernel path.  `rows`
+/* The two remaining fused blocks of a decoder layer as single ops, on the GEMM kernels of the per-kernel path.  `rows`
  * 1..256; activation inputs must be allocated with the rows rounded up to 16/32/64/128/256, as for mtx_linear.
  *
  * Attention.out + the residual add (attentions.py:2017-2030 `out_projection`, llama2.py:139-140):
@@ -700,7 +700,7 @@ int mtx_sample_rows(const float* logits, int rows, long long ld, int vocab, int 
 
 /* Measurement aid: grid-barrier timeline of the persistent step kernel.  While a device buffer of
  * mtx_step_trace_words() 64-bit words is installed with mtx_debug_set_trace, every CTA records
- * %globaltimer at the arrival at and the release from each grid barrier (see tools/mega_trace.py). */
+ * %globaltimer at the arrival at and the release from each grid barrier. */
 size_t mtx_step_trace_words(const mtx_engine* e); /* sized for the engine's grid and layer count (NULL: 148 CTAs, 24 layers) */
 
 /* 1 when the library was built with jaxlib's headers and exports the XLA FFI handler symbols of csrc/mtx_jax_ffi.cc

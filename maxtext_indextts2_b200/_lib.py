@@ -270,7 +270,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
   if not force and not needs_build():
     return LIB_PATH
   nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
-  defines = ["-D" + d for d in os.environ.get("MTX_NVCC_DEFINES", "").split() if d]  # e.g. MTX_PK_EVENTS for tools/mega_trace.py
+  defines = ["-D" + d for d in os.environ.get("MTX_NVCC_DEFINES", "").split() if d]  # e.g. MTX_PK_EVENTS: the persistent step's event log
   os.makedirs(os.path.join(CSRC, "_build"), exist_ok=True)
   flags = [f for f in NVCC_FLAGS if f != "--shared"] + defines + _jaxlib_include() + (["-Xptxas", "-v"] if verbose else [])
   procs = []
@@ -425,7 +425,7 @@ def check(rc: int) -> None:
     return
   msg = last_error()
   if rc in (MTX_ERR_ARG, MTX_ERR_UNSUPPORTED):
-    raise ValueError(msg)  # the reference raises ValueError for bad config / sampling (SURVEY 8b "Errors")
+    raise ValueError(msg)  # the reference raises ValueError for bad config / sampling
   raise RuntimeError(msg)
 
 

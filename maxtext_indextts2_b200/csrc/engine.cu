@@ -556,7 +556,7 @@ bool pk_fill_phase(std::vector<PkTable>& tabs, int ph, int n, int k, bool allow_
   return true;
 }
 
-// Barrier slots of the step trace: 200 (the layout tools/ were written for) or what the layer count needs.
+// Barrier slots of the step trace: 200 (a fixed layout for readers of the trace) or what the layer count needs.
 int pk_trace_bars(int layers) { return 2 + 5 * layers + 2 > 200 ? 2 + 5 * layers + 2 : 200; }
 
 bool pk_usable(const mtx_engine* e, int rows) {

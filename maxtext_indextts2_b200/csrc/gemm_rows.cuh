@@ -1,5 +1,4 @@
-// Dense GEMM for steps of 65..256 rows (batch 128 / 256 decode, prefill chunks): the tensor-core regime of
-// BASELINE configs[2].
+// Dense GEMM for steps of 65..256 rows (batch 128 / 256 decode, prefill chunks): the tensor-core regime.
 //
 //   acc[r, n] = sum_k X[r, k] * W[n, k]        r in a 128-row block of the step's rows (UMMA M = 128),
 //                                               n in a 128-row tile of the weight matrix (UMMA N = 128)
@@ -26,7 +25,7 @@
 //     before griddepcontrol.wait) overlap this kernel's reduction.
 //
 // Per k-block a CTA ingests 16 KB of weights and rows x 128 B of activations (TMA, SWIZZLE_128B); an SM ingests
-// at most ~64 GB/s (profiles/r1f_tma_stream_subset.txt), which bounds the kernel at 256 rows (DESIGN.md).
+// at most ~64 GB/s (profiles/r1f_tma_stream_subset.txt), which bounds the kernel at 256 rows.
 #pragma once
 
 #include "gemm_umma.cuh"

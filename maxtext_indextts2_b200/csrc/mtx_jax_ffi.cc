@@ -6,7 +6,7 @@
 //
 // (maxtext_indextts2_b200/jax_ffi.py does the registration; INTEGRATION.md shows where MaxText calls it.)
 //
-// The reference has no FFI of its own (SURVEY 8b); the handler signatures follow the Python-level seams it does have:
+// The reference has no FFI of its own; the handler signatures follow the Python-level seams it does have:
 //   MtxRaggedAttention  -- AttentionOp.gpu_ragged_attention (MaxText/layers/attentions.py:761-815): (q, k, v, lengths) ->
 //                          (unnormalised out, max, sum), merged by the caller (attentions.py:1454-1464)
 //   MtxDecodeAttention  -- AttentionOp.__call__ in autoregressive mode over this library's two-segment cache

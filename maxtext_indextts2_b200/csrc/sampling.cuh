@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(kSampleThreads) pick_rows_kernel(const SampleA
 
 
 // =============================================================================================================
-// Vocab-parallel top-k / nucleus (SURVEY 8e): every shard extracts its kCandK best logits per row, ONE all-gather
+// Vocab-parallel top-k / nucleus: every shard extracts its kCandK best logits per row, ONE all-gather
 // carries them (kCandFloats floats per row and shard), every rank runs the same final selection.
 //
 //   top-k   : exact for k <= kCandK (the global top-k is a subset of the union of the shards' top-k).
@@ -1027,7 +1027,7 @@ __global__ void __launch_bounds__(kParThreads, 4) par_scan_kernel(const ParSampl
   }
 }
 
-// Vocab-parallel top-k / nucleus (SURVEY 8e): this shard's kCandK best logits of every row as (value, global id) pairs in
+// Vocab-parallel top-k / nucleus: this shard's kCandK best logits of every row as (value, global id) pairs in
 // any order, plus the shard's (max, sum exp) -- what shard_topk_kernel produces with one CTA per row, here from the radix
 // descent above with top_k = kCandK.  The kept set is exactly par_scan_kernel's (cut-off key, ties by index); a kept entry
 // takes the next free slot of its row (the merge on the gathered candidates, commit_topk_kernel, orders by value and id).

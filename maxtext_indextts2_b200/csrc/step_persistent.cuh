@@ -15,7 +15,7 @@
 // RMSNorm is never a phase of its own: the epilogue that produces x (or h) also emits per-row partial
 // sums of squares; the consuming GEMM is computed as rstd[row] * dot(W, bf16(x * scale)): the per-feature
 // scale is applied to the activation k-blocks in shared memory, the per-row factor to the fp32
-// accumulator in the epilogue (normalizations.py:57-69 rounds x * rstd to bf16 first; see DESIGN.md 4.1).
+// accumulator in the epilogue (normalizations.py:57-69 rounds x * rstd to bf16 first).
 //
 // GEMM work tables are built on the host (engine.cu, pk_fill_phase).  CTAs that share a weight tile
 // exchange fp32 partial tiles through an L2-resident workspace WITHOUT flags: a word of a slot is either
@@ -175,7 +175,7 @@ __device__ __forceinline__ PkEv pk_ev_make(const PkParams& p, int role) {
   return e;
 }
 __device__ __forceinline__ void pk_ev(PkEv& e, int id) {
-#ifdef MTX_PK_EVENTS  // per-role event log (tools/mega_trace.py); compiled out by default to keep the kernel small
+#ifdef MTX_PK_EVENTS  // per-role event log; compiled out by default to keep the kernel small
   if (e.base != nullptr && e.on && e.n < 32 && (!e.brief || id == 610 || id == 501)) {
     e.base[2 * e.n] = id;
     e.base[2 * e.n + 1] = (long long)globaltimer_ns();

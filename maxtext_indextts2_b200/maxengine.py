@@ -120,7 +120,7 @@ def fold_norm_scales(dp: DeviceParams) -> DeviceParams:
   ``rstd * dot(x, bf16(scale * W))`` is the same product with the per-feature factor rounded into the weight instead of
   into the activation (one bf16 rounding per term either way; the difference is measured by the parity tests, which
   keep the oracle on the UNFOLDED weights).  What it buys: the decode step no longer touches the activation tiles
-  between their arrival and the MMA (DESIGN.md 4.1).  When every scale is exactly 1 (random init) this is the identity
+  between their arrival and the MMA.  When every scale is exactly 1 (random init) this is the identity
   and nothing is copied."""
   if dp.folded:
     return dp
@@ -822,8 +822,7 @@ class MaxEngine:
   # -- helpers for tests / benchmarks ----------------------------------------------------------
 
   def fill_synthetic_context(self, prefill_lengths, ar_lengths, seed: int = 7) -> dict:
-    """Benchmark set-up: random-normal K/V and per-slot context lengths without running prefill
-    (SURVEY 8d "random-normal bf16 fill allowed for pure bandwidth runs")."""
+    """Benchmark set-up: random-normal K/V and per-slot context lengths without running prefill."""
     cfg = self.config
     B = self.max_concurrent_decodes
     P, R = cfg.max_prefill_predict_length, cfg.max_target_length - cfg.max_prefill_predict_length

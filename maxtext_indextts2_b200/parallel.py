@@ -1,6 +1,6 @@
 """Multi-GPU plumbing of the decode path: one process per GPU, ``torch.distributed`` for rendezvous.
 
-Two ways to use N GPUs (SURVEY 8e):
+Two ways to use N GPUs:
 
 * **Batch-partitioned (default).**  Every rank owns ``per_device_batch_size`` slots, a full weight
   replica and its own KV cache; rows never interact inside a step, so there is NO collective on the

@@ -1,6 +1,6 @@
 """Parameter tree of the llama2-style decoder (and of the gemma3 block), with the reference's names and shapes.
 
-Tree (unscanned layout; SURVEY 5 "Checkpoint / resume", names from
+Tree (unscanned layout; names from
 MaxText/layers/models.py:69, llama2.py:79,102,139, attentions.py:1865-1869,
 linears.py:347,373,388, decoders.py:544,573)::
 

@@ -5,7 +5,7 @@ THIS IS TEST INFRASTRUCTURE, NOT PRODUCT CODE.  Only ``tests/``,
 ``bench.py`` may import it; the product package never does and has no CPU path.
 
 What it restates (file:line are relative to the reference tree
-HyperBlaze456/maxtext-indextts2; the recipe is SURVEY.md Appendix A):
+HyperBlaze456/maxtext-indextts2):
 
 * one decode step        MaxText/maxengine.py:868-936  (``_generate_jit``)
 * decode-state layout     MaxText/maxengine.py:1370-1427

@@ -6,7 +6,7 @@ THIS IS TEST INFRASTRUCTURE, NOT PRODUCT CODE (see the header of ``decode_ref.py
 
 Rows (decode slots) never interact inside a step (attentions.py:587-588 masks per slot), so an
 oracle holding a SUBSET of the engine's slots, with the same shared ring index, reproduces those
-slots exactly.  That keeps the CPU side of a parity check at BASELINE scale (24 layers, V = 264,192,
+slots exactly.  That keeps the CPU side of a parity check at full scale (24 layers, V = 264,192,
 P = 1024 / T = 3072 and larger) to seconds per step.
 """
 
@@ -161,8 +161,8 @@ def bf16_ulp(x: float) -> float:
 
 
 def classify_mismatch(row_f32: torch.Tensor, got: int, want: int) -> dict:
-  """A greedy mismatch judged on the fp32 oracle's logits of that row (SURVEY 8c): the margin between the
-  two candidates in bf16 ulps of the top logit.  `strict` = SURVEY's rule (below one ulp)."""
+  """A greedy mismatch judged on the fp32 oracle's logits of that row: the margin between the
+  two candidates in bf16 ulps of the top logit.  `strict`: below one ulp."""
   top = float(row_f32.max())
   margin = abs(float(row_f32[want]) - float(row_f32[got]))
   ulp = bf16_ulp(top)

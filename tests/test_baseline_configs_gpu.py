@@ -1,4 +1,4 @@
-"""Oracle parity ON THE BASELINE CONFIGURATIONS THEMSELVES (BASELINE.json configs[1..3]).
+"""Oracle parity on the full-size configurations themselves.
 
 The engine runs the full configuration (24 layers, E = 1280, 20/4 heads x 64, M = 5120, V = 264,192; all slots), the
 CPU oracle follows in lock step on the same weights (downloaded from the device) and the same KV cache
@@ -15,15 +15,14 @@ Stated tolerances
 * logits vs the fp32 oracle: ``|d| <= 2^-5 max|logit|``;
 * greedy ids: equal to the faithful oracle's, except where the fp32 oracle's margin between the two candidates is
   within twice the measured logit error of that row (+ one bf16 ulp of the top logit): a near-tie.  Every mismatch
-  is also classified by SURVEY 8c's strict rule (fp32 margin below ONE bf16 ulp of the top logit); the counts and
-  margins are written to ``gpurun_out/parity_stats.jsonl`` and summarised in profiles/ and DESIGN.md.  With 264,192
+  is also classified by the strict rule (fp32 margin below ONE bf16 ulp of the top logit); the counts and
+  margins are printed.  With 264,192
   random-init logits per row near-ties are frequent: the two ORACLES (faithful vs fp32, both CPU) pick different tokens
   on ~5 % of the rows, so the rate bound is stated relative to that: the CUDA path may disagree with the faithful
   oracle at most twice as often as the faithful oracle disagrees with the fp32 one.
 """
 
 import json
-import os
 
 import numpy as np
 import pytest
@@ -35,17 +34,8 @@ from oracle import mirror
 
 pytestmark = pytest.mark.gpu
 
-ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-
 
 def _record(name, stats):
-  out = os.path.join(ROOT, "gpurun_out")
-  try:
-    os.makedirs(out, exist_ok=True)
-    with open(os.path.join(out, "parity_stats.jsonl"), "a", encoding="utf-8") as f:
-      f.write(json.dumps({"test": name, **stats}) + "\n")
-  except OSError:
-    pass
   print(name, json.dumps(stats))
 
 
@@ -134,7 +124,7 @@ def _lockstep(cfg, prefill, ar, slots, steps, name, with_f32=True, expect_launch
 
 
 def test_headline_batch64_full_scale_against_the_oracle():
-  """BASELINE configs[1] / SURVEY C2, the configuration bench.py times: batch 64, P = 1024, T = 3072, V = 264,192, contexts
+  """The configuration bench.py times: batch 64, P = 1024, T = 3072, V = 264,192, contexts
   uniform in [512, 1536] (seed 7), persistent step kernel (3 launches per step), all 64 slots in both oracles."""
   cfg = pyconfig.initialize(None, model_name="indextts2-t2s", per_device_batch_size=64, materialize_logits=True)
   prefill, ar = _contexts(64, 512, 1536, cfg.max_prefill_predict_length)
@@ -144,7 +134,7 @@ def test_headline_batch64_full_scale_against_the_oracle():
 
 @pytest.mark.parametrize("tokens_per_page", [32, 64])
 def test_headline_batch64_paged_against_the_oracle(tokens_per_page):
-  """The same configuration with attention=paged (SURVEY 8f-4; inference/page_manager.py, inference/paged_attention.py): 64 page
+  """The same configuration with attention=paged (inference/page_manager.py, inference/paged_attention.py): 64 page
   groups, pages of 32 / 64 tokens handed out by the page manager, the persistent step kernel reading the page table (3 launches
   per step).  The dense-cache oracles hold 12 of the slots, their rows gathered from the pools through the page map
   (oracle/mirror.py); six steps, so sequences cross page boundaries and get new pages."""
@@ -158,12 +148,12 @@ def test_headline_batch64_paged_against_the_oracle(tokens_per_page):
   slots = [0, 1, 3, 7, 16, 21, 31, 32, 42, 50, 62, 63]
   stats = _lockstep(cfg, prefill, ar, slots, steps=6, name=f"C2_batch64_paged{tokens_per_page}", expect_launches=lambda n: n == 3)
   # 72 tokens are too few for the rate bound of the 64-slot test above (there: 384 tokens); every mismatch has passed the
-  # near-tie rule inside _lockstep, and all but one must be near-ties by SURVEY 8c's strict rule (fp32 margin < 1 bf16 ulp)
+  # near-tie rule inside _lockstep, and all but one must be near-ties by the strict rule (fp32 margin < 1 bf16 ulp)
   assert stats["mismatch"] - stats["strict_near_tie"] <= 1 and stats["mismatch"] <= 8
 
 
 def test_batch256_context2048_against_the_oracle():
-  """BASELINE configs[2] / SURVEY C3: batch 256, every context 2048 (P = 1024 + 1024 ring rows), per-kernel path; the oracle
+  """Batch 256, every context 2048 (P = 1024 + 1024 ring rows), per-kernel path; the oracle
   follows 12 of the 256 slots (first, last and a spread)."""
   cfg = pyconfig.initialize(None, model_name="indextts2-t2s", per_device_batch_size=256, materialize_logits=True)
   prefill = np.full(256, 1024, dtype=np.int64)
@@ -175,7 +165,7 @@ def test_batch256_context2048_against_the_oracle():
 
 @pytest.mark.parametrize("batch", [1, 8])
 def test_long_prompt_config_against_the_oracle(batch):
-  """BASELINE configs[3] / SURVEY C4: P = 4096, T = 5632, prompt length 4000, part of the 1.5k-token decode already done
+  """P = 4096, T = 5632, prompt length 4000, part of the 1.5k-token decode already done
   (ring rows 100..1500): the persistent kernel's long-pair partition (one pair spans many CTAs) against the oracle."""
   cfg = pyconfig.initialize(None, model_name="indextts2-t2s", per_device_batch_size=batch, max_prefill_predict_length=4096,
                             max_target_length=5632, materialize_logits=True)
@@ -188,9 +178,9 @@ def test_long_prompt_config_against_the_oracle(batch):
 
 
 def test_near_tie_rate_tiny_config_320_greedy_steps():
-  """BASELINE configs[0] / SURVEY C1 model (4 layers, E = 256, V = 264,192, batch 1, greedy) decoded for 320 steps (ring of 320
+  """The tiny model (4 layers, E = 256, V = 264,192, batch 1, greedy) decoded for 320 steps (ring of 320
   rows after a 37-token prompt), both oracles in lock step: how often does the CUDA path pick another token than the faithful
-  oracle, and how many of those are near-ties by SURVEY 8c's strict rule?"""
+  oracle, and how many of those are near-ties by the strict rule?"""
   from oracle import decode_ref as ref
   from tests.helpers import make_params
 
@@ -244,7 +234,7 @@ def test_near_tie_rate_tiny_config_320_greedy_steps():
     [("topk", dict(decode_sampling_top_k=50)), ("nucleus", dict(decode_sampling_nucleus_p=0.9)), ("weighted", {})],
 )
 def test_sampling_at_the_expanded_vocabulary(strategy, kw):
-  """inference_utils.py:66-111 over the 264,192-entry vocabulary of BASELINE configs[1] (65 vocabulary slices per row in the
+  """inference_utils.py:66-111 over the 264,192-entry vocabulary (65 vocabulary slices per row in the
   all-SM sampler, the fused Gumbel-max epilogue for `weighted`): every step's token against the oracle's sampler on the SAME
   logits (the GPU's, so model noise plays no role) and the same Philox stream; a different token must be a near-tie of the
   perturbed scores, and must lie inside the oracle's candidate set."""

@@ -1,7 +1,7 @@
 """Engine-level parity on the B200: MaxEngine (CUDA) against the CPU oracle on the same
 random-init weights and synthetic prompts.
 
-Stated tolerances (SURVEY 8c):
+Stated tolerances:
 * logits vs the dtype-faithful oracle: rtol = atol = 1e-1, the reference's own ceiling
   (MaxText/tests/model_test.py:191);
 * logits vs the fp32 oracle: |d| <= 2^-5 * max|logit| (bf16 activations through the stack);
@@ -147,7 +147,7 @@ def test_late_insert_and_ring_wrap():
 
 
 def test_tiny_audio_config_greedy_64_steps():
-  """BASELINE config C1: MaxText decode.py-shaped run -- 4 layers, emb 256, audio-expanded vocabulary,
+  """MaxText decode.py-shaped run -- 4 layers, emb 256, audio-expanded vocabulary,
   batch 1, greedy, 37-token prompt (seed 1234), every one of the 64 decode steps compared."""
   cfg = pyconfig.initialize(None, model_name="tiny-audio", materialize_logits=True)
   params = make_params(cfg, perturb=False)
@@ -188,7 +188,7 @@ def test_weighted_sampling_follows_the_oracle_stream():
 
 
 def test_engine_api_shapes_and_errors():
-  """MaxText/tests/maxengine_test.py:111-164 (shapes / dtypes) and the error behaviour of SURVEY 8b."""
+  """MaxText/tests/maxengine_test.py:111-164 (shapes / dtypes) and the error behaviour."""
   cfg = small_config(per_device_batch_size=2)
   engine = maxengine.MaxEngine(cfg)
   dparams = engine.load_params()  # random init, as decode.py does without load_parameters_path
@@ -294,7 +294,7 @@ def test_topk_ties_keep_the_lowest_index():
 
 
 def test_indextts2_scale_logits_and_greedy_tokens():
-  """BASELINE config C2 shape (24 layers, emb 1280, 20/4 heads x 64, mlp 5120, V = 264,192) with short
+  """Full-size shape (24 layers, emb 1280, 20/4 heads x 64, mlp 5120, V = 264,192) with short
   P/T so the CPU oracle finishes in about a minute: prefill + 6 decode steps, 4 slots."""
   cfg = pyconfig.initialize(None, model_name="indextts2-t2s", per_device_batch_size=4, max_prefill_predict_length=64,
                             max_target_length=128, materialize_logits=True)

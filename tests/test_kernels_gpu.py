@@ -1,6 +1,6 @@
 """Op-level parity on the B200: each fused op, called through the C ABI, against the oracle.
 
-Tolerances (SURVEY 8c): attention |d| <= 2^-7 * max|out| against the fp32-score reference
+Tolerances: attention |d| <= 2^-7 * max|out| against the fp32-score reference
 (one bf16 output rounding + bf16 probabilities), and the reference's own ceiling
 rtol = atol = 1e-2 (MaxText/tests/attention_test.py:406); dense outputs within one bf16 ulp
 of the fp32-accumulated product.
@@ -148,7 +148,7 @@ def test_attention_kernels_test_shape():
 
 
 def test_attention_long_context_many_chunks():
-  # 4k prompt + 1.5k decoded (BASELINE config C4 lengths) for one kv head group
+  # 4k prompt + 1.5k decoded for one kv head group
   _attention_case(B=2, Hq=5, Hkv=1, D=64, P=4096, T=5632, len0=[4000, 4096], ring_first=[0, 1000], ring_len=[1536, 1536])
 
 

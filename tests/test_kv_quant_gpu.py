@@ -1,4 +1,4 @@
-"""int8 KV cache (SURVEY 8f-2; MaxText/inference/kvcache.py:36-90, 658-736; configs/base.yml:104-112) on the B200 against the
+"""int8 KV cache (MaxText/inference/kvcache.py:36-90, 658-736; configs/base.yml:104-112) on the B200 against the
 oracle with the same quantiser: quantize_kvcache=True, kv_quant_dtype=int8, kv_quant_axis=dkv (one scale per token and kv head)
 or heads_and_dkv (the reference's default: one scale per token over all kv heads).
 

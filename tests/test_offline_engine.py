@@ -1,4 +1,4 @@
-"""The callers either side of the decode step (SURVEY 8f-4): the audio-id wire format (CPU) and the continuous-batching loop
+"""The callers either side of the decode step: the audio-id wire format (CPU) and the continuous-batching loop
 (GPU) that mirrors MaxText/inference/offline_engine.py:473-715."""
 
 import json

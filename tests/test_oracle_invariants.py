@@ -1,6 +1,6 @@
 """Pins the CPU oracle with the reference's own invariants for the decode path.
 
-The reference stores no golden vectors for this path (SURVEY 8c); its tests compare
+The reference stores no golden vectors for this path; its tests compare
 the model with itself.  Each test here restates one of them against ``oracle/``:
 
 * AR steps == full-sequence forward    MaxText/tests/attention_test.py:361-406 (1e-2),

@@ -53,7 +53,7 @@ def _random_pages(rng, lengths, tpp, num_pages, max_pages):
         (5, 16, 2, 64, 64, [64, 1, 127, 128, 3000]),     # page = tile
         (4, 20, 4, 64, 128, [5, 128, 129, 1500]),        # a tile is half a page
         (3, 8, 2, 128, 32, [31, 100, 900]),              # head_dim 128 (two 64-wide sub-tiles per box)
-        (64, 20, 4, 64, 32, None),                       # batch 64, lengths 512..1536 (BASELINE configs[1] contexts)
+        (64, 20, 4, 64, 32, None),                       # batch 64, lengths 512..1536
     ],
 )
 def test_paged_attention_matches_oracle(B, Hq, Hkv, D, tpp, lengths):
