@@ -286,8 +286,9 @@ RowsPlan plan_rows(int n, int k, int r_tile, int num_sms, int epi, int forced_sp
 // Whether a decode step's gated up-projection whose K that plan leaves whole takes the pair GEMM (WideEpi<EPI_SWIGLU, true>: the same bits).  The row-major GEMM has one CTA
 // per tile of 128 columns, the pair GEMM tiles as wide as the SMs ask for.  Whole steps, us, row-major / pair: more than 128 rows (a second block of rows for each of its CTAs)
 // 200 rows of 1280 x 5120 579 / 549, of 2048 x 8192 521 / 506, of 4096 x 14336 854 / 805; up to 128 rows where the last wave of its tiles leaves two fifths of the SMs idle: 65 rows of 1280 x
-// 5120 (80 tiles) 486 / 464, of 2048 x 10240 (160) 324 / 308.  Beyond that line it is the slower one (128 tiles 391 / 398, 148 tiles 318 / 325) or no
-// faster (96 tiles 448 / 452, 224 tiles 536 / 537, means of 65 to 128 rows), and up to 64 rows its tiles are mostly padding (1 row 467 / 488, 33 rows 453 / 470, 64 rows 474 / 454).
+// 5120 (80 tiles) 486 / 464, of 2048 x 10240 (160) 324 / 308.  Beyond that line it is the slower one (128 rows: 128 tiles 391 / 398, 148 tiles 318 / 325) or no
+// faster (means of 65 to 128 rows: 96 tiles 450 / 454, 224 tiles 542 / 541).  Up to 64 rows three quarters of its tiles and more are padding, and it is now the slower and now
+// the faster one (1 row of 1280 x 5120 467 / 488, 16 rows 469 / 466, 33 rows 453 / 470, 64 rows 474 / 454): those steps stay where they were.
 bool takes_wide_up(int rows, const RowsPlan& pl, int num_sms) {
   if (rows <= 64 || pl.splits > 1) return false;
   const int waves = (pl.n_tiles + num_sms - 1) / num_sms;
