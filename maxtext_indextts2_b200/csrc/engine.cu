@@ -999,7 +999,7 @@ int enqueue_step(mtx_engine* e, int mode, int rows, const int32_t* chunk_tokens,
   // epilogues leave the row statistics, the consuming epilogues apply rstd; the per-kernel rmsnorm launches disappear)
   const bool fused_norm = rows_k && c.norm_scales_folded && (gemma3 || env_int("MTX_ROWS_FUSED_NORM", 1) != 0);
   // (gemma3's steps stay on the row-major GEMM: not timed on the other one)
-  const bool wide_up = fused_norm && !gemma3 && takes_wide_up(rows, plan_rows(2 * M, E, r_tile, e->num_sms, EPI_SWIGLU), e->num_sms) && env_int("MTX_ROWS_WIDE_UP", 1) != 0;
+  const bool wide_up = fused_norm && !gemma3 && takes_wide_up(rows, E, plan_rows(2 * M, E, r_tile, e->num_sms, EPI_SWIGLU), e->num_sms) && env_int("MTX_ROWS_WIDE_UP", 1) != 0;
   const int ss_tiles = (E + 127) / 128;
   auto ss_args = [&](EpiArgs& ea, const float* in, float* out) {
     ea.ss_in = fused_norm ? in : nullptr;

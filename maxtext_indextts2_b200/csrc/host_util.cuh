@@ -288,9 +288,11 @@ RowsPlan plan_rows(int n, int k, int r_tile, int num_sms, int epi, int forced_sp
 // 200 rows of 1280 x 5120 579 / 549, of 2048 x 8192 521 / 506, of 4096 x 14336 854 / 805; up to 128 rows where the last wave of its tiles leaves two fifths of the SMs idle: 65 rows of 1280 x
 // 5120 (80 tiles) 486 / 464, of 2048 x 10240 (160) 324 / 308.  Beyond that line it is the slower one (128 rows: 128 tiles 391 / 398, 148 tiles 318 / 325) or no
 // faster (means of 65 to 128 rows: 96 tiles 450 / 454, 224 tiles 542 / 541).  Up to 64 rows three quarters of its tiles and more are padding, and it is now the slower and now
-// the faster one (1 row of 1280 x 5120 467 / 488, 16 rows 469 / 466, 33 rows 453 / 470, 64 rows 474 / 454): those steps stay where they were.
-bool takes_wide_up(int rows, const RowsPlan& pl, int num_sms) {
-  if (rows <= 64 || pl.splits > 1) return false;
+// the faster one (1 row of 1280 x 5120 467 / 488, 16 rows 469 / 466, 33 rows 453 / 470, 64 rows 474 / 454): those steps stay where they were.  So do narrow layers (k below
+// 768): their down-projection's few clusters start on the SMs that the row-major tiles leave, which the pairs would take (24 layers of 512 x 5120, 128 rows, 1129 / 1204, the
+// up-projections in it 230 / 196 and the residual ones 389 / 504; of 256 x 4864, 160 rows, 1067 / 1147; 16 layers of 768 x 5120 852 / 874 and, 96 rows, 881 / 823).
+bool takes_wide_up(int rows, int k, const RowsPlan& pl, int num_sms) {
+  if (rows <= 64 || k < 768 || pl.splits > 1) return false;
   const int waves = (pl.n_tiles + num_sms - 1) / num_sms;
   return rows > 128 || pl.n_tiles * 5 <= waves * num_sms * 3;
 }

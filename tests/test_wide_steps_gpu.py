@@ -15,13 +15,13 @@ CACHES = {"bf16": {}, "int8": dict(quantize_kvcache=True, kv_quant_axis="dkv"), 
           "tokens": dict(quantize_kvcache=True, kv_quant_axis="heads_and_dkv"), "paged": dict(attention="paged", pagedattn_tokens_per_page=16)}
 
 
-def _step(cache, dim, rows, mlp=4864, fold=True, graph=True):
+def _step(cache, dim, rows, mlp=4864, fold=True, graph=True, emb=768):
   """The state behind one generated token per slot, and the names of the kernels that ran."""
   kw = dict(attention="dot_product")
   kw.update(CACHES[cache])
   if cache == "paged":
     kw["pagedattn_num_pages"] = 6 * rows + 1
-  cfg = pyconfig.initialize(None, base_num_decoder_layers=2, base_emb_dim=320, base_num_query_heads=6, base_num_kv_heads=2, head_dim=dim, base_mlp_dim=mlp, vocab_size=640,
+  cfg = pyconfig.initialize(None, base_num_decoder_layers=2, base_emb_dim=emb, base_num_query_heads=6, base_num_kv_heads=2, head_dim=dim, base_mlp_dim=mlp, vocab_size=640,
                             per_device_batch_size=rows, max_prefill_predict_length=48, max_target_length=80, weight_dtype="bfloat16", scan_layers=False,
                             materialize_logits=True, return_log_prob=True, decode_sampling_strategy="greedy", fold_norm_scales=fold, **kw)
   engine = maxengine.MaxEngine(cfg, use_cuda_graph=graph)
@@ -36,16 +36,17 @@ def _step(cache, dim, rows, mlp=4864, fold=True, graph=True):
   return dict(got, logits=state["logits"].clone()), {e.name for e in p.events()}
 
 
-@pytest.mark.parametrize("cache,dim,rows,mlp,wide", [
-    ("bf16", 64, 65, 4864, True), ("bf16", 128, 97, 4864, True), ("bf16", 64, 256, 4864, True), ("int8", 64, 129, 4864, True), ("int8", 64, 200, 4864, True),
-    ("fp8", 64, 255, 4864, True), ("tokens", 64, 161, 4864, True), ("paged", 64, 66, 4864, True), ("paged", 128, 224, 4864, True),
-    ("bf16", 64, 200, 9472, True),  # 148 tiles of 128 columns, more than 128 rows
-    ("bf16", 64, 70, 9472, False), ("tokens", 64, 64, 4864, False), ("tokens", 64, 1, 4864, False)])  # (a full wave; rows that fill a quarter of a tile)
-def test_up_projection_has_the_same_bits_on_either_gemm(cache, dim, rows, mlp, wide, monkeypatch):
+@pytest.mark.parametrize("cache,dim,rows,emb,mlp,wide", [
+    ("bf16", 64, 65, 768, 4864, True), ("bf16", 128, 97, 768, 4864, True), ("bf16", 64, 256, 768, 4864, True), ("int8", 64, 129, 768, 4864, True), ("int8", 64, 200, 768, 4864, True),
+    ("fp8", 64, 255, 768, 4864, True), ("tokens", 64, 161, 768, 4864, True), ("paged", 64, 66, 768, 4864, True), ("paged", 128, 224, 768, 4864, True),
+    ("bf16", 64, 200, 768, 9472, True),  # 148 tiles of 128 columns, more than 128 rows
+    ("bf16", 64, 70, 768, 9472, False), ("tokens", 64, 64, 768, 4864, False), ("tokens", 64, 1, 768, 4864, False),  # (a full wave; rows that fill a quarter of a tile)
+    ("bf16", 64, 200, 704, 4864, False), ("bf16", 64, 200, 832, 4864, True)])  # (narrow layers)
+def test_up_projection_has_the_same_bits_on_either_gemm(cache, dim, rows, emb, mlp, wide, monkeypatch):
   """Logits and caches of a step on the GEMM that the rule picks and on the row-major one (MTX_ROWS_WIDE_UP=0)."""
-  got, names = _step(cache, dim, rows, mlp, graph=False)
+  got, names = _step(cache, dim, rows, mlp, graph=False, emb=emb)
   monkeypatch.setenv("MTX_ROWS_WIDE_UP", "0")
-  want, plain = _step(cache, dim, rows, mlp, graph=False)
+  want, plain = _step(cache, dim, rows, mlp, graph=False, emb=emb)
   is_wide = lambda names: any("gemm_wide_kernel" in n for n in names)
   assert any("gemm_rows_kernel" in n for n in plain) and is_wide(names) == wide and not is_wide(plain)
   assert got.keys() == want.keys() and torch.isfinite(got["logits"]).all()
