@@ -118,6 +118,17 @@ struct WideStage {
   __device__ __forceinline__ void place(int n, const uint4 (&v)[kChunks]) const {
     each(n, 32, [&](int i, int r, int j) { *at(r, j) = v[i]; });
   }
+  // the same without registers in between: on its way when this returns, there for the warp behind arrived()
+  __device__ __forceinline__ void bring(int n, const void* p, size_t pitch, int rows) const {
+    each(n, rows, [&](int, int r, int j) {
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(at(r, j))), "l"(static_cast<const char*>(p) + r * pitch + j * 16) : "memory");
+    });
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  __device__ __forceinline__ void arrived() const {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
+  }
   // the buffer's chunks [0, n) of the first `rows` rows to p + r * pitch
   __device__ __forceinline__ void flush(int n, void* p, size_t pitch, int rows) const {
     __syncwarp();
@@ -371,7 +382,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     const int half = (warp - 2) >> 2, quarter = warp & 3;
     const int c0 = half == 0 ? 0 : p.first, c1 = half == 0 ? p.first : p.bn;
     if (!GROUPED) griddep_wait();  // side inputs (residual rows, row statistics) come from earlier kernels
-    const WideStage<EPI::kRowBytes> stage = {staged + (warp - 2) * 32 * EPI::kRowBytes, lane};
+    const typename EPI::Stage stage = {staged + (warp - 2) * 32 * EPI::kRowBytes, lane};
     int buf = 0;
     uint32_t acc_phase = 0;
     auto release = [&]() {  // this warp is done with the accumulator
@@ -494,15 +505,15 @@ __device__ __forceinline__ uint4 wide_pack8(const float* v) {
 template <int KIND, bool STEP = false>
 struct WideEpi {
   static constexpr bool kFragments = KIND == EPI_STORE_BF16 || KIND == EPI_SWIGLU;
-  static constexpr int kRowBytes = KIND == EPI_QKV_ROPE ? 128 : 64;
-  typedef WideStage<kRowBytes> Stage;
-  static constexpr int kPiece = kRowBytes / 2;  // bf16 columns of a staged row
+  static constexpr int kRowBytes = KIND == EPI_QKV_ROPE ? 192 : 64;  // (EPI_QKV_ROPE: 128 of angles, 64 of outputs)
+  typedef WideStage<KIND == EPI_QKV_ROPE ? 128 : 64> Stage;
+  static constexpr int kPiece = 32;  // bf16 columns of a staged row
   EpiArgs e;
 
   struct Pre {
     float rs;                                            // 1 / rms of the row
     int wr, plane;                                       // EPI_QKV_ROPE: its cache row and plane
-    uint4 v[KIND == EPI_RESIDUAL || KIND == EPI_QKV_ROPE ? Stage::kChunks : 1];  // the warp's next residuals, or cosines and sines
+    uint4 v[KIND == EPI_RESIDUAL ? Stage::kChunks : 1];  // the warp's next residuals
   };
 
   __device__ __forceinline__ const char* residuals(const WideTile& w, const Stage& st, int c) const {
@@ -523,7 +534,7 @@ struct WideEpi {
     if constexpr (KIND == EPI_QKV_ROPE) {
       p.wr = w.valid ? e.write_row[w.row] : -1;
       p.plane = w.valid ? e.plane[w.row] : 0;
-      st.fetch(8, angles(w, st, 0), size_t(e.d) * 4, w.rows, p.v);
+      st.bring(8, angles(w, st, 0), size_t(e.d) * 4, w.rows);
     }
     return p;
   }
@@ -582,11 +593,14 @@ struct WideEpi {
       if (e.ss_out != nullptr && w.valid) e.ss_out[(long long)w.slice * e.ss_pitch + w.row] = sq;
     } else if constexpr (KIND == EPI_QKV_ROPE) {
       // dims d .. d + 15 of a head's first half and the same of its second half (d + D / 2), of all the warp's heads: rotated queries, appended keys and values
+      // (The next angles come by asynchronous copies.  In registers, beside these, 140 bytes of a thread's spilled, and a single wave of narrow tiles, whose epilogue nothing
+      // hides, took longer than with angles loaded in place: 495 x 768 x 1472 10.3 us in place, 13.7 in registers, 10.3 so; 389 x 1792 x 1280 10.9, 11.5, 8.8;
+      // 4000 rows of it 30.8, 23.5, 20.4.)
       const int D = e.d, half = D >> 1;
+      const WideStage<64> outs = {st.buf + 32 * 128, st.lane};
+#pragma unroll 1
       for (int d = 0; d < half; d += 16) {
-        st.place(8, p.v);
-        if (d + 16 < half) st.fetch(8, angles(w, st, d + 16), size_t(D) * 4, w.rows, p.v);
-        __syncwarp();
+        st.arrived();
         float cs[32];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -594,6 +608,8 @@ struct WideEpi {
           cs[4 * j] = __uint_as_float(x.x), cs[4 * j + 1] = __uint_as_float(x.y), cs[4 * j + 2] = __uint_as_float(x.z), cs[4 * j + 3] = __uint_as_float(x.w);
         }
         __syncwarp();
+        if (d + 16 < half) st.bring(8, angles(w, st, d + 16), size_t(D) * 4, w.rows);
+#pragma unroll 1
         for (int h = w.c0; h < w.c1; h += D) {
           float a[16], b[16];
           load(h + d, a, h + d + half, b);
@@ -615,11 +631,11 @@ struct WideEpi {
             const int kvh = (head - e.hq) % e.hkv;
             dst = (head < e.hq + e.hkv ? e.k_cache : e.v_cache) + (((long long)p.plane * e.hkv + kvh) * e.t_alloc + p.wr) * D + d;
           }
-          st.put(0, wide_pack8(a));
-          st.put(1, wide_pack8(a + 8));
-          st.put(2, wide_pack8(b));
-          st.put(3, wide_pack8(b + 8));
-          st.flush_pairs(dst, half);
+          outs.put(0, wide_pack8(a));
+          outs.put(1, wide_pack8(a + 8));
+          outs.put(2, wide_pack8(b));
+          outs.put(3, wide_pack8(b + 8));
+          outs.flush_pairs(dst, half);
         }
       }
     }
