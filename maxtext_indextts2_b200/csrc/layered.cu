@@ -985,7 +985,7 @@ int launch_qk_prepare(const QkPrepareArgs<T>& qa, int rows, size_t smem, cudaStr
                     : dn == 64  ? qk_rotate_append_kernel<64, false>
                     : dn == 128 ? qk_rotate_append_kernel<128, false>
                                 : qk_rotate_append_kernel<256, false>,
-                    dim3(rows), dim3(256), 0, st, qa);
+                    dim3(rows), dim3(QkRotatePlan::threads(qa)), 0, st, qa);
     }
   return launch(qk_prepare_append_kernel<T>, dim3(rows), dim3(256), smem, st, qa);
 }
@@ -1014,7 +1014,7 @@ int launch_rope_append(const RopeAppendArgs<T>& ra, int rows, cudaStream_t st) {
     qa.num_pages = ra.num_pages;
     qa.tokens_per_page = ra.tokens_per_page;
     qa.max_pages = ra.max_pages;
-    if (QkRotatePlan::ok(qa)) return launch(qk_rotate_append_kernel<0, true>, dim3(rows), dim3(256), 0, st, qa);
+    if (QkRotatePlan::ok(qa)) return launch(qk_rotate_append_kernel<0, true>, dim3(rows), dim3(QkRotatePlan::threads(qa)), 0, st, qa);
   }
   return launch(rope_append_kernel<T>, dim3(rows), dim3(256), 0, st, ra);
 }

@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(256) qk_prepare_append_kernel(const QkPrepareA
   }
 }
 
-// The same in bf16 for heads whose channels come in eights: a thread takes eight channels of one head (or eight values), a CTA a row, 512 such pieces at a time, all of
+// The same in bf16 for heads whose channels come in eights: a thread takes eight channels of one head (or eight values), a CTA a row, two such pieces per thread at a time, all of
 // them requested before the row's angles are worked out.  The angles go by the position alone and are the row's, not its heads'.  Sums of squares are added up in
 // the order of qk_prepare_append_kernel, so that the bits are its own.
 // DN > 0: heads of DN = 64, 128 or 256 channels are brought to unit RMS first.  ROPE: the sums of a turned pair as rope_append_kernel has them (the other product is
@@ -250,6 +250,13 @@ struct QkRotatePlan {
     return !a.temp && !a.talk && !a.rot_half && !a.norm_whole && a.maps <= 1 && a.dim % 8 == 0 && a.dim <= 256 && a.vdim % 8 == 0 && a.rot_dims % 8 == 0 && a.rot_dims <= a.dim &&
            (!norms || (a.q_norm && a.k_norm && (a.dim == 64 || a.dim == 128 || a.dim == 256) && aligned(a.q_norm) && aligned(a.k_norm))) && a.ld % 4 == 0 && a.q_col % 4 == 0 &&
            a.k_col % 4 == 0 && a.v_col % 4 == 0 && aligned(a.proj) && aligned(a.q_out) && aligned(a.k_pages) && aligned(a.v_pages);
+  }
+  // A piece per thread in 128 threads where that takes the row: a CTA's way is the same, and twice as many rows are in flight.  2700 rows without norms, us, warp by warp / 256
+  // threads / 128: 24 pieces 5.3 / 8.1 / 4.7, 64 pieces 6.6 / 7.8 / 5.0, 128 pieces 9.8 / 7.6 / 5.1.  With two pieces per thread it is slower for few rows (256
+  // pieces, 300 rows 3.0, 3.8 in 128 threads).
+  static int threads(const QkPrepareArgs<bf16>& a) {
+    const int pieces = (a.heads * a.dim + (a.shared_kv ? 0 : a.kv_heads * (a.dim + a.vdim))) / 8;
+    return pieces <= 128 ? 128 : 256;
   }
 };
 
@@ -267,11 +274,12 @@ __global__ void __launch_bounds__(256) qk_rotate_append_kernel(const QkPrepareAr
   const int p = a.pos[r], grp = a.group[r];
   const size_t slot = size_t(a.page_map[size_t(grp) * a.max_pages + p / a.tokens_per_page]) * a.tokens_per_page + p % a.tokens_per_page;
   const size_t pool_rows = size_t(a.num_pages) * a.tokens_per_page;
-  for (int e0 = tid; e0 - tid < n; e0 += kPieces * 256) {
+  const int T = blockDim.x;
+  for (int e0 = tid; e0 - tid < n; e0 += kPieces * T) {
     float x[kPieces][8];
 #pragma unroll
     for (int i = 0; i < kPieces; ++i) {
-      const int e = e0 + i * 256;
+      const int e = e0 + i * T;
       if (e < n) {
         const float* src = row + (e < nq ? a.q_col + e * 8 : e < nq + nk ? a.k_col + (e - nq) * 8 : a.v_col + (e - nq - nk) * 8);
         const float4 lo = *reinterpret_cast<const float4*>(src), hi = *reinterpret_cast<const float4*>(src + 4);
@@ -291,7 +299,7 @@ __global__ void __launch_bounds__(256) qk_rotate_append_kernel(const QkPrepareAr
     }
 #pragma unroll
     for (int i = 0; i < kPieces; ++i) {
-      const int e = e0 + i * 256, u = e < nq ? e : e - nq, c = u % per * 8;  // c: the piece's first channel of its head
+      const int e = e0 + i * T, u = e < nq ? e : e - nq, c = u % per * 8;  // c: the piece's first channel of its head
       if (DN > 0 && e - lane < nq + nk) {  // (uniform in the warp; a head's pieces are neighbours in one)
         constexpr int HW = DN > 0 ? 256 / DN : 1;
         float* ch = channels[DN > 0 ? warp : 0];
