@@ -284,17 +284,19 @@ RowsPlan plan_rows(int n, int k, int r_tile, int num_sms, int epi, int forced_sp
 }
 
 // Whether a decode step's gated up-projection whose K that plan leaves whole takes the pair GEMM (WideEpi<EPI_SWIGLU, true>: the same bits).  The row-major GEMM has one CTA
-// per tile of 128 columns, the pair GEMM tiles as wide as the SMs ask for.  Whole steps, us, row-major / pair: more than 128 rows (a second block of rows for each of its CTAs)
-// 200 rows of 1280 x 5120 579 / 549, of 2048 x 8192 521 / 506, of 4096 x 14336 854 / 805; up to 128 rows where the last wave of its tiles leaves two fifths of the SMs idle: 65 rows of 1280 x
-// 5120 (80 tiles) 486 / 464, of 2048 x 10240 (160) 324 / 308.  Beyond that line it is the slower one (128 rows: 128 tiles 391 / 398, 148 tiles 318 / 325) or no
-// faster (means of 65 to 128 rows: 96 tiles 450 / 454, 224 tiles 542 / 541).  Up to 64 rows three quarters of its tiles and more are padding, and it is now the slower and now
-// the faster one (1 row of 1280 x 5120 467 / 488, 16 rows 469 / 466, 33 rows 453 / 470, 64 rows 474 / 454): those steps stay where they were.  So do narrow layers (k below
-// 768): their down-projection's few clusters start on the SMs that the row-major tiles leave, which the pairs would take (24 layers of 512 x 5120, 128 rows, 1129 / 1204, the
-// up-projections in it 230 / 196 and the residual ones 389 / 504; of 256 x 4864, 160 rows, 1067 / 1147; 16 layers of 768 x 5120 852 / 874 and, 96 rows, 881 / 823).
+// per tile of 128 columns, the pair GEMM tiles as wide as the SMs ask for.  Whole steps, us, row-major / pair:
+//  - more than 128 rows are a second block of rows for each of the row-major CTAs: 200 rows of 1280 x 5120 579 / 549, of 2048 x 8192 521 / 506, of 4096 x 14336 854 / 805;
+//  - up to 128 rows it is the faster one where the row-major tiles leave two fifths of the SMs without one: 65 rows of 1280 x 5120 (80 tiles) 486 / 464, 74 of 768 x 5632 (88) 440 / 421;
+//    with more tiles the slower one (128 rows: 128 tiles 391 / 398, 148 tiles 318 / 325) or no faster (means of 65 to 128 rows: 96 tiles 450 / 454, 224 tiles 542 / 541).  The
+//    same in the last of several waves, if K is long enough for its own second wave: 74 rows of 2048 x 10432 (163 tiles) 395 / 377, of 1280 x 10432 532 / 535, of 768 x 10432 481 / 513;
+//  - up to 64 rows three quarters of its tiles and more are padding, and it is now the slower and now the faster one (1 row of 1280 x 5120 467 / 488, 16 rows 469 / 466, 33 rows
+//    453 / 470, 64 rows 474 / 454): those steps stay where they were;
+//  - so do narrow layers (k below 768), whose down-projection's few clusters start on the SMs that the row-major tiles leave and the pairs would take: 24 layers of 512 x 5120, 128
+//    rows, 1129 / 1204 (up-projections 230 / 196, residual ones 389 / 504), of 256 x 4864, 160 rows, 1067 / 1147.
 bool takes_wide_up(int rows, int k, const RowsPlan& pl, int num_sms) {
   if (rows <= 64 || k < 768 || pl.splits > 1) return false;
   const int waves = (pl.n_tiles + num_sms - 1) / num_sms;
-  return rows > 128 || pl.n_tiles * 5 <= waves * num_sms * 3;
+  return rows > 128 || (pl.n_tiles * 5 <= waves * num_sms * 3 && (waves == 1 || k >= 2048));
 }
 
 template <int EPI>

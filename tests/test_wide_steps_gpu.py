@@ -41,7 +41,8 @@ def _step(cache, dim, rows, mlp=4864, fold=True, graph=True, emb=768):
     ("fp8", 64, 255, 768, 4864, True), ("tokens", 64, 161, 768, 4864, True), ("paged", 64, 66, 768, 4864, True), ("paged", 128, 224, 768, 4864, True),
     ("bf16", 64, 200, 768, 9472, True),  # 148 tiles of 128 columns, more than 128 rows
     ("bf16", 64, 70, 768, 9472, False), ("tokens", 64, 64, 768, 4864, False), ("tokens", 64, 1, 768, 4864, False),  # (a full wave; rows that fill a quarter of a tile)
-    ("bf16", 64, 200, 704, 4864, False), ("bf16", 64, 200, 832, 4864, True)])  # (narrow layers)
+    ("bf16", 64, 200, 704, 4864, False), ("bf16", 64, 200, 832, 4864, True),  # (narrow layers)
+    ("bf16", 64, 74, 768, 9728, False), ("bf16", 64, 74, 2048, 9728, True)])  # (152 tiles: a second wave, a short and a long K)
 def test_up_projection_has_the_same_bits_on_either_gemm(cache, dim, rows, emb, mlp, wide, monkeypatch):
   """Logits and caches of a step on the GEMM that the rule picks and on the row-major one (MTX_ROWS_WIDE_UP=0)."""
   got, names = _step(cache, dim, rows, mlp, graph=False, emb=emb)
